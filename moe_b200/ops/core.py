@@ -48,7 +48,7 @@ def lib():
             "moe_rmsnorm": [P, P, P, P, P, P, I, I, I, F, I, P, P],
             "moe_rmsnorm_combine": [P, P, P, P, I, P, P, P, P, P, P, I, I, I, F, I, P, P],
             "moe_add_inplace": [P, P, LL, P],
-            "moe_gemm_generic": [P, I, I, P, I, P, I, LL, P, I, I, P, P, I, I, I, I, P, P],
+            "moe_gemm_generic": [P, I, I, P, I, P, I, LL, P, I, I, P, P, I, I, I, I, P, P, LL, P],
             "moe_rope_split": [P, P, P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, P, P],
             "moe_kv_commit": [P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
             "moe_attention_generic": [P, P, P, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, F, I, P, I, P],
@@ -101,6 +101,7 @@ def lib():
             fn = getattr(L, name)
             fn.argtypes = argtypes
             fn.restype = c_int
+        L.moe_gemm_scratch_floats.argtypes, L.moe_gemm_scratch_floats.restype = [I, I, I, I], LL
         L.moe_mlstm_state_floats.argtypes, L.moe_mlstm_state_floats.restype = [I, I, I], LL
         L.moe_router_scratch_floats.argtypes = [I, I, I, I]
         L.moe_router_scratch_floats.restype = LL
@@ -752,8 +753,12 @@ def gemm_generic(a, w, out, *, bias=None, a_rows=None, group_offsets=None, statu
         _chk(bias, "bias", torch.float32, 1)
         if bias.numel() != N:
             raise KernelError("gemm: bias size")
+    need = 0
+    if a.dtype == w.dtype == torch.float32:
+        need = lib().moe_gemm_scratch_floats(M, N, K, 0 if group_offsets is None else G)
+    scratch = torch.empty((need,), dtype=torch.float32, device=a.device) if need else None
     _ok(lib().moe_gemm_generic(_p(a), _dt(a), a.stride(0), _p(a_rows), a.shape[0], _p(w), _dt(w), N * K, _p(out),
-                               _dt(out), out.stride(0), _p(bias), _p(group_offsets), G, M, N, K, _p(status),
+                               _dt(out), out.stride(0), _p(bias), _p(group_offsets), G, M, N, K, _p(status), _p(scratch), need,
                                _stream()), "gemm_generic")
 
 
