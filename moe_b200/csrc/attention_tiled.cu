@@ -222,6 +222,196 @@ attn_tiled_kernel(const T* __restrict__ q, const T* __restrict__ k_new, const T*
     }
 }
 
+// ---- the 32-bit path's form for heads of 64 and 128 and steps of many tokens a sequence -------------------------------
+// 128 queries of one (sequence, head) against key tiles of 128 (two pages): an 8 x 8 part of the scores and 8 x HD / 16
+// of the output a thread, so that sixteen 16-byte reads of shared memory feed 256 multiply-adds (the form above: eight
+// feed 64, and the reads, not the multiply-adds, are what bounds it: 13 of 74 TFLOP/s).  Nothing is transposed: queries,
+// keys and values lie in shared memory as they lie in global memory (cp.async), a thread's rows (ty + 16 i) and columns
+// (tx + 16 j) are interleaved so that neighbouring threads read neighbouring rows (a pitch of HD + 4: different banks),
+// and both products walk four of their inner index at a time, in order.  The values arrive under the score product.
+// The heads are the fast index of the grid and a sequence's last queries, which see most keys, come first: one head after
+// another left SMs with long blocks while others had none left (a third of the multiply-add rate on average, 57 % on the
+// fullest SM).
+constexpr int FQ = 128, FK = 128;
+template <int HD>
+__host__ __device__ constexpr int f32_floats() {
+    return FQ * (HD + 4) + FK * (HD + 4) + (HD < FK ? FQ * (FK + 4) : 0) + FK * (HD + 4);
+}
+__device__ __forceinline__ void cp16z(float* dst, const float* src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0)
+                 : "memory");
+}
+
+// PLAIN: neither a cap on the scores nor sigmoid weights; compiled apart because sixty-four inlined copies of those leave no
+// room in the instruction cache for the loops (two thirds of the time was spent waiting for instructions).
+template <int HD, bool PLAIN>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_new, const float* __restrict__ v_new,
+                const float* __restrict__ k_cache, const float* __restrict__ v_cache, float* __restrict__ out,
+                const int* __restrict__ cu_seqlens, const int* __restrict__ seq_start, const int* __restrict__ slots,
+                const int* __restrict__ tables, int table_stride, int ring, int num_pages, int num_seqs, int nh, int nkv,
+                int window, float scale, int use_local, int* status, const AttnVariant var) {
+    constexpr int HP = HD + 4, PP = FK + 4, OC = HD / 16;       // OC: output columns a thread (4 tx + 64 j + 0..3)
+    extern __shared__ __align__(16) float sm[];
+    __shared__ int s_seq, s_tile;
+    float* Q = sm;                                  // [FQ][HP]
+    float* K = Q + FQ * HP;                         // [FK][HP]
+    float* P = HD < FK ? K + FK * HP : K;           // [FQ][PP]: in the keys' place where it fits there
+    float* V = HD < FK ? P + FQ * PP : K + FK * HP; // [FK][HP]
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int h = blockIdx.x, kvh = h / (nh / nkv);
+    if (tid == 0) {
+        int tile = blockIdx.y, seq = -1;
+        for (int s = 0; s < num_seqs; s++) {
+            const int tiles = (cu_seqlens[s + 1] - cu_seqlens[s] + FQ - 1) / FQ;
+            if (tile < tiles) {
+                seq = s, tile = tiles - 1 - tile;
+                break;
+            }
+            tile -= tiles;
+        }
+        s_seq = seq, s_tile = tile;
+    }
+    __syncthreads();
+    const int seq = s_seq;
+    if (seq < 0) return;
+    const int tok0 = cu_seqlens[seq], cnt = cu_seqlens[seq + 1] - tok0, start = seq_start[seq];
+    const int r0 = s_tile * FQ, rows = min(FQ, cnt - r0);
+    const int p_first = start + r0, p_last = p_first + rows - 1;
+    const int local_from = use_local ? start : p_last + 1;
+    const int lo_min = attn_lo(p_first, window, var.chunk), pinned = attn_pinned(var);
+    const int* table = tables + (size_t)slots[seq] * table_stride;
+    for (int idx = tid; idx < FQ * (HD / 4); idx += THREADS) {
+        const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+        cp16z(Q + r * HP + d, q + ((size_t)(tok0 + r0 + (r < rows ? r : 0)) * nh + h) * HD + d, r < rows);
+    }
+    float m[8], l[8], o[8][OC];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+        for (int j = 0; j < OC; j++) o[i][j] = 0.f;
+    }
+    const int tile_lo = lo_min / FK, kept_tiles = min((var.keep + FK - 1) / FK, tile_lo);
+    for (int tile = 0; attn_seen(tile, kept_tiles, tile_lo) * FK <= p_last; tile++) {
+        const int j0 = attn_seen(tile, kept_tiles, tile_lo) * FK;
+        // a thread copies one 16-byte column of every (THREADS * 4 / HD)-th key, then of the values
+        constexpr int STEP = THREADS / (HD / 4);
+        const int d = (tid % (HD / 4)) * 4, c_first = tid / (HD / 4);
+        __syncthreads();                            // K, V and P of the tile before are no longer read
+        const float* vsrc[FK / STEP];
+#pragma unroll
+        for (int i = 0; i < FK / STEP; i++) {
+            const int c = c_first + i * STEP, j = j0 + c;
+            const float* ks = nullptr;
+            vsrc[i] = nullptr;
+            if (j <= p_last && (j >= lo_min || j < var.keep)) {
+                if (j >= local_from) {
+                    const size_t at = ((size_t)(tok0 + (j - start)) * nkv + kvh) * HD + d;
+                    ks = k_new + at, vsrc[i] = v_new + at;
+                } else {
+                    const CachePos cp = cache_pos(j, ring, table, BK, num_pages, status, pinned);
+                    const size_t at = cache_index(cp, kvh, nkv, BK, HD) + d;
+                    ks = k_cache + at, vsrc[i] = v_cache + at;
+                }
+            }
+            cp16z(K + c * HP + d, ks ? ks : q, ks != nullptr);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < FK / STEP; i++) cp16z(V + (c_first + i * STEP) * HP + d, vsrc[i] ? vsrc[i] : q, vsrc[i] != nullptr);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        float s[8][8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) s[i][j] = 0.f;
+#pragma unroll 2
+        for (int e = 0; e < HD; e += 4) {
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4*>(Q + (ty + 16 * i) * HP + e);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float4 b = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * HP + e);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    s[i][j] = fmaf(a[i].x, b.x, s[i][j]), s[i][j] = fmaf(a[i].y, b.y, s[i][j]);
+                    s[i][j] = fmaf(a[i].z, b.z, s[i][j]), s[i][j] = fmaf(a[i].w, b.w, s[i][j]);
+                }
+            }
+        }
+        if (P == K) __syncthreads();                // every thread has read the keys: P may take their place
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int row = ty + 16 * i, p = p_first + row, lo = attn_lo(p, window, var.chunk);
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int key = j0 + tx + 16 * j;
+                const bool seen = row < rows && key <= p && (key >= lo || key < var.keep);
+                s[i][j] = seen ? (PLAIN ? s[i][j] * scale : attn_logit(var, h, s[i][j], scale)) : -INFINITY;
+                mx = fmaxf(mx, s[i][j]);
+            }
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            const float m_new = fmaxf(m[i], mx);
+            float alpha = 1.f, sum = 0.f;
+            if (m_new != -INFINITY) {               // (the same for the 16 threads of the row)
+                alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    s[i][j] = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
+                    sum += s[i][j];
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; j++) s[i][j] = 0.f;
+            }
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            l[i] = l[i] * alpha + sum;
+            m[i] = m_new;
+#pragma unroll
+            for (int j = 0; j < OC; j++) o[i][j] *= alpha;
+#pragma unroll
+            for (int j = 0; j < 8; j++) P[row * PP + tx + 16 * j] = s[i][j];
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+#pragma unroll 1
+        for (int c = 0; c < FK; c += 4) {
+            float4 a[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4*>(P + (ty + 16 * i) * PP + c);
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int j = 0; j < OC; j += 4) {
+                    const float4 v4 = *reinterpret_cast<const float4*>(V + (c + e) * HP + 4 * tx + 16 * j);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const float pv = e == 0 ? a[i].x : e == 1 ? a[i].y : e == 2 ? a[i].z : a[i].w;
+                        o[i][j] = fmaf(pv, v4.x, o[i][j]), o[i][j + 1] = fmaf(pv, v4.y, o[i][j + 1]);
+                        o[i][j + 2] = fmaf(pv, v4.z, o[i][j + 2]), o[i][j + 3] = fmaf(pv, v4.w, o[i][j + 3]);
+                    }
+                }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int row = ty + 16 * i;
+        if (row >= rows) continue;
+        const float inv = l[i] > 0.f ? 1.0f / attn_denominator(m[i], l[i], var.sink, attn_sink_value(var, h)) : 0.f;
+        float* dst = out + ((size_t)(tok0 + r0 + row) * nh + h) * HD;
+#pragma unroll
+        for (int j = 0; j < OC; j += 4)
+            *reinterpret_cast<float4*>(dst + 4 * tx + 16 * j) = make_float4(o[i][j] * inv, o[i][j + 1] * inv, o[i][j + 2] * inv, o[i][j + 3] * inv);
+    }
+}
+
 size_t tiled_smem(int hd) {
     // Q, K (P takes K's place when the head is at least as long as a tile is wide), V
     return ((size_t)hd * (BQ + PAD) + (size_t)hd * (BK + PAD) + (size_t)BK * (hd + PAD) +
@@ -246,6 +436,31 @@ MOE_API int moe_attention_tiled(const void* q, const void* k_new, const void* v_
     if (page_size != BK || (ring % BK) != 0) return -1;
     const size_t align = dt == DT_F32 ? 16 : 8;          // rows are read four elements at a time
     if (((uintptr_t)q | (uintptr_t)k_new | (uintptr_t)v_new | (uintptr_t)k_cache | (uintptr_t)v_cache) % align) return -1;
+    // many new tokens a sequence: 128 of them to a block.  (With fewer than that most of its rows would be padding, and
+    // the form of 64 has twice the blocks.)
+    if (dt == DT_F32 && (hd == 64 || hd == 128) && num_tokens >= FQ * num_seqs &&
+        (num_tokens + FQ - 1) / FQ + num_seqs <= 65535 && !((uintptr_t)out % 16)) {
+        const dim3 grid(nh, (unsigned)((num_tokens + FQ - 1) / FQ + num_seqs));
+#define GO(HD, PLAIN)                                                                                                 \
+    do {                                                                                                              \
+        const int bytes = f32_floats<HD>() * 4;                                                                       \
+        cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<HD, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); \
+        if (e != cudaSuccess) return (int)e;                                                                          \
+        attn_f32_kernel<HD, PLAIN><<<grid, THREADS, bytes, stream>>>(                                                        \
+            (const float*)q, (const float*)k_new, (const float*)v_new, (const float*)k_cache, (const float*)v_cache,  \
+            (float*)out, cu_seqlens, seq_start, slots, tables, table_stride, ring, num_pages, num_seqs, nh, nkv, window, \
+            scale, use_local, status, av);                                                                            \
+        return launch_status();                                                                                       \
+    } while (0)
+        const bool simple = !(softcap > 0.f) && sink != ATTN_SIGMOID;
+        if (hd == 64) {
+            if (simple) GO(64, true);
+            GO(64, false);
+        }
+        if (simple) GO(128, true);
+        GO(128, false);
+#undef GO
+    }
     const size_t smem = tiled_smem(hd);
     const long long tiles = (long long)(num_tokens + BQ - 1) / BQ + num_seqs;
     if (tiles > 0x7fffffffLL) return -1;

@@ -1,8 +1,12 @@
 """The forms of the 32-bit kernels that a size picks, at the sizes where they meet: products of few and of many rows
-(16-byte operands; the tile heights; group counts), against float64."""
+(16-byte operands; the tile heights; group counts), and attention of 128 queries a block, against float64."""
+import math
+
 import numpy as np
 import pytest
 import torch
+
+import gpu_util as G
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -63,4 +67,56 @@ def test_grouped_rows_gathered(core, counts):
         x = a[rows[at:at + c].long()]
         assert bool(((out[at:at + c].double() - x.double() @ w[g].double().T).abs() <= bound(x, w[g])).all()), g
         at += c
+    assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 2, 1), (64, 3, 3)])
+@pytest.mark.parametrize("before,new", [([0, 0], [128, 129]), ([5, 300], [257, 130]), ([64], [511]), ([1000, 0, 127], [150, 260, 128])])
+@pytest.mark.parametrize("opt", [{}, {"window": 100}, {"window": 130, "keep": 70}, {"chunk": 96, "softcap": 5.0}, {"sink": True}])
+def test_attention_of_many_new_tokens(core, hd, nh, nkv, before, new, opt):
+    from moe_b200.cache import KVCache, KVRequest
+
+    torch.manual_seed(hd + sum(new))
+    window, keep, chunk, cap = opt.get("window"), opt.get("keep", 0), opt.get("chunk", 0), opt.get("softcap", 0.0)
+    B = len(new)
+    ring = window or chunk or None
+    cache = KVCache({0: KVRequest(nkv, hd, ring, keep=keep) if keep else KVRequest(nkv, hd, ring)}, {0: None}, max_tokens=64 * 60,
+                    max_slots=B + 1, dtype=torch.float32, device=DEV)
+    cache.groups[0].storage.fill_(3e30)
+    view, slots, st = cache.view(0), [cache.acquire() for _ in range(B)], core.new_status(DEV)
+    K, V = ([torch.randn(a + b, nkv, hd, device=DEV) for a, b in zip(before, new)] for _ in range(2))
+    Q = [2 * torch.randn(b, nh, hd, device=DEV) for b in new]
+    live = [i for i in range(B) if before[i]]
+    for i in live:
+        G.give_pages(cache, slots[i], before[i])
+    if live:
+        b0 = G.make_batch(DEV, [slots[i] for i in live], [0] * len(live), [before[i] for i in live])
+        core.kv_commit(*(torch.cat([x[i][:before[i]] for i in live]).contiguous() for x in (K, V)), view, b0, st)
+    for i in range(B):
+        G.give_pages(cache, slots[i], before[i] + new[i])
+    batch = G.make_batch(DEV, slots, before, new)
+    q, kn, vn = torch.cat(Q).contiguous(), *(torch.cat([x[i][before[i]:] for i in range(B)]).contiguous() for x in (K, V))
+    out = torch.full((q.shape[0], nh * hd), float("nan"), device=DEV)
+    assert core.attention_tiled(q, kn, vn, view, batch, out, nh=nh, window=window, scale=hd ** -0.5, use_local=True, status=st,
+                                chunk=chunk, softcap=cap, sink=opt.get("sink", False), keep=keep)
+    at = 0
+    for i in range(B):
+        n, T = new[i], before[i] + new[i]
+        p, j = torch.arange(before[i], T, device=DEV)[:, None], torch.arange(T, device=DEV)[None]
+        seen = j <= p
+        if chunk:
+            seen &= j >= p // chunk * chunk
+        elif window:
+            seen &= (j > p - window) | (j < keep)
+        for h in range(nh):
+            s = Q[i][:, h].double() @ K[i][:, h // (nh // nkv)].double().T * hd ** -0.5
+            s = cap * torch.tanh(s / cap) if cap else s
+            s = s.masked_fill(~seen, -math.inf)
+            if opt.get("sink"):
+                s = torch.cat([s, torch.zeros(n, 1, dtype=s.dtype, device=DEV)], 1)
+            ref = torch.softmax(s, -1)[:, :T] @ V[i][:, h // (nh // nkv)].double()
+            got = out[at:at + n, h * hd:(h + 1) * hd].double()
+            # scores of up to about 30 are off by 128 half units at most, so a weight is by 30 * 128 * 2^-24 of itself
+            assert float((got - ref).abs().max()) < 3e-4, (i, h)
+        at += n
     assert int(st[0]) == 0
