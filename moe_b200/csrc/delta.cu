@@ -597,7 +597,340 @@ delta_scan_kernel(const DeltaSeq p, float* __restrict__ o) {
     }
 }
 
+// ---- several tokens a sequence: sixteen at a time ---------------------------------------------------------------
+// The same recurrence over chunks of sixteen tokens, in two launches.  What does not need the state is formed for all
+// chunks side by side (delta_chunk_kernel): with L_ij = beta_i (sum_c D_ij k_i k_j) for j < i, the u of a chunk solve
+// (I + L) u = beta (v - (G k) S), so with W = (I + L)^-1 beta (G k) and U = (I + L)^-1 beta v (forward substitution, a
+// column a thread)
+//     u = U - W S,    o = (G q) S + P u,    S <- G_16 S + (D_16 k)^T u,      P_ij = sum_c D_ij q_i k_j, j <= i
+// and the chain over the chunks (delta_chunk_scan_kernel) is three small products.  As above no factor is a quotient of
+// decays.  The chain of the form above is 0.29 us a token of a sequence (2,200 cycles for four tokens, four warps on an
+// SM, most of it the latency of shuffles, shared memory and the triangle inside a group); here it is 0.12 us, bound by the
+// reads of shared memory, and the first launch 0.03 us (16 heads of 128 x 128: 599 -> 298 us for 2,048 tokens).  Error
+// against 64 bits 1.3e-7 (1.1e-7 above).
+constexpr int CC = 16, CS_COLS = 16, CS_THREADS = 256;
+struct DeltaWork {             // what the first launch leaves, a row a (token, value head)
+    float *w, *gq, *kd;        // [T, H, NP]; w and gq in the order chunk_place
+    float *u, *pairs;          // [T, H, dv], [T, H, 16]
+    float* all;                // [chunk, H, NP]: a chunk's decay of a channel
+};
+// where channel c lies in a row of w and gq: a thread's four channels c, c + 16, c + 32, c + 48 are one 16-byte unit
+__device__ __forceinline__ int chunk_place(int c) { return (c & ~63) + (c & 15) * 4 + ((c >> 4) & 3); }
+// number of the chunk that starts at token `tok` (counted in the step) of sequence s: different for all chunks of a step
+__device__ __forceinline__ int chunk_number(int tok, int s) { return tok / CC + s; }
+
+template <int NP, bool CH>
+__global__ void __launch_bounds__(256, 3)
+delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
+    constexpr int PK = NP + 4;
+    __shared__ __align__(16) float sk[CC][PK], sq[CC][PK], sg[CH ? CC : 1][PK];
+    __shared__ float s_l[CC][CC], s_beta[CC], s_lg[CC], s_eb[CC], s_er[CC];
+    __shared__ int s_seq;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, number = blockIdx.x, h = blockIdx.y;
+    if (tid == 0) s_seq = -1;
+    pdl_sync();
+    __syncthreads();
+    for (int s = tid; s < num_seqs; s += blockDim.x) {
+        const int a = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - a, first = chunk_number(a, s);
+        if (n > 0 && number >= first && number < first + (n + CC - 1) / CC) s_seq = s;
+    }
+    __syncthreads();
+    const int s = s_seq;
+    if (s < 0) return;
+    const int a0 = p.cu_seqlens[s], tok = a0 + (number - chunk_number(a0, s)) * CC, cnt = min(CC, p.cu_seqlens[s + 1] - tok);
+    const int d = p.d, dv = p.dv, g = h / (p.H / p.G), channels = 2 * p.G * d + p.H * dv;
+    const float* base = p.qkv + (size_t)tok * channels;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+    for (int e = tid; e < CC * (NP / 4); e += 256) {
+        const int i = e / (NP / 4), c = (e % (NP / 4)) * 4;
+        const bool on = i < cnt && c < d;
+        *reinterpret_cast<float4*>(&sk[i][c]) = on ? *reinterpret_cast<const float4*>(base + (size_t)i * channels + (p.G + g) * d + c) : zero;
+        *reinterpret_cast<float4*>(&sq[i][c]) = on ? *reinterpret_cast<const float4*>(base + (size_t)i * channels + g * d + c) : zero;
+        if (CH) *reinterpret_cast<float4*>(&sg[i][c]) = on ? *reinterpret_cast<const float4*>(p.decay + ((size_t)(tok + i) * p.H + h) * d + c) : one;
+    }
+    if (tid < CC) {
+        s_beta[tid] = tid < cnt ? p.step[(size_t)(tok + tid) * 2 * p.H + h] : 0.f;
+        s_lg[tid] = !CH && tid < cnt ? p.step[(size_t)(tok + tid) * 2 * p.H + p.H + h] : 0.f;
+    }
+    __syncthreads();
+    if (!CH && tid < CC) {             // every exponent is a sum of logarithms, never a difference
+        float b = 0.f, r = 0.f;
+        for (int e = 0; e <= tid; e++) b += s_lg[e];
+        for (int e = tid + 1; e < CC; e++) r += s_lg[e];
+        s_eb[tid] = expf(b), s_er[tid] = expf(r);
+    }
+    // pair sums: a warp takes the pairs of tokens j = warp and 15 - warp with every later one; the thirty-two sums over the
+    // warp cost 31 shuffles, and lane l ends with number l: [0 ... 15] k_i . k_j, [16 ... 31] q_i . k_j, i = l & 15
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+        const int j = half ? CC - 1 - warp : warp;
+        const int e = lane * 4;
+        float4 since = e < NP ? *reinterpret_cast<const float4*>(&sk[j][e]) : zero;        // k_j times the decays after j
+        float v32[32];
+#pragma unroll
+        for (int i = 0; i < CC; i++) {
+            v32[i] = v32[CC + i] = 0.f;
+            if (i >= j && e < NP) {
+                if (CH && i > j) {
+                    const float4 gi = *reinterpret_cast<const float4*>(&sg[CH ? i : 0][e]);
+                    since.x *= gi.x, since.y *= gi.y, since.z *= gi.z, since.w *= gi.w;
+                }
+                const float4 ki = *reinterpret_cast<const float4*>(&sk[i][e]), qi = *reinterpret_cast<const float4*>(&sq[i][e]);
+                v32[i] = fmaf(ki.x, since.x, fmaf(ki.y, since.y, fmaf(ki.z, since.z, ki.w * since.w)));
+                v32[CC + i] = fmaf(qi.x, since.x, fmaf(qi.y, since.y, fmaf(qi.z, since.z, qi.w * since.w)));
+            }
+        }
+        float v16[16], v8[8], v4[4], v2[2];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const bool up = (lane & 16) != 0;
+            v16[i] = (up ? v32[16 + i] : v32[i]) + __shfl_xor_sync(0xffffffffu, up ? v32[i] : v32[16 + i], 16);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const bool up = (lane & 8) != 0;
+            v8[i] = (up ? v16[8 + i] : v16[i]) + __shfl_xor_sync(0xffffffffu, up ? v16[i] : v16[8 + i], 8);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const bool up = (lane & 4) != 0;
+            v4[i] = (up ? v8[4 + i] : v8[i]) + __shfl_xor_sync(0xffffffffu, up ? v8[i] : v8[4 + i], 4);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const bool up = (lane & 2) != 0;
+            v2[i] = (up ? v4[2 + i] : v4[i]) + __shfl_xor_sync(0xffffffffu, up ? v4[i] : v4[2 + i], 2);
+        }
+        const bool up = (lane & 1) != 0;
+        float dot = (up ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, up ? v2[0] : v2[1], 1);
+        const int i = lane & 15;
+        if (!CH) {
+            float between = 0.f;       // the decays' logarithms after j up to i, added up and not subtracted
+            for (int l = j + 1; l <= i; l++) between += s_lg[l];
+            dot *= expf(between);
+        }
+        if (lane < 16)
+            s_l[i][j] = i > j ? s_beta[i] * dot : 0.f;
+        else if (i < cnt)
+            wk.pairs[((size_t)(tok + i) * p.H + h) * CC + j] = i >= j ? dot : 0.f;
+    }
+    __syncthreads();
+    float x[CC];
+    auto solve = [&]() {               // x <- (I + L)^-1 x
+#pragma unroll
+        for (int i = 1; i < CC; i++) {
+            asm volatile("" ::: "memory");       // (or all of L is fetched first: 250 registers, one block an SM)
+#pragma unroll
+            for (int j = 0; j < i; j++) x[i] = fmaf(-s_l[i][j], x[j], x[i]);
+        }
+    };
+    if (tid < NP) {
+        const int c = tid, at = chunk_place(c);
+        const size_t row = ((size_t)tok * p.H + h) * NP, pitch = (size_t)p.H * NP;
+        float all = 1.f;
+#pragma unroll
+        for (int i = 0; i < CC; i++) {
+            if (CH) all *= sg[CH ? i : 0][c]; else all = s_eb[i];
+            x[i] = s_beta[i] * (sk[i][c] * all);
+            if (i < cnt) wk.gq[row + i * pitch + at] = sq[i][c] * all;
+        }
+        wk.all[((size_t)number * p.H + h) * NP + c] = all;
+        float since = 1.f;
+#pragma unroll
+        for (int i = CC - 1; i >= 0; i--) {
+            if (i < cnt) wk.kd[row + i * pitch + c] = sk[i][c] * (CH ? since : s_er[i]);
+            if (CH) since *= sg[CH ? i : 0][c];
+        }
+        solve();
+#pragma unroll
+        for (int i = 0; i < CC; i++)
+            if (i < cnt) wk.w[row + i * pitch + at] = x[i];
+    } else {
+        for (int c = tid - NP; c < dv; c += 256 - NP) {
+            const float* v = base + 2 * p.G * d + (size_t)h * dv + c;
+#pragma unroll
+            for (int i = 0; i < CC; i++) x[i] = i < cnt ? s_beta[i] * v[(size_t)i * channels] : 0.f;
+            solve();
+#pragma unroll
+            for (int i = 0; i < CC; i++)
+                if (i < cnt) wk.u[((size_t)(tok + i) * p.H + h) * dv + c] = x[i];
+        }
+    }
+}
+
+// grid (ceil(dv / 16), heads, sequences): a block carries 16 columns of S in shared memory through its sequence's chunks.
+// A thread of the first product holds 8 of the 32 rows [W; G q] x 4 columns over every 16th channel (the sum over
+// the 16 threads that share them is 30 shuffles); then half of the threads update the state, 4 channels x 4 columns each,
+// and the other half form the outputs.
+template <int NP>
+struct ChunkSmem {
+    static constexpr int STAGE = 3 * CC * NP + 2 * CC * CC + NP;      // W | G q | D k | U | P | decays
+    static constexpr int SPITCH = CS_COLS + 4, XPITCH = CS_COLS + 2;
+    static constexpr int FLOATS = 2 * STAGE + NP * SPITCH + 2 * CC * XPITCH + CC * SPITCH;
+};
+template <int NP>
+__global__ void __launch_bounds__(CS_THREADS, 2)
+delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict__ o) {
+    using L = ChunkSmem<NP>;
+    constexpr int SP = L::SPITCH, XP = L::XPITCH;
+    extern __shared__ __align__(16) float sm[];
+    float* sS = sm + 2 * L::STAGE;     // [NP][SP]
+    float* sX = sS + NP * SP;          // [32][XP]: W S, then (G q) S
+    float* sU = sX + 2 * CC * XP;      // [16][SP]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.y, s = blockIdx.z, c0 = blockIdx.x * CS_COLS, d = p.d, dv = p.dv;
+    pdl_sync();
+    const int tok0 = p.cu_seqlens[s], cnt = p.cu_seqlens[s + 1] - tok0;
+    if (cnt <= 0) return;
+    float* S = p.state + (size_t)p.slots[s] * p.state_pitch + (size_t)h * d * dv;
+    const int ncols = min(CS_COLS, dv - c0);
+    const int number0 = chunk_number(tok0, s);
+    auto stage = [&](int t0, int buf) {
+        float* dst = sm + buf * L::STAGE;
+        const size_t row0 = (size_t)(tok0 + t0) * p.H + h;
+        for (int e = tid; e < 3 * CC * (NP / 4); e += CS_THREADS) {
+            const int which = e / (CC * (NP / 4)), i = e / (NP / 4) % CC, c = (e % (NP / 4)) * 4;
+            const bool on = t0 + i < cnt;
+            const float* src = which == 0 ? wk.w : which == 1 ? wk.gq : wk.kd;
+            cp_zfill(dst + which * CC * NP + i * NP + c, on ? src + (row0 + (size_t)i * p.H) * NP + c : src, 16, on);
+        }
+        float* du = dst + 3 * CC * NP;
+        if (tid < 128) {
+            const int i = (tid & 63) >> 2, c = (tid & 3) * 4, which = tid >> 6;
+            const bool on = t0 + i < cnt && (which || c < ncols);
+            const size_t row = row0 + (size_t)i * p.H;
+            const float* src = which ? wk.pairs + row * CC + c : wk.u + row * dv + c0 + c;
+            cp_zfill(du + which * CC * CC + i * CC + c, on ? src : wk.u, 16, on);
+        } else if (tid < 128 + NP / 4) {
+            const int c = (tid - 128) * 4;
+            cp_zfill(du + 2 * CC * CC + c, wk.all + ((size_t)(number0 + t0 / CC) * p.H + h) * NP + c, 16, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    stage(0, 0);
+    for (int e = tid; e < NP * CS_COLS; e += CS_THREADS) {
+        const int r = e / CS_COLS, c = e % CS_COLS;
+        sS[r * SP + c] = r < d && c < ncols ? S[(size_t)r * dv + c0 + c] : 0.f;
+    }
+    const int ks = lane & 15, cg = ((warp & 1) * 2 + (lane >> 4)) * 4, tg = warp >> 1;
+    for (int t0 = 0, buf = 0; t0 < cnt; t0 += CC, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                               // the chunk is there, the state and the other buffer are at rest
+        if (t0 + CC < cnt) stage(t0 + CC, buf ^ 1);
+        const float* st = sm + buf * L::STAGE;
+        {
+            float acc[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) acc[i] = 0.f;
+            const float* rows = st + tg * 8 * NP + ks * 4;
+#pragma unroll
+            for (int it = 0; it < NP / 64; it++) {
+                float4 sv[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) sv[r] = *reinterpret_cast<const float4*>(sS + (it * 64 + r * 16 + ks) * SP + cg);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const float4 w4 = *reinterpret_cast<const float4*>(rows + i * NP + it * 64);
+                    const float wr[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        acc[4 * i] = fmaf(wr[r], sv[r].x, acc[4 * i]), acc[4 * i + 1] = fmaf(wr[r], sv[r].y, acc[4 * i + 1]);
+                        acc[4 * i + 2] = fmaf(wr[r], sv[r].z, acc[4 * i + 2]), acc[4 * i + 3] = fmaf(wr[r], sv[r].w, acc[4 * i + 3]);
+                    }
+                }
+            }
+            // thirty-two sums over sixteen lanes: a lane ends with two neighbouring ones
+            float v16[16], v8[8], v4[4], v2[2];
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const bool up = (lane & 8) != 0;
+                v16[i] = (up ? acc[16 + i] : acc[i]) + __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[16 + i], 8);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const bool up = (lane & 4) != 0;
+                v8[i] = (up ? v16[8 + i] : v16[i]) + __shfl_xor_sync(0xffffffffu, up ? v16[i] : v16[8 + i], 4);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const bool up = (lane & 2) != 0;
+                v4[i] = (up ? v8[4 + i] : v8[i]) + __shfl_xor_sync(0xffffffffu, up ? v8[i] : v8[4 + i], 2);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const bool up = (lane & 1) != 0;
+                v2[i] = (up ? v4[2 + i] : v4[i]) + __shfl_xor_sync(0xffffffffu, up ? v4[i] : v4[2 + i], 1);
+            }
+            *reinterpret_cast<float2*>(sX + (tg * 8 + (ks >> 1)) * XP + cg + (ks & 1) * 2) = make_float2(v2[0], v2[1]);
+        }
+        __syncthreads();
+        const int i = tid >> 4, c = tid & 15;
+        const float* du = st + 3 * CC * NP;
+        const float mine = du[i * CC + c] - sX[i * XP + c];
+        sU[i * SP + c] = mine;
+        __syncthreads();
+        if (tid < CS_THREADS / 2) {
+            // the state: four neighbouring channels x four columns a thread
+            for (int r0 = (tid >> 2) * 4; r0 < NP; r0 += CS_THREADS / 2) {
+                const int cc = (tid & 3) * 4;
+                float4 a[4];
+                const float4 al = *reinterpret_cast<const float4*>(du + 2 * CC * CC + r0);
+                const float all[4] = {al.x, al.y, al.z, al.w};
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    a[r] = *reinterpret_cast<const float4*>(sS + (r0 + r) * SP + cc);
+                    a[r].x *= all[r], a[r].y *= all[r], a[r].z *= all[r], a[r].w *= all[r];
+                }
+                const float* kd = st + 2 * CC * NP + r0;
+#pragma unroll
+                for (int j = 0; j < CC; j++) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(kd + j * NP), u4 = *reinterpret_cast<const float4*>(sU + j * SP + cc);
+                    const float k[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        a[r].x = fmaf(k[r], u4.x, a[r].x), a[r].y = fmaf(k[r], u4.y, a[r].y);
+                        a[r].z = fmaf(k[r], u4.z, a[r].z), a[r].w = fmaf(k[r], u4.w, a[r].w);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 4; r++) *reinterpret_cast<float4*>(sS + (r0 + r) * SP + cc) = a[r];
+            }
+        } else {
+            // the outputs of two neighbouring columns of a token
+            const int to = (tid & 127) >> 3, co = (tid & 7) * 2;
+            float2 out = *reinterpret_cast<const float2*>(sX + (CC + to) * XP + co);
+            const float* pr = du + CC * CC + to * CC;
+#pragma unroll
+            for (int j = 0; j < CC; j += 4) {
+                const float4 p4 = *reinterpret_cast<const float4*>(pr + j);
+                const float pj[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float2 u2 = *reinterpret_cast<const float2*>(sU + (j + e) * SP + co);
+                    out.x = fmaf(pj[e], u2.x, out.x), out.y = fmaf(pj[e], u2.y, out.y);
+                }
+            }
+            float* dst = o + ((size_t)(tok0 + t0 + to) * p.H + h) * dv + c0 + co;
+            if (t0 + to < cnt) {
+                if (co < ncols) dst[0] = out.x;
+                if (co + 1 < ncols) dst[1] = out.y;
+            }
+        }
+    }
+    __syncthreads();
+    for (int e = tid; e < NP * CS_COLS; e += CS_THREADS) {
+        const int r = e / CS_COLS, c = e % CS_COLS;
+        if (r < d && c < ncols) S[(size_t)r * dv + c0 + c] = sS[r * SP + c];
+    }
+}
+
 bool aligned16(const void* p) { return (uintptr_t)p % 16 == 0; }
+
+// Floats of the first launch's results.
+long long chunk_floats(long long T, int num_seqs, int H, int d, int dv) {
+    const long long NP = d <= 64 ? 64 : 128;
+    return T * H * (3 * NP + dv + CC) + (T / CC + num_seqs + 1) * H * NP;
+}
 
 }  // namespace
 
@@ -677,15 +1010,50 @@ MOE_API int moe_delta_step(const float* qkv, const float* step, float* state, lo
 #undef STEP_C
 }
 
-// Several tokens a sequence; o: [T, H * dv] 32-bit (rows of no sequence are left alone).
+// SMs of the current device.
+MOE_API int moe_scan_sms() { return scan_sms(); }
+
+// Floats of scratch with which moe_delta_scan takes the form over chunks of sixteen tokens; 0: it takes the other one.
+MOE_API long long moe_delta_chunk_floats(long long num_tokens, int num_seqs, int H, int G, int d, int dv) {
+    if (num_tokens <= 0 || num_seqs <= 0 || d <= 0 || d > 128 || d % 4 || dv <= 0 || dv % 4 || H <= 0 || H > 65535 || num_seqs > 65535) return 0;
+    return chunk_floats(num_tokens, num_seqs, H, d, dv);
+}
+
+// Several tokens a sequence; o: [T, H * dv] 32-bit (rows of no sequence are left alone).  `work`: moe_delta_chunk_floats
+// floats, or null for the form of four tokens at a time.
 MOE_API int moe_delta_scan(const float* qkv, const float* step, float* state, long long state_pitch, const int* cu_seqlens,
-                           const int* slots, int num_seqs, int H, int G, int d, int dv, const float* decay, float* o,
-                           cudaStream_t stream) {
+                           const int* slots, int num_tokens, int num_seqs, int H, int G, int d, int dv, const float* decay,
+                           float* o, float* work, cudaStream_t stream) {
     if (num_seqs <= 0) return 0;
     if (!qkv || !step || !state || !cu_seqlens || !slots || !o || H <= 0 || G <= 0 || H % G || d <= 0 || d > 256 || dv <= 0 ||
         state_pitch < (long long)H * d * dv || H > 65535 || num_seqs > 65535)
         return (int)cudaErrorInvalidValue;
     const DeltaSeq p{qkv, step, state, state_pitch, cu_seqlens, slots, H, G, d, dv, decay};
+    if (work && d <= 128 && d % 4 == 0 && dv % 4 == 0 && aligned16(qkv) && aligned16(decay) && aligned16(work)) {
+        const int NP = d <= 64 ? 64 : 128;
+        DeltaWork wk;
+        const size_t rows = (size_t)num_tokens * H;
+        wk.w = work, wk.gq = wk.w + rows * NP, wk.kd = wk.gq + rows * NP, wk.u = wk.kd + rows * NP, wk.pairs = wk.u + rows * dv;
+        wk.all = wk.pairs + rows * CC;
+        const dim3 first(num_tokens / CC + num_seqs + 1, H), chain((dv + CS_COLS - 1) / CS_COLS, H, num_seqs);
+#define CHUNK(NP_, C_)                                                                                                  \
+    do {                                                                                                               \
+        const int rc = launch_pdl(delta_chunk_kernel<NP_, C_>, first, dim3(256), 0, stream, p, wk, num_seqs);          \
+        if (rc) return rc;                                                                                             \
+        const size_t smem = scan_smem(ChunkSmem<NP_>::FLOATS * sizeof(float), (long long)chain.x * chain.y * chain.z); \
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<NP_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (e != cudaSuccess) return (int)e;                                                                           \
+        delta_chunk_scan_kernel<NP_><<<chain, CS_THREADS, smem, stream>>>(p, wk, o);                                   \
+        return launch_status();                                                                                        \
+    } while (0)
+        if (NP == 64) {
+            if (decay) CHUNK(64, true);
+            CHUNK(64, false);
+        }
+        if (decay) CHUNK(128, true);
+        CHUNK(128, false);
+#undef CHUNK
+    }
     // few blocks: the narrow form puts twice as many on the SMs
     const bool narrow = d > 64 && (long long)((dv + dcols(16) - 1) / dcols(16)) * H * num_seqs * 2 <= scan_sms();
     const int cols = dcols(narrow ? 32 : 16);

@@ -91,7 +91,7 @@ def lib():
             "moe_ssd_finish": [P, P, LL, P, F, P, I, I, I, P, I, P],
             "moe_delta_prepare": [P, LL, I, I, P, I, P, LL, P, P, P, P, P, I, I, I, I, I, F, F, I, P, P, P, LL, P, P],
             "moe_delta_step": [P, P, P, LL, P, LL, P, F, P, P, P, I, I, I, I, I, I, P, I, P, I, P],
-            "moe_delta_scan": [P, P, P, LL, P, P, I, I, I, I, I, P, P, P],
+            "moe_delta_scan": [P, P, P, LL, P, P, I, I, I, I, I, I, P, P, P, P],
             "moe_mlstm_scan": [P, LL, I, I, I, I, I, P, P, F, F, P, LL, P, P, I, I, I, I, P, P, I, I, I, P, LL, P, P],
             "moe_mlstm_step": [P, LL, I, I, I, I, I, P, P, F, F, P, LL, P, LL, P, F, P, P, P, I, I, I, I, I, I, P, I, P],
             "moe_post_norm": [P, P, F, P, F, P, P, P, I, P, P, F, P, F, P, P, P, I, I, I, I, P, P],
@@ -101,7 +101,9 @@ def lib():
             fn = getattr(L, name)
             fn.argtypes = argtypes
             fn.restype = c_int
+        L.moe_scan_sms.argtypes, L.moe_scan_sms.restype = [], c_int
         L.moe_gemm_scratch_floats.argtypes, L.moe_gemm_scratch_floats.restype = [I, I, I, I], LL
+        L.moe_delta_chunk_floats.argtypes, L.moe_delta_chunk_floats.restype = [LL, I, I, I, I, I], LL
         L.moe_mlstm_state_floats.argtypes, L.moe_mlstm_state_floats.restype = [I, I, I], LL
         L.moe_router_scratch_floats.argtypes = [I, I, I, I]
         L.moe_router_scratch_floats.restype = LL
@@ -1576,16 +1578,30 @@ def delta_step(qkv, step, state, gate, norm_w, norm_eps, batch, out, *, heads, k
     return True
 
 
-def delta_scan(qkv, step, state, batch, o, *, heads, kv_heads, d, dv, offset=0, decay=None):
+def _delta_chunks(T, num_seqs, heads, dv) -> bool:
+    """Whether the scan goes over chunks: where its blocks (16 columns of a head and sequence) find an SM each.  The chain
+    of a chunk is then short (16 heads of 128 x 128, one sequence of 2,048 tokens: 599 -> 298 us); with more blocks the
+    multiply-adds count, of which a chunk has more (four sequences: 916 against 1,067 us)."""
+    return -(-dv // 16) * heads * num_seqs <= lib().moe_scan_sms()
+
+
+def delta_scan(qkv, step, state, batch, o, *, heads, kv_heads, d, dv, offset=0, decay=None, chunks=None):
     """Per sequence and value head, tokens in order: S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, on
-    what ``delta_prepare`` left (``decay``: a decay a channel, each for its row of S); o: float32 [T, heads * dv]."""
+    what ``delta_prepare`` left (``decay``: a decay a channel, each for its row of S); o: float32 [T, heads * dv].
+    ``chunks``: over chunks of sixteen tokens (scratch of 4 to 6 rows a token) or four tokens at a time; None: by the
+    rule of ``_delta_chunks``."""
     T = _delta_chk(qkv, step, heads, kv_heads, d, dv, decay)
     _chk(o, "o", torch.float32, 2)
     if tuple(o.shape) != (T, heads * dv):
         raise KernelError("delta_scan: shapes")
+    work = None
+    if chunks or (chunks is None and _delta_chunks(T, batch.num_seqs, heads, dv)):
+        n = lib().moe_delta_chunk_floats(T, batch.num_seqs, heads, kv_heads, d, dv)
+        if n:
+            work = torch.empty(n, dtype=torch.float32, device=o.device)
     _ok(lib().moe_delta_scan(_p(qkv), _p(step), _state_at(state, offset, heads * d * dv), state.stride(0),
-                             _p(batch.cu_seqlens), _p(batch.slots), batch.num_seqs, heads, kv_heads, d, dv, _p(decay), _p(o),
-                             _stream()), "delta_scan")
+                             _p(batch.cu_seqlens), _p(batch.slots), T, batch.num_seqs, heads, kv_heads, d, dv, _p(decay), _p(o),
+                             _p(work), _stream()), "delta_scan")
 
 
 def mlstm_state_floats(heads, d, dv) -> int:

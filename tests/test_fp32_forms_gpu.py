@@ -1,5 +1,6 @@
 """The forms of the 32-bit kernels that a size picks, at the sizes where they meet: products of few and of many rows
-(16-byte operands; the tile heights; group counts), and attention of 128 queries a block, against float64."""
+(16-byte operands; the tile heights; group counts), attention of 128 queries a block, and the delta rule over chunks of
+sixteen tokens beside the form of four, against float64."""
 import math
 
 import numpy as np
@@ -120,3 +121,42 @@ def test_attention_of_many_new_tokens(core, hd, nh, nkv, before, new, opt):
             assert float((got - ref).abs().max()) < 3e-4, (i, h)
         at += n
     assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("channel", [True, False])
+@pytest.mark.parametrize("H,Gk,d,dv,lens", [(2, 1, 128, 128, [16, 1, 33]), (3, 3, 64, 96, [15, 17, 200]), (2, 2, 12, 20, [31, 48, 5]),
+                                            (2, 1, 100, 36, [64, 3]), (1, 1, 128, 8, [130])])
+def test_the_delta_rule_over_chunks_and_four_at_a_time(core, channel, H, Gk, d, dv, lens):
+    g = torch.Generator(device=DEV).manual_seed(d + dv)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    T, B = sum(lens), len(lens)
+    unit = torch.nn.functional.normalize
+    q, k, v = unit(r(T, Gk, d), dim=-1) * d ** -0.5, unit(r(T, Gk, d), dim=-1), r(T, H, dv)
+    beta, lg = torch.sigmoid(2 * r(T, H)), -torch.nn.functional.softplus(3 * r(T, H))
+    decay = torch.exp(-torch.nn.functional.softplus(3 * r(T, H * d)))
+    decay[::5, ::3] = 0.0                                   # a channel that forgets everything, and one that forgets nothing
+    decay[1::5, 1::3] = 1.0
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, k, v)], 1).contiguous()
+    step = torch.cat([beta, torch.zeros_like(lg) if channel else lg], 1).contiguous()
+    batch = G.make_batch(DEV, list(range(1, B + 1)), [0] * B, lens)
+    start = r(B + 2, 3 + H * d * dv + 1)[:, :4 + H * d * dv].contiguous()
+    owner = torch.arange(H, device=DEV) // (H // Gk)
+    for chunks in (False, True):
+        state, o = start.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
+        core.delta_scan(qkv, step, state, batch, o, heads=H, kv_heads=Gk, d=d, dv=dv, offset=4, decay=decay if channel else None,
+                        chunks=chunks)
+        assert torch.equal(state[0], start[0]) and torch.equal(state[B + 1], start[B + 1]) and torch.equal(state[:, :4], start[:, :4])
+        at = 0
+        for i, n in enumerate(lens):
+            S, ref = start[i + 1, 4:].double().view(H, d, dv), []
+            for t in range(at, at + n):
+                S = S * (decay[t].double().view(H, d, 1) if channel else torch.exp(lg[t].double())[:, None, None])
+                kk, qq = k[t, owner].double(), q[t, owner].double()
+                S = S + kk[:, :, None] * (beta[t].double()[:, None] * (v[t].double() - torch.einsum("hdv,hd->hv", S, kk)))[:, None]
+                ref.append(torch.einsum("hdv,hd->hv", S, qq))
+            ref = torch.stack(ref)
+            got = o[at:at + n].view(n, H, dv).double()
+            # a state of norm about 10 whose every element passes some d + 16 roundings a chunk
+            assert float((got - ref).abs().max()) < 3e-5 * float(ref.abs().max()), (chunks, i)
+            assert float((state[i + 1, 4:].double().view(H, d, dv) - S).abs().max()) < 3e-5 * float(S.abs().max()), (chunks, i)
+            at += n
