@@ -173,6 +173,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
+                                                 uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+        : "memory");
+}
 // D[256, N] (+)= A[256, 16] B[N, 16]^T over the pair: each CTA holds 128 rows of A and N / 2 rows of B
 // at the same shared-memory offsets, and gets its 128 rows of D in its own tensor memory.
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -926,7 +933,8 @@ template <int BN, int MODE>
 __global__ void __launch_bounds__(P_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
     using C = PairCfg<BN, MODE>;
-    constexpr int PAIR_W = 2 * TILE_W;
+    // features of a tile (two CTAs of 128 weight rows; with gate and up rows interleaved, 64 features each)
+    constexpr int PAIR_W = MODE == MODE_SWIGLU_IL ? TILE_W : 2 * TILE_W;
     extern __shared__ uint8_t smem_raw[];
     __shared__ volatile int s_abort;
     __shared__ uint32_t s_tmem;
@@ -986,7 +994,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             bool ok = true;
             for (int item = pair; item < items && ok; item += pairs) {
                 const Tile t = tile_of<BN, PAIR_W>(item, m_tiles, p, s_prefix, s_offs);
-                const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 15) & ~15);
+                const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31);     // (a pair's N: steps of 32)
                 const int half = n_eff >> 1;
                 const int xchunks = (half + C::XBOX - 1) / C::XBOX;
                 const uint32_t cta_tx = C::NW * C::W_BYTES + xchunks * C::XBOX * BK * 2;
@@ -999,7 +1007,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                     const uint32_t st = base + s * C::STAGE_BYTES;
                     const uint32_t bar = mapa_cluster(full_bar(s), 0);
                     if (rank == 0) mbar_expect_tx(full_bar(s), 2 * cta_tx);
-                    tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
+                    if (MODE == MODE_SWIGLU_IL)
+                        tma_load_5d_pair(st, &tmW, kb * BK, 0, 0, t.n0 / 16 + (int)rank * 4, t.g, bar);
+                    else
+                        tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
                     if (MODE == MODE_SWIGLU) tma_load_2d_pair(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, bar);
                     for (int c = 0; c < xchunks; c++)
                         tma_load_2d_pair(st + C::NW * C::W_BYTES + c * C::XBOX * BK * 2, &tmX, kb * BK,
@@ -1021,8 +1032,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             bool ok = true;
             for (int item = pair; item < items && ok; item += pairs, local++) {
                 const Tile t = tile_of<BN, PAIR_W>(item, m_tiles, p, s_prefix, s_offs);
-                const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 15) & ~15);
-                const uint32_t idesc = instr_desc(n_eff, PAIR_W);
+                const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31);
+                const uint32_t idesc = instr_desc(n_eff, 2 * TILE_W);
                 const int b = local & 1;
                 ok = mbar_wait(acc_empty(b), ((local >> 1) & 1) ^ 1, &s_abort, p.wait_limit, p.status, 0x33);   // both epilogues have drained it
                 if (!ok) break;
@@ -1066,8 +1077,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             const uint32_t taddr = tmem + b * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
             const int rows_here = min(BN, t.row_end - t.row0);
             const int part = ((rows_here + 32 * EPI_GROUPS - 1) / (32 * EPI_GROUPS)) * 32;
-            epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
-                                    min(rows_here, h * part), min(rows_here, (h + 1) * part));
+            if (MODE == MODE_SWIGLU_IL)
+                epilogue_part_il<BN>(p, taddr, t.n0 + (int)rank * (TILE_W / 2) + q * 16 + (lane & 15), (lane & 16) != 0, t.row0,
+                                     t.row_end, min(rows_here, h * part), min(rows_here, (h + 1) * part));
+            else
+                epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
+                                        min(rows_here, h * part), min(rows_here, (h + 1) * part));
             // this warp has read its part of the buffer; the issuer waits for all epilogue warps of the pair
             tc_fence_before();
             __syncwarp();
@@ -1181,7 +1196,7 @@ int launch_persistent(const CUtensorMap& tmW, const CUtensorMap& tmX, const Para
     return launch_pdl(gemm_tc_persistent_kernel<BN, MODE>, dim3(ctas), dim3(P_THREADS), (size_t)C::SMEM, stream, tmW, tmX, p);
 }
 
-int g_pair = 0;
+int g_pair = -1;      // 1 / 0: pairs of CTAs for every persistent product / for none; -1: by size (moe_gemm_tc)
 int g_swiglu_il = 1;
 
 template <int BN, int MODE>
@@ -1244,11 +1259,27 @@ MOE_API int moe_gemm_tc(const void* X, int ldx, const void* W, int num_groups, i
         const int mt = group_offsets ? (M < num_groups ? M : num_groups) + M / pbn : (M + pbn - 1) / pbn;
         const long long max_items = (long long)mt * ((N + TILE_W - 1) / TILE_W);
         const int cap = max_items > (1 << 30) ? (1 << 30) : (int)max_items;
-        if (g_pair && sm_count() >= 2) {
-            // pairs of CTAs on tiles of 256 features: half the activation traffic into shared memory
+        // Pairs of CTAs on tiles of 256 features bring half of the activations' bytes into every SM's shared memory.  Measured,
+        // us, single / pair: qkv (6,144 x 2,048) at 2,048 tokens 49.3 / 49.0, 3,072 65 / 62, 4,096 91 / 85, 8,192 172 / 156; the
+        // shared expert's gate and up 84 / 87, 121 / 124, 156 / 155, 300 / 290; 60 experts' gate and up (four a token) 145 / 147, 168 /
+        // 166, 248 / 250, 408 / 391, their down product 83.5 / 82.3, 95 / 91, 133 / 130, 223 / 204.
+        const int each = group_offsets ? M / num_groups : M;
+        const bool pair = g_pair > 0 || (g_pair < 0 && (group_offsets ? each >= 256 : each >= (mode == MODE_SWIGLU ? 4096 : 3072)));
+        if (pair && sm_count() >= 2) {
             const long long pair_items = (long long)mt * ((N + 2 * TILE_W - 1) / (2 * TILE_W));
             const int pcap = pair_items > (1 << 30) ? (1 << 30) : (int)pair_items;
-            if (mode == MODE_SWIGLU) return launch_pair<128, MODE_SWIGLU>(tmW, tmX, p, pcap, stream);
+            if (mode == MODE_SWIGLU) {
+                CUtensorMap tmG;
+                if (g_swiglu_il && make_map_gate_up(&tmG, W, (uint64_t)num_groups, (uint64_t)N, (uint64_t)K)) {
+                    const int ibn = bn >= 256 ? 256 : 128;
+                    const int imt = group_offsets ? (M < num_groups ? M : num_groups) + M / ibn : (M + ibn - 1) / ibn;
+                    const long long il_items = (long long)imt * ((N + TILE_W - 1) / TILE_W);
+                    const int icap = il_items > (1 << 30) ? (1 << 30) : (int)il_items;
+                    if (ibn == 256) return launch_pair<256, MODE_SWIGLU_IL>(tmG, tmX, p, icap, stream);
+                    return launch_pair<128, MODE_SWIGLU_IL>(tmG, tmX, p, icap, stream);
+                }
+                return launch_pair<128, MODE_SWIGLU>(tmW, tmX, p, pcap, stream);
+            }
             if (act) return pbn == 128 ? launch_pair<128, MODE_ACT>(tmW, tmX, p, pcap, stream) : launch_pair<256, MODE_ACT>(tmW, tmX, p, pcap, stream);
             if (pbn == 128) return launch_pair<128, MODE_PLAIN>(tmW, tmX, p, pcap, stream);
             return launch_pair<256, MODE_PLAIN>(tmW, tmX, p, pcap, stream);
@@ -1306,9 +1337,8 @@ MOE_API void moe_tc_set_wait_test(int fault, unsigned wait_limit) {
     g_wait_limit = wait_limit ? wait_limit : WAIT_LIMIT_US;
 }
 
-// Pairs of CTAs (cta_group::2) for the persistent form on or off (off by default: measured equal or
-// slower than single CTAs at the sizes tried, so what bounds those is not the activation traffic).
-MOE_API void moe_tc_set_pair(int enabled) { g_pair = enabled ? 1 : 0; }
+// Pairs of CTAs (cta_group::2) for every persistent product (1), for none (0), or by size (-1, the default).
+MOE_API void moe_tc_set_pair(int enabled) { g_pair = enabled < 0 ? -1 : enabled ? 1 : 0; }
 
 // How many K splits the kernel will really use for (K, splits asked), and its grid.y for tickets.
 MOE_API int moe_gemm_tc_plan(int K, int splits, int M, int bn, int num_groups, int grouped, int* grid_y) {
