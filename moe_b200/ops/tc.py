@@ -55,8 +55,8 @@ def lib():
             L.moe_tc_set_swiglu_interleaved(0)
         L.moe_tc_set_pair.argtypes = [c_int]
         L.moe_tc_set_pair.restype = None
-        if os.environ.get("MOE_B200_PAIR", "0") == "1":         # pairs of CTAs (cta_group::2) for many tokens
-            L.moe_tc_set_pair(1)
+        if os.environ.get("MOE_B200_PAIR"):     # pairs of CTAs (cta_group::2) for all products of many tokens, or none
+            L.moe_tc_set_pair(1 if os.environ["MOE_B200_PAIR"] == "1" else 0)
         _lib = L
     return _lib
 
@@ -126,10 +126,24 @@ def token_tile(rows_per_group: float, grouped: bool = False) -> int:
     return 256
 
 
+def mid_splits(M: int, n_tiles: int, k_blocks: int, sms: int) -> int:
+    """K splits of a plain dense product of more than 64 rows whose tiles of 64 rows x 128 features all find room on the SMs at
+    once (two CTAs an SM); 0 where they do not, and the persistent form with tiles of 256 rows is the better one.  A
+    persistent launch of 16 to 150 tiles leaves most SMs without work: measured, us, persistent / tiles of 64 with splits, output
+    projection (2,048 x 2,048) at 80, 256, 512 rows 13.3 / 7.3, 16.8 / 10.1, 17.1 / 15.4; the shared expert's down product (5,632 x
+    2,048) 29.0 / 10.5, 35.2 / 14.9, 35.3 / 23.8; qkv (2,048 x 6,144) 14.3 / 14.8, 18.1 / 15.5 and, where its tiles no longer find
+    room (512 rows), 18.9 / 29.8.  Two splits of 32 or fewer k blocks cost what they gain."""
+    tiles = -(-M // 64) * n_tiles
+    if tiles > 2 * sms:
+        return 0
+    splits = max(1, min(8, 256 * sms // (148 * tiles), k_blocks // 4))
+    return 1 if splits == 2 and k_blocks <= 32 else splits
+
+
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swiglu: bool = False,
             bias: Optional[torch.Tensor] = None, group_offsets: Optional[torch.Tensor] = None,
             bn: Optional[int] = None, splits: Optional[int] = None, status=None, early_offsets: bool = False,
-            act: str = "silu", act_param: float = 0.0) -> bool:
+            act: str = "silu", act_param: float = 0.0, beside: bool = False) -> bool:
     """out = x @ w[g].T (PLAIN) or act(x @ gate.T) * (x @ up.T) (SwiGLU, w rows = gate then up; ``act``
     is the gate's activation, one of ``core.GLU_ACTS``, ``act_param`` its constant if it has one).
 
@@ -139,7 +153,8 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swiglu: bool
     out: [M, N] float32 or bfloat16 with N = N' (PLAIN) or N' / 2 (SwiGLU).
     ``early_offsets``: the caller vouches that ``group_offsets`` were written at least two kernels
     before this one on the stream (not by its direct predecessor); the kernel then starts loading
-    weights while the predecessor still runs."""
+    weights while the predecessor still runs.  ``beside``: the product runs beside others on another stream and
+    keeps to few SMs (no ``mid_splits``)."""
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not x.is_cuda:
         return False
     G = w.shape[0] if w.dim() == 3 else 1
@@ -151,11 +166,14 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swiglu: bool
     if (G > 1 or group_offsets is not None) and (group_offsets is None or group_offsets.numel() != G + 1):
         raise core.KernelError("gemm_tc: group_offsets must have G + 1 entries")
     grouped = group_offsets is not None
-    if bn is None:
-        bn = token_tile(M / max(G, 1), True) if grouped else token_tile(min(M, 256))
     L = lib()
     n_tiles = -(-N // 128)
     gy = c_int(0)
+    if bn is None:
+        bn = token_tile(M / max(G, 1), True) if grouped else token_tile(min(M, 256))
+        if splits is None and bn > 64 and not grouped and not swiglu and not beside:
+            splits = mid_splits(M, n_tiles, -(-K // 64), num_sms(x.device)) or None
+            bn = 64 if splits else bn
     if splits is None:
         if bn > 64:
             # many tokens: the product is bound by the tensor cores and by L2, and the split-K

@@ -343,7 +343,9 @@ class RoutedExperts(Part):
             from ..ops import tc
 
             logits = rt.empty((T, self.w_router3.shape[0]), torch.float32)
-            if tc.gemm_tc(core.split3(h.f32), self.w_router3, logits, bn=64, splits=8, status=rt.status):
+            # (one tile of features: the K splits fill the SMs; at 2,048 / 4,096 / 8,192 tokens eight take 11.0 / 21.4 / 43.6 us,
+            # four 13.9 / 14.9 / 33.0)
+            if tc.gemm_tc(core.split3(h.f32), self.w_router3, logits, bn=64, splits=8 if T <= 2048 else 4, status=rt.status):
                 if after_logits is not None:
                     after_logits()
                 core.router_topk(logits, self.k, self.norm_topk, self.scale, topk_idx, topk_w, num_experts=self.E,
@@ -358,7 +360,10 @@ class RoutedExperts(Part):
         return topk_idx, topk_w, sg
 
     def _shared(self, rt, h):
-        return linear(rt, swiglu_linear(rt, h.act, self.ws_gu), self.ws_down)
+        # (up to 256 rows the down product keeps to few SMs: it runs beside the routed products, which want the others; cut into
+        # pieces for all of them a step of three prompts, 145 tokens, took 1,867 instead of 1,795 us.  At 512 rows it is the
+        # longer of the two branches: 2,353 against 2,211 us a step.)
+        return linear(rt, swiglu_linear(rt, h.act, self.ws_gu), self.ws_down, beside=h.act.shape[0] <= 256)
 
     def forward(self, rt, h, batch):
         return self._run(rt, h, batch, None).materialize(rt)

@@ -1,0 +1,94 @@
+"""Which form a tensor-core product takes by its number of rows: tiles of 64 with K splits between the few rows of a decode step
+and the persistent form, pairs of CTAs from some thousand rows on.  Sizes at the edges of tiles, splits and of the rules."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture
+def tc():
+    from moe_b200.ops import tc as t
+
+    t.lib().moe_tc_set_pair(-1)
+    yield t
+    t.lib().moe_tc_set_pair(0)
+
+
+def bound(x, w):
+    """Products of bfloat16 numbers are exact in 32 bits; K of them are added, every sum off by at most one unit."""
+    return (x.shape[1] + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + 1e-30
+
+
+@pytest.mark.parametrize("M", [65, 80, 127, 128, 129, 200, 256, 257, 320, 511, 512, 700])
+@pytest.mark.parametrize("N,K", [(136, 72), (2048, 2048), (256, 5632), (5000, 264)])
+def test_rows_between(tc, M, N, K):
+    from moe_b200.ops import core
+
+    torch.manual_seed(M + N)
+    st, x, w = core.new_status(DEV), torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    b = torch.randn(N, device=DEV)
+    for beside in (False, True):
+        out = torch.full((M + 1, N), float("nan"), device=DEV)
+        assert tc.gemm_tc(x, w, out[:M], bias=b, status=st, beside=beside)
+        ref = x.double() @ w.double().T + b.double()
+        assert bool(((out[:M].double() - ref).abs() <= bound(x, w) + 2.0 ** -23 * ref.abs()).all()) and bool(out[M].isnan().all())
+    assert int(st[0]) == 0
+
+
+def test_splits_between_find_room():
+    from moe_b200.ops.tc import mid_splits
+
+    for M in range(65, 1200, 7):
+        for n_tiles in (1, 2, 16, 28, 36, 48, 88):
+            for kb in (1, 3, 22, 32, 56, 88, 320):
+                s, tiles = mid_splits(M, n_tiles, kb, 148), -(-M // 64) * n_tiles
+                assert (s == 0) == (tiles > 296)
+                assert s == 0 or (1 <= s <= 8 and tiles * s <= 296 and (s == 1 or kb // s >= 4))
+
+
+@pytest.mark.parametrize("M", [3071, 3072, 4095, 4097])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_pairs_by_rows(tc, M, swiglu):
+    from moe_b200.ops import core
+
+    torch.manual_seed(M)
+    N, K = 208, 200
+    st, x, w = core.new_status(DEV), torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N * (2 if swiglu else 1), K, device=DEV).bfloat16()
+    out = torch.full((M, N), float("nan"), device=DEV)
+    assert tc.gemm_tc(x, w, out, swiglu=swiglu, status=st)
+    ref, off = x.double() @ w.double().T, bound(x, w)
+    if swiglu:
+        # |d silu| <= 1.1 |d gate|, then the rounding of silu (a few units) and of the product
+        gate, up = ref[:, :N], ref[:, N:]
+        off = 1.1 * off[:, :N] * (up.abs() + off[:, N:]) + gate.abs() * off[:, N:] + 2.0 ** -20 * (gate * up).abs()
+        ref = torch.nn.functional.silu(gate) * up
+    assert bool(((out.double() - ref).abs() <= off + 2.0 ** -23 * ref.abs()).all())
+    assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("counts", [[300, 0, 470], [256, 257, 255], [1, 900, 0, 513], [200, 200]])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_pairs_of_groups(tc, counts, swiglu):
+    from moe_b200.ops import core
+
+    torch.manual_seed(sum(counts))
+    N, K, E, M = 176, 136, len(counts), sum(counts)
+    st, x = core.new_status(DEV), torch.randn(M, K, device=DEV).bfloat16()
+    w = torch.randn(E, N * (2 if swiglu else 1), K, device=DEV).bfloat16()
+    offs = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
+    out = torch.full((M, N), float("nan"), device=DEV)
+    assert tc.gemm_tc(x, w, out, swiglu=swiglu, group_offsets=offs, status=st)
+    at = 0
+    for e, n in enumerate(counts):
+        r = x[at:at + n].double() @ w[e].double().T
+        off = bound(x[at:at + n], w[e])
+        if swiglu:
+            g, u = r[:, :N], r[:, N:]
+            off = 1.1 * off[:, :N] * (u.abs() + off[:, N:]) + g.abs() * off[:, N:] + 2.0 ** -20 * (g * u).abs()
+            r = torch.nn.functional.silu(g) * u
+        assert bool(((out[at:at + n].double() - r).abs() <= off + 2.0 ** -23 * r.abs()).all()), e
+        at += n
+    assert int(st[0]) == 0
