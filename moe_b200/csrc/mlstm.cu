@@ -481,6 +481,291 @@ mlstm_scan_kernel(const MemSeq p, float* __restrict__ o, const MemSegments sg) {
     }
 }
 
+// ---- several tokens a sequence: chunks of sixty-four side by side ------------------------------------------------------
+// The same sums with a chunk in the place of a group of four: what a chunk adds to S and n (mlstm_chunk_add_kernel) and its
+// outputs from the state before it (mlstm_chunk_out_kernel) are products of 64 tokens, formed for all chunks side by side; only
+// the state's way through the chunks is a chain, one multiply-add an element and chunk (mlstm_chunk_state_kernel, which puts
+// the state before a chunk in the place of what the chunk adds).  The scan above is bound by its
+// shuffles and reads of shared memory (2,048 tokens, 16 heads of 64 x 128, in eight segments: 108 + 184 us; here 39 + 34 + 92 us).
+// Factors are products of a.
+constexpr int QC = 64, QV = 128;       // tokens a chunk; columns of S a block
+struct MemChunks {
+    float* add;              // [chunk][H][d][dv]: what the chunk adds, then the state before it
+    float* norm;             // [chunk][H][d]: the same of n
+    float* keep;             // [chunk][H]: the product of the chunk's a
+};
+// number of the chunk that starts at token `tok` (counted in the step) of sequence s: different for all chunks of a step
+__device__ __forceinline__ int mem_chunk(int tok, int s) { return tok / QC + s; }
+// the sequence whose chunk `number` is, or -1; by the whole block
+__device__ __forceinline__ int mem_chunk_seq(const MemSeq& p, int num_seqs, int number, int* s_seq) {
+    if (threadIdx.x == 0) *s_seq = -1;
+    __syncthreads();
+    for (int s = threadIdx.x; s < num_seqs; s += blockDim.x) {
+        const int a = p.cu_seqlens[s], n = p.cu_seqlens[s + 1] - a, first = mem_chunk(a, s);
+        if (n > 0 && number >= first && number < first + (n + QC - 1) / QC) *s_seq = s;
+    }
+    __syncthreads();
+    return *s_seq;
+}
+
+// grid (chunks, heads, ceil(dv / 128)): a thread 4 rows x 8 columns of a 64-row part of S
+__global__ void __launch_bounds__(256)
+mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
+    extern __shared__ __align__(16) float sm[];               // k [64][d + 4], scaled | v [64][132]
+    __shared__ float s_a[QC], s_b[QC];
+    __shared__ int s_seq;
+    const int tid = threadIdx.x, number = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
+    pdl_sync();
+    const int s = mem_chunk_seq(p, num_seqs, number, &s_seq);
+    if (s < 0) return;
+    const int a0 = p.cu_seqlens[s], tok = a0 + (number - mem_chunk(a0, s)) * QC, cnt = min(QC, p.cu_seqlens[s + 1] - tok);
+    const int ncols = min(QV, dv - c0);
+    float* sk = sm;
+    float* sv = sm + QC * dp;
+    if (tid < QC) {
+        const float* st = p.steps + (size_t)(tok + tid) * 3 * p.H + h;
+        s_a[tid] = tid < cnt ? st[0] : 1.f, s_b[tid] = tid < cnt ? st[p.H] : 0.f;
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int e = tid; e < QC * (QV / 4); e += 256) {
+        const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
+        *reinterpret_cast<float4*>(sv + i * (QV + 4) + x) =
+            i < cnt && x < ncols ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.v_at + h * dv + c0 + x) : zero;
+    }
+    __syncthreads();
+    for (int e = tid; e < QC * (d / 4); e += 256) {
+        const int i = e / (d / 4), x = (e % (d / 4)) * 4;
+        float4 k4 = i < cnt ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.k_at + h * d + x) : zero;
+        float f = s_b[i];
+        for (int l = i + 1; l < cnt; l++) f *= s_a[l];
+        k4.x *= f, k4.y *= f, k4.z *= f, k4.w *= f;
+        *reinterpret_cast<float4*>(sk + i * dp + x) = k4;
+    }
+    __syncthreads();
+    const size_t at = ((size_t)number * p.H + h) * d;
+    if (blockIdx.z == 0) {
+        for (int x = tid; x < d; x += 256) {
+            float n = 0.f;
+            for (int i = 0; i < QC; i++) n += sk[i * dp + x];
+            c.norm[at + x] = n;
+        }
+        if (tid == 0) {
+            float a = 1.f;
+            for (int i = 0; i < cnt; i++) a *= s_a[i];
+            c.keep[(size_t)number * p.H + h] = a;
+        }
+    }
+    const int rg = (tid >> 4) * 4, cg = (tid & 15) * 4;
+    for (int r0 = rg; r0 < d; r0 += 64) {
+        float acc[4][8];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int e = 0; e < 8; e++) acc[r][e] = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < QC; i++) {
+            const float4 k4 = *reinterpret_cast<const float4*>(sk + i * dp + r0);
+            const float4 va = *reinterpret_cast<const float4*>(sv + i * (QV + 4) + cg), vb = *reinterpret_cast<const float4*>(sv + i * (QV + 4) + 64 + cg);
+            const float k[4] = {k4.x, k4.y, k4.z, k4.w}, v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int e = 0; e < 8; e++) acc[r][e] = fmaf(k[r], v[e], acc[r][e]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int x = e * 64 + cg;
+                if (r0 + r < d && x < ncols)
+                    *reinterpret_cast<float4*>(c.add + (at + r0 + r) * dv + c0 + x) =
+                        make_float4(acc[r][4 * e], acc[r][4 * e + 1], acc[r][4 * e + 2], acc[r][4 * e + 3]);
+            }
+    }
+}
+
+// grid (ceil((d dv / 4 + d) / 256), heads, sequences): an element of S (four) or of n a thread, through its sequence's chunks
+__global__ void __launch_bounds__(256)
+mlstm_chunk_state_kernel(const MemSeq p, const MemChunks c) {
+    pdl_sync();
+    const int h = blockIdx.y, s = blockIdx.z, d = p.d, dv = p.dv, quads = d * dv / 4;
+    const int a0 = p.cu_seqlens[s], cnt = p.cu_seqlens[s + 1] - a0, e = blockIdx.x * 256 + threadIdx.x;
+    if (cnt <= 0 || e >= quads + d) return;
+    const int first = mem_chunk(a0, s), chunks = (cnt + QC - 1) / QC;
+    float* state = p.state + (size_t)p.slots[s] * p.state_pitch;
+    const float* keep = c.keep + (size_t)first * p.H + h;
+    if (e < quads) {
+        float4* from = reinterpret_cast<float4*>(state + (size_t)h * d * dv) + e;
+        float4* at = reinterpret_cast<float4*>(c.add + ((size_t)first * p.H + h) * d * dv) + e;
+        const size_t step = (size_t)p.H * quads;
+        float4 S = *from;
+        for (int i = 0; i < chunks; i += 4) {                 // (the loads of four chunks in flight)
+            float4 x[4];
+            float k[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (i + j < chunks) x[j] = at[(i + j) * step], k[j] = keep[(size_t)(i + j) * p.H];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (i + j < chunks) {
+                    at[(i + j) * step] = S;
+                    S.x = fmaf(k[j], S.x, x[j].x), S.y = fmaf(k[j], S.y, x[j].y), S.z = fmaf(k[j], S.z, x[j].z), S.w = fmaf(k[j], S.w, x[j].w);
+                }
+        }
+        *from = S;
+    } else {
+        const int x = e - quads;
+        float* at = c.norm + ((size_t)first * p.H + h) * d + x;
+        float n = state[p.n_at(0, h) + x];
+        for (int i = 0; i < chunks; i++) {
+            const float y = at[(size_t)i * p.H * d];
+            at[(size_t)i * p.H * d] = n;
+            n = fmaf(keep[(size_t)i * p.H], n, y);
+        }
+        for (int i = 0; i < p.copies; i++) state[p.n_at(i, h) + x] = n;
+    }
+}
+
+// grid (chunks, heads, ceil(dv / 128)): the pair products of a chunk, 4 x 4 a thread; the outputs, 4 rows x 8 columns a thread
+constexpr int QP = QC + 4;
+__host__ __device__ constexpr size_t mlstm_chunk_out_floats(int d) {
+    return (size_t)2 * QC * (d + 4) + QC * QP + QC * (QV + 4) + (size_t)d * (QV + 4) + d;
+}
+__global__ void __launch_bounds__(256)
+mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* __restrict__ o) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float s_a[QC], s_b[QC], s_all[QC], s_den[QC];
+    __shared__ int s_seq;
+    const int tid = threadIdx.x, number = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
+    float* sq = sm;                    // [64][d + 4]
+    float* sk = sq + QC * dp;          // [64][d + 4]
+    float* sP = sk + QC * dp;          // [64][68]
+    float* sv = sP + QC * QP;          // [64][132]
+    float* sS = sv + QC * (QV + 4);    // [d][132]
+    float* sn = sS + d * (QV + 4);     // [d]
+    pdl_sync();
+    const int s = mem_chunk_seq(p, num_seqs, number, &s_seq);
+    if (s < 0) return;
+    const int a0 = p.cu_seqlens[s], tok = a0 + (number - mem_chunk(a0, s)) * QC, cnt = min(QC, p.cu_seqlens[s + 1] - tok);
+    const int ncols = min(QV, dv - c0);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const size_t at = ((size_t)number * p.H + h) * d;
+    if (tid < QC) {
+        const float* st = p.steps + (size_t)(tok + tid) * 3 * p.H + h;
+        s_a[tid] = tid < cnt ? st[0] : 1.f, s_b[tid] = tid < cnt ? st[p.H] : 0.f, s_den[tid] = tid < cnt ? st[2 * p.H] : 1.f;
+    }
+    for (int e = tid; e < QC * (d / 4); e += 256) {
+        const int i = e / (d / 4), x = (e % (d / 4)) * 4;
+        const float* row = p.proj + (size_t)(tok + i) * p.ld + h * d + x;
+        float4 q4 = i < cnt ? *reinterpret_cast<const float4*>(row + p.q_at) : zero;
+        q4.x *= p.q_scale, q4.y *= p.q_scale, q4.z *= p.q_scale, q4.w *= p.q_scale;
+        *reinterpret_cast<float4*>(sq + i * dp + x) = q4;
+        *reinterpret_cast<float4*>(sk + i * dp + x) = i < cnt ? *reinterpret_cast<const float4*>(row + p.k_at) : zero;
+    }
+    for (int e = tid; e < QC * (QV / 4); e += 256) {
+        const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
+        *reinterpret_cast<float4*>(sv + i * (QV + 4) + x) =
+            i < cnt && x < ncols ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.v_at + h * dv + c0 + x) : zero;
+    }
+    for (int e = tid; e < d * (QV / 4); e += 256) {
+        const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
+        *reinterpret_cast<float4*>(sS + i * (QV + 4) + x) = x < ncols ? *reinterpret_cast<const float4*>(c.add + (at + i) * dv + c0 + x) : zero;
+    }
+    for (int x = tid; x < d; x += 256) sn[x] = c.norm[at + x];
+    __syncthreads();
+    if (tid < QC) {                    // column j of the pair factors: b_j times the a after j, 0 above the diagonal
+        float run = s_b[tid];
+        for (int i = 0; i < QC; i++) {
+            if (i > tid) run *= s_a[i];
+            sP[i * QP + tid] = i >= tid ? run : 0.f;
+        }
+    } else if (tid < 2 * QC) {         // from the chunk's first token to its i-th
+        float run = 1.f;
+        for (int i = 0; i <= tid - QC; i++) run *= s_a[i];
+        s_all[tid - QC] = run;
+    }
+    __syncthreads();
+    const int ty = tid >> 4, tx = tid & 15;
+    {
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+#pragma unroll 2
+        for (int x = 0; x < d; x += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(sq + (ty + 16 * i) * dp + x);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 b = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * dp + x);
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    acc[i][j] = fmaf(a[i].x, b.x, fmaf(a[i].y, b.y, fmaf(a[i].z, b.z, fmaf(a[i].w, b.w, acc[i][j]))));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) sP[(ty + 16 * i) * QP + tx + 16 * j] *= acc[i][j];
+    }
+    __syncthreads();
+    {                                  // n . q of a token by four neighbouring threads
+        const int i = tid >> 2, part = tid & 3;
+        float in = 0.f, held = 0.f;
+        for (int j = part; j < QC; j += 4) in += sP[i * QP + j];
+        for (int x = part; x < d; x += 4) held = fmaf(sq[i * dp + x], sn[x], held);
+        float n = fmaf(s_all[i], held, in);
+        n += __shfl_xor_sync(0xffffffffu, n, 1);
+        n += __shfl_xor_sync(0xffffffffu, n, 2);
+        __syncwarp();
+        if (part == 0) s_den[i] = fmaxf(fabsf(n), s_den[i]) + READ_EPS;
+    }
+    float in[4][8], held[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int e = 0; e < 8; e++) in[i][e] = held[i][e] = 0.f;
+    auto product = [&](const float* left, int pitch, int n, const float* right, float (&acc)[4][8]) {
+#pragma unroll 2
+        for (int x = 0; x < n; x += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(left + (ty + 16 * i) * pitch + x);
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                const float* row = right + (x + z) * (QV + 4) + tx * 4;
+                const float4 va = *reinterpret_cast<const float4*>(row), vb = *reinterpret_cast<const float4*>(row + 64);
+                const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
+#pragma unroll
+                    for (int e = 0; e < 8; e++) acc[i][e] = fmaf(f, v[e], acc[i][e]);
+                }
+            }
+        }
+    };
+    product(sP, QP, QC, sv, in);
+    product(sq, dp, d, sS, held);
+    __syncthreads();                   // the denominators are there
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int t = ty + 16 * i;
+        if (t >= cnt) continue;
+        const float all = s_all[t], den = s_den[t];
+        float* dst = o + ((size_t)(tok + t) * p.H + h) * dv + c0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int x = e * 64 + tx * 4;
+            if (x < ncols)
+                *reinterpret_cast<float4*>(dst + x) = make_float4(fmaf(all, held[i][4 * e], in[i][4 * e]) / den, fmaf(all, held[i][4 * e + 1], in[i][4 * e + 1]) / den,
+                                                                  fmaf(all, held[i][4 * e + 2], in[i][4 * e + 2]) / den, fmaf(all, held[i][4 * e + 3], in[i][4 * e + 3]) / den);
+        }
+    }
+}
+
 bool aligned16(const void* p) { return (uintptr_t)p % 16 == 0; }
 
 }  // namespace
@@ -562,6 +847,48 @@ MOE_API int moe_mlstm_scan(const float* proj, long long ld, int q_at, int k_at, 
 #undef SCAN
 #undef SCAN_V
 #undef SCAN_P
+}
+
+// Floats of scratch of moe_mlstm_chunks; 0 for sizes it does not take.
+MOE_API long long moe_mlstm_chunk_floats(long long num_tokens, int num_seqs, int H, int d, int dv) {
+    if (num_tokens <= 0 || num_seqs <= 0 || num_seqs > 65535 || H <= 0 || H > 65535 || d <= 0 || d > 128 || d % 4 || dv <= 0 || dv % 4 ||
+        (dv + QV - 1) / QV > 65535)
+        return 0;
+    const long long chunks = num_tokens / QC + num_seqs + 1;
+    return chunks * H * d * dv + (chunks * H * d + 3) / 4 * 4 + chunks * H;
+}
+
+// The same as moe_mlstm_scan, over chunks of sixty-four tokens; `work`: moe_mlstm_chunk_floats floats.  Returns -1, with nothing
+// launched, for rows that are not whole 16-byte units and sizes it does not take.
+MOE_API int moe_mlstm_chunks(const float* proj, long long ld, int q_at, int k_at, int v_at, int i_at, int f_at,
+                             const float* i_bias, const float* f_bias, float cap, float q_scale, float* state,
+                             long long state_pitch, const int* cu_seqlens, const int* slots, int num_tokens, int num_seqs, int H,
+                             int d, int dv, float* steps, float* o, int longest, float* work, cudaStream_t stream) {
+    if (num_seqs <= 0 || num_tokens <= 0) return 0;
+    if (!steps || !o || !work ||
+        mlstm_bad(proj, ld, q_at, k_at, v_at, i_at, f_at, i_bias, f_bias, state, state_pitch, cu_seqlens, slots, H, d, dv, cap))
+        return (int)cudaErrorInvalidValue;
+    if (!moe_mlstm_chunk_floats(num_tokens, num_seqs, H, d, dv) || ld % 4 || q_at % 4 || k_at % 4 || v_at % 4 || state_pitch % 4 ||
+        !aligned16(proj) || !aligned16(state) || !aligned16(o) || !aligned16(work))
+        return -1;
+    const MemSeq p{proj, ld, q_at, k_at, v_at, i_at, f_at, i_bias, f_bias, state, state_pitch, cu_seqlens, slots, steps,
+                   H, d, dv, cap, q_scale, (dv + COPY_COLS - 1) / COPY_COLS};
+    const int chunks = num_tokens / QC + num_seqs + 1;
+    MemChunks c;
+    c.add = work, c.norm = work + (size_t)chunks * H * d * dv, c.keep = c.norm + ((size_t)chunks * H * d + 3) / 4 * 4;
+    const int threads = longest > 0 && longest < 1024 ? (longest + 31) / 32 * 32 : 1024;
+    int code = launch_pdl(mlstm_gates_kernel, dim3(H, num_seqs), dim3(threads), 0, stream, p);
+    if (code) return code;
+    const dim3 grid(chunks, H, (dv + QV - 1) / QV);
+    const size_t add = ((size_t)QC * (d + 4) + QC * (QV + 4)) * 4, out = mlstm_chunk_out_floats(d) * 4;
+    cudaError_t e = cudaFuncSetAttribute(mlstm_chunk_add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)add);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
+    if (e != cudaSuccess) return (int)e;
+    code = launch_pdl(mlstm_chunk_add_kernel, grid, dim3(256), add, stream, p, c, num_seqs);
+    if (code) return code;
+    code = launch_pdl(mlstm_chunk_state_kernel, dim3((d * dv / 4 + d + 255) / 256, H, num_seqs), dim3(256), 0, stream, p, c);
+    if (code) return code;
+    return launch_pdl(mlstm_chunk_out_kernel, grid, dim3(256), out, stream, p, c, num_seqs, o);
 }
 
 // One token a sequence: gates, recurrence, head norm (norm_w [H * dv]) and gate (gate: [T, H * dv] 32-bit logits, rows of

@@ -127,14 +127,14 @@ def token_tile(rows_per_group: float, grouped: bool = False) -> int:
 
 
 def mid_splits(M: int, n_tiles: int, k_blocks: int, sms: int) -> int:
-    """K splits of a plain dense product of more than 64 rows whose tiles of 64 rows x 128 features all find room on the SMs at
-    once (two CTAs an SM); 0 where they do not, and the persistent form with tiles of 256 rows is the better one.  A
+    """K splits of a plain dense product of 65 to 512 rows whose tiles of 64 rows x 128 features all find room on the SMs at
+    once (two CTAs an SM); 0 where they do not, or with more rows, and the persistent form with tiles of 256 rows is the better one.  A
     persistent launch of 16 to 150 tiles leaves most SMs without work: measured, us, persistent / tiles of 64 with splits, output
     projection (2,048 x 2,048) at 80, 256, 512 rows 13.3 / 7.3, 16.8 / 10.1, 17.1 / 15.4; the shared expert's down product (5,632 x
     2,048) 29.0 / 10.5, 35.2 / 14.9, 35.3 / 23.8; qkv (2,048 x 6,144) 14.3 / 14.8, 18.1 / 15.5 and, where its tiles no longer find
     room (512 rows), 18.9 / 29.8.  Two splits of 32 or fewer k blocks cost what they gain."""
     tiles = -(-M // 64) * n_tiles
-    if tiles > 2 * sms:
+    if M > 512 or tiles > 2 * sms:
         return 0
     splits = max(1, min(8, 256 * sms // (148 * tiles), k_blocks // 4))
     return 1 if splits == 2 and k_blocks <= 32 else splits

@@ -1,6 +1,6 @@
 """The forms of the 32-bit kernels that a size picks, at the sizes where they meet: products of few and of many rows
-(16-byte operands; the tile heights; group counts), attention of 128 queries a block, and the delta rule over chunks of
-sixteen tokens beside the form of four, against float64."""
+(16-byte operands; the tile heights; group counts), attention of 128 queries a block, the delta rule over chunks of
+sixteen tokens and the mLSTM memory over chunks of sixty-four beside their forms of four, against float64."""
 import math
 
 import numpy as np
@@ -160,3 +160,45 @@ def test_the_delta_rule_over_chunks_and_four_at_a_time(core, channel, H, Gk, d, 
             assert float((got - ref).abs().max()) < 3e-5 * float(ref.abs().max()), (chunks, i)
             assert float((state[i + 1, 4:].double().view(H, d, dv) - S).abs().max()) < 3e-5 * float(S.abs().max()), (chunks, i)
             at += n
+
+
+@pytest.mark.parametrize("H,d,dv,lens", [(2, 64, 128, [1, 63, 64]), (3, 12, 20, [65, 130]), (1, 100, 36, [200]), (2, 128, 260, [70, 5])])
+def test_the_memory_over_chunks_and_four_at_a_time(core, H, d, dv, lens):
+    g = torch.Generator(device=DEV).manual_seed(d + dv)
+    T, B, cap = sum(lens), len(lens), 9.0
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    proj = torch.randn(T, -(-(at["f"] + H) // 4) * 4, device=DEV, generator=g)
+    ib, fb = (torch.randn(H, device=DEV, generator=g) + b for b in (-0.5, 2.0))
+    floats = core.mlstm_state_floats(H, d, dv)
+    copies = -(-dv // 16)
+    start = torch.zeros(B + 2, -(-(floats + 4) // 4) * 4, device=DEV)
+    start[:, 4:4 + H * d * dv] = 0.3 * torch.randn(B + 2, H * d * dv, device=DEV, generator=g)
+    norm = 0.3 * torch.randn(B + 2, 1, H * d, device=DEV, generator=g)
+    start[:, 4 + H * d * dv:4 + H * d * (dv + copies)] = norm.expand(-1, copies, -1).reshape(B + 2, -1)
+    batch = G.make_batch(DEV, list(range(1, B + 1)), [0] * B, lens)
+    for segments in (None, 1):
+        state, o = start.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
+        core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, offset=4, segments=segments)
+        assert torch.equal(state[0], start[0]) and torch.equal(state[B + 1], start[B + 1]) and torch.equal(state[:, :4], start[:, :4])
+        t0 = 0
+        for i, n in enumerate(lens):
+            x = proj[t0:t0 + n].double()
+            q, k = (x[:, at[c]:at[c] + H * d].view(n, H, d) for c in "qk")
+            v = x[:, at["v"]:at["v"] + H * dv].view(n, H, dv)
+            li = cap * torch.tanh((x[:, at["i"]:at["i"] + H] + ib.double()) / cap)
+            lf = torch.nn.functional.logsigmoid(cap * torch.tanh((x[:, at["f"]:at["f"] + H] + fb.double()) / cap))
+            S, z, m, ref = start[i + 1, 4:4 + H * d * dv].double().view(H, d, dv), norm[i + 1, 0].double().view(H, d), torch.zeros(H, device=DEV, dtype=torch.float64), []
+            for t in range(n):
+                new = torch.maximum(lf[t] + m, li[t])
+                a, b = torch.exp(lf[t] + m - new), torch.exp(li[t] - new)
+                m, S, z = new, a[:, None, None] * S + b[:, None, None] * k[t][:, :, None] * v[t][:, None], a[:, None] * z + b[:, None] * k[t]
+                den = torch.maximum((z * q[t]).sum(-1).abs() * d ** -0.5, torch.exp(-m)) + 1e-6
+                ref.append(torch.einsum("hdv,hd->hv", S, q[t]) * d ** -0.5 / den[:, None])
+            ref, got = torch.stack(ref), o[t0:t0 + n].view(n, H, dv).double()
+            # sums of up to 200 terms of size 1 over a denominator of at least e^(-m): relative to the largest output
+            assert float((got - ref).abs().max()) < 3e-5 * float(ref.abs().max()), (segments, i)
+            assert float((state[i + 1, 4:4 + H * d * dv].double().view(H, d, dv) - S).abs().max()) < 3e-5 * float(S.abs().max()), (segments, i)
+            held = state[i + 1, 4 + H * d * dv:4 + H * d * (dv + copies)].double().view(copies, H, d)
+            assert float((held - z).abs().max()) < 3e-5 * float(z.abs().max()), (segments, i)
+            assert float((state[i + 1, 4 + H * d * (dv + copies):4 + floats].double() - m).abs().max()) < 1e-5 * max(1.0, float(m.abs().max()))
+            t0 += n

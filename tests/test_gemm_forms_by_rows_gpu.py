@@ -22,7 +22,7 @@ def bound(x, w):
     return (x.shape[1] + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T) + 1e-30
 
 
-@pytest.mark.parametrize("M", [65, 80, 127, 128, 129, 200, 256, 257, 320, 511, 512, 700])
+@pytest.mark.parametrize("M", [65, 80, 127, 128, 129, 200, 256, 257, 320, 511, 512, 513])
 @pytest.mark.parametrize("N,K", [(136, 72), (2048, 2048), (256, 5632), (5000, 264)])
 def test_rows_between(tc, M, N, K):
     from moe_b200.ops import core
@@ -45,7 +45,7 @@ def test_splits_between_find_room():
         for n_tiles in (1, 2, 16, 28, 36, 48, 88):
             for kb in (1, 3, 22, 32, 56, 88, 320):
                 s, tiles = mid_splits(M, n_tiles, kb, 148), -(-M // 64) * n_tiles
-                assert (s == 0) == (tiles > 296)
+                assert (s == 0) == (tiles > 296 or M > 512)
                 assert s == 0 or (1 <= s <= 8 and tiles * s <= 296 and (s == 1 or kb // s >= 4))
 
 
