@@ -12,6 +12,8 @@
 //   mlstm_step    one token a sequence: gates, recurrence with the state read once and written once, and the output's
 //                 norm and gate behind it, a block a (head, sequence).
 // Everything is 32-bit arithmetic; only the normed, gated output of mlstm_step is rounded.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -708,7 +710,11 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) sP[(ty + 16 * i) * QP + tx + 16 * j] *= acc[i][j];
+            for (int j = 0; j < 4; j++) {
+                // (picked, not multiplied by 0: what a later token brings, infinite or NaN, reaches no earlier one)
+                float& at = sP[(ty + 16 * i) * QP + tx + 16 * j];
+                at = tx + 16 * j <= ty + 16 * i ? at * acc[i][j] : 0.f;
+            }
     }
     __syncthreads();
     {                                  // n . q of a token by four neighbouring threads
@@ -727,7 +733,9 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int e = 0; e < 8; e++) in[i][e] = held[i][e] = 0.f;
-    auto product = [&](const float* left, int pitch, int n, const float* right, float (&acc)[4][8]) {
+    // CAUSAL: row i takes the right side's rows up to i, later ones not even with a factor of 0
+    auto product = [&](auto causal, const float* left, int pitch, int n, const float* right, float (&acc)[4][8]) {
+        constexpr bool CAUSAL = decltype(causal)::value;
 #pragma unroll 2
         for (int x = 0; x < n; x += 4) {
             float4 a[4];
@@ -740,6 +748,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
                 const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
+                    if (CAUSAL && x + z > ty + 16 * i) continue;
                     const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
 #pragma unroll
                     for (int e = 0; e < 8; e++) acc[i][e] = fmaf(f, v[e], acc[i][e]);
@@ -747,8 +756,8 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
             }
         }
     };
-    product(sP, QP, QC, sv, in);
-    product(sq, dp, d, sS, held);
+    product(std::true_type(), sP, QP, QC, sv, in);
+    product(std::false_type(), sq, dp, d, sS, held);
     __syncthreads();                   // the denominators are there
 #pragma unroll
     for (int i = 0; i < 4; i++) {

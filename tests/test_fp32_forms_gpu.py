@@ -202,3 +202,27 @@ def test_the_memory_over_chunks_and_four_at_a_time(core, H, d, dv, lens):
             assert float((held - z).abs().max()) < 3e-5 * float(z.abs().max()), (segments, i)
             assert float((state[i + 1, 4 + H * d * (dv + copies):4 + floats].double() - m).abs().max()) < 1e-5 * max(1.0, float(m.abs().max()))
             t0 += n
+
+
+@pytest.mark.parametrize("column", ["k", "v"])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+@pytest.mark.parametrize("d,dv,n,where", [(64, 128, 200, 64), (64, 128, 200, 130), (20, 36, 64, 63), (128, 130 * 2, 70, 5)])
+def test_what_a_token_brings_reaches_no_earlier_output_of_the_memory(core, column, bad, d, dv, n, where):
+    H = 2
+    g = torch.Generator(device=DEV).manual_seed(where)
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    proj = torch.randn(n, -(-(at["f"] + H) // 4) * 4, device=DEV, generator=g)
+    ib, fb = torch.randn(H, device=DEV, generator=g), torch.randn(H, device=DEV, generator=g) + 2
+    batch = G.make_batch(DEV, [1], [0], [n])
+
+    def run():
+        state = torch.zeros(2, -(-core.mlstm_state_floats(H, d, dv) // 4) * 4, device=DEV)
+        o = torch.full((n, H * dv), 7.0, device=DEV)
+        core.mlstm_scan(proj, at, ib, fb, 9.0, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv)
+        return o
+
+    plain = run()
+    proj[where, at[column]] = bad
+    got = run()
+    assert torch.equal(got[:where], plain[:where])
+    assert not bool(got[where].isfinite().all()) and bool(plain.isfinite().all())
