@@ -900,14 +900,15 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
             const int to = (tid & 127) >> 3, co = (tid & 7) * 2;
             float2 out = *reinterpret_cast<const float2*>(sX + (CC + to) * XP + co);
             const float* pr = du + CC * CC + to * CC;
-#pragma unroll
-            for (int j = 0; j < CC; j += 4) {
+            // (a warp's four tokens stand together: no group of four behind them, and inside it each ends at its own place,
+            // so that what a later token brings, infinite or NaN, reaches no earlier one)
+            for (int j = 0; j <= to; j += 4) {
                 const float4 p4 = *reinterpret_cast<const float4*>(pr + j);
                 const float pj[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const float2 u2 = *reinterpret_cast<const float2*>(sU + (j + e) * SP + co);
-                    out.x = fmaf(pj[e], u2.x, out.x), out.y = fmaf(pj[e], u2.y, out.y);
+                    if (j + e <= to) out.x = fmaf(pj[e], u2.x, out.x), out.y = fmaf(pj[e], u2.y, out.y);
                 }
             }
             float* dst = o + ((size_t)(tok0 + t0 + to) * p.H + h) * dv + c0 + co;

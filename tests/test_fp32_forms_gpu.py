@@ -226,3 +226,30 @@ def test_what_a_token_brings_reaches_no_earlier_output_of_the_memory(core, colum
     got = run()
     assert torch.equal(got[:where], plain[:where])
     assert not bool(got[where].isfinite().all()) and bool(plain.isfinite().all())
+
+
+@pytest.mark.parametrize("chunks", [False, True])
+@pytest.mark.parametrize("channel", [True, False])
+@pytest.mark.parametrize("column", ["k", "v"])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+@pytest.mark.parametrize("d,dv,n,where", [(128, 128, 50, 31), (128, 128, 50, 33), (12, 20, 15, 14)])
+def test_what_a_token_brings_reaches_no_earlier_output_of_the_delta_rule(core, chunks, channel, column, bad, d, dv, n, where):
+    H = 2
+    g = torch.Generator(device=DEV).manual_seed(where)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    unit = torch.nn.functional.normalize
+    qkv = torch.cat([x.reshape(n, -1) for x in (unit(r(n, H, d), dim=-1) * d ** -0.5, unit(r(n, H, d), dim=-1), r(n, H, dv))], 1).contiguous()
+    step = torch.cat([torch.sigmoid(r(n, H)), torch.zeros(n, H, device=DEV) if channel else -torch.rand(n, H, device=DEV, generator=g)], 1).contiguous()
+    decay = torch.rand(n, H * d, device=DEV, generator=g) if channel else None
+    batch, start = G.make_batch(DEV, [1], [0], [n]), r(2, H * d * dv)
+
+    def run():
+        o = torch.full((n, H * dv), 7.0, device=DEV)
+        core.delta_scan(qkv, step, start.clone(), batch, o, heads=H, kv_heads=H, d=d, dv=dv, decay=decay, chunks=chunks)
+        return o
+
+    plain = run()
+    qkv[where, H * d if column == "k" else 2 * H * d] = bad
+    got = run()
+    assert torch.equal(got[:where], plain[:where])
+    assert not bool(got[where].isfinite().all()) and bool(plain.isfinite().all())
