@@ -600,31 +600,38 @@ delta_scan_kernel(const DeltaSeq p, float* __restrict__ o) {
 // ---- several tokens a sequence: sixteen at a time ---------------------------------------------------------------
 // The same recurrence over chunks of sixteen tokens, in two launches.  What does not need the state is formed for all
 // chunks side by side (delta_chunk_kernel): with L_ij = beta_i (sum_c D_ij k_i k_j) for j < i, the u of a chunk solve
-// (I + L) u = beta (v - (G k) S), so with W = (I + L)^-1 beta (G k) and U = (I + L)^-1 beta v (forward substitution, a
-// column a thread)
-//     u = U - W S,    o = (G q) S + P u,    S <- G_16 S + (D_16 k)^T u,      P_ij = sum_c D_ij q_i k_j, j <= i
-// and the chain over the chunks (delta_chunk_scan_kernel) is three small products.  As above no factor is a quotient of
-// decays.  The chain of the form above is 0.29 us a token of a sequence (2,200 cycles for four tokens, four warps on an
-// SM, most of it the latency of shuffles, shared memory and the triangle inside a group); here it is 0.12 us, bound by the
-// reads of shared memory, and the first launch 0.03 us (16 heads of 128 x 128: 599 -> 298 us for 2,048 tokens).  Error
-// against 64 bits 1.3e-7 (1.1e-7 above).
+// (I + L) u = beta (v - (G k) S), so with W = (I + L)^-1 beta (G k), U = (I + L)^-1 beta v (forward substitution, a
+// column a thread) and P_ij = sum_c D_ij q_i k_j, j <= i,
+//     u = U - W S,    o = (G q) S + P u = Q S + P U with Q = G q - P W,    S <- G_16 S + (D_16 k)^T u
+// and the chain over the chunks (delta_chunk_scan_kernel) is two products with S and its update.  As above no factor is a
+// quotient of decays.  The first launch computes in 64 bits and rounds what it leaves: sixteen tokens' substitution and
+// the terms that cancel between G q and P u cost more than four tokens' do, and in 32 bits the outputs were 1.2 to 1.8 times as
+// far from the exact ones as those of the form above (correlated keys the most); so they are at 0.3 to 0.6 of its error (0.4 -
+// 1.2e-7 against 0.9 - 2.2e-7), for all that is left in 32 bits is the chain's own sums.  A token's places in W, U, Q and P U
+// hang on no later token.
+// The chain of the form above is 0.29 us a token of a sequence (2,200 cycles for four tokens, four warps on an
+// SM, most of it the latency of shuffles, shared memory and the triangle inside a group); here it is bound by the
+// reads of shared memory.  2,048 tokens of 16 heads of 128 x 128: 595 us (500 with one decay a head) there, 316 here; in 32 bits
+// throughout it was 295.
 constexpr int CC = 16, CS_COLS = 16, CS_THREADS = 256;
 struct DeltaWork {             // what the first launch leaves, a row a (token, value head)
-    float *w, *gq, *kd;        // [T, H, NP]; w and gq in the order chunk_place
-    float *u, *pairs;          // [T, H, dv], [T, H, 16]
+    float *w, *q, *kd;         // [T, H, NP]; w and q in the order chunk_place
+    float *u, *pu;             // [T, H, dv]
     float* all;                // [chunk, H, NP]: a chunk's decay of a channel
 };
-// where channel c lies in a row of w and gq: a thread's four channels c, c + 16, c + 32, c + 48 are one 16-byte unit
+// where channel c lies in a row of w and q: a thread's four channels c, c + 16, c + 32, c + 48 are one 16-byte unit
 __device__ __forceinline__ int chunk_place(int c) { return (c & ~63) + (c & 15) * 4 + ((c >> 4) & 3); }
 // number of the chunk that starts at token `tok` (counted in the step) of sequence s: different for all chunks of a step
 __device__ __forceinline__ int chunk_number(int tok, int s) { return tok / CC + s; }
+__device__ __forceinline__ double shfl_xor(double v, int lanes) { return __shfl_xor_sync(0xffffffffu, v, lanes); }
 
 template <int NP, bool CH>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(256, 2)
 delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     constexpr int PK = NP + 4;
     __shared__ __align__(16) float sk[CC][PK], sq[CC][PK], sg[CH ? CC : 1][PK];
-    __shared__ float s_l[CC][CC], s_beta[CC], s_lg[CC], s_eb[CC], s_er[CC];
+    __shared__ __align__(16) double s_l[CC][CC], s_p[CC][CC];      // L, P; both 0 where j is later
+    __shared__ double s_beta[CC], s_lg[CC], s_eb[CC], s_er[CC];
     __shared__ int s_seq;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, number = blockIdx.x, h = blockIdx.y;
     if (tid == 0) s_seq = -1;
@@ -653,11 +660,14 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
         s_lg[tid] = !CH && tid < cnt ? p.step[(size_t)(tok + tid) * 2 * p.H + p.H + h] : 0.f;
     }
     __syncthreads();
-    if (!CH && tid < CC) {             // every exponent is a sum of logarithms, never a difference
-        float b = 0.f, r = 0.f;
-        for (int e = 0; e <= tid; e++) b += s_lg[e];
-        for (int e = tid + 1; e < CC; e++) r += s_lg[e];
-        s_eb[tid] = expf(b), s_er[tid] = expf(r);
+    if (!CH && tid < 2 * CC) {         // every exponent is a sum of logarithms, never a difference
+        const int i = tid & (CC - 1);
+        double x = 0.;
+        if (tid < CC)
+            for (int e = 0; e <= i; e++) x += s_lg[e];
+        else
+            for (int e = i + 1; e < CC; e++) x += s_lg[e];
+        (tid < CC ? s_eb : s_er)[i] = exp(x);
     }
     // pair sums: a warp takes the pairs of tokens j = warp and 15 - warp with every later one; the thirty-two sums over the
     // warp cost 31 shuffles, and lane l ends with number l: [0 ... 15] k_i . k_j, [16 ... 31] q_i . k_j, i = l & 15
@@ -665,106 +675,118 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     for (int half = 0; half < 2; half++) {
         const int j = half ? CC - 1 - warp : warp;
         const int e = lane * 4;
-        float4 since = e < NP ? *reinterpret_cast<const float4*>(&sk[j][e]) : zero;        // k_j times the decays after j
-        float v32[32];
+        double since[4];               // k_j times the decays after j
+        {
+            const float4 kj = e < NP ? *reinterpret_cast<const float4*>(&sk[j][e]) : zero;
+            since[0] = kj.x, since[1] = kj.y, since[2] = kj.z, since[3] = kj.w;
+        }
+        double v32[32];
 #pragma unroll
         for (int i = 0; i < CC; i++) {
-            v32[i] = v32[CC + i] = 0.f;
+            v32[i] = v32[CC + i] = 0.;
             if (i >= j && e < NP) {
                 if (CH && i > j) {
                     const float4 gi = *reinterpret_cast<const float4*>(&sg[CH ? i : 0][e]);
-                    since.x *= gi.x, since.y *= gi.y, since.z *= gi.z, since.w *= gi.w;
+                    since[0] *= gi.x, since[1] *= gi.y, since[2] *= gi.z, since[3] *= gi.w;
                 }
                 const float4 ki = *reinterpret_cast<const float4*>(&sk[i][e]), qi = *reinterpret_cast<const float4*>(&sq[i][e]);
-                v32[i] = fmaf(ki.x, since.x, fmaf(ki.y, since.y, fmaf(ki.z, since.z, ki.w * since.w)));
-                v32[CC + i] = fmaf(qi.x, since.x, fmaf(qi.y, since.y, fmaf(qi.z, since.z, qi.w * since.w)));
+                v32[i] = fma((double)ki.x, since[0], fma((double)ki.y, since[1], fma((double)ki.z, since[2], ki.w * since[3])));
+                v32[CC + i] = fma((double)qi.x, since[0], fma((double)qi.y, since[1], fma((double)qi.z, since[2], qi.w * since[3])));
             }
         }
-        float v16[16], v8[8], v4[4], v2[2];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const bool up = (lane & 16) != 0;
-            v16[i] = (up ? v32[16 + i] : v32[i]) + __shfl_xor_sync(0xffffffffu, up ? v32[i] : v32[16 + i], 16);
-        }
+        for (int n = 16; n >= 1; n >>= 1) {
+            const bool up = (lane & n) != 0;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const bool up = (lane & 8) != 0;
-            v8[i] = (up ? v16[8 + i] : v16[i]) + __shfl_xor_sync(0xffffffffu, up ? v16[i] : v16[8 + i], 8);
+            for (int i = 0; i < 16; i++)
+                if (i < n) v32[i] = (up ? v32[n + i] : v32[i]) + shfl_xor(up ? v32[i] : v32[n + i], n);
         }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const bool up = (lane & 4) != 0;
-            v4[i] = (up ? v8[4 + i] : v8[i]) + __shfl_xor_sync(0xffffffffu, up ? v8[i] : v8[4 + i], 4);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const bool up = (lane & 2) != 0;
-            v2[i] = (up ? v4[2 + i] : v4[i]) + __shfl_xor_sync(0xffffffffu, up ? v4[i] : v4[2 + i], 2);
-        }
-        const bool up = (lane & 1) != 0;
-        float dot = (up ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, up ? v2[0] : v2[1], 1);
+        double dot = v32[0];
         const int i = lane & 15;
         if (!CH) {
-            float between = 0.f;       // the decays' logarithms after j up to i, added up and not subtracted
+            double between = 0.;       // the decays' logarithms after j up to i, added up and not subtracted
             for (int l = j + 1; l <= i; l++) between += s_lg[l];
-            dot *= expf(between);
+            dot *= exp(between);
         }
         if (lane < 16)
-            s_l[i][j] = i > j ? s_beta[i] * dot : 0.f;
-        else if (i < cnt)
-            wk.pairs[((size_t)(tok + i) * p.H + h) * CC + j] = i >= j ? dot : 0.f;
+            s_l[i][j] = i > j ? s_beta[i] * dot : 0.;
+        else
+            s_p[i][j] = i >= j ? dot : 0.;
     }
     __syncthreads();
-    float x[CC];
+    double x[CC];
     auto solve = [&]() {               // x <- (I + L)^-1 x
 #pragma unroll
         for (int i = 1; i < CC; i++) {
-            asm volatile("" ::: "memory");       // (or all of L is fetched first: 250 registers, one block an SM)
+            asm volatile("" ::: "memory");       // (or all of L is fetched first)
 #pragma unroll
-            for (int j = 0; j < i; j++) x[i] = fmaf(-s_l[i][j], x[j], x[i]);
+            for (int j = 0; j < i; j += 2) {
+                const double2 l2 = *reinterpret_cast<const double2*>(&s_l[i][j]);
+                x[i] = fma(-l2.x, x[j], x[i]);
+                if (j + 1 < i) x[i] = fma(-l2.y, x[j + 1], x[i]);
+            }
         }
+    };
+    auto pair_sum = [&](int i) {       // (P x)_i
+        double r = 0.;
+#pragma unroll
+        for (int j = 0; j < CC; j += 2)
+            if (j <= i) {
+                const double2 p2 = *reinterpret_cast<const double2*>(&s_p[i][j]);
+                r = fma(p2.x, x[j], r);
+                if (j + 1 <= i) r = fma(p2.y, x[j + 1], r);
+            }
+        return r;
     };
     if (tid < NP) {
         const int c = tid, at = chunk_place(c);
         const size_t row = ((size_t)tok * p.H + h) * NP, pitch = (size_t)p.H * NP;
-        float all = 1.f;
+        double all = 1.;
 #pragma unroll
         for (int i = 0; i < CC; i++) {
             if (CH) all *= sg[CH ? i : 0][c]; else all = s_eb[i];
             x[i] = s_beta[i] * (sk[i][c] * all);
-            if (i < cnt) wk.gq[row + i * pitch + at] = sq[i][c] * all;
         }
-        wk.all[((size_t)number * p.H + h) * NP + c] = all;
-        float since = 1.f;
+        wk.all[((size_t)number * p.H + h) * NP + c] = (float)all;
+        double since = 1.;
 #pragma unroll
         for (int i = CC - 1; i >= 0; i--) {
-            if (i < cnt) wk.kd[row + i * pitch + c] = sk[i][c] * (CH ? since : s_er[i]);
+            if (i < cnt) wk.kd[row + i * pitch + c] = (float)(sk[i][c] * (CH ? since : s_er[i]));
             if (CH) since *= sg[CH ? i : 0][c];
         }
         solve();
+        all = 1.;
 #pragma unroll
-        for (int i = 0; i < CC; i++)
-            if (i < cnt) wk.w[row + i * pitch + at] = x[i];
+        for (int i = 0; i < CC; i++) {
+            asm volatile("" ::: "memory");
+            if (CH) all *= sg[CH ? i : 0][c]; else all = s_eb[i];
+            const double q = sq[i][c] * all - pair_sum(i);
+            if (i < cnt) wk.w[row + i * pitch + at] = (float)x[i], wk.q[row + i * pitch + at] = (float)q;
+        }
     } else {
         for (int c = tid - NP; c < dv; c += 256 - NP) {
             const float* v = base + 2 * p.G * d + (size_t)h * dv + c;
 #pragma unroll
-            for (int i = 0; i < CC; i++) x[i] = i < cnt ? s_beta[i] * v[(size_t)i * channels] : 0.f;
+            for (int i = 0; i < CC; i++) x[i] = i < cnt ? s_beta[i] * v[(size_t)i * channels] : 0.;
             solve();
+            const size_t row = ((size_t)tok * p.H + h) * dv + c, pitch = (size_t)p.H * dv;
 #pragma unroll
-            for (int i = 0; i < CC; i++)
-                if (i < cnt) wk.u[((size_t)(tok + i) * p.H + h) * dv + c] = x[i];
+            for (int i = 0; i < CC; i++) {
+                asm volatile("" ::: "memory");
+                const double r = pair_sum(i);
+                if (i < cnt) wk.u[row + i * pitch] = (float)x[i], wk.pu[row + i * pitch] = (float)r;
+            }
         }
     }
 }
 
 // grid (ceil(dv / 16), heads, sequences): a block carries 16 columns of S in shared memory through its sequence's chunks.
-// A thread of the first product holds 8 of the 32 rows [W; G q] x 4 columns over every 16th channel (the sum over
-// the 16 threads that share them is 30 shuffles); then half of the threads update the state, 4 channels x 4 columns each,
-// and the other half form the outputs.
+// A thread of the first product holds 8 of the 32 rows [W; Q] x 4 columns over every 16th channel (the sum over
+// the 16 threads that share them is 30 shuffles); then a thread forms an output and an element of u, and half of the threads
+// update the state, 4 channels x 4 columns each.
 template <int NP>
 struct ChunkSmem {
-    static constexpr int STAGE = 3 * CC * NP + 2 * CC * CC + NP;      // W | G q | D k | U | P | decays
+    static constexpr int STAGE = 3 * CC * NP + 2 * CC * CS_COLS + NP;      // W | Q | D k | U | P U | decays
     static constexpr int SPITCH = CS_COLS + 4, XPITCH = CS_COLS + 2;
     static constexpr int FLOATS = 2 * STAGE + NP * SPITCH + 2 * CC * XPITCH + CC * SPITCH;
 };
@@ -775,7 +797,7 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
     constexpr int SP = L::SPITCH, XP = L::XPITCH;
     extern __shared__ __align__(16) float sm[];
     float* sS = sm + 2 * L::STAGE;     // [NP][SP]
-    float* sX = sS + NP * SP;          // [32][XP]: W S, then (G q) S
+    float* sX = sS + NP * SP;          // [32][XP]: W S, then Q S
     float* sU = sX + 2 * CC * XP;      // [16][SP]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int h = blockIdx.y, s = blockIdx.z, c0 = blockIdx.x * CS_COLS, d = p.d, dv = p.dv;
@@ -791,19 +813,18 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
         for (int e = tid; e < 3 * CC * (NP / 4); e += CS_THREADS) {
             const int which = e / (CC * (NP / 4)), i = e / (NP / 4) % CC, c = (e % (NP / 4)) * 4;
             const bool on = t0 + i < cnt;
-            const float* src = which == 0 ? wk.w : which == 1 ? wk.gq : wk.kd;
+            const float* src = which == 0 ? wk.w : which == 1 ? wk.q : wk.kd;
             cp_zfill(dst + which * CC * NP + i * NP + c, on ? src + (row0 + (size_t)i * p.H) * NP + c : src, 16, on);
         }
         float* du = dst + 3 * CC * NP;
         if (tid < 128) {
             const int i = (tid & 63) >> 2, c = (tid & 3) * 4, which = tid >> 6;
-            const bool on = t0 + i < cnt && (which || c < ncols);
-            const size_t row = row0 + (size_t)i * p.H;
-            const float* src = which ? wk.pairs + row * CC + c : wk.u + row * dv + c0 + c;
-            cp_zfill(du + which * CC * CC + i * CC + c, on ? src : wk.u, 16, on);
+            const bool on = t0 + i < cnt && c < ncols;
+            const float* src = which ? wk.pu : wk.u;
+            cp_zfill(du + which * CC * CS_COLS + i * CS_COLS + c, on ? src + (row0 + (size_t)i * p.H) * dv + c0 + c : src, 16, on);
         } else if (tid < 128 + NP / 4) {
             const int c = (tid - 128) * 4;
-            cp_zfill(du + 2 * CC * CC + c, wk.all + ((size_t)(number0 + t0 / CC) * p.H + h) * NP + c, 16, true);
+            cp_zfill(du + 2 * CC * CS_COLS + c, wk.all + ((size_t)(number0 + t0 / CC) * p.H + h) * NP + c, 16, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -864,23 +885,22 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
             *reinterpret_cast<float2*>(sX + (tg * 8 + (ks >> 1)) * XP + cg + (ks & 1) * 2) = make_float2(v2[0], v2[1]);
         }
         __syncthreads();
-        const int i = tid >> 4, c = tid & 15;
         const float* du = st + 3 * CC * NP;
-        const float mine = du[i * CC + c] - sX[i * XP + c];
-        sU[i * SP + c] = mine;
+        {
+            const int i = tid >> 4, c = tid & 15;
+            sU[i * SP + c] = du[i * CS_COLS + c] - sX[i * XP + c];
+            if (t0 + i < cnt && c < ncols)
+                o[((size_t)(tok0 + t0 + i) * p.H + h) * dv + c0 + c] = sX[(CC + i) * XP + c] + du[CC * CS_COLS + i * CS_COLS + c];
+        }
         __syncthreads();
         if (tid < CS_THREADS / 2) {
-            // the state: four neighbouring channels x four columns a thread
+            // the state: four neighbouring channels x four columns a thread; what the chunk adds is summed by itself, so that the
+            // state is rounded once a chunk
             for (int r0 = (tid >> 2) * 4; r0 < NP; r0 += CS_THREADS / 2) {
                 const int cc = (tid & 3) * 4;
                 float4 a[4];
-                const float4 al = *reinterpret_cast<const float4*>(du + 2 * CC * CC + r0);
-                const float all[4] = {al.x, al.y, al.z, al.w};
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    a[r] = *reinterpret_cast<const float4*>(sS + (r0 + r) * SP + cc);
-                    a[r].x *= all[r], a[r].y *= all[r], a[r].z *= all[r], a[r].w *= all[r];
-                }
+                for (int r = 0; r < 4; r++) a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
                 const float* kd = st + 2 * CC * NP + r0;
 #pragma unroll
                 for (int j = 0; j < CC; j++) {
@@ -892,29 +912,15 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
                         a[r].z = fmaf(k[r], u4.z, a[r].z), a[r].w = fmaf(k[r], u4.w, a[r].w);
                     }
                 }
+                const float4 al = *reinterpret_cast<const float4*>(du + 2 * CC * CS_COLS + r0);
+                const float all[4] = {al.x, al.y, al.z, al.w};
 #pragma unroll
-                for (int r = 0; r < 4; r++) *reinterpret_cast<float4*>(sS + (r0 + r) * SP + cc) = a[r];
-            }
-        } else {
-            // the outputs of two neighbouring columns of a token
-            const int to = (tid & 127) >> 3, co = (tid & 7) * 2;
-            float2 out = *reinterpret_cast<const float2*>(sX + (CC + to) * XP + co);
-            const float* pr = du + CC * CC + to * CC;
-            // (a warp's four tokens stand together: no group of four behind them, and inside it each ends at its own place,
-            // so that what a later token brings, infinite or NaN, reaches no earlier one)
-            for (int j = 0; j <= to; j += 4) {
-                const float4 p4 = *reinterpret_cast<const float4*>(pr + j);
-                const float pj[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const float2 u2 = *reinterpret_cast<const float2*>(sU + (j + e) * SP + co);
-                    if (j + e <= to) out.x = fmaf(pj[e], u2.x, out.x), out.y = fmaf(pj[e], u2.y, out.y);
+                for (int r = 0; r < 4; r++) {
+                    float4* at = reinterpret_cast<float4*>(sS + (r0 + r) * SP + cc);
+                    const float4 before = *at;
+                    *at = make_float4(fmaf(all[r], before.x, a[r].x), fmaf(all[r], before.y, a[r].y), fmaf(all[r], before.z, a[r].z),
+                                      fmaf(all[r], before.w, a[r].w));
                 }
-            }
-            float* dst = o + ((size_t)(tok0 + t0 + to) * p.H + h) * dv + c0 + co;
-            if (t0 + to < cnt) {
-                if (co < ncols) dst[0] = out.x;
-                if (co + 1 < ncols) dst[1] = out.y;
             }
         }
     }
@@ -930,7 +936,7 @@ bool aligned16(const void* p) { return (uintptr_t)p % 16 == 0; }
 // Floats of the first launch's results.
 long long chunk_floats(long long T, int num_seqs, int H, int d, int dv) {
     const long long NP = d <= 64 ? 64 : 128;
-    return T * H * (3 * NP + dv + CC) + (T / CC + num_seqs + 1) * H * NP;
+    return T * H * (3 * NP + 2 * dv) + (T / CC + num_seqs + 1) * H * NP;
 }
 
 }  // namespace
@@ -1034,8 +1040,8 @@ MOE_API int moe_delta_scan(const float* qkv, const float* step, float* state, lo
         const int NP = d <= 64 ? 64 : 128;
         DeltaWork wk;
         const size_t rows = (size_t)num_tokens * H;
-        wk.w = work, wk.gq = wk.w + rows * NP, wk.kd = wk.gq + rows * NP, wk.u = wk.kd + rows * NP, wk.pairs = wk.u + rows * dv;
-        wk.all = wk.pairs + rows * CC;
+        wk.w = work, wk.q = wk.w + rows * NP, wk.kd = wk.q + rows * NP, wk.u = wk.kd + rows * NP, wk.pu = wk.u + rows * dv;
+        wk.all = wk.pu + rows * dv;
         const dim3 first(num_tokens / CC + num_seqs + 1, H), chain((dv + CS_COLS - 1) / CS_COLS, H, num_seqs);
 #define CHUNK(NP_, C_)                                                                                                  \
     do {                                                                                                               \

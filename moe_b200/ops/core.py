@@ -1582,7 +1582,7 @@ def delta_step(qkv, step, state, gate, norm_w, norm_eps, batch, out, *, heads, k
 
 def _delta_chunks(T, num_seqs, heads, dv) -> bool:
     """Whether the scan goes over chunks: where its blocks (16 columns of a head and sequence) find an SM each.  The chain
-    of a chunk is then short (16 heads of 128 x 128, one sequence of 2,048 tokens: 599 -> 298 us); with more blocks the
+    of a chunk is then short (16 heads of 128 x 128, one sequence of 2,048 tokens: 595 -> 316 us); with more blocks the
     multiply-adds count, of which a chunk has more (four sequences: 916 against 1,067 us)."""
     return -(-dv // 16) * heads * num_seqs <= lib().moe_scan_sms()
 

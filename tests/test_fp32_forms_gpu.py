@@ -253,3 +253,32 @@ def test_what_a_token_brings_reaches_no_earlier_output_of_the_delta_rule(core, c
     got = run()
     assert torch.equal(got[:where], plain[:where])
     assert not bool(got[where].isfinite().all()) and bool(plain.isfinite().all())
+
+
+@pytest.mark.parametrize("channel", [True, False])
+@pytest.mark.parametrize("alike", [0.0, 1.0, 3.0])          # how much the keys resemble one another
+@pytest.mark.parametrize("forget", [2.0, 5.0])              # decays around sigmoid(this)
+def test_the_delta_rule_over_chunks_is_no_further_off_than_four_at_a_time(core, channel, alike, forget):
+    H, d, dv, n = 4, 128, 64, 400
+    g = torch.Generator(device=DEV).manual_seed(5)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    unit, soft = torch.nn.functional.normalize, torch.nn.functional.softplus
+    common = alike * r(1, H, d)
+    q, k, v = unit(r(n, H, d) + common, dim=-1) * d ** -0.5, unit(r(n, H, d) + common, dim=-1), r(n, H, dv)
+    beta, lg = torch.sigmoid(2 * r(n, H) + 2 * (alike > 0)), -soft(r(n, H) - forget)
+    decay = torch.exp(-soft(r(n, H * d) - forget)) if channel else None
+    qkv = torch.cat([x.reshape(n, -1) for x in (q, k, v)], 1).contiguous()
+    step = torch.cat([beta, torch.zeros_like(lg) if channel else lg], 1).contiguous()
+    batch, start = G.make_batch(DEV, [1], [0], [n]), 0.1 * r(2, H * d * dv)
+    S, ref = start[1].double().view(H, d, dv), []
+    for t in range(n):
+        S = S * (decay[t].double().view(H, d, 1) if channel else torch.exp(lg[t].double())[:, None, None])
+        u = beta[t].double()[:, None] * (v[t].double() - torch.einsum("hdv,hd->hv", S, k[t].double()))
+        S = S + k[t].double()[:, :, None] * u[:, None]
+        ref.append(torch.einsum("hdv,hd->hv", S, q[t].double()))
+    ref, off = torch.stack(ref).view(n, -1), {}
+    for chunks in (False, True):
+        state, o = start.clone(), torch.empty(n, H * dv, device=DEV)
+        core.delta_scan(qkv, step, state, batch, o, heads=H, kv_heads=H, d=d, dv=dv, decay=decay, chunks=chunks)
+        off[chunks] = [float((a.double() - b).norm() / b.norm()) for a, b in ((o, ref), (state[1], S.flatten()))]
+    assert off[True][0] <= off[False][0] and off[True][1] <= off[False][1], off
