@@ -488,7 +488,7 @@ mlstm_scan_kernel(const MemSeq p, float* __restrict__ o, const MemSegments sg) {
 // outputs from the state before it (mlstm_chunk_out_kernel) are products of 64 tokens, formed for all chunks side by side; only
 // the state's way through the chunks is a chain, one multiply-add an element and chunk (mlstm_chunk_state_kernel, which puts
 // the state before a chunk in the place of what the chunk adds).  The scan above is bound by its
-// shuffles and reads of shared memory (2,048 tokens, 16 heads of 64 x 128, in eight segments: 108 + 184 us; here 39 + 34 + 92 us).
+// shuffles and reads of shared memory (2,048 tokens, 16 heads of 64 x 128, gates included: 243 us in four segments, 139 here).
 // Factors are products of a.
 constexpr int QC = 64, QV = 128;       // tokens a chunk; columns of S a block
 struct MemChunks {
@@ -628,7 +628,10 @@ mlstm_chunk_state_kernel(const MemSeq p, const MemChunks c) {
     }
 }
 
-// grid (chunks, heads, ceil(dv / 128)): the pair products of a chunk, 4 x 4 a thread; the outputs, 4 rows x 8 columns a thread
+// grid (chunks, heads, ceil(dv / 128)): the pair products of a chunk, 4 x 4 a thread; the outputs, 4 rows x 8 columns a thread.
+// The pair products and n . q are sums in 64 bits: an output is divided by n . q, which cancels, and whatever is lost in it
+// counts as often as that is small beside its terms.  An output's own error (the median over tokens) is 0.7 - 0.8 of the
+// form's of four tokens; with 32-bit sums throughout, 118 us instead of 139, it was 1.2 - 1.3 times that.
 constexpr int QP = QC + 4;
 __host__ __device__ constexpr size_t mlstm_chunk_out_floats(int d) {
     return (size_t)2 * QC * (d + 4) + QC * QP + QC * (QV + 4) + (size_t)d * (QV + 4) + d;
@@ -636,7 +639,8 @@ __host__ __device__ constexpr size_t mlstm_chunk_out_floats(int d) {
 __global__ void __launch_bounds__(256)
 mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* __restrict__ o) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ float s_a[QC], s_b[QC], s_all[QC], s_den[QC];
+    __shared__ float s_a[QC], s_b[QC], s_den[QC];
+    __shared__ double s_all[QC], s_in[QC];
     __shared__ int s_seq;
     const int tid = threadIdx.x, number = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
     float* sq = sm;                    // [64][d + 4]
@@ -675,85 +679,107 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     }
     for (int x = tid; x < d; x += 256) sn[x] = c.norm[at + x];
     __syncthreads();
-    if (tid < QC) {                    // column j of the pair factors: b_j times the a after j, 0 above the diagonal
-        float run = s_b[tid];
-        for (int i = 0; i < QC; i++) {
+    if (tid < QC) {                    // column j of the pair factors: b_j times the a after j
+        double run = s_b[tid];
+        for (int i = tid; i < QC; i++) {
             if (i > tid) run *= s_a[i];
-            sP[i * QP + tid] = i >= tid ? run : 0.f;
+            sP[i * QP + tid] = (float)run;
         }
     } else if (tid < 2 * QC) {         // from the chunk's first token to its i-th
-        float run = 1.f;
+        double run = 1.;
         for (int i = 0; i <= tid - QC; i++) run *= s_a[i];
         s_all[tid - QC] = run;
     }
     __syncthreads();
     const int ty = tid >> 4, tx = tid & 15;
     {
-        float acc[4][4];
+        double acc[4][4];              // of rows ty + 16 i, columns tx + 16 j; j > i lies above the diagonal
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-#pragma unroll 2
+            for (int j = 0; j < 4; j++) acc[i][j] = 0.;
+#pragma unroll 1
         for (int x = 0; x < d; x += 4) {
-            float4 a[4];
+            double a[4][4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(sq + (ty + 16 * i) * dp + x);
+            for (int i = 0; i < 4; i++) {
+                const float4 v = *reinterpret_cast<const float4*>(sq + (ty + 16 * i) * dp + x);
+                a[i][0] = v.x, a[i][1] = v.y, a[i][2] = v.z, a[i][3] = v.w;
+            }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float4 b = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * dp + x);
+                const float4 v = *reinterpret_cast<const float4*>(sk + (tx + 16 * j) * dp + x);
+                const double b[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-                    acc[i][j] = fmaf(a[i].x, b.x, fmaf(a[i].y, b.y, fmaf(a[i].z, b.z, fmaf(a[i].w, b.w, acc[i][j]))));
+                for (int i = j; i < 4; i++)
+#pragma unroll
+                    for (int z = 0; z < 4; z++) acc[i][j] = fma(a[i][z], b[z], acc[i][j]);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < 4; i++) {
+            double sum = 0.;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 // (picked, not multiplied by 0: what a later token brings, infinite or NaN, reaches no earlier one)
                 float& at = sP[(ty + 16 * i) * QP + tx + 16 * j];
-                at = tx + 16 * j <= ty + 16 * i ? at * acc[i][j] : 0.f;
+                const double pair = j <= i && tx + 16 * j <= ty + 16 * i ? at * acc[i][j] : 0.;
+                at = (float)pair, sum += pair;
             }
+#pragma unroll
+            for (int off = 8; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+            if (tx == 0) s_in[ty + 16 * i] = sum;
+        }
     }
     __syncthreads();
     {                                  // n . q of a token by four neighbouring threads
         const int i = tid >> 2, part = tid & 3;
-        float in = 0.f, held = 0.f;
-        for (int j = part; j < QC; j += 4) in += sP[i * QP + j];
-        for (int x = part; x < d; x += 4) held = fmaf(sq[i * dp + x], sn[x], held);
-        float n = fmaf(s_all[i], held, in);
-        n += __shfl_xor_sync(0xffffffffu, n, 1);
-        n += __shfl_xor_sync(0xffffffffu, n, 2);
+        double held = 0.;
+        for (int x = part; x < d; x += 4) held = fma((double)sq[i * dp + x], (double)sn[x], held);
+        held += __shfl_xor_sync(0xffffffffu, held, 1);
+        held += __shfl_xor_sync(0xffffffffu, held, 2);
         __syncwarp();
-        if (part == 0) s_den[i] = fmaxf(fabsf(n), s_den[i]) + READ_EPS;
+        if (part == 0) s_den[i] = fmaxf(fabsf((float)fma(s_all[i], held, s_in[i])), s_den[i]) + READ_EPS;
     }
     float in[4][8], held[4][8];
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
         for (int e = 0; e < 8; e++) in[i][e] = held[i][e] = 0.f;
+    // Sixteen terms at a time, then their sums (one accumulator over 64 or 128 terms would be about twice as far off).
     // CAUSAL: row i takes the right side's rows up to i, later ones not even with a factor of 0
     auto product = [&](auto causal, const float* left, int pitch, int n, const float* right, float (&acc)[4][8]) {
         constexpr bool CAUSAL = decltype(causal)::value;
+#pragma unroll 1
+        for (int x0 = 0; x0 < n; x0 += 16) {
+            float part[4][8];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int e = 0; e < 8; e++) part[i][e] = 0.f;
 #pragma unroll 2
-        for (int x = 0; x < n; x += 4) {
-            float4 a[4];
+            for (int x = x0; x < min(n, x0 + 16); x += 4) {
+                float4 a[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(left + (ty + 16 * i) * pitch + x);
+                for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4*>(left + (ty + 16 * i) * pitch + x);
 #pragma unroll
-            for (int z = 0; z < 4; z++) {
-                const float* row = right + (x + z) * (QV + 4) + tx * 4;
-                const float4 va = *reinterpret_cast<const float4*>(row), vb = *reinterpret_cast<const float4*>(row + 64);
-                const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+                for (int z = 0; z < 4; z++) {
+                    const float* row = right + (x + z) * (QV + 4) + tx * 4;
+                    const float4 va = *reinterpret_cast<const float4*>(row), vb = *reinterpret_cast<const float4*>(row + 64);
+                    const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    if (CAUSAL && x + z > ty + 16 * i) continue;
-                    const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
+                    for (int i = 0; i < 4; i++) {
+                        if (CAUSAL && x + z > ty + 16 * i) continue;
+                        const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
 #pragma unroll
-                    for (int e = 0; e < 8; e++) acc[i][e] = fmaf(f, v[e], acc[i][e]);
+                        for (int e = 0; e < 8; e++) part[i][e] = fmaf(f, v[e], part[i][e]);
+                    }
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int e = 0; e < 8; e++) acc[i][e] += part[i][e];
         }
     };
     product(std::true_type(), sP, QP, QC, sv, in);
@@ -763,7 +789,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     for (int i = 0; i < 4; i++) {
         const int t = ty + 16 * i;
         if (t >= cnt) continue;
-        const float all = s_all[t], den = s_den[t];
+        const float all = (float)s_all[t], den = s_den[t];
         float* dst = o + ((size_t)(tok + t) * p.H + h) * dv + c0;
 #pragma unroll
         for (int e = 0; e < 2; e++) {

@@ -282,3 +282,38 @@ def test_the_delta_rule_over_chunks_is_no_further_off_than_four_at_a_time(core, 
         core.delta_scan(qkv, step, state, batch, o, heads=H, kv_heads=H, d=d, dv=dv, decay=decay, chunks=chunks)
         off[chunks] = [float((a.double() - b).norm() / b.norm()) for a, b in ((o, ref), (state[1], S.flatten()))]
     assert off[True][0] <= off[False][0] and off[True][1] <= off[False][1], off
+
+
+@pytest.mark.parametrize("forget", [0.0, 2.5, 6.0])         # the forget gate's bias
+@pytest.mark.parametrize("n", [40, 300])
+def test_the_memory_over_chunks_is_no_further_off_than_four_at_a_time(core, forget, n):
+    H, d, dv, cap = 16, 64, 128, 15.0
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    off = {None: [], 1: []}
+    for seed in range(4):
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        proj = torch.randn(n, at["f"] + H, device=DEV, generator=g)
+        ib, fb = (torch.randn(H, device=DEV, generator=g) + b for b in (-0.5, forget))
+        batch, x = G.make_batch(DEV, [1], [0], [n]), proj.double()
+        q, k = (x[:, at[c]:at[c] + H * d].view(n, H, d) for c in "qk")
+        v = x[:, at["v"]:at["v"] + H * dv].view(n, H, dv)
+        li = cap * torch.tanh((x[:, at["i"]:at["i"] + H] + ib.double()) / cap)
+        lf = torch.nn.functional.logsigmoid(cap * torch.tanh((x[:, at["f"]:at["f"] + H] + fb.double()) / cap))
+        S, z, m, ref = torch.zeros(H, d, dv, device=DEV, dtype=torch.float64), 0.0, torch.zeros(H, device=DEV, dtype=torch.float64), []
+        for t in range(n):
+            new = torch.maximum(lf[t] + m, li[t])
+            a, b = torch.exp(lf[t] + m - new)[:, None], torch.exp(li[t] - new)[:, None]
+            m, S, z = new, a[:, None] * S + b[:, None] * k[t][:, :, None] * v[t][:, None], a * z + b * k[t]
+            den = torch.maximum((z * q[t]).sum(-1).abs() * d ** -0.5, torch.exp(-m)) + 1e-6
+            ref.append((torch.einsum("hdv,hd->hv", S, q[t]) * d ** -0.5 / den[:, None]).flatten())
+        ref = torch.stack(ref)
+        for segments in off:
+            state, o = torch.zeros(2, core.mlstm_state_floats(H, d, dv), device=DEV), torch.empty(n, H * dv, device=DEV)
+            core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, segments=segments)
+            # (a token's own relative error: where n . q cancels an output is far off in any form, and such outputs, few,
+            # would decide a norm over all)
+            e, r = (o.double() - ref).view(n, H, dv).norm(dim=2), ref.view(n, H, dv).norm(dim=2)
+            off[segments].append(e / r)
+    four, chunks = (float(torch.cat(off[s]).median()) for s in (1, None))
+    # the medians of 4 x 16 x n errors are known to about 1 / sqrt(2,560) of themselves; both share what the gates' rounding brings
+    assert chunks <= 1.02 * four, (chunks, four)
