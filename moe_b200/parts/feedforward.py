@@ -343,9 +343,10 @@ class RoutedExperts(Part):
             from ..ops import tc
 
             logits = rt.empty((T, self.w_router3.shape[0]), torch.float32)
-            # (one tile of features: the K splits fill the SMs; at 2,048 / 4,096 / 8,192 tokens eight take 11.0 / 21.4 / 43.6 us,
-            # four 13.9 / 14.9 / 33.0)
-            if tc.gemm_tc(core.split3(h.f32), self.w_router3, logits, bn=64, splits=8 if T <= 2048 else 4, status=rt.status):
+            # (one tile of features: the K splits fill the SMs, and eight of them for any number of tokens: with four the logits of
+            # more than 4,096 tokens took 33 instead of 44 us, but were twice as far off, 1.5e-6 instead of 7.3e-7, and a token's
+            # picks would have hung on how many others came along)
+            if tc.gemm_tc(core.split3(h.f32), self.w_router3, logits, bn=64, splits=8, status=rt.status):
                 if after_logits is not None:
                     after_logits()
                 core.router_topk(logits, self.k, self.norm_topk, self.scale, topk_idx, topk_w, num_experts=self.E,

@@ -92,3 +92,21 @@ def test_pairs_of_groups(tc, counts, swiglu):
         assert bool(((out[at:at + n].double() - r).abs() <= off + 2.0 ** -23 * r.abs()).all()), e
         at += n
     assert int(st[0]) == 0
+
+
+def test_a_token_is_routed_alike_in_a_short_and_in_a_long_prompt():
+    """The router's logits, from which picks and weights are formed, are the same to the bit for any number of tokens that the
+    tensor-core form takes."""
+    import moe_b200
+    from moe_b200.parts.base import Activations
+
+    H = 2048
+    cfg = dict(architectures=["Qwen2MoeForCausalLM"], model_type="qwen2_moe", num_hidden_layers=1, hidden_size=H, num_attention_heads=1,
+               num_key_value_heads=1, head_dim=128, num_experts=60, num_experts_per_tok=4, moe_intermediate_size=16,
+               shared_expert_intermediate_size=16, norm_topk_prob=False, decoder_sparse_step=1, intermediate_size=16, vocab_size=64)
+    model = moe_b200.random_model(cfg, seed=0, dtype="bfloat16", device=DEV)
+    part = model.blocks[0].ffn
+    x = torch.randn(4500, H, device=DEV)
+    short, *longer = [part.route(model.rt, Activations(act=x[:T].bfloat16(), f32=x[:T].contiguous()), None) for T in (300, 2048, 2100, 4500)]
+    for got in longer:
+        assert all(torch.equal(a, b[:300]) for a, b in zip(short, got))
