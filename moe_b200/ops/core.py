@@ -1452,11 +1452,15 @@ def table_route(table, batch, top_k, num_experts, topk_idx, topk_w, status):
                               _p(topk_idx), _p(topk_w), _p(status), _stream()), "table_route")
 
 
+def _forced_segments() -> int:
+    return int(os.environ.get("MOE_B200_SCAN_SEGMENTS", "0"))
+
+
 def scan_segments(batch, blocks_per_sequence: int, device) -> int:
     """Into how many segments a sequence's tokens are cut for ``ssd_scan``, ``wkv_scan`` and ``mlstm_scan``: one where the launch fills
     the GPU anyway or the sequences are short; else enough to fill it, of at least 128 tokens each, eight
     at most.  (``MOE_B200_SCAN_SEGMENTS``: 0 this rule, n > 0 that many.)"""
-    forced = int(os.environ.get("MOE_B200_SCAN_SEGMENTS", "0"))
+    forced = _forced_segments()
     longest = int(getattr(batch, "max_new", 0) or 0)
     if forced > 0:
         return max(1, min(forced, 64))
@@ -1628,7 +1632,7 @@ def mlstm_scan(proj, at, i_bias, f_bias, cap, q_scale, state, batch, o, *, heads
     of q, k, v and of the gates' logits i and f start at ``at``; queries are multiplied by ``q_scale``; ``state`` rows hold
     ``mlstm_state_floats`` floats from ``offset``; o: float32 [T, heads * dv].  ``segments``: into how many pieces that run
     side by side every sequence's tokens are cut, four tokens at a time (None: chunks of sixty-four tokens where the sizes
-    allow it, else ``scan_segments`` decides)."""
+    allow it and ``MOE_B200_SCAN_SEGMENTS`` gives no number, else ``scan_segments`` decides)."""
     _chk(o, "o", torch.float32, 2)
     T = proj.shape[0]
     if tuple(o.shape) != (T, heads * dv):
@@ -1636,7 +1640,7 @@ def mlstm_scan(proj, at, i_bias, f_bias, cap, q_scale, state, batch, o, *, heads
     args = _mlstm_args(proj, at, i_bias, f_bias, cap, q_scale, state, offset, batch, heads, d, dv)
     steps = torch.empty((T, 3 * heads), dtype=torch.float32, device=o.device)
     longest = int(getattr(batch, "max_new", 0) or 0)
-    need = lib().moe_mlstm_chunk_floats(T, batch.num_seqs, heads, d, dv) if segments is None else 0
+    need = lib().moe_mlstm_chunk_floats(T, batch.num_seqs, heads, d, dv) if segments is None and _forced_segments() <= 0 else 0
     if need:
         # chunks of sixty-four tokens side by side (one sequence of 2,048 tokens, 16 heads of 64 x 128: 243 -> 139 us)
         work = torch.empty((need,), dtype=torch.float32, device=o.device)

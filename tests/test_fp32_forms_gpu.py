@@ -317,3 +317,20 @@ def test_the_memory_over_chunks_is_no_further_off_than_four_at_a_time(core, forg
     four, chunks = (float(torch.cat(off[s]).median()) for s in (1, None))
     # the medians of 4 x 16 x n errors are known to about 1 / sqrt(2,560) of themselves; both share what the gates' rounding brings
     assert chunks <= 1.02 * four, (chunks, four)
+
+
+def test_segments_asked_for_by_the_environment_reach_the_memory(core, monkeypatch):
+    H, d, dv, n = 2, 64, 128, 600
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    g = torch.Generator(device=DEV).manual_seed(1)
+    proj, ib, fb = torch.randn(n, at["f"] + H, device=DEV, generator=g), torch.zeros(H, device=DEV), torch.ones(H, device=DEV)
+    batch = G.make_batch(DEV, [1], [0], [n])
+
+    def run(segments):
+        state, o = torch.zeros(2, -(-core.mlstm_state_floats(H, d, dv) // 4) * 4, device=DEV), torch.empty(n, H * dv, device=DEV)
+        core.mlstm_scan(proj, at, ib, fb, 9.0, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, segments=segments)
+        return o
+
+    for n_seg in (1, 3):
+        monkeypatch.setenv("MOE_B200_SCAN_SEGMENTS", str(n_seg))
+        assert torch.equal(run(None), run(n_seg))
