@@ -1627,12 +1627,22 @@ def _mlstm_args(proj, at, i_bias, f_bias, cap, q_scale, state, offset, batch, he
             float(q_scale), st, state.stride(0))
 
 
-def mlstm_scan(proj, at, i_bias, f_bias, cap, q_scale, state, batch, o, *, heads, d, dv, offset=0, segments=None):
+def _memory_chunks(T, num_seqs, heads, dv) -> bool:
+    """Whether the memory goes over chunks: with 256 tokens a sequence or more on average, where the blocks of the form of four
+    (32 columns of a head and sequence) leave SMs idle.  Four launches and a chunk's states through memory are what a step of few
+    tokens need not pay, and full SMs gain nothing.  Measured, us, chunks / four at a time: one sequence of 64, 128, 256, 2,048 tokens,
+    16 heads of 64 x 128: 38 / 20, 38 / 33, 39 / 60, 139 / 243; 4 heads of 128 x 256: 54 / 20, 54 / 35, 55 / 63, 109 / 175; eight
+    sequences (512 blocks) of 256 and 2,048: 130 / 107, 1,020 / 813; 32 of 64: 153 / 102."""
+    return T >= 256 * num_seqs and -(-dv // 32) * heads * num_seqs <= lib().moe_scan_sms()
+
+
+def mlstm_scan(proj, at, i_bias, f_bias, cap, q_scale, state, batch, o, *, heads, d, dv, offset=0, segments=None, chunks=None):
     """Several tokens a sequence of the exponentially gated memory (csrc/mlstm.cu) on 32-bit projection rows whose columns
     of q, k, v and of the gates' logits i and f start at ``at``; queries are multiplied by ``q_scale``; ``state`` rows hold
     ``mlstm_state_floats`` floats from ``offset``; o: float32 [T, heads * dv].  ``segments``: into how many pieces that run
-    side by side every sequence's tokens are cut, four tokens at a time (None: chunks of sixty-four tokens where the sizes
-    allow it and ``MOE_B200_SCAN_SEGMENTS`` gives no number, else ``scan_segments`` decides)."""
+    side by side every sequence's tokens are cut, four tokens at a time (None: ``scan_segments`` decides).  ``chunks``: over chunks
+    of sixty-four tokens side by side, where the kernels take the sizes; None: by the rule of ``_memory_chunks``, unless ``segments``
+    or ``MOE_B200_SCAN_SEGMENTS`` give a number."""
     _chk(o, "o", torch.float32, 2)
     T = proj.shape[0]
     if tuple(o.shape) != (T, heads * dv):
@@ -1640,9 +1650,10 @@ def mlstm_scan(proj, at, i_bias, f_bias, cap, q_scale, state, batch, o, *, heads
     args = _mlstm_args(proj, at, i_bias, f_bias, cap, q_scale, state, offset, batch, heads, d, dv)
     steps = torch.empty((T, 3 * heads), dtype=torch.float32, device=o.device)
     longest = int(getattr(batch, "max_new", 0) or 0)
-    need = lib().moe_mlstm_chunk_floats(T, batch.num_seqs, heads, d, dv) if segments is None and _forced_segments() <= 0 else 0
+    if chunks is None:
+        chunks = segments is None and _forced_segments() <= 0 and _memory_chunks(T, batch.num_seqs, heads, dv)
+    need = lib().moe_mlstm_chunk_floats(T, batch.num_seqs, heads, d, dv) if chunks else 0
     if need:
-        # chunks of sixty-four tokens side by side (one sequence of 2,048 tokens, 16 heads of 64 x 128: 243 -> 139 us)
         work = torch.empty((need,), dtype=torch.float32, device=o.device)
         code = lib().moe_mlstm_chunks(*args, _p(batch.cu_seqlens), _p(batch.slots), T, batch.num_seqs, heads, d, dv, _p(steps),
                                       _p(o), longest, _p(work), _stream())

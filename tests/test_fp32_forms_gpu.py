@@ -178,7 +178,8 @@ def test_the_memory_over_chunks_and_four_at_a_time(core, H, d, dv, lens):
     batch = G.make_batch(DEV, list(range(1, B + 1)), [0] * B, lens)
     for segments in (None, 1):
         state, o = start.clone(), torch.full((T, H * dv), float("nan"), device=DEV)
-        core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, offset=4, segments=segments)
+        core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, offset=4, segments=segments,
+                        chunks=segments is None)
         assert torch.equal(state[0], start[0]) and torch.equal(state[B + 1], start[B + 1]) and torch.equal(state[:, :4], start[:, :4])
         t0 = 0
         for i, n in enumerate(lens):
@@ -218,7 +219,7 @@ def test_what_a_token_brings_reaches_no_earlier_output_of_the_memory(core, colum
     def run():
         state = torch.zeros(2, -(-core.mlstm_state_floats(H, d, dv) // 4) * 4, device=DEV)
         o = torch.full((n, H * dv), 7.0, device=DEV)
-        core.mlstm_scan(proj, at, ib, fb, 9.0, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv)
+        core.mlstm_scan(proj, at, ib, fb, 9.0, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, chunks=True)
         return o
 
     plain = run()
@@ -309,7 +310,8 @@ def test_the_memory_over_chunks_is_no_further_off_than_four_at_a_time(core, forg
         ref = torch.stack(ref)
         for segments in off:
             state, o = torch.zeros(2, core.mlstm_state_floats(H, d, dv), device=DEV), torch.empty(n, H * dv, device=DEV)
-            core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, segments=segments)
+            core.mlstm_scan(proj, at, ib, fb, cap, d ** -0.5, state, batch, o, heads=H, d=d, dv=dv, segments=segments,
+                            chunks=segments is None)
             # (a token's own relative error: where n . q cancels an output is far off in any form, and such outputs, few,
             # would decide a norm over all)
             e, r = (o.double() - ref).view(n, H, dv).norm(dim=2), ref.view(n, H, dv).norm(dim=2)
@@ -334,3 +336,17 @@ def test_segments_asked_for_by_the_environment_reach_the_memory(core, monkeypatc
     for n_seg in (1, 3):
         monkeypatch.setenv("MOE_B200_SCAN_SEGMENTS", str(n_seg))
         assert torch.equal(run(None), run(n_seg))
+
+
+def test_short_steps_and_many_sequences_keep_the_form_of_four(core, monkeypatch):
+    """A step of few tokens a sequence, or one whose blocks fill the SMs anyway, launches what it did before there were chunks."""
+    H, d, dv = 16, 64, 128
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    taken, L = [], core.lib()
+    monkeypatch.setattr(core, "lib", lambda: type("Spy", (), {"__getattr__": lambda _, name: (taken.append(name), getattr(L, name))[1]})())
+    for B, n, over_chunks in ((1, 2, False), (64, 2, False), (1, 128, False), (8, 300, False), (1, 256, True), (2, 300, True)):
+        proj, z = torch.randn(B * n, at["f"] + H, device=DEV), torch.zeros(H, device=DEV)
+        state, o = torch.zeros(B + 1, core.mlstm_state_floats(H, d, dv), device=DEV), torch.empty(B * n, H * dv, device=DEV)
+        taken.clear()
+        core.mlstm_scan(proj, at, z, z, 9.0, d ** -0.5, state, G.make_batch(DEV, list(range(1, B + 1)), [0] * B, [n] * B), o, heads=H, d=d, dv=dv)
+        assert ("moe_mlstm_chunks" in taken) == over_chunks, (B, n)
