@@ -360,11 +360,12 @@ class RoutedExperts(Part):
             after_logits()
         return topk_idx, topk_w, sg
 
-    def _shared(self, rt, h):
+    def _shared(self, rt, h, beside=True):
+        # ``beside``: on a side stream, beside the routed products; else it runs alone.
         # (up to 256 rows the down product keeps to few SMs: it runs beside the routed products, which want the others; cut into
         # pieces for all of them a step of three prompts, 145 tokens, took 1,867 instead of 1,795 us.  At 512 rows it is the
         # longer of the two branches: 2,353 against 2,211 us a step.)
-        return linear(rt, swiglu_linear(rt, h.act, self.ws_gu), self.ws_down, beside=h.act.shape[0] <= 256)
+        return linear(rt, swiglu_linear(rt, h.act, self.ws_gu), self.ws_down, beside=beside and h.act.shape[0] <= 256)
 
     def forward(self, rt, h, batch):
         return self._run(rt, h, batch, None).materialize(rt)
@@ -461,7 +462,7 @@ class RoutedExperts(Part):
         # (the offsets were written before the product above: the second product may start on its weights early)
         y = grouped_linear(rt, act, self.w_down, offsets, P, early_offsets=True)
         if self.ws_gu is not None and side is None:
-            ys = self._shared(rt, h)
+            ys = self._shared(rt, h, beside=False)
         if side is not None:
             torch.cuda.current_stream().wait_stream(side)
             ys.record_stream(torch.cuda.current_stream())

@@ -110,3 +110,29 @@ def test_a_token_is_routed_alike_in_a_short_and_in_a_long_prompt():
     short, *longer = [part.route(model.rt, Activations(act=x[:T].bfloat16(), f32=x[:T].contiguous()), None) for T in (300, 2048, 2100, 4500)]
     for got in longer:
         assert all(torch.equal(a, b[:300]) for a, b in zip(short, got))
+
+
+@pytest.mark.parametrize("on_a_side_stream", [True, False])
+def test_the_shared_experts_product_keeps_to_few_sms_only_beside_others(on_a_side_stream, monkeypatch):
+    import moe_b200
+    from moe_b200.ops import tc
+
+    cfg = dict(architectures=["Qwen2MoeForCausalLM"], model_type="qwen2_moe", num_hidden_layers=1, hidden_size=128, num_attention_heads=1,
+               num_key_value_heads=1, head_dim=128, num_experts=4, num_experts_per_tok=2, moe_intermediate_size=64,
+               shared_expert_intermediate_size=256, norm_topk_prob=False, decoder_sparse_step=1, intermediate_size=16, vocab_size=64)
+    model = moe_b200.random_model(cfg, seed=0, dtype="bfloat16", device=DEV)
+    model.blocks[0].ffn.shared_beside = on_a_side_stream
+    product, seen = tc.gemm_tc, []
+
+    def spy(x, w, out, **k):
+        if w.shape == (128, 256):
+            seen.append((x.shape[0], k["beside"]))
+        return product(x, w, out, **k)
+
+    monkeypatch.setattr(tc, "gemm_tc", spy)
+    eng = moe_b200.Engine(model, max_tokens=2048, max_slots=2)
+    for n in (200, 512):
+        slot = eng.new_sequence()
+        eng.step([slot], [[1] * n], check=True)
+        eng.release(slot)
+    assert set(seen) == {(256, on_a_side_stream), (512, False)}
