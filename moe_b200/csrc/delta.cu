@@ -614,10 +614,12 @@ delta_scan_kernel(const DeltaSeq p, float* __restrict__ o) {
 // reads of shared memory.  2,048 tokens of 16 heads of 128 x 128: 595 us (500 with one decay a head) there, 316 here; in 32 bits
 // throughout it was 295.
 constexpr int CC = 16, CS_COLS = 16, CS_THREADS = 256;
-struct DeltaWork {             // what the first launch leaves, a row a (token, value head)
-    float *w, *q, *kd;         // [T, H, NP]; w and q in the order chunk_place
-    float *u, *pu;             // [T, H, dv]
+constexpr long long CHUNK_SCRATCH = 1ll << 25;      // floats of DeltaWork at most (128 MB): a step of more chunks goes window by window
+struct DeltaWork {             // what the first launch leaves of the window's chunks, sixteen rows each, a row a (token, value head)
+    float *w, *q, *kd;         // [16 chunks, H, NP]; w and q in the order chunk_place
+    float *u, *pu;             // [16 chunks, H, dv]
     float* all;                // [chunk, H, NP]: a chunk's decay of a channel
+    int first, chunks;         // the window: numbers of chunks
 };
 // where channel c lies in a row of w and q: a thread's four channels c, c + 16, c + 32, c + 48 are one 16-byte unit
 __device__ __forceinline__ int chunk_place(int c) { return (c & ~63) + (c & 15) * 4 + ((c >> 4) & 3); }
@@ -633,7 +635,7 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     __shared__ __align__(16) double s_l[CC][CC], s_p[CC][CC];      // L, P; both 0 where j is later
     __shared__ double s_beta[CC], s_lg[CC], s_eb[CC], s_er[CC];
     __shared__ int s_seq;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, number = blockIdx.x, h = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, at_chunk = blockIdx.x, number = wk.first + at_chunk, h = blockIdx.y;
     if (tid == 0) s_seq = -1;
     pdl_sync();
     __syncthreads();
@@ -740,14 +742,14 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     };
     if (tid < NP) {
         const int c = tid, at = chunk_place(c);
-        const size_t row = ((size_t)tok * p.H + h) * NP, pitch = (size_t)p.H * NP;
+        const size_t row = ((size_t)at_chunk * CC * p.H + h) * NP, pitch = (size_t)p.H * NP;
         double all = 1.;
 #pragma unroll
         for (int i = 0; i < CC; i++) {
             if (CH) all *= sg[CH ? i : 0][c]; else all = s_eb[i];
             x[i] = s_beta[i] * (sk[i][c] * all);
         }
-        wk.all[((size_t)number * p.H + h) * NP + c] = (float)all;
+        wk.all[((size_t)at_chunk * p.H + h) * NP + c] = (float)all;
         double since = 1.;
 #pragma unroll
         for (int i = CC - 1; i >= 0; i--) {
@@ -769,7 +771,7 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
 #pragma unroll
             for (int i = 0; i < CC; i++) x[i] = i < cnt ? s_beta[i] * v[(size_t)i * channels] : 0.;
             solve();
-            const size_t row = ((size_t)tok * p.H + h) * dv + c, pitch = (size_t)p.H * dv;
+            const size_t row = ((size_t)at_chunk * CC * p.H + h) * dv + c, pitch = (size_t)p.H * dv;
 #pragma unroll
             for (int i = 0; i < CC; i++) {
                 asm volatile("" ::: "memory");
@@ -780,7 +782,8 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     }
 }
 
-// grid (ceil(dv / 16), heads, sequences): a block carries 16 columns of S in shared memory through its sequence's chunks.
+// grid (ceil(dv / 16), heads, sequences): a block carries 16 columns of S in shared memory through its sequence's chunks in the
+// window.
 // A thread of the first product holds 8 of the 32 rows [W; Q] x 4 columns over every 16th channel (the sum over
 // the 16 threads that share them is 30 shuffles); then a thread forms an output and an element of u, and half of the threads
 // update the state, 4 channels x 4 columns each.
@@ -803,13 +806,14 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
     const int h = blockIdx.y, s = blockIdx.z, c0 = blockIdx.x * CS_COLS, d = p.d, dv = p.dv;
     pdl_sync();
     const int tok0 = p.cu_seqlens[s], cnt = p.cu_seqlens[s + 1] - tok0;
-    if (cnt <= 0) return;
+    const int number0 = chunk_number(tok0, s);        // (counted from the window's first chunk the sequence's first is number0 - first)
+    const int begin = max(0, wk.first - number0) * CC, end = min(cnt, (wk.first + wk.chunks - number0) * CC);
+    if (begin >= end) return;
     float* S = p.state + (size_t)p.slots[s] * p.state_pitch + (size_t)h * d * dv;
     const int ncols = min(CS_COLS, dv - c0);
-    const int number0 = chunk_number(tok0, s);
     auto stage = [&](int t0, int buf) {
         float* dst = sm + buf * L::STAGE;
-        const size_t row0 = (size_t)(tok0 + t0) * p.H + h;
+        const size_t at_chunk = number0 - wk.first + t0 / CC, row0 = at_chunk * CC * p.H + h;
         for (int e = tid; e < 3 * CC * (NP / 4); e += CS_THREADS) {
             const int which = e / (CC * (NP / 4)), i = e / (NP / 4) % CC, c = (e % (NP / 4)) * 4;
             const bool on = t0 + i < cnt;
@@ -824,20 +828,20 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
             cp_zfill(du + which * CC * CS_COLS + i * CS_COLS + c, on ? src + (row0 + (size_t)i * p.H) * dv + c0 + c : src, 16, on);
         } else if (tid < 128 + NP / 4) {
             const int c = (tid - 128) * 4;
-            cp_zfill(du + 2 * CC * CS_COLS + c, wk.all + ((size_t)(number0 + t0 / CC) * p.H + h) * NP + c, 16, true);
+            cp_zfill(du + 2 * CC * CS_COLS + c, wk.all + (at_chunk * p.H + h) * NP + c, 16, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    stage(0, 0);
+    stage(begin, 0);
     for (int e = tid; e < NP * CS_COLS; e += CS_THREADS) {
         const int r = e / CS_COLS, c = e % CS_COLS;
         sS[r * SP + c] = r < d && c < ncols ? S[(size_t)r * dv + c0 + c] : 0.f;
     }
     const int ks = lane & 15, cg = ((warp & 1) * 2 + (lane >> 4)) * 4, tg = warp >> 1;
-    for (int t0 = 0, buf = 0; t0 < cnt; t0 += CC, buf ^= 1) {
+    for (int t0 = begin, buf = 0; t0 < end; t0 += CC, buf ^= 1) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                               // the chunk is there, the state and the other buffer are at rest
-        if (t0 + CC < cnt) stage(t0 + CC, buf ^ 1);
+        if (t0 + CC < end) stage(t0 + CC, buf ^ 1);
         const float* st = sm + buf * L::STAGE;
         {
             float acc[32];
@@ -933,10 +937,16 @@ delta_chunk_scan_kernel(const DeltaSeq p, const DeltaWork wk, float* __restrict_
 
 bool aligned16(const void* p) { return (uintptr_t)p % 16 == 0; }
 
-// Floats of the first launch's results.
-long long chunk_floats(long long T, int num_seqs, int H, int d, int dv) {
+// Chunk numbers of a step, and floats that the first launch leaves of one chunk.
+long long chunk_numbers(long long T, int num_seqs) { return T / CC + num_seqs + 1; }
+long long chunk_floats(int H, int d, int dv) {
     const long long NP = d <= 64 ? 64 : 128;
-    return T * H * (3 * NP + 2 * dv) + (T / CC + num_seqs + 1) * H * NP;
+    return H * (CC * (3 * NP + 2ll * dv) + NP);
+}
+// Chunks of a window: all of the step's if their results find room, as many as do otherwise.
+long long chunk_window(long long T, int num_seqs, int H, int d, int dv) {
+    const long long n = chunk_numbers(T, num_seqs), room = CHUNK_SCRATCH / chunk_floats(H, d, dv);
+    return n < room ? n : room;
 }
 
 }  // namespace
@@ -1023,7 +1033,7 @@ MOE_API int moe_scan_sms() { return scan_sms(); }
 // Floats of scratch with which moe_delta_scan takes the form over chunks of sixteen tokens; 0: it takes the other one.
 MOE_API long long moe_delta_chunk_floats(long long num_tokens, int num_seqs, int H, int G, int d, int dv) {
     if (num_tokens <= 0 || num_seqs <= 0 || d <= 0 || d > 128 || d % 4 || dv <= 0 || dv % 4 || H <= 0 || H > 65535 || num_seqs > 65535) return 0;
-    return chunk_floats(num_tokens, num_seqs, H, d, dv);
+    return chunk_window(num_tokens, num_seqs, H, d, dv) * chunk_floats(H, d, dv);
 }
 
 // Several tokens a sequence; o: [T, H * dv] 32-bit (rows of no sequence are left alone).  `work`: moe_delta_chunk_floats
@@ -1036,22 +1046,27 @@ MOE_API int moe_delta_scan(const float* qkv, const float* step, float* state, lo
         state_pitch < (long long)H * d * dv || H > 65535 || num_seqs > 65535)
         return (int)cudaErrorInvalidValue;
     const DeltaSeq p{qkv, step, state, state_pitch, cu_seqlens, slots, H, G, d, dv, decay};
-    if (work && d <= 128 && d % 4 == 0 && dv % 4 == 0 && aligned16(qkv) && aligned16(decay) && aligned16(work)) {
+    if (work && moe_delta_chunk_floats(num_tokens, num_seqs, H, G, d, dv) > 0 && aligned16(qkv) && aligned16(decay) && aligned16(work)) {
         const int NP = d <= 64 ? 64 : 128;
         DeltaWork wk;
-        const size_t rows = (size_t)num_tokens * H;
+        const long long numbers = chunk_numbers(num_tokens, num_seqs), window = chunk_window(num_tokens, num_seqs, H, d, dv);
+        const size_t rows = (size_t)window * CC * H;
         wk.w = work, wk.q = wk.w + rows * NP, wk.kd = wk.q + rows * NP, wk.u = wk.kd + rows * NP, wk.pu = wk.u + rows * dv;
         wk.all = wk.pu + rows * dv;
-        const dim3 first(num_tokens / CC + num_seqs + 1, H), chain((dv + CS_COLS - 1) / CS_COLS, H, num_seqs);
+        const dim3 chain((dv + CS_COLS - 1) / CS_COLS, H, num_seqs);
 #define CHUNK(NP_, C_)                                                                                                  \
     do {                                                                                                               \
-        const int rc = launch_pdl(delta_chunk_kernel<NP_, C_>, first, dim3(256), 0, stream, p, wk, num_seqs);          \
-        if (rc) return rc;                                                                                             \
         const size_t smem = scan_smem(ChunkSmem<NP_>::FLOATS * sizeof(float), (long long)chain.x * chain.y * chain.z); \
         cudaError_t e = cudaFuncSetAttribute(delta_chunk_scan_kernel<NP_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         if (e != cudaSuccess) return (int)e;                                                                           \
-        delta_chunk_scan_kernel<NP_><<<chain, CS_THREADS, smem, stream>>>(p, wk, o);                                   \
-        return launch_status();                                                                                        \
+        for (long long at = 0; at < numbers; at += window) {                                                           \
+            wk.first = (int)at, wk.chunks = (int)(numbers - at < window ? numbers - at : window);                      \
+            int rc = launch_pdl(delta_chunk_kernel<NP_, C_>, dim3(wk.chunks, H), dim3(256), 0, stream, p, wk, num_seqs); \
+            if (rc) return rc;                                                                                         \
+            delta_chunk_scan_kernel<NP_><<<chain, CS_THREADS, smem, stream>>>(p, wk, o);                               \
+            if ((rc = launch_status())) return rc;                                                                     \
+        }                                                                                                              \
+        return 0;                                                                                                      \
     } while (0)
         if (NP == 64) {
             if (decay) CHUNK(64, true);

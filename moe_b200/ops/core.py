@@ -1597,8 +1597,8 @@ def _delta_chunks(T, num_seqs, heads, dv) -> bool:
 def delta_scan(qkv, step, state, batch, o, *, heads, kv_heads, d, dv, offset=0, decay=None, chunks=None):
     """Per sequence and value head, tokens in order: S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q, on
     what ``delta_prepare`` left (``decay``: a decay a channel, each for its row of S); o: float32 [T, heads * dv].
-    ``chunks``: over chunks of sixteen tokens (scratch of 4 to 6 rows a token) or four tokens at a time; None: by the
-    rule of ``_delta_chunks``."""
+    ``chunks``: over chunks of sixteen tokens (scratch of five rows a token, 128 MB at most: a longer step goes window by
+    window) or four tokens at a time; None: by the rule of ``_delta_chunks``."""
     T = _delta_chk(qkv, step, heads, kv_heads, d, dv, decay)
     _chk(o, "o", torch.float32, 2)
     if tuple(o.shape) != (T, heads * dv):

@@ -362,3 +362,23 @@ def test_short_steps_of_the_delta_rule_keep_the_form_of_four(core, monkeypatch):
         asked.clear()
         core.delta_scan(qkv, step, state, G.make_batch(DEV, list(range(1, B + 1)), [0] * B, [n] * B), o, heads=H, kv_heads=H, d=d, dv=dv)
         assert ("moe_delta_chunk_floats" in asked) == over_chunks, (B, n)
+
+
+def test_a_long_delta_step_goes_window_by_window(core):
+    """The scratch of the chunks is bounded; a step that needs more of it gives what its sequences give alone, to the bit."""
+    H, d, dv, lens = 16, 128, 128, [3000, 517]
+    T, r = sum(lens), lambda *s: torch.randn(*s, device=DEV)
+    unit = torch.nn.functional.normalize
+    qkv = torch.cat([x.reshape(T, -1) for x in (unit(r(T, H, d), dim=-1), unit(r(T, H, d), dim=-1), r(T, H, dv))], 1).contiguous()
+    step, decay, start = torch.sigmoid(r(T, 2 * H)), torch.sigmoid(r(T, H * d) + 2), r(3, H * d * dv)
+    floats = core.lib().moe_delta_chunk_floats
+    assert floats(10 * T, 2, H, H, d, dv) == floats(T, 2, H, H, d, dv) <= 1 << 25 and floats(3000, 1, H, H, d, dv) < floats(T, 2, H, H, d, dv)
+    run = lambda a, b, state, slots, o: core.delta_scan(  # noqa: E731
+        qkv[a:b], step[a:b], state, G.make_batch(DEV, slots, [0] * len(slots), [lens[s - 1] for s in slots]), o, heads=H, kv_heads=H,
+        d=d, dv=dv, decay=decay[a:b], chunks=True)
+    whole, state = torch.full((T, H * dv), float("nan"), device=DEV), start.clone()
+    run(0, T, state, [1, 2], whole)
+    apart, one = torch.empty_like(whole), start.clone()
+    run(0, 3000, one, [1], apart[:3000])
+    run(3000, T, one, [2], apart[3000:])
+    assert torch.equal(whole, apart) and torch.equal(state, one)
