@@ -491,10 +491,12 @@ mlstm_scan_kernel(const MemSeq p, float* __restrict__ o, const MemSegments sg) {
 // shuffles and reads of shared memory (2,048 tokens, 16 heads of 64 x 128, gates included: 243 us in four segments, 139 here).
 // Factors are products of a.
 constexpr int QC = 64, QV = 128;       // tokens a chunk; columns of S a block
-struct MemChunks {
+constexpr long long MEM_SCRATCH = 1ll << 25;        // floats of MemChunks at most (128 MB): a step of more chunks goes window by window
+struct MemChunks {             // of a window's chunks
     float* add;              // [chunk][H][d][dv]: what the chunk adds, then the state before it
     float* norm;             // [chunk][H][d]: the same of n
     float* keep;             // [chunk][H]: the product of the chunk's a
+    int first, chunks;       // the window: numbers of chunks
 };
 // number of the chunk that starts at token `tok` (counted in the step) of sequence s: different for all chunks of a step
 __device__ __forceinline__ int mem_chunk(int tok, int s) { return tok / QC + s; }
@@ -516,7 +518,7 @@ mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
     extern __shared__ __align__(16) float sm[];               // k [64][d + 4], scaled | v [64][132]
     __shared__ float s_a[QC], s_b[QC];
     __shared__ int s_seq;
-    const int tid = threadIdx.x, number = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
+    const int tid = threadIdx.x, number = c.first + blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
     pdl_sync();
     const int s = mem_chunk_seq(p, num_seqs, number, &s_seq);
     if (s < 0) return;
@@ -544,7 +546,7 @@ mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
         *reinterpret_cast<float4*>(sk + i * dp + x) = k4;
     }
     __syncthreads();
-    const size_t at = ((size_t)number * p.H + h) * d;
+    const size_t at = ((size_t)blockIdx.x * p.H + h) * d;
     if (blockIdx.z == 0) {
         for (int x = tid; x < d; x += 256) {
             float n = 0.f;
@@ -554,7 +556,7 @@ mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
         if (tid == 0) {
             float a = 1.f;
             for (int i = 0; i < cnt; i++) a *= s_a[i];
-            c.keep[(size_t)number * p.H + h] = a;
+            c.keep[(size_t)blockIdx.x * p.H + h] = a;
         }
     }
     const int rg = (tid >> 4) * 4, cg = (tid & 15) * 4;
@@ -586,14 +588,17 @@ mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
     }
 }
 
-// grid (ceil((d dv / 4 + d) / 256), heads, sequences): an element of S (four) or of n a thread, through its sequence's chunks
+// grid (ceil((d dv / 4 + d) / 256), heads, sequences): an element of S (four) or of n a thread, through its sequence's chunks in
+// the window
 __global__ void __launch_bounds__(256)
 mlstm_chunk_state_kernel(const MemSeq p, const MemChunks c) {
     pdl_sync();
     const int h = blockIdx.y, s = blockIdx.z, d = p.d, dv = p.dv, quads = d * dv / 4;
     const int a0 = p.cu_seqlens[s], cnt = p.cu_seqlens[s + 1] - a0, e = blockIdx.x * 256 + threadIdx.x;
     if (cnt <= 0 || e >= quads + d) return;
-    const int first = mem_chunk(a0, s), chunks = (cnt + QC - 1) / QC;
+    const int number0 = mem_chunk(a0, s), begin = max(number0, c.first), end = min(number0 + (cnt + QC - 1) / QC, c.first + c.chunks);
+    if (begin >= end) return;
+    const int first = begin - c.first, chunks = end - begin;
     float* state = p.state + (size_t)p.slots[s] * p.state_pitch;
     const float* keep = c.keep + (size_t)first * p.H + h;
     if (e < quads) {
@@ -642,7 +647,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     __shared__ float s_a[QC], s_b[QC], s_den[QC];
     __shared__ double s_all[QC], s_in[QC];
     __shared__ int s_seq;
-    const int tid = threadIdx.x, number = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
+    const int tid = threadIdx.x, number = c.first + blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
     float* sq = sm;                    // [64][d + 4]
     float* sk = sq + QC * dp;          // [64][d + 4]
     float* sP = sk + QC * dp;          // [64][68]
@@ -655,7 +660,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     const int a0 = p.cu_seqlens[s], tok = a0 + (number - mem_chunk(a0, s)) * QC, cnt = min(QC, p.cu_seqlens[s + 1] - tok);
     const int ncols = min(QV, dv - c0);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const size_t at = ((size_t)number * p.H + h) * d;
+    const size_t at = ((size_t)blockIdx.x * p.H + h) * d;
     if (tid < QC) {
         const float* st = p.steps + (size_t)(tok + tid) * 3 * p.H + h;
         s_a[tid] = tid < cnt ? st[0] : 1.f, s_b[tid] = tid < cnt ? st[p.H] : 0.f, s_den[tid] = tid < cnt ? st[2 * p.H] : 1.f;
@@ -884,13 +889,19 @@ MOE_API int moe_mlstm_scan(const float* proj, long long ld, int q_at, int k_at, 
 #undef SCAN_P
 }
 
+// Chunks of a window: all of the step's if what they leave finds room, as many as do otherwise.
+static long long mem_window(long long num_tokens, int num_seqs, int H, int d, int dv) {
+    const long long n = num_tokens / QC + num_seqs + 1, room = MEM_SCRATCH / ((long long)H * (d * dv + d + 1));
+    return n < room ? n : room;
+}
+
 // Floats of scratch of moe_mlstm_chunks; 0 for sizes it does not take.
 MOE_API long long moe_mlstm_chunk_floats(long long num_tokens, int num_seqs, int H, int d, int dv) {
     if (num_tokens <= 0 || num_seqs <= 0 || num_seqs > 65535 || H <= 0 || H > 65535 || d <= 0 || d > 128 || d % 4 || dv <= 0 || dv % 4 ||
         (dv + QV - 1) / QV > 65535)
         return 0;
-    const long long chunks = num_tokens / QC + num_seqs + 1;
-    return chunks * H * d * dv + (chunks * H * d + 3) / 4 * 4 + chunks * H;
+    const long long window = mem_window(num_tokens, num_seqs, H, d, dv);
+    return window * H * d * dv + window * H * d + window * H;
 }
 
 // The same as moe_mlstm_scan, over chunks of sixty-four tokens; `work`: moe_mlstm_chunk_floats floats.  Returns -1, with nothing
@@ -908,22 +919,24 @@ MOE_API int moe_mlstm_chunks(const float* proj, long long ld, int q_at, int k_at
         return -1;
     const MemSeq p{proj, ld, q_at, k_at, v_at, i_at, f_at, i_bias, f_bias, state, state_pitch, cu_seqlens, slots, steps,
                    H, d, dv, cap, q_scale, (dv + COPY_COLS - 1) / COPY_COLS};
-    const int chunks = num_tokens / QC + num_seqs + 1;
+    const int chunks = num_tokens / QC + num_seqs + 1, window = (int)mem_window(num_tokens, num_seqs, H, d, dv);
     MemChunks c;
-    c.add = work, c.norm = work + (size_t)chunks * H * d * dv, c.keep = c.norm + ((size_t)chunks * H * d + 3) / 4 * 4;
+    c.add = work, c.norm = work + (size_t)window * H * d * dv, c.keep = c.norm + (size_t)window * H * d;
     const int threads = longest > 0 && longest < 1024 ? (longest + 31) / 32 * 32 : 1024;
     int code = launch_pdl(mlstm_gates_kernel, dim3(H, num_seqs), dim3(threads), 0, stream, p);
     if (code) return code;
-    const dim3 grid(chunks, H, (dv + QV - 1) / QV);
     const size_t add = ((size_t)QC * (d + 4) + QC * (QV + 4)) * 4, out = mlstm_chunk_out_floats(d) * 4;
     cudaError_t e = cudaFuncSetAttribute(mlstm_chunk_add_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)add);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)out);
     if (e != cudaSuccess) return (int)e;
-    code = launch_pdl(mlstm_chunk_add_kernel, grid, dim3(256), add, stream, p, c, num_seqs);
-    if (code) return code;
-    code = launch_pdl(mlstm_chunk_state_kernel, dim3((d * dv / 4 + d + 255) / 256, H, num_seqs), dim3(256), 0, stream, p, c);
-    if (code) return code;
-    return launch_pdl(mlstm_chunk_out_kernel, grid, dim3(256), out, stream, p, c, num_seqs, o);
+    for (int at = 0; at < chunks && !code; at += window) {
+        c.first = at, c.chunks = chunks - at < window ? chunks - at : window;
+        const dim3 grid(c.chunks, H, (dv + QV - 1) / QV);
+        code = launch_pdl(mlstm_chunk_add_kernel, grid, dim3(256), add, stream, p, c, num_seqs);
+        if (!code) code = launch_pdl(mlstm_chunk_state_kernel, dim3((d * dv / 4 + d + 255) / 256, H, num_seqs), dim3(256), 0, stream, p, c);
+        if (!code) code = launch_pdl(mlstm_chunk_out_kernel, grid, dim3(256), out, stream, p, c, num_seqs, o);
+    }
+    return code;
 }
 
 // One token a sequence: gates, recurrence, head norm (norm_w [H * dv]) and gate (gate: [T, H * dv] 32-bit logits, rows of

@@ -382,3 +382,21 @@ def test_a_long_delta_step_goes_window_by_window(core):
     run(0, 3000, one, [1], apart[:3000])
     run(3000, T, one, [2], apart[3000:])
     assert torch.equal(whole, apart) and torch.equal(state, one)
+
+
+def test_a_long_step_of_the_memory_goes_window_by_window(core):
+    H, d, dv, lens = 32, 128, 256, [1500, 1003]
+    T, floats = sum(lens), core.lib().moe_mlstm_chunk_floats
+    assert floats(20 * T, 2, H, d, dv) == floats(T, 2, H, d, dv) <= 1 << 25 and floats(1500, 1, H, d, dv) < floats(T, 2, H, d, dv)
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    proj, ib, fb = torch.randn(T, at["f"] + H, device=DEV), torch.randn(H, device=DEV), torch.randn(H, device=DEV) + 2
+    state = torch.zeros(3, -(-core.mlstm_state_floats(H, d, dv) // 4) * 4, device=DEV)
+    one = state.clone()
+    run = lambda a, b, st, slots, o: core.mlstm_scan(  # noqa: E731
+        proj[a:b], at, ib, fb, 9.0, d ** -0.5, st, G.make_batch(DEV, slots, [0] * len(slots), [lens[s - 1] for s in slots]), o,
+        heads=H, d=d, dv=dv, chunks=True)
+    whole, apart = torch.full((T, H * dv), float("nan"), device=DEV), torch.empty(T, H * dv, device=DEV)
+    run(0, T, state, [1, 2], whole)
+    run(0, 1500, one, [1], apart[:1500])
+    run(1500, T, one, [2], apart[1500:])
+    assert torch.equal(whole, apart) and torch.equal(state, one)
