@@ -721,7 +721,7 @@ template <typename AT, typename WT, typename OT>
 int launch(const void* A, int lda, const int* a_rows, int a_src_rows, const void* W, long long w_group_stride, void* C,
            int ldc, const float* bias, const int* group_offsets, int num_groups, int M, int N, int K, int* status,
            float* scratch, long long scratch_floats, cudaStream_t stream) {
-    if (M <= 0 || N <= 0) return 0;
+    if (M <= 0 || N <= 0 || (group_offsets && num_groups <= 0)) return 0;      // (rows of no group are left alone)
     const int a_vec = (K % 4 == 0) && (lda % 4 == 0) && ((uintptr_t)A % 16 == 0);
     const int w_vec = (K % 4 == 0) && ((uintptr_t)W % 16 == 0) && ((w_group_stride * (long long)sizeof(WT)) % 16 == 0);
     if constexpr (sizeof(AT) == 4 && sizeof(WT) == 4) {

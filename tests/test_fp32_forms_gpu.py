@@ -400,3 +400,10 @@ def test_a_long_step_of_the_memory_goes_window_by_window(core):
     run(0, 1500, one, [1], apart[:1500])
     run(1500, T, one, [2], apart[1500:])
     assert torch.equal(whole, apart) and torch.equal(state, one)
+
+
+def test_a_stack_of_no_weights_leaves_the_rows_alone(core):
+    st, out = core.new_status(DEV), torch.full((5, 8), 3.0, device=DEV)
+    core.gemm_generic(torch.ones(5, 16, device=DEV), torch.empty(0, 8, 16, device=DEV), out, group_offsets=torch.zeros(1, dtype=torch.int32, device=DEV),
+                      status=st)
+    assert bool((out == 3).all()) and int(st[0]) == 0
