@@ -469,14 +469,15 @@ sgemm_tile_kernel(const float* __restrict__ A, int lda, const int* __restrict__ 
 }
 static_assert(CHUNK % TK == 0, "a chunk is whole stages");
 
-// C[r, n] = the chunks' sums of (r, n) in order (+ bias[n]); with groups, rows past the last group are left alone
+// C[r, n] = the chunks' sums of (r, n) in order (+ bias[n]); with groups, rows of none (before the first, past the last) are left alone
 template <typename OT>
 __global__ void __launch_bounds__(256)
 sum_chunks_kernel(const float* __restrict__ part, int chunks, OT* __restrict__ C, int ldc, const float* __restrict__ bias,
                   const int* __restrict__ group_offsets, int num_groups, int M, int N) {
     const size_t n = (size_t)M * N, i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const size_t from = group_offsets ? (size_t)max(0, group_offsets[0]) * N : 0;
     const size_t live = group_offsets ? (size_t)min(M, group_offsets[num_groups]) * N : n;
-    if (i >= live) return;
+    if (i < from || i >= live) return;
     float t = 0.f;
 #pragma unroll 4
     for (int c = 0; c < chunks; c++) t += part[(size_t)c * n + i];

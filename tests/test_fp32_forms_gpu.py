@@ -407,3 +407,18 @@ def test_a_stack_of_no_weights_leaves_the_rows_alone(core):
     core.gemm_generic(torch.ones(5, 16, device=DEV), torch.empty(0, 8, 16, device=DEV), out, group_offsets=torch.zeros(1, dtype=torch.int32, device=DEV),
                       status=st)
     assert bool((out == 3).all()) and int(st[0]) == 0
+
+
+@pytest.mark.parametrize("counts,before,after", [([40, 0, 70], 7, 5), ([3, 2], 4, 6), ([20, 300], 1, 0)])
+def test_rows_of_no_group_are_left_alone(core, counts, before, after):
+    torch.manual_seed(before)
+    E, N, K, M = len(counts), 132, 772, before + sum(counts) + after
+    a, w, st = torch.randn(M, K, device=DEV), torch.randn(E, N, K, device=DEV), core.new_status(DEV)
+    offs = torch.tensor(np.cumsum([before] + counts), dtype=torch.int32, device=DEV)
+    out = torch.full((M, N), 7.0, device=DEV)
+    core.gemm_generic(a, w, out, group_offsets=offs, status=st)
+    assert bool((out[:before] == 7).all()) and bool((out[M - after:] == 7).all())
+    for g in range(E):
+        x = a[offs[g]:offs[g + 1]]
+        assert bool(((out[offs[g]:offs[g + 1]].double() - x.double() @ w[g].double().T).abs() <= bound(x, w[g])).all()), g
+    assert int(st[0]) == 0
