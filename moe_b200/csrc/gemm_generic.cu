@@ -631,13 +631,18 @@ sgemm_rows_kernel(const float* __restrict__ A, int lda, const int* __restrict__ 
 }
 
 // Which form a product of 32-bit operands takes.
+constexpr long long SCRATCH_FLOATS = 1ll << 25;      // chunk sums a launch may leave (128 MB)
 struct Plan {
     int rows;            // > 0: sgemm_rows_kernel with so many rows a tile; else sgemm_tile_kernel
     int tile;            // 128, 64 or 32 rows a tile
     int splits, per;     // K splits and chunks a split
+    int pass;            // rows a launch (all, or with splits as many as SCRATCH_FLOATS has room for)
 };
+long long plan_floats(const Plan& p, int N, int K) {
+    return p.splits > 1 ? (long long)((K + CHUNK - 1) / CHUNK) * p.pass * N : 0;
+}
 Plan plan_f32(int M, int N, int K, bool grouped, int num_groups) {
-    Plan p = {0, 0, 1, 0};
+    Plan p = {0, 0, 1, 0, M};
     const int groups = grouped ? num_groups : 1, each = M / groups, chunks = (K + CHUNK - 1) / CHUNK;
     // Few rows a group: the weight stream is the time.  (Measured, us: 60 groups of 2,048 x 2,816 with 7 rows each 297
     // against 814 in tiles of 32; beyond 16 rows a tile of it would have to read the weights twice.)
@@ -646,27 +651,39 @@ Plan plan_f32(int M, int N, int K, bool grouped, int num_groups) {
         return p;
     }
     // The tile whose waves take least: blocks over the blocks the SMs hold, times a wave's rows, by the rate the
-    // form reaches with all SMs full (TFLOP/s, measured).  A group's last tile is half empty on average.
+    // form reaches with all SMs full (TFLOP/s, measured).  A group's last tile is half empty on average.  Less than half a wave:
+    // the chunks of k side by side (2,048 x 6,144 weights at 24 / 64 / 100 rows: 53 / 56 / 97 us, 243 / 201 / 185 without); every chunk's
+    // sums go through memory, so a product without groups whose sums find no room goes over its rows in passes.
     const int cols = (N + TN - 1) / TN, tms[3] = {128, 64, 32}, slots[3] = {2, 3, 6};
     const float rate[3] = {54.f, 50.f, 43.6f};
     float best = 0.f;
     for (int f = 0; f < 3; f++) {
-        const long long tiles = grouped ? M / tms[f] + (num_groups + 1) / 2 : (M + tms[f] - 1) / tms[f];
-        const long long blocks = tiles * cols, room = (long long)slots[f] * scan_sms();
-        // less than a wave: the chunks of k side by side (2,048 x 6,144 weights at 24 / 64 / 100 rows: 53 / 56 / 97 us, 243 /
-        // 201 / 185 without)
-        int splits = blocks * 2 <= room ? (int)(room / blocks) : 1;
-        if (splits > chunks) splits = chunks;
-        const int per = (chunks + splits - 1) / splits;
-        splits = (chunks + per - 1) / per;
-        const float waves = (float)((blocks * splits + room - 1) / room) * per / chunks;
-        const float cost = waves * slots[f] * tms[f] / rate[f];
-        if (!p.tile || cost < best) p.tile = tms[f], p.splits = splits, p.per = per, best = cost;
+        const long long room = (long long)slots[f] * scan_sms();
+        // the plan for `pass` rows a launch, with K splits if asked for and two blocks or more find room
+        auto consider = [&](int pass, bool split) {
+            const long long blocks = cols * (long long)(grouped ? M / tms[f] + (num_groups + 1) / 2 : (pass + tms[f] - 1) / tms[f]);
+            int splits = split ? (int)(room / blocks < chunks ? room / blocks : chunks) : 1;
+            if (split && splits < 2) return;
+            const int per = (chunks + splits - 1) / splits;
+            splits = (chunks + per - 1) / per;
+            const float waves = (float)((blocks * splits + room - 1) / room) * per / chunks;
+            // us: a wave's multiply-adds at the form's rate; the chunks' sums written and read at some 8 TB/s, and a launch more
+            float cost = waves * slots[f] * tms[f] / rate[f] * scan_sms() * TN * 2e-6f * K;
+            if (splits > 1) cost += 8.f * chunks * pass * N / 8e6f + 3.f;
+            const int passes = (M + pass - 1) / pass;
+            if (passes > 1) cost *= 1.25f * passes;          // (as measured: the weights come from memory again, the last one is not whole)
+            if (!p.tile || cost < best) p.tile = tms[f], p.splits = splits, p.per = per, p.pass = pass, best = cost;
+        };
+        consider(M, false);
+        const long long fit = SCRATCH_FLOATS / ((long long)chunks * N);      // rows whose sums find room
+        if (fit >= M)
+            consider(M, true);
+        else if (!grouped && fit >= tms[f]) {
+            const int most = (int)(fit / tms[f]) * tms[f], passes = (M + most - 1) / most;
+            consider(((M + passes - 1) / passes + tms[f] - 1) / tms[f] * tms[f], true);
+        }
     }
     return p;
-}
-long long plan_floats(const Plan& p, int M, int N, int K) {
-    return p.splits > 1 ? (long long)((K + CHUNK - 1) / CHUNK) * M * N : 0;
 }
 
 // The forms above, for 32-bit operands whose rows are whole 16-byte units; -1 where they do not apply.
@@ -675,16 +692,18 @@ int launch_f32(const float* A, int lda, const int* a_rows, int a_src_rows, const
                int ldc, const float* bias, const int* group_offsets, int num_groups, int M, int N, int K, int* status,
                float* scratch, long long scratch_floats, cudaStream_t stream) {
     Plan p = plan_f32(M, N, K, group_offsets != nullptr, num_groups);
-    if (plan_floats(p, M, N, K) > scratch_floats) p.splits = 1;
+    if (plan_floats(p, N, K) > scratch_floats) p.splits = 1, p.pass = M;
 #define RUN(kernel, bytes, grid, threads, ...)                                                                              \
     {                                                                                                                      \
         const dim3 gr = grid;                                                                                              \
         if (gr.y > 65535) return -1;                                                                                       \
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);                  \
         if (e != cudaSuccess) return (int)e;                                                                               \
-        kernel<<<gr, threads, bytes, stream>>>(A, lda, a_rows, a_src_rows, W, w_group_stride, C, ldc, bias, group_offsets, \
-                                               num_groups, M, N, K, status __VA_OPT__(, ) __VA_ARGS__);                    \
+        kernel<<<gr, threads, bytes, stream>>>(a_rows ? A : A + (size_t)r0 * lda, lda, a_rows ? a_rows + r0 : nullptr,      \
+                                               a_rows ? a_src_rows : a_src_rows - r0, W, w_group_stride, C + (size_t)r0 * ldc, ldc, \
+                                               bias, group_offsets, num_groups, m, N, K, status __VA_OPT__(, ) __VA_ARGS__); \
     }
+    int r0 = 0, m = M;              // the rows of a pass
     if (p.rows) {
         const int tiles = group_offsets ? (M < num_groups ? M : num_groups) + M / p.rows : (M + p.rows - 1) / p.rows;
 #define ROWS(R, FL) RUN((sgemm_rows_kernel<R, FL, OT>), (RowsForm<R, FL>::BYTES), dim3((N + 16 * FL - 1) / (16 * FL), tiles), SWARPS * 32)
@@ -699,23 +718,28 @@ int launch_f32(const float* A, int lda, const int* a_rows, int a_src_rows, const
         return launch_status();
     }
     const int cols = (N + TN - 1) / TN;
-    const int tiles = (M + p.tile - 1) / p.tile + (group_offsets ? (M < num_groups ? M : num_groups) : 0);
+    for (; r0 < M; r0 += p.pass) {
+        m = M - r0 < p.pass ? M - r0 : p.pass;
+        const int tiles = (m + p.tile - 1) / p.tile + (group_offsets ? (m < num_groups ? m : num_groups) : 0);
 #define TILE(F)                                                                                                            \
     {                                                                                                                      \
         if (p.splits > 1) RUN((sgemm_tile_kernel<F, OT, true>), F::SPLIT_BYTES, dim3(cols, tiles, p.splits), F::NT, p.per, scratch) \
         else RUN((sgemm_tile_kernel<F, OT, false>), F::BYTES, dim3(cols, tiles), F::NT, 0, nullptr)                        \
     }
-    if (p.tile == 128) TILE(Tile128)
-    else if (p.tile == 64) TILE(Tile64)
-    else TILE(Tile32)
+        if (p.tile == 128) TILE(Tile128)
+        else if (p.tile == 64) TILE(Tile64)
+        else TILE(Tile32)
 #undef TILE
 #undef RUN
-    if (p.splits > 1) {
-        const long long n = (long long)M * N;
-        sum_chunks_kernel<OT><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(scratch, (K + CHUNK - 1) / CHUNK, C, ldc, bias,
-                                                                              group_offsets, num_groups, M, N);
+        if (p.splits > 1) {
+            const long long n = (long long)m * N;
+            sum_chunks_kernel<OT><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(scratch, (K + CHUNK - 1) / CHUNK, C + (size_t)r0 * ldc, ldc,
+                                                                                  bias, group_offsets, num_groups, m, N);
+        }
+        const int rc = launch_status();
+        if (rc) return rc;
     }
-    return launch_status();
+    return 0;
 }
 
 template <typename AT, typename WT, typename OT>
@@ -752,11 +776,16 @@ int launch(const void* A, int lda, const int* a_rows, int a_src_rows, const void
 
 }  // namespace
 
-// Floats of scratch that moe_gemm_generic can use for such a product of 32-bit operands (without them it takes the
-// form that needs none: the same result, fewer blocks).
+// Floats of scratch that moe_gemm_generic can use for such a product of 32-bit operands, 2^25 at most (without them it takes
+// the form that needs none: the same result, fewer blocks).
 MOE_API long long moe_gemm_scratch_floats(int M, int N, int K, int num_groups) {
     if (M <= 0 || N <= 0 || K <= 0 || K % 4) return 0;
-    return plan_floats(plan_f32(M, N, K, num_groups > 0, num_groups), M, N, K);
+    return plan_floats(plan_f32(M, N, K, num_groups > 0, num_groups), N, K);
+}
+// The form such a product takes: rows a tile of the form for few rows (or 0), rows a tile, K splits, chunks a split, rows a pass.
+MOE_API void moe_gemm_plan(int M, int N, int K, int num_groups, int* out) {
+    const Plan p = plan_f32(M, N, K, num_groups > 0, num_groups);
+    out[0] = p.rows, out[1] = p.rows ? 0 : p.tile, out[2] = p.splits, out[3] = p.per, out[4] = p.pass;
 }
 
 // A: [*, lda] of a_dt; W: [G][N, K] of w_dt; C: [M, ldc] of c_dt.  `a_rows` (may be

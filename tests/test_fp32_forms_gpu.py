@@ -422,3 +422,19 @@ def test_rows_of_no_group_are_left_alone(core, counts, before, after):
         x = a[offs[g]:offs[g + 1]]
         assert bool(((out[offs[g]:offs[g + 1]].double() - x.double() @ w[g].double().T).abs() <= bound(x, w[g])).all()), g
     assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1152, 2048, 5632), (520, 3584, 20480), (333, 6145, 4100)])
+def test_the_sums_of_k_splits_find_room(core, M, N, K):
+    """The chunks' sums of K splits take 128 MB at most: a product that would need more goes over its rows in passes.  The result is
+    the same to the bit as its rows' alone."""
+    torch.manual_seed(M)
+    assert all(core.lib().moe_gemm_scratch_floats(m, N, K, 0) <= 1 << 25 for m in range(1, 4 * M, 7))
+    a, w, st = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), core.new_status(DEV)
+    out = torch.full((M + 1, N), float("nan"), device=DEV)
+    core.gemm_generic(a, w, out[:M], status=st)
+    few = torch.empty(8, N, device=DEV)
+    for r in (0, M // 2, M - 8):
+        core.gemm_generic(a[r:r + 8], w, few, status=st)
+        assert torch.equal(few, out[r:r + 8]), r
+    assert bool(out[M].isnan().all()) and int(st[0]) == 0
