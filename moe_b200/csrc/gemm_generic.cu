@@ -654,21 +654,25 @@ Plan plan_f32(int M, int N, int K, bool grouped, int num_groups) {
     // form reaches with all SMs full (TFLOP/s, measured).  A group's last tile is half empty on average.  Less than half a wave:
     // the chunks of k side by side (2,048 x 6,144 weights at 24 / 64 / 100 rows: 53 / 56 / 97 us, 243 / 201 / 185 without); every chunk's
     // sums go through memory, so a product without groups whose sums find no room goes over its rows in passes.
-    const int cols = (N + TN - 1) / TN, tms[3] = {128, 64, 32}, slots[3] = {2, 3, 6};
-    const float rate[3] = {54.f, 50.f, 43.6f};
+    const int cols = (N + TN - 1) / TN, tms[3] = {128, 64, 32};
+    // blocks an SM holds: with the totals in shared memory (no splits) the form of 32 rows is at five.  (Room for a sixth, the few bytes that
+    // say which tile it is in the padding, leaves L1 too little: 60 groups of 17 rows, 2,816 x 2,048, 592 -> 683 us.)
+    auto slots = [](int f, bool split) { return f == 0 ? 2 : f == 1 ? 3 : split ? 6 : 5; };
+    auto rate = [](int f, bool split) { return f == 0 ? 54.f : f == 1 ? 50.f : split ? 43.6f : 36.3f; };
     float best = 0.f;
     for (int f = 0; f < 3; f++) {
-        const long long room = (long long)slots[f] * scan_sms();
         // the plan for `pass` rows a launch, with K splits if asked for and two blocks or more find room
         auto consider = [&](int pass, bool split) {
             const long long blocks = cols * (long long)(grouped ? M / tms[f] + (num_groups + 1) / 2 : (pass + tms[f] - 1) / tms[f]);
+            const int here = slots(f, split);
+            const long long room = (long long)here * scan_sms();
             int splits = split ? (int)(room / blocks < chunks ? room / blocks : chunks) : 1;
             if (split && splits < 2) return;
             const int per = (chunks + splits - 1) / splits;
             splits = (chunks + per - 1) / per;
             const float waves = (float)((blocks * splits + room - 1) / room) * per / chunks;
             // us: a wave's multiply-adds at the form's rate; the chunks' sums written and read at some 8 TB/s, and a launch more
-            float cost = waves * slots[f] * tms[f] / rate[f] * scan_sms() * TN * 2e-6f * K;
+            float cost = waves * here * tms[f] / rate(f, split) * scan_sms() * TN * 2e-6f * K;
             if (splits > 1) cost += 8.f * chunks * pass * N / 8e6f + 3.f;
             const int passes = (M + pass - 1) / pass;
             if (passes > 1) cost *= 1.25f * passes;          // (as measured: the weights come from memory again, the last one is not whole)
@@ -781,6 +785,23 @@ int launch(const void* A, int lda, const int* a_rows, int a_src_rows, const void
 MOE_API long long moe_gemm_scratch_floats(int M, int N, int K, int num_groups) {
     if (M <= 0 || N <= 0 || K <= 0 || K % 4) return 0;
     return plan_floats(plan_f32(M, N, K, num_groups > 0, num_groups), N, K);
+}
+// Blocks of the tile form of `tile` rows that an SM holds (split: with K splits).
+MOE_API int moe_gemm_tile_room(int tile, int split) {
+    int n = -1;
+#define ROOM(F)                                                                                                            \
+    {                                                                                                                      \
+        auto kernel = split ? sgemm_tile_kernel<F, float, true> : sgemm_tile_kernel<F, float, false>;                      \
+        const int bytes = split ? F::SPLIT_BYTES : F::BYTES;                                                               \
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess ||             \
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, F::NT, bytes) != cudaSuccess)                        \
+            return -1;                                                                                                     \
+    }
+    if (tile == 128) ROOM(Tile128)
+    else if (tile == 64) ROOM(Tile64)
+    else if (tile == 32) ROOM(Tile32)
+#undef ROOM
+    return n;
 }
 // The form such a product takes: rows a tile of the form for few rows (or 0), rows a tile, K splits, chunks a split, rows a pass.
 MOE_API void moe_gemm_plan(int M, int N, int K, int num_groups, int* out) {

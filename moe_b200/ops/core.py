@@ -103,6 +103,7 @@ def lib():
             fn.argtypes = argtypes
             fn.restype = c_int
         L.moe_scan_sms.argtypes, L.moe_scan_sms.restype = [], c_int
+        L.moe_gemm_tile_room.argtypes, L.moe_gemm_tile_room.restype = [I, I], c_int
         L.moe_gemm_plan.argtypes, L.moe_gemm_plan.restype = [I, I, I, I, P], None
         L.moe_gemm_scratch_floats.argtypes, L.moe_gemm_scratch_floats.restype = [I, I, I, I], LL
         L.moe_delta_chunk_floats.argtypes, L.moe_delta_chunk_floats.restype = [LL, I, I, I, I, I], LL

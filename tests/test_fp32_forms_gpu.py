@@ -438,3 +438,8 @@ def test_the_sums_of_k_splits_find_room(core, M, N, K):
         core.gemm_generic(a[r:r + 8], w, few, status=st)
         assert torch.equal(few, out[r:r + 8]), r
     assert bool(out[M].isnan().all()) and int(st[0]) == 0
+
+
+@pytest.mark.parametrize("tile,split,blocks", [(128, 0, 2), (128, 1, 2), (64, 0, 3), (64, 1, 3), (32, 0, 5), (32, 1, 6)])
+def test_an_sm_holds_the_blocks_the_plan_counts_with(core, tile, split, blocks):
+    assert core.lib().moe_gemm_tile_room(tile, split) >= blocks
