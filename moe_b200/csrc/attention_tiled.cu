@@ -292,6 +292,9 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_new, co
 #pragma unroll
         for (int j = 0; j < OC; j++) o[i][j] = 0.f;
     }
+    // The first 64 queries take no value behind the last of them and the others none in front of their window, not even with a
+    // weight of 0: an infinite or NaN value reaches as many queries that do not see it as in the form above, and no more.
+    const int low_to = p_first + FQ / 2 - 1, high_from = attn_lo(p_first + FQ / 2, window, var.chunk);
     const int tile_lo = lo_min / FK, kept_tiles = min((var.keep + FK - 1) / FK, tile_lo);
     for (int tile = 0; attn_seen(tile, kept_tiles, tile_lo) * FK <= p_last; tile++) {
         const int j0 = attn_seen(tile, kept_tiles, tile_lo) * FK;
@@ -381,8 +384,32 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_new, co
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
+        // keys [c_lo, c_hi) are for both halves of the queries; a key outside for the half that may take it
+        const int c_lo = high_from > j0 && j0 + FK > var.keep ? min(FK, (high_from - j0 + 3) & ~3) : 0;
+        const int c_hi = max(c_lo, min(FK, (low_to - j0 + 1) & ~3));
+        auto for_one_half = [&](int from, int to) {
 #pragma unroll 1
-        for (int c = 0; c < FK; c += 4) {
+            for (int c = from; c < to; c++) {
+                const int key = j0 + c;
+                const bool low = key <= low_to, high = key >= high_from || key < var.keep;
+                float4 v4[OC / 4];
+#pragma unroll
+                for (int j = 0; j < OC; j += 4) v4[j / 4] = *reinterpret_cast<const float4*>(V + c * HP + 4 * tx + 16 * j);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    if (!(i < 4 ? low : high)) continue;
+                    const float pv = P[(ty + 16 * i) * PP + c];
+#pragma unroll
+                    for (int j = 0; j < OC; j += 4) {
+                        o[i][j] = fmaf(pv, v4[j / 4].x, o[i][j]), o[i][j + 1] = fmaf(pv, v4[j / 4].y, o[i][j + 1]);
+                        o[i][j + 2] = fmaf(pv, v4[j / 4].z, o[i][j + 2]), o[i][j + 3] = fmaf(pv, v4[j / 4].w, o[i][j + 3]);
+                    }
+                }
+            }
+        };
+        for_one_half(0, c_lo);
+#pragma unroll 1
+        for (int c = c_lo; c < c_hi; c += 4) {
             float4 a[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4*>(P + (ty + 16 * i) * PP + c);
@@ -399,6 +426,7 @@ attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_new, co
                     }
                 }
         }
+        for_one_half(c_hi, min(FK, p_last - j0 + 1));
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) {

@@ -443,3 +443,39 @@ def test_the_sums_of_k_splits_find_room(core, M, N, K):
 @pytest.mark.parametrize("tile,split,blocks", [(128, 0, 2), (128, 1, 2), (64, 0, 3), (64, 1, 3), (32, 0, 5), (32, 1, 6)])
 def test_an_sm_holds_the_blocks_the_plan_counts_with(core, tile, split, blocks):
     assert core.lib().moe_gemm_tile_room(tile, split) >= blocks
+
+
+@pytest.mark.parametrize("hd", [128, 64])
+@pytest.mark.parametrize("before,new,window,keep,where", [(0, 256, None, 0, 100), (0, 256, None, 0, 200), (70, 300, None, 0, 140), (0, 400, 50, 0, 10),
+                                                          (0, 400, 50, 0, 150), (37, 290, 130, 70, 90)])
+def test_a_value_reaches_no_query_of_another_tile_that_does_not_see_it(core, hd, before, new, window, keep, where):
+    """An infinite or NaN value of one key: the queries of a tile of 64 none of which sees the key are the same to the bit."""
+    from moe_b200.cache import KVCache, KVRequest
+
+    torch.manual_seed(where)
+    T = before + new
+    cache = KVCache({0: KVRequest(1, hd, window, keep=keep) if keep else KVRequest(1, hd, window)}, {0: None}, max_tokens=64 * 30, max_slots=2,
+                    dtype=torch.float32, device=DEV)
+    view, slot, st = cache.view(0), cache.acquire(), core.new_status(DEV)
+    K, V, q = torch.randn(T, 1, hd, device=DEV), torch.randn(T, 1, hd, device=DEV), torch.randn(new, 1, hd, device=DEV)
+    if before:
+        G.give_pages(cache, slot, before)
+        core.kv_commit(K[:before].contiguous(), V[:before].contiguous(), view, G.make_batch(DEV, [slot], [0], [before]), st)
+    G.give_pages(cache, slot, T)
+    batch, outs = G.make_batch(DEV, [slot], [before], [new]), []
+    assert where >= before
+    for bad in (None, math.inf, math.nan):
+        vn = V[before:].clone()
+        if bad is not None:
+            vn[where - before] = bad
+        outs.append(torch.empty(new, hd, device=DEV))
+        assert core.attention_tiled(q, K[before:].contiguous(), vn, view, batch, outs[-1], nh=1, window=window, scale=hd ** -0.5, use_local=True,
+                                    status=st, keep=keep)
+    clean = 0
+    for r0 in range(0, new, 64):
+        p = torch.arange(before + r0, before + min(r0 + 64, new))
+        lo = (p + 1 - window).clamp(min=0) if window else torch.zeros_like(p)
+        if not bool(((where <= p) & ((where >= lo) | (where < keep))).any()):
+            clean += 1
+            assert torch.equal(outs[1][r0:r0 + 64], outs[0][r0:r0 + 64]) and torch.equal(outs[2][r0:r0 + 64], outs[0][r0:r0 + 64]), r0
+    assert clean > 0 and not bool(outs[1].isfinite().all()) and bool(outs[0].isfinite().all()) and int(st[0]) == 0
