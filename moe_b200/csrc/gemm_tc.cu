@@ -74,7 +74,8 @@ struct Params {
     int* tickets;               // one per (grid.y, grid.x), zero before and after the launch
     int* status;
     uint32_t wait_limit;        // microseconds a wait on a barrier may take (WAIT_LIMIT_US, less in the wait test)
-    int test_fault;             // 0; the wait test: 1 = the producer loads nothing, 2 = no MMA is issued
+    int test_fault;             // 0; the wait test: 1 = the producer loads nothing, 2 = no MMA is issued, 3 and 4 = the producer of a pair's
+                                // second or first CTA loads nothing
     int act;                    // SWIGLU: the gate's activation (ACT_* in common.cuh)
     float act_param;            // its constant, if it has one (the limit of ACT_CLAMPED_SIGMOID)
 };
@@ -87,6 +88,10 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// counts bytes as arrived that nobody will copy
+__device__ __forceinline__ void mbar_complete_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
@@ -148,6 +153,14 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
+}
+__device__ __forceinline__ int ld_cluster_s32(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_cluster_s32(uint32_t addr, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
@@ -914,6 +927,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
 //   empty[s]     in each CTA: the MMA issuer's commit, multicast to both
 //   acc_full[b]  in each CTA: likewise
 //   acc_empty[b] in the first CTA: the epilogue warps of both CTAs
+//   mma_done     in each CTA: only where a wait ran out, the issuer's last commit
+// A role whose wait runs out tells both CTAs, all roles end, and before the pair gives its memory back the first CTA sees to it
+// that every copy either of them asked for has landed (one may have asked for stages the other did not) and that no MMA runs.
 template <int BN, int MODE>
 struct PairCfg {
     static constexpr int NW = MODE == MODE_SWIGLU ? 2 : 1;
@@ -937,6 +953,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     constexpr int PAIR_W = MODE == MODE_SWIGLU_IL ? TILE_W : 2 * TILE_W;
     extern __shared__ uint8_t smem_raw[];
     __shared__ volatile int s_abort;
+    __shared__ int s_issued;                        // stages this CTA's producer has asked for
     __shared__ uint32_t s_tmem;
     __shared__ int s_offs[MAX_SMEM_GROUPS + 1], s_prefix[MAX_SMEM_GROUPS + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -968,7 +985,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     auto empty_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };
     auto acc_full = [&](int b) { return bar_base + 8u * (2 * C::STAGES + b); };
     auto acc_empty = [&](int b) { return bar_base + 8u * (2 * C::STAGES + 2 + b); };
+    const uint32_t mma_done = bar_base + 8u * (2 * C::STAGES + 4);
     if (threadIdx.x == 0) {
+        s_issued = 0;
+        mbar_init(mma_done, 1);
         for (int s = 0; s < C::STAGES; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
@@ -986,13 +1006,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     const int kbs = (p.K + BK - 1) / BK;
+    auto give_up = [&]() {       // (the other CTA is there until the cluster's barrier below)
+        atomicOr(p.status, ST_WAIT_TIMEOUT);
+        s_abort = 1;
+        st_cluster_s32(mapa_cluster(smem_u32((const void*)&s_abort), rank ^ 1), 1);
+    };
 
     if (warp == 0) {
         // ---- producer (in both CTAs): own weight rows, own half of the tokens --------------------
         if (lane == 0) {
             int issued = 0;
             bool ok = true;
-            for (int item = pair; item < items && ok; item += pairs) {
+            const bool idle = p.test_fault == 1 || p.test_fault == 4 - (int)rank;
+            for (int item = pair; item < items && ok && !idle; item += pairs) {
                 const Tile t = tile_of<BN, PAIR_W>(item, m_tiles, p, s_prefix, s_offs);
                 const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31);     // (a pair's N: steps of 32)
                 const int half = n_eff >> 1;
@@ -1017,20 +1043,15 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                                          x_row + c * C::XBOX, bar);
                 }
             }
-            if (!ok) {
-                atomicOr(p.status, ST_WAIT_TIMEOUT);
-                s_abort = 1;
-                if (rank == 0)
-                    for (int i = max(0, issued - C::STAGES); i < issued; i++)     // copies in flight must land
-                        mbar_wait(full_bar(i % C::STAGES), (i / C::STAGES) & 1, nullptr, p.wait_limit, p.status, 0x32);
-            }
+            s_issued = issued;
+            if (!ok) give_up();
         }
     } else if (warp == 1) {
         // ---- MMA issuer (first CTA only): accumulator buffer (tile & 1) ---------------------------
         if (lane == 0 && rank == 0) {
             int consumed = 0, local = 0;
             bool ok = true;
-            for (int item = pair; item < items && ok; item += pairs, local++) {
+            for (int item = pair; item < items && ok && p.test_fault != 2; item += pairs, local++) {
                 const Tile t = tile_of<BN, PAIR_W>(item, m_tiles, p, s_prefix, s_offs);
                 const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31);
                 const uint32_t idesc = instr_desc(n_eff, 2 * TILE_W);
@@ -1058,10 +1079,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                 }
                 if (ok) umma_commit_pair(acc_full(b));
             }
-            if (!ok) {
-                atomicOr(p.status, ST_WAIT_TIMEOUT);
-                s_abort = 1;
-            }
+            if (!ok) give_up();
         }
     } else {
         // ---- epilogue (in both CTAs): this CTA's 128 features of the tile; warps as in the single form --
@@ -1088,14 +1106,32 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_cluster(acc_empty(b), 0));
         }
-        if (!ok && lane == 0) {
-            atomicOr(p.status, ST_WAIT_TIMEOUT);
-            s_abort = 1;
-        }
+        if (!ok && lane == 0) give_up();
     }
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();          // neither CTA frees tensor memory or leaves while the other may still use it
+    if (s_abort) {               // (the same in both)
+        if (warp == 1 && lane == 0) {
+            if (rank == 0) umma_commit_pair(mma_done);
+            mbar_wait(mma_done, 0, nullptr, p.wait_limit, p.status, 0x36);
+        }
+        if (warp == 0 && lane == 0 && rank == 0) {
+            const int mine = s_issued, theirs = ld_cluster_s32(mapa_cluster(smem_u32(&s_issued), 1)), most = max(mine, theirs);
+            for (int i = max(0, most - C::STAGES); i < most; i++) {
+                const Tile t = tile_of<BN, PAIR_W>(pair + i / kbs * pairs, m_tiles, p, s_prefix, s_offs);
+                const int half = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31) >> 1;
+                const uint32_t cta_tx = C::NW * C::W_BYTES + (half + C::XBOX - 1) / C::XBOX * C::XBOX * BK * 2;
+                const uint32_t bar = full_bar(i % C::STAGES);
+                if (i >= theirs) mbar_complete_tx(bar, cta_tx);      // announced for both, but the other half was never asked for
+                if (i >= mine) mbar_expect_tx(bar, cta_tx);          // asked for by the other CTA alone, and not yet announced
+                mbar_wait(bar, (i / C::STAGES) & 1, nullptr, p.wait_limit, p.status, 0x32);
+            }
+        }
+        __syncthreads();
+        cluster_sync_all();
+        tc_fence_after();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem, C::TMEM_COLS);
@@ -1327,13 +1363,13 @@ MOE_API void moe_tc_set_persistent(int enabled) { g_persistent = enabled ? 1 : 0
 // The one-accumulator SwiGLU form of the persistent kernel on or off (on by default).
 MOE_API void moe_tc_set_swiglu_interleaved(int enabled) { g_swiglu_il = enabled ? 1 : 0; }
 
-// For the test of the bounded waits only: ``fault`` 1 makes the producer of the single-CTA kernels
-// load nothing, 2 makes their MMA issuer issue nothing, so that the other roles' waits run out after
+// For the test of the bounded waits only: ``fault`` 1 makes the kernels' producers load nothing, 2 makes their
+// MMA issuer issue nothing, 3 and 4 the producer of the second and of the first CTA of a pair load nothing, so that the other roles' waits run out after
 // ``wait_limit`` microseconds (0: the normal limit); the CTAs then set ST_WAIT_TIMEOUT in the status word,
 // wait for their own copies in flight, free their tensor memory and return.  (0, 0) restores the
 // normal behaviour.  Nothing faults and nothing waits without a limit.
 MOE_API void moe_tc_set_wait_test(int fault, unsigned wait_limit) {
-    g_test_fault = (fault == 1 || fault == 2) ? fault : 0;
+    g_test_fault = (fault >= 1 && fault <= 4) ? fault : 0;
     g_wait_limit = wait_limit ? wait_limit : WAIT_LIMIT_US;
 }
 

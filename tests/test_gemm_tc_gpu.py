@@ -241,3 +241,41 @@ def test_the_products_of_a_small_model_with_a_width_of_264(tc, tokens):
     bn = token_tile(P / E)
     check(torch.randn(P, H, device=DEV).to(torch.bfloat16), rnd(E, 2 * mi, H), mi, swiglu=True, offs=offs, bn=bn)
     check(torch.randn(P, mi, device=DEV).to(torch.bfloat16), rnd(E, H, mi), H, offs=offs, bn=bn)
+
+
+@pytest.mark.parametrize("swiglu,offs", [(False, None), (True, None), (False, [0, 260, 260, 700])])
+@pytest.mark.parametrize("fault", [1, 2, 3, 4])
+def test_a_wait_that_runs_out_in_a_pair_of_ctas_is_reported(fault, swiglu, offs):
+    """The same on pairs of CTAs: both producers load nothing, no MMA is issued, or one CTA's producer alone loads nothing, so
+    that the other has asked for stages which never fill.  Every wait is bounded: both CTAs return, the status says so, and the
+    next product is right."""
+    from moe_b200.ops import core, tc
+
+    torch.manual_seed(0)
+    K, N, M = 1024, 384, 700
+    G = 3 if offs else 1
+    x = (torch.randn(M, K, device=DEV) * 0.5).to(torch.bfloat16)
+    w = (torch.randn(G, N * (2 if swiglu else 1), K, device=DEV) * 0.05).to(torch.bfloat16)
+    ref = torch.cat([x[a:b].float() @ w[g].float().T for g, (a, b) in enumerate(zip(offs[:-1], offs[1:]) if offs else [(0, M)])])
+    if swiglu:
+        ref = torch.nn.functional.silu(ref[:, :N]) * ref[:, N:]
+    args = dict(swiglu=swiglu, group_offsets=torch.tensor(offs, dtype=torch.int32, device=DEV) if offs else None, bn=256, splits=1)
+    w = w if offs else w[0]
+    status, out, L = core.new_status(DEV), torch.zeros(M, N, device=DEV), tc.lib()
+    L.moe_tc_set_wait_test.argtypes, L.moe_tc_set_wait_test.restype = [ctypes.c_int, ctypes.c_uint], None
+    L.moe_tc_set_pair(1)
+    L.moe_tc_set_wait_test(fault, 2000)
+    try:
+        assert tc.gemm_tc(x, w, out, status=status, **args)
+        torch.cuda.synchronize()
+    finally:
+        L.moe_tc_set_wait_test(0, 0)
+    assert int(status[0]) & 8, "the wait that ran out was not reported"
+    with pytest.raises(core.KernelError) as e:
+        core.check_status(status)
+    assert "pairs of CTAs" in str(e.value)
+    for _ in range(3):
+        assert tc.gemm_tc(x, w, out, status=status, **args)
+    torch.cuda.synchronize()
+    core.check_status(status)
+    assert float((out - ref).abs().max()) < 2e-2 * float(ref.abs().max())
