@@ -186,13 +186,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
-__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
-                                                 uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
-        : "memory");
-}
 // D[256, N] (+)= A[256, 16] B[N, 16]^T over the pair: each CTA holds 128 rows of A and N / 2 rows of B
 // at the same shared-memory offsets, and gets its 128 rows of D in its own tensor memory.
 __device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -949,8 +942,7 @@ template <int BN, int MODE>
 __global__ void __launch_bounds__(P_THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
     using C = PairCfg<BN, MODE>;
-    // features of a tile (two CTAs of 128 weight rows; with gate and up rows interleaved, 64 features each)
-    constexpr int PAIR_W = MODE == MODE_SWIGLU_IL ? TILE_W : 2 * TILE_W;
+    constexpr int PAIR_W = 2 * TILE_W;
     extern __shared__ uint8_t smem_raw[];
     __shared__ volatile int s_abort;
     __shared__ int s_issued;                        // stages this CTA's producer has asked for
@@ -1033,10 +1025,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                     const uint32_t st = base + s * C::STAGE_BYTES;
                     const uint32_t bar = mapa_cluster(full_bar(s), 0);
                     if (rank == 0) mbar_expect_tx(full_bar(s), 2 * cta_tx);
-                    if (MODE == MODE_SWIGLU_IL)
-                        tma_load_5d_pair(st, &tmW, kb * BK, 0, 0, t.n0 / 16 + (int)rank * 4, t.g, bar);
-                    else
-                        tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
+                    tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
                     if (MODE == MODE_SWIGLU) tma_load_2d_pair(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, bar);
                     for (int c = 0; c < xchunks; c++)
                         tma_load_2d_pair(st + C::NW * C::W_BYTES + c * C::XBOX * BK * 2, &tmX, kb * BK,
@@ -1054,7 +1043,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             for (int item = pair; item < items && ok && p.test_fault != 2; item += pairs, local++) {
                 const Tile t = tile_of<BN, PAIR_W>(item, m_tiles, p, s_prefix, s_offs);
                 const int n_eff = min(BN, (min(BN, t.row_end - t.row0) + 31) & ~31);
-                const uint32_t idesc = instr_desc(n_eff, 2 * TILE_W);
+                const uint32_t idesc = instr_desc(n_eff, PAIR_W);
                 const int b = local & 1;
                 ok = mbar_wait(acc_empty(b), ((local >> 1) & 1) ^ 1, &s_abort, p.wait_limit, p.status, 0x33);   // both epilogues have drained it
                 if (!ok) break;
@@ -1095,12 +1084,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             const uint32_t taddr = tmem + b * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
             const int rows_here = min(BN, t.row_end - t.row0);
             const int part = ((rows_here + 32 * EPI_GROUPS - 1) / (32 * EPI_GROUPS)) * 32;
-            if (MODE == MODE_SWIGLU_IL)
-                epilogue_part_il<BN>(p, taddr, t.n0 + (int)rank * (TILE_W / 2) + q * 16 + (lane & 15), (lane & 16) != 0, t.row0,
-                                     t.row_end, min(rows_here, h * part), min(rows_here, (h + 1) * part));
-            else
-                epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
-                                        min(rows_here, h * part), min(rows_here, (h + 1) * part));
+            epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
+                                    min(rows_here, h * part), min(rows_here, (h + 1) * part));
             // this warp has read its part of the buffer; the issuer waits for all epilogue warps of the pair
             tc_fence_before();
             __syncwarp();
@@ -1235,6 +1220,18 @@ int launch_persistent(const CUtensorMap& tmW, const CUtensorMap& tmX, const Para
 int g_pair = -1;      // 1 / 0: pairs of CTAs for every persistent product / for none; -1: by size (moe_gemm_tc)
 int g_swiglu_il = 1;
 
+// Pairs of CTAs on tiles of 256 features bring half of the activations' bytes into every SM's shared memory.  Measured in
+// turn, us, single / pair: qkv (6,144 x 2,048) at 2,048 tokens 55 / 53, 3,072 75 / 71, 4,096 109 / 101, 8,192 177 / 161; output
+// projection (2,048 x 2,048) 22.6 / 23.4, 37.6 / 37.3, 39.2 / 38.9, 66 / 62; shared down (5,632 -> 2,048) 49 / 49, 89 / 86, 90 / 86, 166 /
+// 148; 60 experts' down product at 137, 205, 256, 320, 546 rows an expert 82 / 80, 102 / 95, 129 / 119, 140 / 136, 247 / 230, 64 wider ones
+// 285 / 282, 318 / 289, 399 / 376, 479 / 491, 742 / 731.  SwiGLU products, whose gate and up rows share a tile, gain nothing: the shared
+// expert's 123 / 126, 159 / 164, 307 / 318, 60 experts' 239 / 248 at 256 rows and 444 / 467 at 546.  A prompt of 8,192 tokens:
+// 13.77 ms without pairs, 13.35 with, 13.47 with SwiGLU pairs too.
+bool takes_pairs(int M, int num_groups, int mode) {       // num_groups: 0 for a product without groups
+    if (g_pair >= 0) return g_pair > 0;
+    return mode != MODE_SWIGLU && (num_groups ? M / num_groups >= 256 : M >= 3072);
+}
+
 template <int BN, int MODE>
 int launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const Params& p, int max_items, cudaStream_t stream) {
     using C = PairCfg<BN, MODE>;
@@ -1295,27 +1292,11 @@ MOE_API int moe_gemm_tc(const void* X, int ldx, const void* W, int num_groups, i
         const int mt = group_offsets ? (M < num_groups ? M : num_groups) + M / pbn : (M + pbn - 1) / pbn;
         const long long max_items = (long long)mt * ((N + TILE_W - 1) / TILE_W);
         const int cap = max_items > (1 << 30) ? (1 << 30) : (int)max_items;
-        // Pairs of CTAs on tiles of 256 features bring half of the activations' bytes into every SM's shared memory.  Measured,
-        // us, single / pair: qkv (6,144 x 2,048) at 2,048 tokens 49.3 / 49.0, 3,072 65 / 62, 4,096 91 / 85, 8,192 172 / 156; the
-        // shared expert's gate and up 84 / 87, 121 / 124, 156 / 155, 300 / 290; 60 experts' gate and up (four a token) 145 / 147, 168 /
-        // 166, 248 / 250, 408 / 391, their down product 83.5 / 82.3, 95 / 91, 133 / 130, 223 / 204.
-        const int each = group_offsets ? M / num_groups : M;
-        const bool pair = g_pair > 0 || (g_pair < 0 && (group_offsets ? each >= 256 : each >= (mode == MODE_SWIGLU ? 4096 : 3072)));
+        const bool pair = takes_pairs(M, group_offsets ? num_groups : 0, mode);
         if (pair && sm_count() >= 2) {
             const long long pair_items = (long long)mt * ((N + 2 * TILE_W - 1) / (2 * TILE_W));
             const int pcap = pair_items > (1 << 30) ? (1 << 30) : (int)pair_items;
-            if (mode == MODE_SWIGLU) {
-                CUtensorMap tmG;
-                if (g_swiglu_il && make_map_gate_up(&tmG, W, (uint64_t)num_groups, (uint64_t)N, (uint64_t)K)) {
-                    const int ibn = bn >= 256 ? 256 : 128;
-                    const int imt = group_offsets ? (M < num_groups ? M : num_groups) + M / ibn : (M + ibn - 1) / ibn;
-                    const long long il_items = (long long)imt * ((N + TILE_W - 1) / TILE_W);
-                    const int icap = il_items > (1 << 30) ? (1 << 30) : (int)il_items;
-                    if (ibn == 256) return launch_pair<256, MODE_SWIGLU_IL>(tmG, tmX, p, icap, stream);
-                    return launch_pair<128, MODE_SWIGLU_IL>(tmG, tmX, p, icap, stream);
-                }
-                return launch_pair<128, MODE_SWIGLU>(tmW, tmX, p, pcap, stream);
-            }
+            if (mode == MODE_SWIGLU) return launch_pair<128, MODE_SWIGLU>(tmW, tmX, p, pcap, stream);
             if (act) return pbn == 128 ? launch_pair<128, MODE_ACT>(tmW, tmX, p, pcap, stream) : launch_pair<256, MODE_ACT>(tmW, tmX, p, pcap, stream);
             if (pbn == 128) return launch_pair<128, MODE_PLAIN>(tmW, tmX, p, pcap, stream);
             return launch_pair<256, MODE_PLAIN>(tmW, tmX, p, pcap, stream);
@@ -1375,6 +1356,9 @@ MOE_API void moe_tc_set_wait_test(int fault, unsigned wait_limit) {
 
 // Pairs of CTAs (cta_group::2) for every persistent product (1), for none (0), or by size (-1, the default).
 MOE_API void moe_tc_set_pair(int enabled) { g_pair = enabled < 0 ? -1 : enabled ? 1 : 0; }
+
+// Whether a persistent product of M rows (in num_groups groups; 0: none) runs on pairs of CTAs.
+MOE_API int moe_gemm_tc_pairs(int M, int num_groups, int mode) { return takes_pairs(M, num_groups, mode) ? 1 : 0; }
 
 // How many K splits the kernel will really use for (K, splits asked), and its grid.y for tickets.
 MOE_API int moe_gemm_tc_plan(int K, int splits, int M, int bn, int num_groups, int grouped, int* grid_y) {
