@@ -20,12 +20,14 @@ def _use_tc(rt, a: torch.Tensor, w: torch.Tensor) -> bool:
 
 def linear(rt, a: torch.Tensor, w: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
            out_dtype: torch.dtype = torch.float32, beside: bool = False) -> torch.Tensor:
-    """a: [M, K]; w: [N, K]; returns [M, N] in ``out_dtype``.  ``beside``: see ``tc.gemm_tc``."""
+    """a: [M, K]; w: [N, K]; returns [M, N] in ``out_dtype``.  ``beside``: see ``tc.gemm_tc``; so, from 257 rows on, on the runtime
+    of a branch (``Runtime.beside``): the other branch wants the SMs that the splits would fill"""
     out = torch.empty((a.shape[0], w.shape[0]), dtype=out_dtype, device=a.device)
     if _use_tc(rt, a, w):
         from . import tc
 
-        if tc.gemm_tc(a, w, out, bias=bias, status=rt.status, beside=beside):
+        if tc.gemm_tc(a, w, out, bias=bias, status=rt.status,
+                      beside=beside or (getattr(rt, "forked", False) and a.shape[0] > 256)):
             return out
     core.gemm_generic(a, w, out, bias=bias, status=rt.status)
     return out

@@ -23,6 +23,7 @@ A pending delta may be a ``LazyDelta``; ``delta_for(norm, delta, rt)`` gives wha
 """
 from __future__ import annotations
 
+import copy
 from dataclasses import dataclass
 from typing import Callable, Dict, Optional, Tuple
 
@@ -113,6 +114,8 @@ class Runtime:
             raise ValueError("compute dtype must be float32 or bfloat16")
         self.device = torch.device(device)
         self.compute_dtype = compute_dtype
+        self.forked = False            # see ``beside``
+        self._sides = {}
         self.status = None
         if self.device.type == "cuda":
             from ..ops import core
@@ -126,8 +129,6 @@ class Runtime:
     def side_stream(self, index: int = 0) -> "torch.cuda.Stream":
         """A further stream of this runtime, for a branch that may run beside the main one (``index``
         tells several apart: a branch that itself forks takes another number)."""
-        if getattr(self, "_sides", None) is None:
-            self._sides = {}
         if index not in self._sides:
             from ..ops import tc
 
@@ -136,6 +137,13 @@ class Runtime:
             self._sides[index] = torch.cuda.Stream(device=self.device)
             tc.register_side_stream(self._sides[index])     # its products get a split-K workspace of their own
         return self._sides[index]
+
+    def beside(self) -> "Runtime":
+        """This runtime for the parts of two branches that run beside one another: the same device, status and streams, but
+        products of more than 256 rows do not spread over all SMs, which the other branch wants too (``ops.linear.linear``)."""
+        rt = copy.copy(self)           # (the streams' dict is shared)
+        rt.forked = True
+        return rt
 
     def empty(self, shape, dtype=None) -> torch.Tensor:
         return torch.empty(shape, dtype=dtype or self.compute_dtype, device=self.device)

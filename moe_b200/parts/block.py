@@ -174,11 +174,11 @@ class ParallelBlock:
             # the two sublayers share nothing but the stream they read: the feed-forward runs on a second
             # stream beside the mixer (inside a captured step: a fork and a join)
             main = torch.cuda.current_stream()
-            side = rt.side_stream(2)
+            side, forked = rt.side_stream(2), rt.beside()
             side.wait_stream(main)
             with torch.cuda.stream(side):
-                b = self.ffn.forward(rt, h2, batch)
-            a = self.mixer.forward(rt, h, batch, cache_view, state)
+                b = self.ffn.forward(forked, h2, batch)
+            a = self.mixer.forward(forked, h, batch, cache_view, state)
             main.wait_stream(side)
             b.record_stream(main)
             return x, ScaledPairDelta(a, self._factor(rt, self.scale1, a), b, self._factor(rt, self.scale2, a))

@@ -670,6 +670,7 @@ class SideBySideMixer(Part):
         if self.beside and h.act.is_cuda:
             main = torch.cuda.current_stream()
             side = rt.side_stream(1)
+            rt = rt.beside()
             side.wait_stream(main)
             with torch.cuda.stream(side):
                 b = right.forward(rt, h, batch, views[1], states[1])

@@ -136,3 +136,30 @@ def test_the_shared_experts_product_keeps_to_few_sms_only_beside_others(on_a_sid
         eng.step([slot], [[1] * n], check=True)
         eng.release(slot)
     assert set(seen) == {(256, on_a_side_stream), (512, False)}
+
+
+def test_branches_beside_one_another_do_not_spread_over_all_sms(monkeypatch):
+    """The two mixers of a layer run side by side: from 257 rows on their products keep to the SMs they need.  The other layers' do not."""
+    import kulanex_util
+    import moe_b200
+    from moe_b200.ops import tc
+
+    cfg = {"architecture": "Kulanex", "vocab": 64, "width": 128, "norm": {"eps": 1e-5}, "residual_mult": 0.5,
+           "layers": [kulanex_util.layer(kulanex_util.parallel(2, 1, 64, 3, 16, size=64, keep=5, rheads=2, rdim=16, rvdim=32), 0),
+                      kulanex_util.layer(kulanex_util.delta(2, 2, 16, 32, 4), 0)]}
+    model = moe_b200.random_model(cfg, seed=0, dtype="bfloat16", device=DEV)
+    product, seen = tc.gemm_tc, []
+
+    def spy(x, w, out, **k):
+        seen.append((x.shape[0], bool(k.get("beside"))))
+        return product(x, w, out, **k)
+
+    monkeypatch.setattr(tc, "gemm_tc", spy)
+    eng = moe_b200.Engine(model, max_tokens=2048, max_slots=2)
+    for n, rows, marked in ((200, 256, False), (300, 512, True)):
+        seen.clear()
+        slot = eng.new_sequence()
+        eng.step([slot], [[1] * n], check=True)
+        eng.release(slot)
+        of_rows = [b for r, b in seen if r == rows]
+        assert any(of_rows) == marked and not all(of_rows), (n, seen)
