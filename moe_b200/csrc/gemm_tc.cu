@@ -1355,7 +1355,12 @@ MOE_API void moe_tc_set_wait_test(int fault, unsigned wait_limit) {
 }
 
 // Pairs of CTAs (cta_group::2) for every persistent product (1), for none (0), or by size (-1, the default).
-MOE_API void moe_tc_set_pair(int enabled) { g_pair = enabled < 0 ? -1 : enabled ? 1 : 0; }
+// Returns what was set before.
+MOE_API int moe_tc_set_pair(int enabled) {
+    const int before = g_pair;
+    g_pair = enabled < 0 ? -1 : enabled ? 1 : 0;
+    return before;
+}
 
 // Whether a persistent product of M rows (in num_groups groups; 0: none) runs on pairs of CTAs.
 MOE_API int moe_gemm_tc_pairs(int M, int num_groups, int mode) { return takes_pairs(M, num_groups, mode) ? 1 : 0; }

@@ -54,7 +54,7 @@ def lib():
         if os.environ.get("MOE_B200_SWIGLU_IL", "1") == "0":    # many tokens: SwiGLU with two accumulators
             L.moe_tc_set_swiglu_interleaved(0)
         L.moe_tc_set_pair.argtypes = [c_int]
-        L.moe_tc_set_pair.restype = None
+        L.moe_tc_set_pair.restype = c_int
         if os.environ.get("MOE_B200_PAIR"):     # pairs of CTAs (cta_group::2) for all products of many tokens, or none
             L.moe_tc_set_pair(1 if os.environ["MOE_B200_PAIR"] == "1" else 0)
         _lib = L

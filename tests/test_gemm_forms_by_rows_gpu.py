@@ -12,9 +12,9 @@ DEV = "cuda:0"
 def tc():
     from moe_b200.ops import tc as t
 
-    t.lib().moe_tc_set_pair(-1)
+    before = t.lib().moe_tc_set_pair(-1)
     yield t
-    t.lib().moe_tc_set_pair(0)
+    t.lib().moe_tc_set_pair(before)
 
 
 def bound(x, w):
@@ -163,3 +163,21 @@ def test_branches_beside_one_another_do_not_spread_over_all_sms(monkeypatch):
         eng.release(slot)
         of_rows = [b for r, b in seen if r == rows]
         assert any(of_rows) == marked and not all(of_rows), (n, seen)
+
+
+def test_a_prompt_of_more_than_4096_tokens_is_the_same_with_and_without_pairs(tc):
+    """A whole step under the default rule: a pair's products add the same terms in the same order."""
+    import moe_b200
+
+    cfg = dict(architectures=["Qwen2MoeForCausalLM"], model_type="qwen2_moe", num_hidden_layers=2, hidden_size=256, num_attention_heads=2,
+               num_key_value_heads=2, head_dim=128, num_experts=4, num_experts_per_tok=2, moe_intermediate_size=128,
+               shared_expert_intermediate_size=512, norm_topk_prob=False, decoder_sparse_step=1, intermediate_size=16, vocab_size=128)
+    model = moe_b200.random_model(cfg, seed=0, dtype="bfloat16", device=DEV)
+    eng = moe_b200.Engine(model, max_tokens=5120, max_slots=2)
+    logits = []
+    for pairs in (-1, 0):
+        tc.lib().moe_tc_set_pair(pairs)
+        slot = eng.new_sequence()
+        logits.append(eng.step([slot], [[(i * 7 + 3) % 128 for i in range(4300)]], check=True).clone())
+        eng.release(slot)
+    assert torch.equal(*logits) and bool(logits[0].isfinite().all())

@@ -23,10 +23,10 @@ def pairing(request, tc):
     """Many tokens take pairs of CTAs on tiles of 256 features (cta_group::2), or, switched off, one
     CTA per tile; SwiGLU for many tokens has one accumulator (gate and up rows interleaved by the
     loads) or, switched off, two: every test runs all ways."""
-    tc.lib().moe_tc_set_pair(1 if request.param == "pairs" else 0)
+    before = tc.lib().moe_tc_set_pair(1 if request.param == "pairs" else 0)
     tc.lib().moe_tc_set_swiglu_interleaved(0 if request.param == "two-accumulators" else 1)
     yield
-    tc.lib().moe_tc_set_pair(0)
+    tc.lib().moe_tc_set_pair(before)
     tc.lib().moe_tc_set_swiglu_interleaved(1)
 
 
@@ -177,7 +177,7 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_product_is_right(fault, t
     status = core.new_status(DEV)
     out = torch.zeros(tokens, N, device=DEV)
     L = tc.lib()
-    L.moe_tc_set_pair(0)                        # (the form on pairs of CTAs, off by default, has no such switch)
+    L.moe_tc_set_pair(0)                        # (pairs of CTAs have a test of their own below)
     L.moe_tc_set_wait_test.argtypes = [ctypes.c_int, ctypes.c_uint]
     L.moe_tc_set_wait_test.restype = None
     L.moe_tc_set_wait_test(fault, 2000)
