@@ -73,7 +73,8 @@ def test_grouped_rows_gathered(core, counts):
 
 @pytest.mark.parametrize("hd,nh,nkv", [(128, 2, 1), (64, 3, 3)])
 @pytest.mark.parametrize("before,new", [([0, 0], [128, 129]), ([5, 300], [257, 130]), ([64], [511]), ([1000, 0, 127], [150, 260, 128])])
-@pytest.mark.parametrize("opt", [{}, {"window": 100}, {"window": 130, "keep": 70}, {"chunk": 96, "softcap": 5.0}, {"sink": True}])
+@pytest.mark.parametrize("opt", [{}, {"window": 100}, {"window": 130, "keep": 70}, {"chunk": 96, "softcap": 5.0}, {"sink": True},
+                                 {"sigmoid": True}, {"sigmoid": True, "chunk": 96}])
 def test_attention_of_many_new_tokens(core, hd, nh, nkv, before, new, opt):
     from moe_b200.cache import KVCache, KVRequest
 
@@ -97,9 +98,10 @@ def test_attention_of_many_new_tokens(core, hd, nh, nkv, before, new, opt):
         G.give_pages(cache, slots[i], before[i] + new[i])
     batch = G.make_batch(DEV, slots, before, new)
     q, kn, vn = torch.cat(Q).contiguous(), *(torch.cat([x[i][before[i]:] for i in range(B)]).contiguous() for x in (K, V))
-    out = torch.full((q.shape[0], nh * hd), float("nan"), device=DEV)
+    out, bias = torch.full((q.shape[0], nh * hd), float("nan"), device=DEV), torch.randn(nh, device=DEV)
+    sink = core.SigmoidWeights(bias) if opt.get("sigmoid") else opt.get("sink", False)
     assert core.attention_tiled(q, kn, vn, view, batch, out, nh=nh, window=window, scale=hd ** -0.5, use_local=True, status=st,
-                                chunk=chunk, softcap=cap, sink=opt.get("sink", False), keep=keep)
+                                chunk=chunk, softcap=cap, sink=sink, keep=keep)
     at = 0
     for i in range(B):
         n, T = new[i], before[i] + new[i]
@@ -115,10 +117,13 @@ def test_attention_of_many_new_tokens(core, hd, nh, nkv, before, new, opt):
             s = s.masked_fill(~seen, -math.inf)
             if opt.get("sink"):
                 s = torch.cat([s, torch.zeros(n, 1, dtype=s.dtype, device=DEV)], 1)
-            ref = torch.softmax(s, -1)[:, :T] @ V[i][:, h // (nh // nkv)].double()
+            weights = torch.sigmoid(s + bias[h].double()) if opt.get("sigmoid") else torch.softmax(s, -1)[:, :T]
+            values = V[i][:, h // (nh // nkv)].double()
+            ref, size = weights @ values, (weights @ values.abs()).clamp(min=1.0) if opt.get("sigmoid") else 1.0
             got = out[at:at + n, h * hd:(h + 1) * hd].double()
-            # scores of up to about 30 are off by 128 half units at most, so a weight is by 30 * 128 * 2^-24 of itself
-            assert float((got - ref).abs().max()) < 3e-4, (i, h)
+            # scores of up to about 30 are off by 128 half units at most, so a weight is by 30 * 128 * 2^-24 of itself (sigmoid
+            # weights do not sum to 1: an output is off by that part of its terms)
+            assert float(((got - ref).abs() / size).max()) < 3e-4, (i, h)
         at += n
     assert int(st[0]) == 0
 
@@ -479,3 +484,60 @@ def test_a_value_reaches_no_query_of_another_tile_that_does_not_see_it(core, hd,
             clean += 1
             assert torch.equal(outs[1][r0:r0 + 64], outs[0][r0:r0 + 64]) and torch.equal(outs[2][r0:r0 + 64], outs[0][r0:r0 + 64]), r0
     assert clean > 0 and not bool(outs[1].isfinite().all()) and bool(outs[0].isfinite().all()) and int(st[0]) == 0
+
+
+def form(core, M, N, K, groups=0):
+    import ctypes
+
+    out = (ctypes.c_int * 5)()
+    core.lib().moe_gemm_plan(M, N, K, groups, ctypes.addressof(out))
+    return list(out)             # rows a tile of the form for few rows (or 0), rows a tile, K splits, chunks a split, rows a pass
+
+
+# one size for every form on 148 SMs: (rows a tile, with K splits or not, chunks a split more than one or not)
+@pytest.mark.parametrize("M,N,K,tile,split,several", [
+    (4921, 6145, 2052, 128, False, True), (4920, 2048, 2048, 64, False, True), (640, 6144, 2048, 128, False, True),
+    (512, 2048, 5632, 128, True, True), (200, 2048, 2048, 128, True, False), (100, 6145, 2052, 128, True, True),
+    (300, 2048, 2048, 64, True, True), (40, 6144, 2048, 64, True, False), (400, 2049, 2044, 32, True, True),
+    (17, 11264, 2048, 32, True, False), (1152, 2047, 5632, 64, True, True)])
+def test_every_tile_form_gives_the_same_bits(core, M, N, K, tile, split, several):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        rows, t, splits, per, _ = form(core, M, N, K)
+        assert rows == 0 and (t, splits > 1, per > 1) == (tile, split, several), (t, splits, per)
+    torch.manual_seed(M + N)
+    a, w, b, st = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.randn(N, device=DEV), core.new_status(DEV)
+    out = torch.full((M + 1, N), float("nan"), device=DEV)
+    core.gemm_generic(a, w, out[:M], bias=b, status=st)
+    assert bool(out[M].isnan().all())
+    some = torch.tensor(sorted({0, 1, 31, 32, 63, 64, 127, 128, M // 2, M - 2, M - 1} & set(range(M))), device=DEV)
+    ref = a[some].double() @ w.double().T + b.double()
+    assert bool(((out[some].double() - ref).abs() <= bound(a[some], w) + 2 * EPS * ref.abs()).all())
+    few = torch.empty(1, N, device=DEV)
+    for r in some.tolist():
+        core.gemm_generic(a[r:r + 1], w, few, bias=b, status=st)
+        assert torch.equal(few, out[r:r + 1]), r
+    assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("G,each,N,K,tile,splits", [(24, 20, 1284, 516, 32, 3), (24, 24, 1284, 516, 64, 2), (24, 40, 1410, 516, 64, 1),
+                                                    (24, 90, 1284, 772, 128, 1), (60, 40, 2816, 516, 32, 1), (24, 600, 1284, 516, 128, 1)])
+def test_every_tile_form_of_many_groups(core, G, each, N, K, tile, splits):
+    """Several hundred blocks and more; groups of unequal size, empty ones among them."""
+    counts = [0 if g % 7 == 3 else each + (g * 37) % (each + 1) - each // 2 for g in range(G)]
+    M = sum(counts)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert form(core, M, N, K, G)[:3] == [0, tile, splits], form(core, M, N, K, G)
+    torch.manual_seed(G + each)
+    a, w, st = torch.randn(M, K, device=DEV), torch.randn(G, N, K, device=DEV), core.new_status(DEV)
+    offs = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int32, device=DEV)
+    out, few = torch.full((M + 1, N), float("nan"), device=DEV), torch.empty(1, N, device=DEV)
+    core.gemm_generic(a, w, out[:M], group_offsets=offs, status=st)
+    assert bool(out[M].isnan().all())
+    for g in range(0, G, max(1, G // 8)):
+        if counts[g]:
+            x = a[offs[g]:offs[g + 1]]
+            assert bool(((out[offs[g]:offs[g + 1]].double() - x.double() @ w[g].double().T).abs() <= bound(x, w[g])).all()), g
+            for r in {0, counts[g] // 2, counts[g] - 1}:
+                core.gemm_generic(x[r:r + 1], w[g], few, status=st)
+                assert torch.equal(few[0], out[int(offs[g]) + r]), (g, r)
+    assert int(st[0]) == 0
