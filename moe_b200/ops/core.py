@@ -1587,13 +1587,13 @@ def delta_step(qkv, step, state, gate, norm_w, norm_eps, batch, out, *, heads, k
 
 
 def _delta_chunks(T, num_seqs, heads, dv) -> bool:
-    """Whether the scan goes over chunks: with 128 tokens a sequence or more on average, where its blocks (16 columns of a head
-    and sequence) find an SM each.  The chain of a chunk is then short; with more blocks the multiply-adds count, of which a chunk
+    """Whether the scan goes over chunks: with 160 tokens a sequence or more on average, where its blocks (16 columns of a head
+    and sequence) find an SM each.  (A step of 65 to 128 tokens is padded to 128 rows; at 66 it is 2 % slower over chunks, at 128 1 % faster.)  The chain of a chunk is then short; with more blocks the multiply-adds count, of which a chunk
     has more, and a step of few tokens need not pay for a second launch.  Measured, us, chunks / four at a time, 16 heads of 128 x
     128, a decay a channel: one sequence of 16, 64, 128, 2,048 tokens 15 / 7, 23 / 21, 30 / 40, 316 / 595 (a decay a head: 16 / 6, 23 / 18, 30 /
     33, 316 / 500); two sequences of 128 and 2,048 39 / 44, 525 / 662; three 62 / 61, 819 / 914; four 74 / 61, 1,039 / 912.  8 heads of 64 x
     64, four sequences of 64, 128, 2,048: 19 / 18, 24 / 33, 298 / 496."""
-    return T >= 128 * num_seqs and -(-dv // 16) * heads * num_seqs <= lib().moe_scan_sms()
+    return T >= 160 * num_seqs and -(-dv // 16) * heads * num_seqs <= lib().moe_scan_sms()
 
 
 def delta_scan(qkv, step, state, batch, o, *, heads, kv_heads, d, dv, offset=0, decay=None, chunks=None):

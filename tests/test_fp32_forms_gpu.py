@@ -361,7 +361,7 @@ def test_short_steps_of_the_delta_rule_keep_the_form_of_four(core, monkeypatch):
     H, d, dv = 16, 128, 128
     asked, L = [], core.lib()
     monkeypatch.setattr(core, "lib", lambda: type("Spy", (), {"__getattr__": lambda _, name: (asked.append(name), getattr(L, name))[1]})())
-    for B, n, over_chunks in ((1, 2, False), (1, 64, False), (2, 200, False), (1, 128, True)):
+    for B, n, over_chunks in ((1, 2, False), (1, 64, False), (1, 128, False), (2, 200, False), (1, 160, True)):
         qkv, step = torch.zeros(B * n, 2 * H * d + H * dv, device=DEV), torch.zeros(B * n, 2 * H, device=DEV)
         state, o = torch.zeros(B + 1, H * d * dv, device=DEV), torch.empty(B * n, H * dv, device=DEV)
         asked.clear()
