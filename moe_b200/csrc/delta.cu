@@ -12,9 +12,12 @@
 //   delta_step      one token a sequence: the recurrence with the state read once and written once, and
 //                   the output's norm and gate behind it, a block a (head, sequence).
 //   delta_scan      several tokens a sequence, four at a time, the state in registers.
+//   delta_chunk, delta_chunk_scan   the same for few long sequences: chunks of sixteen tokens, first what needs no state for
+//                   all of them side by side, then the state's way through them.
 // The decay g is one number a value head, or one a value head and key channel (the rows of S then shrink each by their
 // own): delta_prepare forms those from a product's rows of their own, g = exp(-exp(A_log_h) softplus(a + dt_bias)).
-// Everything here is 32-bit arithmetic; only the normed, gated output of delta_step is rounded.
+// Everything here is 32-bit arithmetic (delta_chunk's in 64 bits, its results in 32); only the normed, gated output of delta_step
+// is rounded.
 #include "common.cuh"
 
 namespace {

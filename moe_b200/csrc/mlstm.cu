@@ -9,9 +9,12 @@
 //   mlstm_gates   a, b and e^(-m) of every token, and the sequences' m moved on: a block a (head, sequence), a token a
 //                 thread (the pairs (lf, li) compose as m -> max(lf + m, li), an associative operation).
 //   mlstm_scan    several tokens a sequence, four at a time, state and normaliser in registers.
+//   mlstm_chunk_add, _state, _out   the same for few long sequences: chunks of sixty-four tokens side by side, only the state's
+//                   way through them a chain.
 //   mlstm_step    one token a sequence: gates, recurrence with the state read once and written once, and the output's
 //                 norm and gate behind it, a block a (head, sequence).
-// Everything is 32-bit arithmetic; only the normed, gated output of mlstm_step is rounded.
+// Everything is 32-bit arithmetic (but for mlstm_chunk_out's pair products and n . q, sums in 64 bits); only the normed, gated output
+// of mlstm_step is rounded.
 #include <type_traits>
 
 #include "common.cuh"

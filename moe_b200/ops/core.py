@@ -1459,7 +1459,8 @@ def _forced_segments() -> int:
 
 
 def scan_segments(batch, blocks_per_sequence: int, device) -> int:
-    """Into how many segments a sequence's tokens are cut for ``ssd_scan``, ``wkv_scan`` and ``mlstm_scan``: one where the launch fills
+    """Into how many segments a sequence's tokens are cut for ``ssd_scan``, ``wkv_scan`` and ``mlstm_scan`` (there where it does not go
+    over chunks): one where the launch fills
     the GPU anyway or the sequences are short; else enough to fill it, of at least 128 tokens each, eight
     at most.  (``MOE_B200_SCAN_SEGMENTS``: 0 this rule, n > 0 that many.)"""
     forced = _forced_segments()

@@ -362,9 +362,10 @@ class RoutedExperts(Part):
 
     def _shared(self, rt, h, beside=True):
         # ``beside``: on a side stream, beside the routed products; else it runs alone.
-        # (up to 256 rows the down product keeps to few SMs: it runs beside the routed products, which want the others; cut into
-        # pieces for all of them a step of three prompts, 145 tokens, took 1,867 instead of 1,795 us.  At 512 rows it is the
-        # longer of the two branches: 2,353 against 2,211 us a step.)
+        # (up to 256 rows the down product keeps to few SMs: it runs beside the routed products, which want the others.  Measured, us a
+        # step, few SMs / cut into pieces for all of them: 128 rows 1,850 / 1,929 (6 layers, 60 experts of 1,408, width 2,048), 978 / 1,019
+        # and 1,298 / 1,353 (32 experts of 704 and 1,408, widths 2,048 and 4,096); 256 rows 1,070 / 1,168 and 1,503 / 1,509 there,
+        # though 2,270 / 2,105 with the 60 experts.  At 512 rows it is the longer of the two branches: 2,353 against 2,211.)
         return linear(rt, swiglu_linear(rt, h.act, self.ws_gu), self.ws_down, beside=beside and h.act.shape[0] <= 256)
 
     def forward(self, rt, h, batch):
