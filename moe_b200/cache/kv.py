@@ -21,6 +21,7 @@ from typing import Dict, List, Optional, Tuple
 
 import torch
 
+from ..ops import core
 from .allocator import PAGE_TOKENS, CacheError, CacheLedger
 
 
@@ -149,8 +150,12 @@ class KVCache:
     # ---- slots -----------------------------------------------------------------
     def acquire(self) -> int:
         s = self.ledger.acquire()
-        for t in self._states.values():
-            t[s].zero_()
+        rows = [t[s] for t in self._states.values()]
+        if rows and rows[0].is_cuda:
+            core.clear_rows(rows)
+        else:
+            for row in rows:
+                row.zero_()
         return s
 
     def release(self, slot: int) -> None:

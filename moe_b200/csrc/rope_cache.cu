@@ -229,6 +229,25 @@ __global__ void table_update_kernel(int* __restrict__ table, int stride, const i
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) table[(size_t)upd[3 * i] * stride + upd[3 * i + 1]] = upd[3 * i + 2];
 }
+
+// The state of a new sequence: its rows in the layers' state buffers become zero, all of them in one launch (a launch a layer
+// cost 4 us each while a batch of requests is taken in).  grid (pieces of 16 KB of the longest row, rows).
+constexpr int CLEAR_ROWS = 32, CLEAR_PIECE = 16384;
+struct ClearRows {
+    unsigned char* row[CLEAR_ROWS];
+    long long bytes[CLEAR_ROWS];
+};
+__global__ void __launch_bounds__(256) clear_rows_kernel(const ClearRows p) {
+    pdl_sync();
+    unsigned char* row = p.row[blockIdx.y];
+    const long long from = (long long)blockIdx.x * CLEAR_PIECE, to = min(p.bytes[blockIdx.y], from + CLEAR_PIECE);
+    if ((((uintptr_t)row | (uintptr_t)p.bytes[blockIdx.y]) & 15) == 0) {
+        for (long long i = from + 16 * threadIdx.x; i < to; i += 16 * 256) *reinterpret_cast<uint4*>(row + i) = make_uint4(0, 0, 0, 0);
+    } else {
+        for (long long i = from + threadIdx.x; i < to; i += 256) row[i] = 0;
+    }
+}
+
 // A decode step (one token per sequence): rotate, write the query, and append key and value
 // straight into the cache, in one launch.  Same arithmetic as rope_split_kernel followed by
 // kv_commit_kernel.  One block per token.
@@ -312,4 +331,23 @@ MOE_API int moe_rope_commit(const float* qkv, const int* pos, const float* inv_f
 MOE_API int moe_table_update(int* table, int stride, const int* upd, int n, cudaStream_t stream) {
     if (n <= 0) return 0;
     return launch_pdl(table_update_kernel, (n + 127) / 128, 128, 0, stream, table, stride, upd, n);
+}
+
+// rows[i] points to bytes[i] bytes on the device (host arrays); all of them become zero.
+MOE_API int moe_clear_rows(void* const* rows, const long long* bytes, int n, cudaStream_t stream) {
+    for (int at = 0; at < n; at += CLEAR_ROWS) {
+        ClearRows p = {};
+        const int here = n - at < CLEAR_ROWS ? n - at : CLEAR_ROWS;
+        long long longest = 0;
+        for (int i = 0; i < here; i++) {
+            p.row[i] = (unsigned char*)rows[at + i], p.bytes[i] = bytes[at + i];
+            if (bytes[at + i] > longest) longest = bytes[at + i];
+        }
+        const long long pieces = (longest + CLEAR_PIECE - 1) / CLEAR_PIECE;
+        if (pieces <= 0) continue;
+        if (pieces > 0x7fffffffll) return (int)cudaErrorInvalidValue;
+        const int code = launch_pdl(clear_rows_kernel, dim3((unsigned)pieces, here), 256, 0, stream, p);
+        if (code) return code;
+    }
+    return 0;
 }

@@ -77,6 +77,7 @@ def lib():
             "moe_logprobs": [P, I, I, P, I, P, P, P, P],
             "moe_seed_rng": [P, P, P, I, P],
             "moe_table_update": [P, I, P, I, P],
+            "moe_clear_rows": [P, P, I, P],
             "moe_whole_prepare": [P, I, P, P, P, P, F, P, I, P, I, I, I, I, I, I, P, P, P, LL, LL, I, P, P, P, P, P, I, I, I, I,
                                   I, P, P],
             "moe_whole_conv_prepare": [P, I, P, I, P, LL, I, P, P, P, P, P, P, F, P, I, I, I, I, I, I, I, I, I, P, P, P, LL, LL,
@@ -1146,6 +1147,18 @@ def table_update(table, updates, n):
     if updates.numel() < 3 * n:
         raise KernelError("table_update: updates too short")
     _ok(lib().moe_table_update(_p(table), table.stride(0), _p(updates), n, _stream()), "table_update")
+
+
+def clear_rows(rows):
+    """Every tensor of ``rows`` (contiguous, of any type) becomes zero, all in one launch (32 to a launch)."""
+    rows = [t for t in rows if t.numel()]
+    if not rows:
+        return
+    for t in rows:
+        _chk(t, "clear_rows")
+    n = len(rows)
+    _ok(lib().moe_clear_rows((c_void_p * n)(*[t.data_ptr() for t in rows]),
+                             (c_longlong * n)(*[t.numel() * t.element_size() for t in rows]), n, _stream()), "clear_rows")
 
 
 def rope_commit(qkv, pos, inv_freq, nh, nkv, hd, rot, q, view, batch, status):
