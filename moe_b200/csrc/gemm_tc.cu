@@ -43,6 +43,7 @@ constexpr int BK = 64;        // K elements per stage = one 128-byte swizzle row
 constexpr int UMMA_K = 16;
 constexpr int MAX_SMEM_GROUPS = 256;
 constexpr int MAX_SPLITS = 16;
+constexpr int MAX_CLUSTER = 8;   // portable cluster size
 
 // MODE_SWIGLU_IL (persistent form only): gate and up rows of the same 16 features alternate within a
 // 128-row weight tile (see gemm_tc_persistent_kernel), so that SwiGLU needs ONE accumulator.
@@ -70,6 +71,7 @@ struct Params {
     int kb_per_split;
     int cluster;                // 1: the splits of a tile are one cluster and add up through shared memory
     int early_offsets;          // 1: group_offsets were written at least two kernels ago (see the kernel)
+    int late_dependents;        // 1: the successor is let onto the SMs when this kernel has asked for its last stage, not at its start
     float* partials;            // [splits][M][cols] float32, cols = N or 2 N (not with cluster)
     int* tickets;               // one per (grid.y, grid.x), zero before and after the launch
     int* status;
@@ -133,11 +135,39 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
         : "memory");
 }
+// The same with a say in what stays in L2.  Weights that one CTA reads once go first: a step streams more of them than L2 holds, and
+// what it pushes out otherwise are activations, the small weights and the kernels' instructions, which the chain of small kernels waits for.
+// (us a step of 6 layers, without / with: one sequence 509 / 478, eight 970 / 954, sixty-four 1,922 / 1,884, prompts of 113 tokens 1,675 / 1,635.)
+__device__ __forceinline__ uint64_t l2_policy(bool read_once) {
+    uint64_t first, normal;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+    return read_once ? first : normal;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar), "l"(policy)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
+                                            uint32_t bar, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar), "l"(policy)
+        : "memory");
+}
 // ---- thread-block clusters (the K splits of one tile) ----
 __device__ __forceinline__ uint32_t cluster_ctarank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
+}
+// (the same in two halves)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -277,18 +307,137 @@ struct Cfg {
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : (STAGES_RAW < 2 ? 2 : STAGES_RAW);
     static constexpr int TMEM_COLS_RAW = NW * BN;
     static constexpr int TMEM_COLS = TMEM_COLS_RAW < 32 ? 32 : TMEM_COLS_RAW;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
+    // Where a cluster's other K splits put their rows of the partial tile (see cluster_epilogue).  Room for eight tokens (SwiGLU, with two numbers
+    // a feature: for one to three) and no more: with two CTAs on an SM the small kernels of the chain must still fit beside them.
+    static constexpr int ROW_BYTES = NW * TILE_W * 4;
+    static constexpr int RECV_BYTES = BN > 64 ? 0 : MODE == MODE_SWIGLU ? 3 * 1024 : 4 * 1024;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + RECV_BYTES;
     // the partial tile of a K split fits in the (then free) pipeline stages
     static constexpr bool CLUSTER_OK = NW * BN * TILE_W * 4 <= STAGES * STAGE_BYTES;
 };
 
+// The end of a K split's CTA of a cluster, for tiles of few rows, by the four epilogue warps: rows t = r, r + S, ... of the tile belong to the
+// split of rank r; every CTA writes the others' rows of its partial tile into their shared memory (recv: distributed stores, one barrier, and
+// nobody reads a peer's memory, so nobody waits to leave), keeps its own (in the pipeline stages, which are free by then) and adds its rows
+// up in split order.  The loop goes through the additions once BEFORE the accumulator is ready, on whatever lies there and without storing:
+// that brings the instructions to the SM while the main loop runs (read for the first time behind the barrier they took 1 - 2 us).  A step of one
+// sequence, 6 layers: 478 us, 488 where every CTA reads its peers' memory instead.
+// false: the wait for the accumulator ran out (the barriers are passed all the same).
+template <int BN, int MODE>
+__device__ __forceinline__ bool cluster_epilogue(const Params& p, uint32_t base, float* stage, const float* recv, uint32_t tmem, uint32_t acc_bar,
+                                                 volatile int* s_abort, int n0, int row0, int rows_here, int quarter, int lane) {
+    using C = Cfg<BN, MODE>;
+    constexpr int NW = C::NW, ROW = NW * TILE_W;
+    const int S = p.splits, rank = (int)cluster_ctarank(), f = quarter * 32 + lane, n = n0 + f;
+    const float bias = (plain_mode(MODE) && p.bias && n < p.N) ? p.bias[n] : 0.f;
+    bool ok = true;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        int real;
+        asm volatile("mov.u32 %0, %1;" : "=r"(real) : "r"(pass));      // (or the first pass is found to have no effect and dropped)
+        if (real) {
+            ok = mbar_wait(acc_bar, 0, s_abort, p.wait_limit, p.status, 0x15);
+            __syncwarp();
+            cluster_wait();                                            // every CTA of the cluster runs
+            if (ok) {
+                tc_fence_after();
+                const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16), mine = smem_u32(recv);
+                int owner = 0, slot = 0;
+                for (int c0 = 0; c0 < rows_here; c0 += 16) {
+                    float a[16], b[16];
+                    __syncwarp();
+                    tmem_ld16(taddr + c0, a);
+                    if (MODE == MODE_SWIGLU) tmem_ld16(taddr + BN + c0, b);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        if (c0 + j >= rows_here) break;
+                        if (owner == rank) {
+                            stage[(c0 + j) * ROW + f] = a[j];
+                            if (MODE == MODE_SWIGLU) stage[(c0 + j) * ROW + TILE_W + f] = b[j];
+                        } else {
+                            const uint32_t at = mapa_cluster(mine, owner) + (uint32_t)((slot * (S - 1) + (rank < owner ? rank : rank - 1)) * ROW + f) * 4u;
+                            st_cluster_f32(at, a[j]);
+                            if (MODE == MODE_SWIGLU) st_cluster_f32(at + TILE_W * 4u, b[j]);
+                        }
+                        if (++owner == S) owner = 0, slot++;
+                    }
+                }
+            }
+            __syncwarp();
+            cluster_arrive();
+            cluster_wait();
+        }
+        for (int i = 0, t = rank; t < rows_here || !real; i++, t += S) {
+            float sa = 0.f, sb = 0.f;
+#pragma unroll
+            for (int s = 0; s < MAX_CLUSTER; s++) {
+                if (s >= S) break;
+                const float* src = (s == rank ? stage + t * ROW : recv + (i * (S - 1) + (s < rank ? s : s - 1)) * ROW) + f;
+                sa += src[0];
+                if (MODE == MODE_SWIGLU) sb += src[TILE_W];
+            }
+            const float v = MODE == MODE_SWIGLU ? glu_mul(p.act, p.act_param, sa, sb) : plain_out<MODE>(p.act, sa + bias);
+            if (real && ok && n < p.N) {
+                if (p.out_bf16)
+                    ((__nv_bfloat16*)p.out)[(size_t)(row0 + t) * p.ldo + n] = __float2bfloat16_rn(v);
+                else
+                    ((float*)p.out)[(size_t)(row0 + t) * p.ldo + n] = v;
+            }
+            if (!real) break;
+        }
+    }
+    return ok;
+}
+
+
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
+// Tile `tile` of bn rows in order of groups: (group, its first row, end of the group's rows), group -1 for none.  By one warp,
+// 32 groups at a time (one thread that walked the offsets took 20 - 25 cycles a group: a microsecond for 60 experts, in front
+// of the first load).
+struct GroupTile {
+    int g, row0, row_end, first;     // first: the group's first row
+};
+__device__ __forceinline__ GroupTile find_group_tile(const int* offsets, int num_groups, int tile, int bn, int M, int lane) {
+    GroupTile t{-1, 0, 0, 0};
+    if (!offsets) {
+        if (tile * bn < M) t.g = 0, t.row0 = tile * bn, t.row_end = M;
+        return t;
+    }
+    int before = 0;                                    // tiles of the groups already passed
+    for (int g0 = 0; g0 < num_groups; g0 += 32) {
+        const int g = g0 + lane;
+        const int b = g < num_groups ? offsets[g] : 0, e = g < num_groups ? offsets[g + 1] : 0;
+        const int tiles = (e - b + bn - 1) / bn;
+        int upto = tiles;                              // tiles up to and with this lane's group
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += n;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, tile < before + upto);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            t.row0 = __shfl_sync(0xffffffffu, b + (tile - before - (upto - tiles)) * bn, l);
+            t.row_end = __shfl_sync(0xffffffffu, e, l);
+            t.first = __shfl_sync(0xffffffffu, b, l);
+            t.g = g0 + l;
+            return t;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return t;
+}
 
 template <int BN, int MODE>
-__global__ void __launch_bounds__(192)
+__global__ void __launch_bounds__(192, 3)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
     using C = Cfg<BN, MODE>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_work[4];          // group, first row, end row, is_last
+    __shared__ int s_once;             // this tile holds all rows of its group: nobody else reads its weights
     __shared__ volatile int s_abort;
     __shared__ uint32_t s_tmem;
 
@@ -304,62 +453,49 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     // experts: its offsets were written before the first) may do the same.
     const bool grouped = p.group_offsets != nullptr;
     const bool wait_first = grouped && !p.early_offsets;
-    if (wait_first) pdl_sync();
 
-    // ---- which rows of X this CTA owns -------------------------------------------------
-    // (the offsets are fetched by all threads at once: a scan straight from global memory would
-    // pay one memory latency per group)
-    __shared__ int s_offs[MAX_SMEM_GROUPS + 1];
-    const bool offs_in_smem = p.group_offsets && p.num_groups <= MAX_SMEM_GROUPS;
-    if (offs_in_smem) {
-        for (int i = threadIdx.x; i <= p.num_groups; i += blockDim.x) s_offs[i] = p.group_offsets[i];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        int g = 0, r0 = 0, r1 = p.M, tile = blockIdx.y;
-        if (p.group_offsets) {
-            g = -1;
-            const int* offs = offs_in_smem ? s_offs : p.group_offsets;
-            for (int i = 0; i < p.num_groups; i++) {
-                const int b = offs[i], e = offs[i + 1];
-                const int tiles = (e - b + BN - 1) / BN;
-                if (tile < tiles) {
-                    g = i, r0 = b + tile * BN, r1 = e;
-                    break;
-                }
-                tile -= tiles;
-            }
-        } else {
-            r0 = tile * BN;
-            if (r0 >= p.M) g = -1;
-        }
-        s_work[0] = g, s_work[1] = r0, s_work[2] = r1, s_work[3] = 0;
-        s_abort = 0;
-    }
-    __syncthreads();
-    const int g = s_work[0];
-    if (g < 0) return;                 // uniform: nothing to do for this tile index
-    const int row0 = s_work[1], row_end = s_work[2];
-
+    // What hangs on nobody comes before the wait: the descriptors of the two operands, and the barriers.
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar_base = base + C::STAGES * C::STAGE_BYTES;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };
     const uint32_t acc_bar = bar_base + 8u * (2 * C::STAGES);
-
     if (threadIdx.x == 0) {
+        prefetch_map(&tmW);
+        prefetch_map(&tmX);
         for (int s = 0; s < C::STAGES; s++) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
         mbar_init(acc_bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    if (wait_first) {
+        pdl_wait();
+        if (!p.late_dependents) pdl_launch_dependents();
     }
     if (warp == 1) tmem_alloc(smem_u32(&s_tmem), C::TMEM_COLS);
+
+    // ---- which rows of X this CTA owns -------------------------------------------------
+    if (warp == 0) {
+        const GroupTile t = find_group_tile(p.group_offsets, p.num_groups, blockIdx.y, BN, p.M, lane);
+        if (lane == 0) s_work[0] = t.g, s_work[1] = t.row0, s_work[2] = t.row_end, s_work[3] = 0, s_once = t.row_end - t.first <= BN;
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    const int g = s_work[0];
+    if (g < 0) {                       // uniform (and the same in a whole cluster): nothing to do for this tile index
+        if (warp == 1) tmem_dealloc(tmem, C::TMEM_COLS);
+        return;
+    }
+    const int row0 = s_work[1], row_end = s_work[2];
+    // few rows in a cluster: see cluster_epilogue
+    const int rows_tile = min(BN, row_end - row0);
+    const bool push = p.cluster && (p.splits - 1) * ((rows_tile + p.splits - 1) / p.splits) * C::ROW_BYTES <= C::RECV_BYTES;
+    if (push) cluster_arrive();
 
     const int kb_total = (p.K + BK - 1) / BK;
     const int kb0 = split * p.kb_per_split;
@@ -379,11 +515,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     if (warp == 0) {
         // ---- producer ---------------------------------------------------------------------
         if (lane == 0) {
+            const uint64_t policy = l2_policy(s_once != 0);
             int issued = 0;
             bool ok = true;
             int kb_next = kb0;
             if (p.test_fault == 1) {
-                if (!wait_first) pdl_sync();
+                if (!wait_first) pdl_wait();
                 kb_next = kb1;                   // the wait test: nothing is loaded, the MMA issuer's wait runs out
             } else if (!wait_first) {
                 // weight tiles of the first stages, then wait for the predecessor, then their activations
@@ -391,10 +528,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                 for (int i = 0; i < pre; i++) {
                     const uint32_t st = base + i * C::STAGE_BYTES;
                     mbar_expect_tx(full_bar(i), stage_tx);
-                    tma_load_2d(st, &tmW, (kb0 + i) * BK, w_row, full_bar(i));
-                    if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, (kb0 + i) * BK, w_row + p.N, full_bar(i));
+                    tma_load_2d(st, &tmW, (kb0 + i) * BK, w_row, full_bar(i), policy);
+                    if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, (kb0 + i) * BK, w_row + p.N, full_bar(i), policy);
                 }
-                pdl_sync();
+                pdl_wait();
+                if (!p.late_dependents) pdl_launch_dependents();
                 for (int i = 0; i < pre; i++) load_x(base + i * C::STAGE_BYTES, kb0 + i, full_bar(i));
                 issued = pre;
                 kb_next = kb0 + pre;
@@ -406,10 +544,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                 if (!ok) break;
                 const uint32_t st = base + s * C::STAGE_BYTES;
                 mbar_expect_tx(full_bar(s), stage_tx);
-                tma_load_2d(st, &tmW, kb * BK, w_row, full_bar(s));
-                if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, full_bar(s));
+                tma_load_2d(st, &tmW, kb * BK, w_row, full_bar(s), policy);
+                if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, full_bar(s), policy);
                 load_x(st, kb, full_bar(s));
             }
+            pdl_launch_dependents();             // (a second time it does nothing)
             if (!ok) {
                 atomicOr(p.status, ST_WAIT_TIMEOUT);
                 s_abort = 1;
@@ -449,6 +588,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                 atomicOr(p.status, ST_WAIT_TIMEOUT);
                 s_abort = 1;
             }
+        }
+    } else if (push) {
+        uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
+        if (!cluster_epilogue<BN, MODE>(p, base, reinterpret_cast<float*>(aligned), reinterpret_cast<const float*>(aligned + C::STAGES * C::STAGE_BYTES + 256),
+                                        tmem, acc_bar, &s_abort, n0, row0, rows_tile, warp & 3, lane) && lane == 0) {
+            atomicOr(p.status, ST_WAIT_TIMEOUT);
+            s_abort = 1;
         }
     } else {
         // ---- epilogue -----------------------------------------------------------------------
@@ -574,9 +720,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
             }
         }
     }
+    if (push && warp < 2) {                            // (the epilogue warps pass the cluster's barriers on their way)
+        __syncwarp();
+        cluster_wait();
+        cluster_arrive();
+        cluster_wait();
+    }
     tc_fence_before();
     __syncthreads();
-    if (p.cluster) {
+    if (p.cluster && !push) {
         // Every thread of every CTA of the cluster comes here (all waits above are bounded), so the
         // two cluster barriers always complete.  Between them CTA r adds, for the rows r, r + S, ...
         // of the tile, the S partial values in split order (reading its peers' shared memory) and
@@ -713,6 +865,7 @@ struct PCfg {
 
 struct Tile {
     int g, row0, row_end, n0;
+    bool once;               // the tile holds all rows of its group: its weights are read once
 };
 
 // item -> tile.  prefix[i]: token tiles of the groups before i (grouped), in shared memory.
@@ -722,7 +875,7 @@ __device__ __forceinline__ Tile tile_of(int item, int m_tiles, const Params& p, 
     if (!p.group_offsets) {
         // all token tiles of one feature tile first: CTAs running together share weight tiles in L2
         const int nt = item / m_tiles, m = item % m_tiles;
-        t.n0 = nt * TW, t.g = 0, t.row0 = m * BN, t.row_end = p.M;
+        t.n0 = nt * TW, t.g = 0, t.row0 = m * BN, t.row_end = p.M, t.once = p.M <= BN;
         return t;
     }
     // grouped: all feature tiles of one token tile first.  A group's weights are read once anyway;
@@ -735,7 +888,7 @@ __device__ __forceinline__ Tile tile_of(int item, int m_tiles, const Params& p, 
         const int mid = (lo + hi) >> 1;
         if (prefix[mid] <= m) lo = mid; else hi = mid;
     }
-    t.g = lo, t.row0 = offs[lo] + (m - prefix[lo]) * BN, t.row_end = offs[lo + 1];
+    t.g = lo, t.row0 = offs[lo] + (m - prefix[lo]) * BN, t.row_end = offs[lo + 1], t.once = t.row_end - offs[lo] <= BN;
     return t;
 }
 
@@ -807,6 +960,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
                 const int xchunks = (n_eff + C::XBOX - 1) / C::XBOX;
                 const uint32_t stage_tx = C::NW * C::W_BYTES + xchunks * C::XBOX * BK * 2;
                 const int w_row = t.g * p.w_rows_per_group + t.n0;
+                const uint64_t policy = l2_policy(t.once);
                 for (int kb = 0; kb < kbs; kb++, issued++) {
                     const int s = issued % C::STAGES;
                     ok = mbar_wait(empty_bar(s), ((issued / C::STAGES) & 1) ^ 1, &s_abort, p.wait_limit, p.status, 0x21);
@@ -816,11 +970,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
                     if (MODE == MODE_SWIGLU_IL) {
                         // tmW is five-dimensional here, (k, row of 16, gate|up, block of 16 features, group):
                         // one box is four times [16 gate rows, the 16 up rows of the same features]
-                        tma_load_5d(st, &tmW, kb * BK, 0, 0, t.n0 / 16, t.g, full_bar(s));
+                        tma_load_5d(st, &tmW, kb * BK, 0, 0, t.n0 / 16, t.g, full_bar(s), policy);
                     } else {
-                        tma_load_2d(st, &tmW, kb * BK, w_row, full_bar(s));
+                        tma_load_2d(st, &tmW, kb * BK, w_row, full_bar(s), policy);
                     }
-                    if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, full_bar(s));
+                    if (MODE == MODE_SWIGLU) tma_load_2d(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, full_bar(s), policy);
                     for (int c = 0; c < xchunks; c++)
                         tma_load_2d(st + C::NW * C::W_BYTES + c * C::XBOX * BK * 2, &tmX, kb * BK,
                                     t.row0 + c * C::XBOX, full_bar(s));
@@ -1170,8 +1324,6 @@ bool make_map_gate_up(CUtensorMap* map, const void* ptr, uint64_t groups, uint64
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-constexpr int MAX_CLUSTER = 8;   // portable cluster size
-
 template <int BN, int MODE>
 int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, Params p, dim3 grid, cudaStream_t stream) {
     using C = Cfg<BN, MODE>;
@@ -1280,6 +1432,9 @@ MOE_API int moe_gemm_tc(const void* X, int ldx, const void* W, int num_groups, i
     splits = (kb_total + per - 1) / per;
     Params p;
     p.cluster = 0, p.early_offsets = (group_offsets && early_offsets) ? 1 : 0;
+    // The routed experts' first product: its successor's CTAs, let in at its start, took the places of the shared expert's, which run beside it.
+    // (us a step, 6 layers, late / at the start: one sequence 509 / 511, eight 907 / 924.)
+    p.late_dependents = mode == MODE_SWIGLU && group_offsets && !early_offsets;
     p.out = out, p.out_bf16 = out_bf16, p.ldo = ldo, p.bias = bias, p.group_offsets = group_offsets;
     p.num_groups = num_groups, p.M = M, p.N = N, p.K = K, p.w_rows_per_group = w_rows, p.splits = splits;
     p.kb_per_split = per, p.partials = partials, p.tickets = tickets, p.status = status;

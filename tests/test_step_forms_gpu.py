@@ -1,4 +1,6 @@
-"""The kernels and forms of a step that a size or a pitch picks, at the sizes where they meet."""
+"""The kernels and forms of a step that a size or a pitch picks, at the sizes where they meet: clearing a new sequence's state, a grouped
+product's search for its rows, the fused norm and router with several blocks a token, the norm that leaves three terms, rows gathered from a
+pitch, the router's logits, the delta rule's preparation over runs of tokens, and queries, keys and values in one product."""
 from __future__ import annotations
 
 import pytest
@@ -39,3 +41,23 @@ def test_a_slot_used_again_starts_with_a_clear_state():
     for i in range(3):
         t = cache.state(i).float()
         assert float(t[b].abs().sum()) == 0.0 and int((t == 1).sum()) == t.numel() - t[b].numel()
+
+
+@pytest.mark.parametrize("groups", [1, 31, 33, 70, 300])
+def test_a_grouped_product_finds_its_rows_among_any_number_of_groups(groups):
+    """Few rows a group, empty groups among them, tiles that end inside a group; in one CTA a tile and on persistent CTAs."""
+    from moe_b200.ops import core as c, tc
+
+    torch.manual_seed(groups)
+    counts = [0 if g % 5 == 2 else 1 + (g * 7) % 23 for g in range(groups)]
+    offs = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    M, K, N = sum(counts), 136, 72
+    x, w, st = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(groups, N, K, device=DEV).bfloat16(), c.new_status(DEV)
+    ref = torch.cat([x[int(offs[g]):int(offs[g + 1])].double() @ w[g].double().T for g in range(groups)])
+    for bn in (16, 32, 128):
+        for early in (False, True):
+            out = torch.full((M, N), float("nan"), device=DEV)
+            assert tc.gemm_tc(x, w, out, group_offsets=offs, bn=bn, splits=1, status=st, early_offsets=early)
+            # 136 products of bfloat16 numbers of size 1, added in 32 bits
+            assert float((out.double() - ref).abs().max()) < 136 * 8 * 2.0 ** -23 * 8, (bn, early)
+    assert int(st[0]) == 0
