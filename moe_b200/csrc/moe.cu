@@ -298,18 +298,18 @@ __device__ __forceinline__ void route_token(const float* __restrict__ lg, float*
     }
     float wsum = 0.f;
     for (int j = 0; j < top_k; j++) {
+        // Scores are >= 0 and so ordered as their bit patterns; the best one and, among equals, the lowest expert are one
+        // warp-wide reduction each (five rounds of two shuffles took 250 cycles a pick).
         float best = -1.f;
         int bi = 0x7fffffff;
         for (int e = lane; e < num_experts; e += 32) {
             const float v = sc[e];
             if (v > best) best = v, bi = e;   // ascending e: first maximum kept
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) best = ob, bi = oi;
-        }
+        const unsigned key = best >= 0.f ? __float_as_uint(best + 0.f) + 1u : 0u;      // 0: no score at all (taken, or NaN)
+        const unsigned top = __reduce_max_sync(0xffffffffu, key);
+        bi = (int)__reduce_min_sync(0xffffffffu, key == top ? (unsigned)bi : 0x7fffffffu);
+        best = top ? __uint_as_float(top - 1u) : -1.f;
         if (bi < 0 || bi >= num_experts) bi = j % num_experts;   // only with NaN scores
         const float w = fmaxf(best, 0.f);
         wsum += w;
@@ -556,10 +556,10 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const int* __res
 }
 
 // Few tokens (a decode step): the norm before the feed-forward, the router and the dispatch in
-// ONE launch.  A block per token adds the pending delta to the stream, normalises the row
-// (as rmsnorm_kernel), forms the token's router logits from the 32-bit normalised row in shared
+// ONE launch, in two forms.  norm_route_kernel (9 tokens and more): a block per token adds the pending delta to the stream, normalises
+// the row (as rmsnorm_kernel), forms the token's router logits from the 32-bit normalised row in shared
 // memory (one warp per router row) and picks its experts; the block that finishes last inverts
-// the table and gathers the picked tokens' activations (as route_dispatch_kernel).
+// the table and gathers the picked tokens' activations (as route_dispatch_kernel).  norm_route_cluster_kernel: up to 8 tokens.
 int g_norm_route_cluster = 1;
 
 struct NormRouteParams {
@@ -586,7 +586,7 @@ struct NormRouteParams {
     int* ticket;              // one int, zero before and after
     int* status;
     int vec_ok;
-    int cluster;              // 1: the tokens' blocks are one cluster (at most 8 tokens), see the kernel
+    int per_token;            // cluster form: blocks a token
     int groups, keep;         // experts picked within the best `keep` of `groups` groups (0: no groups)
     // A norm on what is pending instead of a norm in front of the router (post_w not null; norm_w is then not read):
     // x += rms(delta sa + delta_b sb) post_w, and the router reads the stream itself.
@@ -597,28 +597,240 @@ struct NormRouteParams {
     int weight_input;         // the gathered rows are multiplied by their pick's weight
 };
 
+// Asks for the router's weights (the `blocks` blocks share its lines among them) and the norm's in L2: they do not hang on the predecessor.
+template <typename WT>
+__device__ __forceinline__ void prefetch_router(const NormRouteParams& p, int block, int blocks, const float* norm_w) {
+    const size_t line = 128, w_bytes = (size_t)p.num_experts * p.hidden * sizeof(WT);
+    for (size_t off = ((size_t)block * blockDim.x + threadIdx.x) * line; off < w_bytes; off += (size_t)blocks * blockDim.x * line)
+        prefetch_l2((const char*)p.wr + off);
+    for (size_t off = threadIdx.x * line; off < (size_t)p.hidden * sizeof(float); off += blockDim.x * line)
+        prefetch_l2((const char*)norm_w + off);
+    if (p.wsg)
+        for (size_t off = threadIdx.x * line; off < (size_t)p.hidden * sizeof(WT); off += blockDim.x * line)
+            prefetch_l2((const char*)p.wsg + off);
+}
+
+__device__ __forceinline__ void router_add8(const float* x, const float* wv, float& sum) {
+    const float4 a = *reinterpret_cast<const float4*>(x), b = *reinterpret_cast<const float4*>(x + 4);
+    sum = fmaf(a.x, wv[0], sum), sum = fmaf(a.y, wv[1], sum), sum = fmaf(a.z, wv[2], sum);
+    sum = fmaf(a.w, wv[3], sum), sum = fmaf(b.x, wv[4], sum), sum = fmaf(b.y, wv[5], sum);
+    sum = fmaf(b.z, wv[6], sum), sum = fmaf(b.w, wv[7], sum);
+}
+// The products of the 32-bit row with router rows r = first, first + step, ..., handed to out(r, v) by the whole warp: one warp a row, 32-bit
+// products and sums in an order that hangs on H alone.  (A warp takes two rows at a time, so that the loads of both are in flight together.)
+template <typename WT, typename Out>
+__device__ __forceinline__ void router_rows(const NormRouteParams& p, const float* row, int first, int step, int lane, Out out) {
+    const int H = p.hidden, E = p.num_experts, groups = p.vec_ok ? H / 8 : 0;
+    for (int r = first; r < p.rows; r += 2 * step) {
+        const int r2 = r + step;
+        const bool two = r2 < p.rows;
+        const WT* w = r < E ? (const WT*)p.wr + (size_t)r * H : (const WT*)p.wsg;
+        const WT* w2 = !two ? w : (r2 < E ? (const WT*)p.wr + (size_t)r2 * H : (const WT*)p.wsg);
+        float acc = 0.f, acc2 = 0.f;
+        if (two) {
+#pragma unroll 4
+            for (int gi = lane; gi < groups; gi += 32) {
+                float wv[8], wv2[8];
+                w_load8<WT>(w + gi * 8, wv);
+                w_load8<WT>(w2 + gi * 8, wv2);
+                router_add8(row + gi * 8, wv, acc);
+                router_add8(row + gi * 8, wv2, acc2);
+            }
+        } else {
+#pragma unroll 8
+            for (int gi = lane; gi < groups; gi += 32) {
+                float wv[8];
+                w_load8<WT>(w + gi * 8, wv);
+                router_add8(row + gi * 8, wv, acc);
+            }
+        }
+        for (int c = groups * 8 + lane; c < H; c += 32) {
+            acc = fmaf(row[c], ld_f(w + c), acc);
+            if (two) acc2 = fmaf(row[c], ld_f(w2 + c), acc2);
+        }
+        out(r, warp_sum(acc));
+        if (two) out(r2, warp_sum(acc2));
+    }
+}
+// Up to 8 tokens: ONE cluster of at most 8 blocks.  What bounds it is a chain of trips: between SMs, to L2, and, in code that an SM
+// has not run for a while, to the instructions themselves (the pick of one token, some 1,000 cycles of work, took 3 us).  So
+//  * few tokens: every token has per_token blocks, each of which normalises the row and forms the logits of every per_token-th router row
+//    (the router is 250 KB, and an SM takes in about 110 GB/s: 2.3 us where a token has one block);
+//  * the logits are written into all blocks' shared memory (distributed stores, one barrier; nobody reads a peer's memory, so nobody waits to
+//    leave).  Every block then picks for ALL tokens (a warp each) and counts the places of all pairs for itself, in pair order, so the
+//    result does not depend on timing.  A token's blocks share its gathered rows; block 0 writes the tables;
+//  * where a warp has no router row, it runs the pick once on whatever is there, which brings its instructions to the SM while nothing hangs on them.
+// A step of one / eight sequences, 6 layers: 491 / 922 -> 478 / 915 us.  (512 threads, so that two blocks fit an SM, or the router's rows shared
+// among all blocks for all tokens, each row of the stream sent to every block first: eight sequences 934 to 954.)
 // POST: post_w and what goes with it (a form of its own, so that the other carries nothing of it).
+constexpr int NRC_THREADS = 1024;
+__device__ __noinline__ void route_token_once(const float* lg, float* sc, int lane, bool padding, const NormRouteParams* p, int* idx, float* w,
+                                              float* gate, float* wk) {
+    route_token(lg, sc, lane, padding, p->num_experts, p->rows, p->top_k, p->norm_topk, p->scale, idx, w, gate, wk, nullptr, p->groups, p->keep);
+}
+__device__ __forceinline__ unsigned peer_addr(const void* local, unsigned rank) {
+    unsigned pa;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(pa) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+    return pa;
+}
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 template <typename WT, bool POST>
+__global__ void __launch_bounds__(NRC_THREADS) norm_route_cluster_kernel(const __grid_constant__ NormRouteParams p) {
+    extern __shared__ __align__(16) float nr_smem[];
+    __shared__ float red[32];
+    const int H = p.hidden, E = p.num_experts, T = p.num_tokens, C = p.per_token, B = gridDim.z;
+    const int rank = blockIdx.z, t = rank / C, part = rank % C;                  // (the cluster lies along z)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const int H4 = (H + 3) & ~3, pairs = T * p.top_k;
+    float* row = nr_smem;                              // [H4]
+    float* before = row + H4;                          // [H4]: the stream's row, where several blocks of a token read it and one writes it
+    float* all = before + (C > 1 ? H4 : 0);            // [T][rows]: the logits
+    float* sc = all + T * p.rows;                      // [T][E]
+    float* wk = sc + T * E;                            // [T][top_k]
+    float* w_pick = wk + pairs;                        // [T][top_k]
+    float* gate = w_pick + pairs;                      // [T]
+    int* picks = reinterpret_cast<int*>(gate + T);     // [pairs]
+    int* place = picks + pairs;                        // [pairs]
+    cl_arrive();                                       // (a peer's memory may be written once it runs)
+    const float* norm_w = POST ? p.post_w : p.norm_w;
+    prefetch_router<WT>(p, rank, B, norm_w);
+    constexpr int NV = 4;
+    float nw[NV];                                      // this thread's first weights of the norm
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int j = threadIdx.x + i * blockDim.x;
+        nw[i] = j < H ? norm_w[j] : 0.f;
+    }
+    pdl_sync();
+
+    // ---- the norm --------------------------------------------------------------------------
+    float* xr = p.x + (size_t)t * H;
+    const float* dr = p.delta ? p.delta + (size_t)t * H : nullptr;
+    float ss = 0.f;
+    if (POST) {
+        const float* br = p.delta_b ? p.delta_b + (size_t)t * H : nullptr;
+        for (int j = threadIdx.x; j < H; j += blockDim.x) {
+            float y = p.sa * dr[j];
+            if (br) y = fmaf(p.sb, br[j], y);
+            if (C > 1) before[j] = xr[j];
+            row[j] = y;
+            ss = fmaf(y, y, ss);
+        }
+        ss = block_sum(ss, red);
+        const float rs = 1.0f / sqrtf(ss / (float)H + p.post_eps);
+        auto one = [&](int j, float w) {
+            const float v = fmaf(row[j] * rs, w, C > 1 ? before[j] : xr[j]);
+            if (C == 1) xr[j] = v;
+            row[j] = v;
+        };
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int j = threadIdx.x + i * blockDim.x;
+            if (j < H) one(j, nw[i]);
+        }
+        for (int j = threadIdx.x + NV * blockDim.x; j < H; j += blockDim.x) one(j, norm_w[j]);
+    } else {
+        for (int j = threadIdx.x; j < H; j += blockDim.x) {
+            float v = xr[j];
+            if (dr) {
+                v += dr[j];
+                if (C == 1) xr[j] = v; else before[j] = v;
+            }
+            row[j] = v;
+            ss += v * v;
+        }
+        ss = block_sum(ss, red);
+        const float rs = 1.0f / sqrtf(ss / (float)H + p.eps);
+        auto one = [&](int j, float w) {
+            const float y = row[j] * rs * w;
+            row[j] = y;
+            if (part == 0 && p.out32) p.out32[(size_t)t * H + j] = y;
+            if (part == 0 && p.out16) p.out16[(size_t)t * H + j] = __float2bfloat16_rn(y);
+        };
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int j = threadIdx.x + i * blockDim.x;
+            if (j < H) one(j, nw[i]);
+        }
+        for (int j = threadIdx.x + NV * blockDim.x; j < H; j += blockDim.x) one(j, norm_w[j]);
+    }
+    __syncthreads();
+    cl_wait();
+
+    // ---- the router's logits, into everybody's shared memory ------------------------------------
+    if (warp == nwarps - 1 && warp * C + part >= p.rows)       // (a warp without a router row: see above)
+        route_token_once(all, sc, lane, false, &p, picks, w_pick, gate, wk);
+    router_rows<WT>(p, row, warp * C + part, nwarps * C, lane, [&](int r, float v) {
+        if (lane < B) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_addr(all + t * p.rows + r, (unsigned)lane)), "f"(v) : "memory");
+    });
+    __syncwarp();
+    cl_arrive();
+    cl_wait();                                         // (and all blocks of a token have read its row of the stream)
+    if (warp < T)
+        route_token_once(all + warp * p.rows, sc + warp * E, lane, p.seq_of_token && p.seq_of_token[warp] < 0, &p, picks + warp * p.top_k,
+                         w_pick + warp * p.top_k, p.shared_gate ? gate + warp : nullptr, wk + warp * p.top_k);
+    else if (C > 1 && part == 0 && (POST || dr))       // (one block a token wrote it above)
+        for (int j = threadIdx.x - 32 * T; j < H; j += blockDim.x - 32 * T) xr[j] = POST ? row[j] : before[j];
+    __syncthreads();
+
+    // ---- the table inverted: a pair's place is the number of pairs of lower experts and of earlier pairs of its own --------
+    // (a warp an item: the pairs, then, in block 0, the experts' first places and their end)
+    for (int i = warp; i < pairs + (rank == 0 ? E + 1 : 0); i += nwarps) {
+        const int e = i < pairs ? picks[i] : i - pairs;
+        int n = 0;
+        for (int j = lane; j < pairs; j += 32) n += picks[j] >= 0 && (picks[j] < e || (i < pairs && picks[j] == e && j < i));
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane) continue;
+        if (i >= pairs) {
+            p.offsets[e] = n;
+            continue;
+        }
+        const bool on = e >= 0 && e < E;
+        if (!on && e != -1) atomicOr(p.status, ST_BAD_EXPERT);
+        place[i] = on ? n : -1;
+        if (rank == 0) {
+            p.pos_of_pair[i] = on ? n : -1;
+            if (on) p.sorted_token[n] = i / p.top_k;
+        }
+    }
+    if (part == 0) {
+        for (int j = threadIdx.x; j < p.top_k; j += blockDim.x) {
+            p.topk_idx[(size_t)t * p.top_k + j] = picks[t * p.top_k + j];
+            p.topk_w[(size_t)t * p.top_k + j] = w_pick[t * p.top_k + j];
+        }
+        if (p.shared_gate && threadIdx.x == 0 && (p.rows > E || (p.seq_of_token && p.seq_of_token[t] < 0))) p.shared_gate[t] = gate[t];
+    }
+    __syncthreads();
+    if (rank == 0 && warp == 0) {      // places past the last routed pair: a valid row, never used
+        int total = 0;
+        for (int j = lane; j < pairs; j += 32) total += picks[j] >= 0;
+        total = __reduce_add_sync(0xffffffffu, total);
+        for (int i = total + lane; i < pairs; i += 32) p.sorted_token[i] = 0;
+    }
+    if (p.xs) {
+        const int units = H / 8;                       // (xs comes with rows of whole 16-byte units only)
+        for (int i = threadIdx.x + part * blockDim.x; i < p.top_k * units; i += C * blockDim.x) {
+            const int j = i / units, c = i % units, q = place[t * p.top_k + j];
+            if (q < 0) continue;
+            const float f = (POST && p.weight_input) ? w_pick[t * p.top_k + j] : 1.0f;
+            const float4 a = *reinterpret_cast<const float4*>(row + 8 * c), b = *reinterpret_cast<const float4*>(row + 8 * c + 4);
+            alignas(16) const __nv_bfloat162 v[4] = {__floats2bfloat162_rn(f * a.x, f * a.y), __floats2bfloat162_rn(f * a.z, f * a.w),
+                                                     __floats2bfloat162_rn(f * b.x, f * b.y), __floats2bfloat162_rn(f * b.z, f * b.w)};
+            p.xs[(size_t)q * p.row_units + c] = *reinterpret_cast<const uint4*>(v);
+        }
+    }
+}
+
+template <typename WT>
 __global__ void __launch_bounds__(1024) norm_route_kernel(const NormRouteParams p) {
     extern __shared__ __align__(16) float nr_smem[];
     __shared__ float red[32];
     __shared__ int s_last;
-    __shared__ int s_mine[64];                         // this token's picks, for the other blocks of a cluster
-    const int t = blockIdx.x + blockIdx.z, H = p.hidden, E = p.num_experts;      // (a cluster lies along z)
+    const int t = blockIdx.x, H = p.hidden, E = p.num_experts;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    {
-        // the weights do not depend on the predecessor: they are asked into L2 before the wait
-        // (the blocks share the router's lines among them)
-        const size_t line = 128, w_bytes = (size_t)E * H * sizeof(WT);
-        for (size_t off = ((size_t)t * blockDim.x + threadIdx.x) * line; off < w_bytes;
-             off += (size_t)p.num_tokens * blockDim.x * line)
-            prefetch_l2((const char*)p.wr + off);
-        for (size_t off = threadIdx.x * line; off < (size_t)H * sizeof(float); off += blockDim.x * line)
-            prefetch_l2((const char*)(POST ? p.post_w : p.norm_w) + off);
-        if (p.wsg)
-            for (size_t off = threadIdx.x * line; off < (size_t)H * sizeof(WT); off += blockDim.x * line)
-                prefetch_l2((const char*)p.wsg + off);
-    }
+    prefetch_router<WT>(p, t, p.num_tokens, p.norm_w);
     pdl_sync();
     float* row = nr_smem;                              // [H] (H rounded up to 4)
     float* logit = row + ((H + 3) & ~3);               // [rows]
@@ -633,76 +845,27 @@ __global__ void __launch_bounds__(1024) norm_route_kernel(const NormRouteParams 
     float* xr = p.x + (size_t)t * H;
     const float* dr = p.delta ? p.delta + (size_t)t * H : nullptr;
     float ss = 0.f;
-    if (POST) {
-        const float* br = p.delta_b ? p.delta_b + (size_t)t * H : nullptr;
-        for (int j = threadIdx.x; j < H; j += blockDim.x) {
-            float y = p.sa * dr[j];
-            if (br) y = fmaf(p.sb, br[j], y);
-            row[j] = y;
-            ss = fmaf(y, y, ss);
-        }
-        ss = block_sum(ss, red);
-        const float rs = 1.0f / sqrtf(ss / (float)H + p.post_eps);
-        for (int j = threadIdx.x; j < H; j += blockDim.x) {
-            const float v = fmaf(row[j] * rs, p.post_w[j], xr[j]);
+    for (int j = threadIdx.x; j < H; j += blockDim.x) {
+        float v = xr[j];
+        if (dr) {
+            v += dr[j];
             xr[j] = v;
-            row[j] = v;
         }
-    } else {
-        for (int j = threadIdx.x; j < H; j += blockDim.x) {
-            float v = xr[j];
-            if (dr) {
-                v += dr[j];
-                xr[j] = v;
-            }
-            row[j] = v;
-            ss += v * v;
-        }
-        ss = block_sum(ss, red);
-        const float rs = 1.0f / sqrtf(ss / (float)H + p.eps);
-        for (int j = threadIdx.x; j < H; j += blockDim.x) {
-            const float y = row[j] * rs * p.norm_w[j];
-            row[j] = y;
-            if (p.out32) p.out32[(size_t)t * H + j] = y;
-            if (p.out16) p.out16[(size_t)t * H + j] = __float2bfloat16_rn(y);
-        }
+        row[j] = v;
+        ss += v * v;
+    }
+    ss = block_sum(ss, red);
+    const float rs = 1.0f / sqrtf(ss / (float)H + p.eps);
+    for (int j = threadIdx.x; j < H; j += blockDim.x) {
+        const float y = row[j] * rs * p.norm_w[j];
+        row[j] = y;
+        if (p.out32) p.out32[(size_t)t * H + j] = y;
+        if (p.out16) p.out16[(size_t)t * H + j] = __float2bfloat16_rn(y);
     }
     __syncthreads();
-
-    // ---- router logits: one warp per router row, 32-bit products and sums in a fixed order ----
-    // (a warp takes two rows at a time, so that the loads of both are in flight together)
-    const int groups = p.vec_ok ? H / 8 : 0;
-    for (int r = warp; r < p.rows; r += 2 * nwarps) {
-        const int r2 = r + nwarps;
-        const bool two = r2 < p.rows;
-        const WT* w = r < E ? (const WT*)p.wr + (size_t)r * H : (const WT*)p.wsg;
-        const WT* w2 = !two ? w : (r2 < E ? (const WT*)p.wr + (size_t)r2 * H : (const WT*)p.wsg);
-        float acc = 0.f, acc2 = 0.f;
-#pragma unroll 4
-        for (int gi = lane; gi < groups; gi += 32) {
-            float wv[8], wv2[8];
-            w_load8<WT>(w + gi * 8, wv);
-            w_load8<WT>(w2 + gi * 8, wv2);
-            const float4 a = *reinterpret_cast<const float4*>(row + gi * 8);
-            const float4 b = *reinterpret_cast<const float4*>(row + gi * 8 + 4);
-            acc = fmaf(a.x, wv[0], acc), acc = fmaf(a.y, wv[1], acc), acc = fmaf(a.z, wv[2], acc);
-            acc = fmaf(a.w, wv[3], acc), acc = fmaf(b.x, wv[4], acc), acc = fmaf(b.y, wv[5], acc);
-            acc = fmaf(b.z, wv[6], acc), acc = fmaf(b.w, wv[7], acc);
-            acc2 = fmaf(a.x, wv2[0], acc2), acc2 = fmaf(a.y, wv2[1], acc2), acc2 = fmaf(a.z, wv2[2], acc2);
-            acc2 = fmaf(a.w, wv2[3], acc2), acc2 = fmaf(b.x, wv2[4], acc2), acc2 = fmaf(b.y, wv2[5], acc2);
-            acc2 = fmaf(b.z, wv2[6], acc2), acc2 = fmaf(b.w, wv2[7], acc2);
-        }
-        for (int c = groups * 8 + lane; c < H; c += 32) {
-            acc = fmaf(row[c], ld_f(w + c), acc);
-            acc2 = fmaf(row[c], ld_f(w2 + c), acc2);
-        }
-        acc = warp_sum(acc);
-        acc2 = warp_sum(acc2);
-        if (lane == 0) {
-            logit[r] = acc;
-            if (two) logit[r2] = acc2;
-        }
-    }
+    router_rows<WT>(p, row, warp, nwarps, lane, [&](int r, float v) {
+        if (lane == 0) logit[r] = v;
+    });
     __syncthreads();
 
     // ---- this token's experts ------------------------------------------------------------------
@@ -710,77 +873,6 @@ __global__ void __launch_bounds__(1024) norm_route_kernel(const NormRouteParams 
         route_token(logit, sc, lane, p.seq_of_token && p.seq_of_token[t] < 0, E, p.rows, p.top_k, p.norm_topk, p.scale,
                     p.topk_idx + (size_t)t * p.top_k, p.topk_w + (size_t)t * p.top_k,
                     p.shared_gate ? p.shared_gate + t : nullptr, wk, nullptr, p.groups, p.keep);
-
-    if (p.cluster) {
-        // ---- one cluster: every block learns all picks through distributed shared memory, inverts
-        // the table for itself (in pair order, so the result does not depend on timing) and writes
-        // the gathered rows of ITS token from the row it still holds; block 0 writes the tables
-        __syncthreads();
-        for (int j = threadIdx.x; j < p.top_k; j += blockDim.x) s_mine[j] = p.topk_idx[(size_t)t * p.top_k + j];
-        cl_sync();
-        for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-            picks[i] = (int)cl_peer_u32(&s_mine[i % p.top_k], (unsigned)(i / p.top_k));
-        __syncthreads();
-        for (int e = threadIdx.x; e < E; e += blockDim.x) {
-            int c = 0;
-            for (int i = 0; i < pairs; i++) c += picks[i] == e;
-            counts[e] = c;
-        }
-        for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-            if (picks[i] != -1 && (picks[i] < 0 || picks[i] >= E)) atomicOr(p.status, ST_BAD_EXPERT);
-        __syncthreads();
-        int* start = counts + E;
-        if (warp == 0) {   // exclusive scan of the counts, 32 experts at a time
-            int run = 0;
-            for (int e0 = 0; e0 < E; e0 += 32) {
-                const int e = e0 + lane;
-                const int c = e < E ? counts[e] : 0;
-                int inc = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int n = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += n;
-                }
-                if (e < E) {
-                    start[e] = run + inc - c;
-                    if (t == 0) p.offsets[e] = run + inc - c;
-                }
-                run += __shfl_sync(0xffffffffu, inc, 31);
-            }
-            if (lane == 0) {
-                if (t == 0) p.offsets[E] = run;
-                s_last = run;
-            }
-        }
-        __syncthreads();
-        const int total = s_last;
-        for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-            const int e = picks[i];
-            int q = -1;
-            if (e >= 0 && e < E) {
-                q = start[e];
-                for (int j = 0; j < i; j++) q += picks[j] == e;      // pairs of the same expert before this one
-                if (t == 0) p.sorted_token[q] = i / p.top_k;
-            }
-            sorted[i] = q;                                          // here: the place of pair i
-            if (t == 0) p.pos_of_pair[i] = q;
-        }
-        if (t == 0)
-            for (int i = total + threadIdx.x; i < pairs; i += blockDim.x) p.sorted_token[i] = 0;
-        __syncthreads();
-        if (p.xs) {
-            for (int j = 0; j < p.top_k; j++) {
-                const int q = sorted[t * p.top_k + j];
-                if (q < 0) continue;
-                __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.xs) + (size_t)q * H;
-                const float f = (POST && p.weight_input) ? p.topk_w[(size_t)t * p.top_k + j] : 1.0f;
-                for (int c = threadIdx.x * 2; c < H; c += blockDim.x * 2)
-                    *reinterpret_cast<__nv_bfloat162*>(dst + c) = __floats2bfloat162_rn(f * row[c], f * row[c + 1]);
-            }
-        }
-        cl_sync();      // no block leaves while another may still read its picks
-        return;
-    }
 
     // ---- the block that finishes last inverts the table and gathers ----------------------------
     __threadfence();
@@ -890,19 +982,25 @@ MOE_API int moe_norm_route(float* x, const float* delta, const float* norm_w, fl
     const size_t elt = w_dt == DT_F32 ? 4 : 2;
     p.vec_ok = (hidden % 8 == 0) && ((uintptr_t)wr % 16 == 0) && (!wsg || (uintptr_t)wsg % 16 == 0) &&
                ((hidden * elt) % 16 == 0);
-    const size_t smem = ((size_t)((hidden + 3) & ~3) + p.rows + num_experts + top_k) * sizeof(float) +
-                        ((size_t)2 * pairs + 2 * num_experts) * sizeof(int);
+    // up to 8 tokens: one cluster, no ticket, no second reading of what other blocks wrote
+    const bool cluster = num_tokens <= 8 && top_k <= 64 && hidden % 2 == 0 && g_norm_route_cluster;
+    if (post_w && !cluster) return -1;                       // (the ticket form gathers normed rows only)
+    const size_t row_bytes = (size_t)((hidden + 3) & ~3) * sizeof(float);
+    p.per_token = cluster && row_bytes <= 64 * 1024 ? 8 / num_tokens : 1;
+    const size_t smem = cluster ? (p.per_token > 1 ? 2 : 1) * row_bytes +
+                                      ((size_t)p.rows * num_tokens + (size_t)num_tokens * (num_experts + 1) + 4 * (size_t)pairs) * 4
+                                : row_bytes + ((size_t)p.rows + num_experts + top_k) * sizeof(float) +
+                                      ((size_t)2 * pairs + 2 * num_experts) * sizeof(int);
     if (smem > 200 * 1024) return -1;
-    auto kernel = post_w ? (w_dt == DT_F32 ? norm_route_kernel<float, true> : norm_route_kernel<__nv_bfloat16, true>)
-                         : (w_dt == DT_F32 ? norm_route_kernel<float, false> : norm_route_kernel<__nv_bfloat16, false>);
+    auto kernel = !cluster ? (w_dt == DT_F32 ? norm_route_kernel<float> : norm_route_kernel<__nv_bfloat16>)
+                  : post_w ? (w_dt == DT_F32 ? norm_route_cluster_kernel<float, true> : norm_route_cluster_kernel<__nv_bfloat16, true>)
+                           : (w_dt == DT_F32 ? norm_route_cluster_kernel<float, false> : norm_route_cluster_kernel<__nv_bfloat16, false>);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    // up to 8 tokens: one cluster, no ticket, no second reading of what other blocks wrote
-    p.cluster = (num_tokens <= 8 && top_k <= 64 && hidden % 2 == 0 && g_norm_route_cluster) ? 1 : 0;
-    if (post_w && !p.cluster) return -1;                     // (the ticket form gathers normed rows only)
-    if (p.cluster) return launch_pdl_cluster(kernel, dim3(1, 1, num_tokens), 1024, smem, stream, num_tokens, p);
+    const int blocks = num_tokens * p.per_token;
+    if (cluster) return launch_pdl_cluster(kernel, dim3(1, 1, blocks), NRC_THREADS, smem, stream, blocks, p);
     return launch_pdl(kernel, num_tokens, 1024, smem, stream, p);
 }
 

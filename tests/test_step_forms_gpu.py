@@ -61,3 +61,52 @@ def test_a_grouped_product_finds_its_rows_among_any_number_of_groups(groups):
             # 136 products of bfloat16 numbers of size 1, added in 32 bits
             assert float((out.double() - ref).abs().max()) < 136 * 8 * 2.0 ** -23 * 8, (bn, early)
     assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 7, 8])
+@pytest.mark.parametrize("E,k,H,post", [(61, 4, 2048, False), (16, 2, 2056, True), (256, 8, 4104, False), (3, 3, 40, True)])
+def test_norm_and_router_with_several_blocks_a_token(core, T, E, k, H, post):
+    """Against 64 bits, for every number of blocks a token (eight blocks among the tokens)."""
+    torch.manual_seed(T + E)
+    x0, a, b = (torch.randn(T, H, device=DEV) for _ in range(3))
+    w, wr = 1 + 0.1 * torch.randn(H, device=DEV), (torch.randn(E, H, device=DEV) * H ** -0.5).bfloat16()
+    wsg = None if post else (torch.randn(H, device=DEV) * H ** -0.5).bfloat16()
+    seq, st, x = torch.zeros(T, dtype=torch.int32, device=DEV), core.new_status(DEV), x0.clone()
+    if T > 2:
+        seq[1] = -1
+    if post:
+        res = core.norm_route(x, a, None, 0.0, wr, k, True, 1.0, bf16=True, seq_of_token=seq, status=st, delta_b=b, sa=0.5, sb=0.25,
+                              post=(w, 1e-5), weight_input=True)
+        y = 0.5 * a.double() + 0.25 * b.double()
+        ref = x0.double() + y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * w.double()
+        assert torch.allclose(x.double(), ref, rtol=1e-5, atol=1e-6)
+        row = x
+    else:
+        res = core.norm_route(x, a, w, 1e-5, wr, k, True, 1.0, bf16=True, shared_gate_w=wsg, seq_of_token=seq, status=st)
+        assert torch.equal(x, x0 + a)
+        y = x.double()
+        row = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * w.double()).float()
+        assert float((res[1].float() - row).abs().max()) <= 2.0 ** -8 * float(row.abs().max())
+    out32, out16, idx, wt, sg, offs, sorted_token, pos, xs = res
+    live = (seq >= 0).tolist()
+    probs = torch.softmax(row.double() @ wr.double().T, -1)
+    pairs, want = idx.tolist(), torch.topk(probs, k, -1)
+    flat = [(e, t * k + j) for t in range(T) for j, e in enumerate(pairs[t]) if live[t]]
+    for t in range(T):
+        if not live[t]:
+            assert pairs[t] == [-1] * k and float(wt[t].abs().sum()) == 0.0
+            continue
+        # (a pick of another expert only where the two are as likely to rounding)
+        assert torch.allclose(probs[t][idx[t].long()], want.values[t], rtol=1e-5)
+        ref_w = probs[t][idx[t].long()] / probs[t][idx[t].long()].sum()
+        assert torch.allclose(wt[t].double(), ref_w, rtol=1e-5)
+        if sg is not None:
+            assert abs(float(sg[t]) - float(torch.sigmoid(row[t].double() @ wsg.double()))) < 1e-5
+    order = {p: i for i, (_, p) in enumerate(sorted(flat))}              # places: by expert, then in pair order
+    assert pos.reshape(-1).tolist() == [order.get(p, -1) for p in range(T * k)]
+    assert offs.tolist() == [sum(e < g for e, _ in flat) for g in range(E + 1)]
+    for p, i in order.items():
+        assert int(sorted_token[i]) == p // k
+        src = row[p // k] * (wt.reshape(-1)[p] if post else 1.0)
+        assert float((xs[i].float() - src).abs().max()) <= 2.0 ** -8 * float(src.abs().max())
+    assert int(st[0]) == 0
