@@ -196,6 +196,8 @@ class RoutedExperts(Part):
         # from 16 on, where its single gathering block is the bottleneck
         self.fused_norm_tokens = int(os.environ.get("MOE_B200_NORM_ROUTE_MAX", "8"))
         self.shared_beside = os.environ.get("MOE_B200_SHARED_BESIDE", "1") != "0"
+        # up to this many tokens the shared expert's products start with the router's kernels, not behind them (see _run)
+        self.shared_first_tokens = int(os.environ.get("MOE_B200_SHARED_FIRST", "512"))
         # up to this many tokens one block picks, inverts and gathers (one launch after the logits);
         # beyond, a warp per token picks and the inversion and the gather are launches of their own
         # (measured on a B200, ms a decode step at 16 / 32 / 64 tokens: 4.65 / 5.89 / 7.38 with one
@@ -407,20 +409,71 @@ class RoutedExperts(Part):
 
     def _run(self, rt, h, batch, routed):
         T = h.act.shape[0]
-        P = T * self.k
-        few = T <= 64 and self.E <= 256
-        ys = side = None
-        if self.ws_gu is not None and few:
-            # few tokens: neither branch fills the GPU, so the shared expert runs beside the routed
-            # ones on a second stream (inside a captured graph this becomes a fork and a join)
-            main = torch.cuda.current_stream()
-            side = rt.side_stream()
-            side.wait_stream(main)
+        if self.ws_gu is None:
+            return self._routed(rt, h, batch, routed, self._record)
+        if not (T <= 64 and self.E <= 256) and not (self.shared_beside and rt.is_bf16 and T <= self.shared_first_tokens):
+            # Many tokens: pick, table inversion and gather are small launches that leave the GPU
+            # idle (37 us of a layer at 2,048 tokens), so the shared expert starts beside them on
+            # a second stream.  (Not before the logits' product: the shared expert's CTAs fill every
+            # SM's shared memory, and that product would wait for them to end.)
+            ys = side = None
+
+            def shared_beside():
+                nonlocal ys, side
+                main = torch.cuda.current_stream()
+                side = rt.side_stream()
+                side.wait_stream(main)
+                with torch.cuda.stream(side):
+                    ys = self._shared(rt, h)
+
+            out = self._routed(rt, h, batch, routed, self._record, shared_beside if self.shared_beside else None)
+            if side is None:
+                ys = self._shared(rt, h, beside=False)
+            else:
+                torch.cuda.current_stream().wait_stream(side)
+                ys.record_stream(torch.cuda.current_stream())
+            out.shared = ys
+            return out
+        # Fewer: neither branch fills the GPU, so they run beside one another (inside a captured graph a fork and a join).  In bfloat16 the
+        # shared expert's products follow the norm on the main stream, where a programmatic launch lets them fetch their first weights before
+        # it has ended; what hangs on the picks (and, with 9 tokens and more, the picks themselves) runs on the second.  Measured, us a step
+        # of 6 layers, this way / the shared expert on the second stream: one sequence 465 / 478, eight 914 / 915, sixty-four 1,821 / 1,836.
+        # (In 32 bits, whose products have no such launch, eight sequences take 1,069 / 1,055 us: there it is the shared expert's.)
+        main = torch.cuda.current_stream()
+        side = rt.side_stream()
+        side.wait_stream(main)
+        if not rt.is_bf16:
             with torch.cuda.stream(side):
                 ys = self._shared(rt, h)
+            out = self._routed(rt, h, batch, routed, self._record)
+            main.wait_stream(side)
+            ys.record_stream(main)
+            out.shared = ys
+            return out
+        picks = []
+        with torch.cuda.stream(side):
+            out = self._routed(rt, h, batch, routed, lambda *pair: picks.extend(pair))
+        ys = self._shared(rt, h)
+        main.wait_stream(side)
+        for t in (out.y, out.pos_of_pair, out.shared_gate, *picks):
+            if t is not None:
+                t.record_stream(main)
+        self._record(*picks)
+        out.shared = ys
+        return out
+
+    def _record(self, topk_idx, topk_w):
+        if self.trace is not None:
+            self.trace.append((topk_idx.clone(), topk_w.clone()))
+
+    def _routed(self, rt, h, batch, routed, picked, after_logits=None):
+        """The routed experts' outputs, not combined yet.  ``routed``: what ``core.norm_route`` returned behind the two norms, or None;
+        ``picked`` is called with the picks and their weights, ``after_logits`` once the logits' product is launched."""
+        T = h.act.shape[0]
+        P = T * self.k
         if routed is not None:
             topk_idx, topk_w, sg, offsets, sorted_token, pos_of_pair, xs = routed
-        elif few and T <= self.route_dispatch_tokens and not self.table:
+        elif T <= 64 and self.E <= 256 and T <= self.route_dispatch_tokens and not self.table:
             # pick, table inversion and gather in one launch after the logits
             topk_idx, topk_w, sg, offsets, sorted_token, pos_of_pair, xs = core.route_dispatch(
                 h.f32, self.w_router, self.k, self.norm_topk, self.scale, shared_gate_w=self.w_sgate,
@@ -430,27 +483,13 @@ class RoutedExperts(Part):
                 bias=self.b_router, **self._grp)
             # (more tokens: the gather by that one block would take longer than a launch of its own)
         else:
-            def shared_beside():
-                # Many tokens: pick, table inversion and gather are small launches that leave the GPU
-                # idle (37 us of a layer at 2,048 tokens), so the shared expert starts beside them on
-                # a second stream.  (Not before the logits' product: the shared expert's CTAs fill every
-                # SM's shared memory, and that product would wait for them to end.)
-                nonlocal ys, side
-                main = torch.cuda.current_stream()
-                side = rt.side_stream()
-                side.wait_stream(main)
-                with torch.cuda.stream(side):
-                    ys = self._shared(rt, h)
-
-            topk_idx, topk_w, sg = self.route(rt, h, batch,
-                                              after_logits=shared_beside if self.ws_gu is not None and side is None and self.shared_beside else None)
+            topk_idx, topk_w, sg = self.route(rt, h, batch, after_logits=after_logits)
             offsets = rt.empty((self.E + 1,), torch.int32)
             sorted_token = rt.empty((P,), torch.int32)
             pos_of_pair = rt.empty((P,), torch.int32)
             core.moe_align(topk_idx, T, self.k, self.E, offsets, sorted_token, pos_of_pair, rt.status)
             xs = None
-        if self.trace is not None:
-            self.trace.append((topk_idx.clone(), topk_w.clone()))
+        picked(topk_idx, topk_w)
         if self.weight_input:
             # what expert e reads for a token is w x: formed from the 32-bit row and rounded once, in expert order
             if xs is None:
@@ -462,12 +501,7 @@ class RoutedExperts(Part):
         act = grouped_swiglu_linear(rt, h.act, self.w_gu, offsets, sorted_token, P, gathered=xs)
         # (the offsets were written before the product above: the second product may start on its weights early)
         y = grouped_linear(rt, act, self.w_down, offsets, P, early_offsets=True)
-        if self.ws_gu is not None and side is None:
-            ys = self._shared(rt, h, beside=False)
-        if side is not None:
-            torch.cuda.current_stream().wait_stream(side)
-            ys.record_stream(torch.cuda.current_stream())
-        return CombineDelta(y, pos_of_pair, topk_w, self.k, ys, sg, T, self.hidden)
+        return CombineDelta(y, pos_of_pair, topk_w, self.k, None, sg, T, self.hidden)
 
 
 register_part("ffn", "dense_swiglu", DenseSwiGLU)
