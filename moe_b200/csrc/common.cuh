@@ -54,6 +54,23 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Four neighbouring numbers as three bfloat16 terms each, v = p0 + p1 + p2 exactly (8 + 8 + 8 bits of mantissa), term k at out + k * pitch.
+__device__ __forceinline__ void split_store4(const float4 v, __nv_bfloat16* out, int pitch) {
+    const float in[4] = {v.x, v.y, v.z, v.w};
+    __nv_bfloat16 p[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        float r = in[e];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            p[k][e] = __float2bfloat16_rn(r);
+            r -= __bfloat162float(p[k][e]);          // exact: the difference fits in float32
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) *reinterpret_cast<uint2*>(out + (size_t)k * pitch) = *reinterpret_cast<const uint2*>(p[k]);
+}
+
 // Block-wide sum; `red` is shared memory of at least 32 floats.  All threads get
 // the result.  Order of additions is fixed, so the result is reproducible.
 __device__ __forceinline__ float block_sum(float v, float* red) {

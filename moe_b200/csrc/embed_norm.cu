@@ -65,7 +65,8 @@ struct CombineSrc {
 // MINB: blocks of 512 threads that must fit an SM.  4 for many rows (a prompt: the kernel is bound by
 // how many loads are in flight, and 32 registers a thread cost a few spills that do not matter there:
 // 26.7 -> 20.5 us for 2,048 rows of 2,048), 1 for few rows (a decode step: every instruction counts).
-template <int MINB>
+// SPLIT: out16 is [rows, 3 hidden] and takes y as three bfloat16 terms (split_store4); the first is the rounded y.
+template <int MINB, bool SPLIT = false>
 __global__ void __launch_bounds__(512, MINB) rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ delta, const float* __restrict__ w,
                                const int* __restrict__ rows, float* __restrict__ out32,
                                __nv_bfloat16* __restrict__ out16, int hidden, float eps, int write_back,
@@ -178,6 +179,10 @@ __global__ void __launch_bounds__(512, MINB) rmsnorm_kernel(float* __restrict__ 
         for (int j = threadIdx.x; j < hidden / 4; j += blockDim.x) {
             const float4 v = reinterpret_cast<const float4*>(row)[j], g = reinterpret_cast<const float4*>(w)[j];
             const float4 y = make_float4(v.x * scale * g.x, v.y * scale * g.y, v.z * scale * g.z, v.w * scale * g.w);
+            if (SPLIT) {
+                split_store4(y, out16 + (size_t)i * 3 * hidden + 4 * j, hidden);
+                continue;
+            }
             if (out32) reinterpret_cast<float4*>(out32 + (size_t)i * hidden)[j] = y;
             if (out16) {
                 __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
@@ -188,6 +193,7 @@ __global__ void __launch_bounds__(512, MINB) rmsnorm_kernel(float* __restrict__ 
         }
         return;
     }
+    if (SPLIT) return;       // (the host asks for it with rows of whole units only)
     for (int j = threadIdx.x; j < hidden; j += blockDim.x) {
         float v = xr[j];
         if (dr) {
@@ -235,6 +241,19 @@ MOE_API int moe_rmsnorm(float* x, const float* delta, const float* w, const int*
     CombineSrc none = {};
     return rmsnorm_launch(x, delta, w, rows, out32, out16, num_out_rows, num_src_rows, hidden, eps, write_back, status,
                           none, stream);
+}
+
+// The norm of every row for a consumer that wants it in 32 bits on the tensor cores (the router) and rounded (everybody else): out3 [rows,
+// 3 hidden] takes the three terms of split3, the first of which is the rounded row.  This kernel instead of
+// norm (with a 32-bit output) and split: a pass of 400 tokens, 6 layers of 2,048 features, 2,243 -> 2,158 us.  Returns -1, with nothing launched, where rows are not whole 16-byte units.
+MOE_API int moe_rmsnorm_split(float* x, const float* delta, const float* w, void* out3, int num_rows, int hidden, float eps,
+                              int write_back, int* status, cudaStream_t stream) {
+    if (num_rows <= 0) return 0;
+    const size_t smem = (size_t)hidden * sizeof(float);
+    if (hidden % 4 || ((uintptr_t)x | (uintptr_t)delta | (uintptr_t)w) % 16 || (uintptr_t)out3 % 8 || smem > 47 * 1024) return -1;
+    CombineSrc none = {};
+    return launch_pdl(rmsnorm_kernel<4, true>, num_rows, hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128), smem, stream, x, delta, w,
+                      (const int*)nullptr, (float*)nullptr, (__nv_bfloat16*)out3, hidden, eps, write_back, num_rows, status, 1, none);
 }
 
 // The same with the delta still uncombined (see CombineSrc).  Returns -1, with nothing launched, if

@@ -1530,8 +1530,8 @@ MOE_API int moe_gemm_tc_plan(int K, int splits, int M, int bn, int num_groups, i
     return (kb_total + per - 1) / per;
 }
 
-// dst[i, :] = src[rows[i], :] for bf16 rows of `width` elements (expert dispatch before the grouped product)
-__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ rows,
+// dst[i, :] = src[rows[i], :] for bf16 rows of `width` elements, `pitch` apart in src (expert dispatch before the grouped product)
+__global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, int pitch, const int* __restrict__ rows,
                                    __nv_bfloat16* __restrict__ dst, int width, int src_rows, int* status) {
     pdl_sync();
     const int i = blockIdx.x;
@@ -1540,14 +1540,14 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const 
         if (threadIdx.x == 0) atomicOr(status, ST_BAD_ROW);
         r = 0;
     }
-    const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)r * width);
+    const uint4* s = reinterpret_cast<const uint4*>(src + (size_t)r * pitch);
     uint4* d = reinterpret_cast<uint4*>(dst + (size_t)i * width);
     for (int j = threadIdx.x; j < width / 8; j += blockDim.x) d[j] = s[j];
 }
-MOE_API int moe_gather_rows_bf16(const void* src, const int* rows, void* dst, int n, int width, int src_rows,
+MOE_API int moe_gather_rows_bf16(const void* src, int pitch, const int* rows, void* dst, int n, int width, int src_rows,
                                  int* status, cudaStream_t stream) {
     if (n <= 0) return 0;
-    if (width % 8) return (int)cudaErrorInvalidValue;
-    return launch_pdl(gather_rows_kernel, n, 128, 0, stream, (const __nv_bfloat16*)src, rows, (__nv_bfloat16*)dst,
+    if (width % 8 || pitch % 8 || ((uintptr_t)src & 15) || ((uintptr_t)dst & 15)) return (int)cudaErrorInvalidValue;
+    return launch_pdl(gather_rows_kernel, n, 128, 0, stream, (const __nv_bfloat16*)src, pitch, rows, (__nv_bfloat16*)dst,
                       width, src_rows, status);
 }

@@ -1144,21 +1144,7 @@ __global__ void split3_kernel(const float* __restrict__ x, __nv_bfloat16* __rest
     if (i >= n4) return;
     const long long t = (i * 4) / hidden;
     const int c = (int)((i * 4) % hidden);
-    const float4 v = reinterpret_cast<const float4*>(x)[i];
-    const float in[4] = {v.x, v.y, v.z, v.w};
-    __nv_bfloat16 p[3][4];
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        float r = in[e];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            p[k][e] = __float2bfloat16_rn(r);
-            r -= __bfloat162float(p[k][e]);          // exact: the difference fits in float32
-        }
-    }
-    __nv_bfloat16* o = out + t * 3 * hidden + c;
-#pragma unroll
-    for (int k = 0; k < 3; k++) *reinterpret_cast<uint2*>(o + (size_t)k * hidden) = *reinterpret_cast<const uint2*>(p[k]);
+    split_store4(reinterpret_cast<const float4*>(x)[i], out + t * 3 * hidden + c, hidden);
 }
 MOE_API int moe_split3(const float* x, void* out, long long num_tokens, int hidden, cudaStream_t stream) {
     if (num_tokens <= 0) return 0;

@@ -56,6 +56,7 @@ def lib():
             "moe_router_logits": [P, P, P, I, I, I, I, P, P, LL, P],
             "moe_router_topk": [P, P, I, I, I, I, I, F, P, P, P, P, I, I, P],
             "moe_split3": [P, P, LL, I, P],
+            "moe_rmsnorm_split": [P, P, P, P, I, I, F, I, P, P],
             "moe_route_dispatch": [P, P, I, I, I, I, I, F, P, P, P, P, P, P, P, P, I, P, P, I, I, P],
             "moe_rope_commit": [P, P, P, I, I, I, I, I, P, P, P, I, P, P, P, I, I, I, I, P, P],
             "moe_attention_decode": [P, P, P, P, P, I, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, I, P, I, F, I, P, I, P],
@@ -263,6 +264,25 @@ def rmsnorm(x, weight, eps, *, delta=None, rows=None, out32=None, out16=None, wr
                 raise KernelError("rmsnorm: output shape")
     _ok(lib().moe_rmsnorm(_p(x), _p(delta), _p(weight), _p(rows), _p(out32), _p(out16), n_out, S, H, float(eps),
                           1 if (write_back and rows is None) else 0, _p(status), _stream()), "rmsnorm")
+
+
+def rmsnorm_split(x, weight, eps, *, delta=None, status=None) -> Optional[torch.Tensor]:
+    """y = rmsnorm(x (+ delta)) of every row, the sum stored back into ``x``, as [T, 3 H] bfloat16 with y = p0 + p1 + p2 exactly (see
+    ``split3``); the first H columns are the rounded y.  None, with nothing launched, for rows that are no whole 16-byte units."""
+    _chk(x, "x", torch.float32, 2), _chk(weight, "weight", torch.float32, 1)
+    T, H = x.shape
+    if weight.numel() != H:
+        raise KernelError("rmsnorm: weight size")
+    if delta is not None:
+        _chk(delta, "delta", torch.float32, 2)
+        if delta.shape != x.shape:
+            raise KernelError("rmsnorm: delta shape")
+    out = torch.empty((T, 3 * H), dtype=torch.bfloat16, device=x.device)
+    code = lib().moe_rmsnorm_split(_p(x), _p(delta), _p(weight), _p(out), T, H, float(eps), 1, _p(status), _stream())
+    if code == -1:
+        return None
+    _ok(code, "rmsnorm_split")
+    return out
 
 
 def layernorm(x, weight, eps, *, bias=None, delta=None, rows=None, out32=None, out16=None, write_back=True, status=None):

@@ -29,7 +29,7 @@ def lib():
         L.moe_gemm_tc.restype = c_int
         L.moe_gemm_tc_plan.argtypes = [I, I, I, I, I, I, P]
         L.moe_gemm_tc_plan.restype = c_int
-        L.moe_gather_rows_bf16.argtypes = [P, P, P, I, I, I, P, P]
+        L.moe_gather_rows_bf16.argtypes = [P, I, P, P, I, I, I, P, P]
         L.moe_gather_rows_bf16.restype = c_int
         from ctypes import c_float
 
@@ -295,10 +295,10 @@ def _packed(out, T: int, nh: int, hd: int, dv: int, gate):
 
 
 def gather_rows(src: torch.Tensor, rows: torch.Tensor, n: int, status) -> torch.Tensor:
-    """dst[i] = src[rows[i]] for bf16 rows (expert dispatch)."""
-    if src.dtype != torch.bfloat16 or src.shape[1] % 8:
+    """dst[i] = src[rows[i]] for bf16 rows (expert dispatch); ``src`` may be a column slice."""
+    if src.dtype != torch.bfloat16 or src.shape[1] % 8 or src.stride(1) != 1 or src.stride(0) % 8:
         raise core.KernelError("gather_rows: bfloat16 rows of a multiple of 8 elements")
     dst = torch.empty((n, src.shape[1]), dtype=torch.bfloat16, device=src.device)
-    core._ok(lib().moe_gather_rows_bf16(src.data_ptr(), rows.data_ptr(), dst.data_ptr(), n, src.shape[1],
+    core._ok(lib().moe_gather_rows_bf16(src.data_ptr(), src.stride(0), rows.data_ptr(), dst.data_ptr(), n, src.shape[1],
                                         src.shape[0], status.data_ptr(), core._stream()), "gather_rows")
     return dst

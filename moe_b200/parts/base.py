@@ -161,6 +161,8 @@ class Activations:
 
     act: torch.Tensor
     f32: Optional[torch.Tensor] = None
+    # the 32-bit state as three bfloat16 terms side by side (``core.split3``), where a norm was asked for it instead of f32
+    split: Optional[torch.Tensor] = None
 
 
 class Part:

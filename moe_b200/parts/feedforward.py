@@ -327,6 +327,9 @@ class RoutedExperts(Part):
             rows = [self.w_router] + ([self.w_sgate.reshape(1, -1)] if self.w_sgate is not None else [])
             one = torch.cat(rows, dim=0)
             self.w_router3 = torch.cat([one, one, one], dim=1).contiguous()
+        # every product that reads the normed rows takes them on the tensor cores, from rows of any pitch
+        self.split_router = self.w_router3 is not None and all(
+            w is None or (w.dtype == torch.bfloat16 and w.data_ptr() % 16 == 0) for w in (self.w_gu, self.ws_gu, self.w_router3))
 
     def route(self, rt, h, batch, after_logits=None):
         """-> (topk_idx [T, k] int32, topk_w [T, k] float32, shared_gate [T] float32 or None)
@@ -348,7 +351,7 @@ class RoutedExperts(Part):
             # (one tile of features: the K splits fill the SMs, and eight of them for any number of tokens: with four the logits of
             # more than 4,096 tokens took 33 instead of 44 us, but were twice as far off, 1.5e-6 instead of 7.3e-7, and a token's
             # picks would have hung on how many others came along)
-            if tc.gemm_tc(core.split3(h.f32), self.w_router3, logits, bn=64, splits=8, status=rt.status):
+            if tc.gemm_tc(h.split if h.split is not None else core.split3(h.f32), self.w_router3, logits, bn=64, splits=8, status=rt.status):
                 if after_logits is not None:
                     after_logits()
                 core.router_topk(logits, self.k, self.norm_topk, self.scale, topk_idx, topk_w, num_experts=self.E,
@@ -381,6 +384,11 @@ class RoutedExperts(Part):
         """The block's offer to take the norm before this feed-forward along: for a step of few
         tokens, norm, router and dispatch are one launch.  None if the sizes or the kind of norm do
         not allow it (the block then runs the norm itself and calls ``forward``)."""
+        if x.shape[0] >= self.tc_router_tokens and self.split_router and not self.weight_input:
+            # a prompt: the norm leaves the three terms that the router's product reads, and no 32-bit row
+            split = getattr(norm, "forward_split", None)
+            h = split(rt, x, delta) if split is not None else None
+            return None if h is None else self._run(rt, h, batch, None)
         if x.shape[0] > self.fused_norm_tokens or self.E > 256 or self.b_router is not None or self.table:
             return None
         if norm.kind == "none" and self.weight_input and isinstance(delta, LazyDelta) and delta.kind == "post_rmsnorm":

@@ -55,6 +55,14 @@ class RMSNorm(Part):
         core.rmsnorm(t, self.weight, self.eps, out32=out, write_back=False, status=rt.status)
         return out
 
+    def forward_split(self, rt, x, delta):
+        """``forward`` of every row for a consumer that wants the 32-bit result on the tensor cores: its three bfloat16 terms
+        (``Activations.split``), of which the first is ``act``, in one kernel; None where that is not possible."""
+        if not rt.is_bf16 or isinstance(delta, LazyDelta):
+            return None
+        split = core.rmsnorm_split(x, self.weight, self.eps, delta=delta, status=rt.status)
+        return None if split is None else Activations(act=split[:, :self.size], split=split)
+
     def forward_pair(self, rt, x, delta, other):
         """This norm and ``other`` (an RMS norm of the same size and eps with a weight of its own) of the
         same x + delta in one kernel with one statistic: (Activations, Activations), both 32-bit only, or

@@ -43,6 +43,34 @@ def test_a_slot_used_again_starts_with_a_clear_state():
         assert float(t[b].abs().sum()) == 0.0 and int((t == 1).sum()) == t.numel() - t[b].numel()
 
 
+@pytest.mark.parametrize("T,H", [(1, 4), (300, 2048), (257, 264), (3, 12032)])
+@pytest.mark.parametrize("with_delta", [True, False])
+def test_the_norm_that_leaves_three_terms(core, T, H, with_delta):
+    """The same as norm and split, to the bit; a row pitch that is no whole unit is left to them."""
+    torch.manual_seed(T)
+    x, w = torch.randn(T, H, device=DEV), torch.randn(H, device=DEV)
+    delta = torch.randn(T, H, device=DEV) if with_delta else None
+    x1, x2, o32, st = x.clone(), x.clone(), torch.empty(T, H, device=DEV), core.new_status(DEV)
+    core.rmsnorm(x1, w, 1e-6, delta=delta, out32=o32, status=st)
+    got = core.rmsnorm_split(x2, w, 1e-6, delta=delta, status=st)
+    assert torch.equal(x1, x2)
+    if T >= 256:        # (fewer rows: the norm beside it is another instance, whose products may be contracted otherwise)
+        assert torch.equal(got, core.split3(o32))
+    y = got.float().view(T, 3, H)
+    assert torch.allclose((y[:, 0] + y[:, 1]) + y[:, 2], o32, rtol=3e-7, atol=1e-12) and int(st[0]) == 0
+    assert core.rmsnorm_split(torch.randn(2, 6, device=DEV), torch.ones(6, device=DEV), 1e-6, status=st) is None
+
+
+def test_gather_rows_from_a_pitch(core):
+    from moe_b200.ops import tc
+
+    src, st = torch.randn(9, 3 * 72, device=DEV).bfloat16(), core.new_status(DEV)
+    rows = torch.tensor([8, 0, 3, 3], dtype=torch.int32, device=DEV)
+    for lo in (0, 72):
+        assert torch.equal(tc.gather_rows(src[:, lo:lo + 72], rows, 4, st), src[:, lo:lo + 72][rows.long()])
+    assert int(st[0]) == 0
+
+
 @pytest.mark.parametrize("groups", [1, 31, 33, 70, 300])
 def test_a_grouped_product_finds_its_rows_among_any_number_of_groups(groups):
     """Few rows a group, empty groups among them, tiles that end inside a group; in one CTA a tile and on persistent CTAs."""
