@@ -99,54 +99,86 @@ router_logits_kernel(const float* __restrict__ h, const WT* __restrict__ wr, con
     }
 }
 
-// The same product for many tokens (a prompt): a block takes 8 router rows (one per warp) and 16
-// tokens, and walks the hidden dimension in chunks of 512 that are staged in shared memory, so
-// that an activation is read from global memory once per 8 rows and a weight once per 16 tokens.
-// hidden must be a multiple of 8.  Grid: (ceil(rows / 8), ceil(T / 16)).
-constexpr int PT = 16, PKC = 512;
+// The same product for 65 to 256 tokens, hidden a multiple of 8: a block takes 4 tokens and 16 router rows, a warp two of the rows.  What bounds
+// it is the chain of loads, so all rows of the block's tokens are asked for at once (cp.async; a row's 16-byte units of even and of odd
+// number lie apart, so that a lane's 8 elements are two reads without bank conflicts) and a lane's weights in batches of eight, asked into
+// L2 before the wait.  A lane's elements and the order of its sums are those of router_logits_kernel with KSPLIT = 1.  (Not for fewer tokens:
+// its shared memory does not fit beside the shared expert's CTAs of a decode step.)  128 rows, 6 layers: a pass 1,746 -> 1,665 us
+// against staging the tokens in chunks of 512 features, a barrier each.  Grid: (ceil(rows / 16), ceil(T / 4)).
+constexpr int RS_TOKENS = 4, RS_ROWS = 16;
 template <typename WT>
 __global__ void __launch_bounds__(256)
-router_logits_tiled_kernel(const float* __restrict__ h, const WT* __restrict__ wr, const WT* __restrict__ wsg,
-                           int num_tokens, int hidden, int num_experts, int rows, float* __restrict__ logits) {
-    __shared__ __align__(16) float xs[PT][PKC];
+router_logits_staged_kernel(const float* __restrict__ h, const WT* __restrict__ wr, const WT* __restrict__ wsg,
+                            int num_tokens, int hidden, int num_experts, int rows, float* __restrict__ logits) {
+    extern __shared__ __align__(16) float4 rs_x[];           // [RS_TOKENS][even | odd units][hidden / 8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * 8 + warp;
-    const int t0 = blockIdx.y * PT;
-    const int nt = min(PT, num_tokens - t0);
-    const WT* w = r < num_experts ? wr + (size_t)r * hidden : wsg;
-    float acc[PT];
+    const int r0 = blockIdx.x * RS_ROWS + warp * 2, t0 = blockIdx.y * RS_TOKENS, nt = min(RS_TOKENS, num_tokens - t0);
+    const int groups = hidden / 8;
+    const WT* w[2];
 #pragma unroll
-    for (int i = 0; i < PT; i++) acc[i] = 0.f;
-    for (int c0 = 0; c0 < hidden; c0 += PKC) {
-        const int kc = min(PKC, hidden - c0);            // a multiple of 8
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < PT * (PKC / 4); idx += blockDim.x) {
-            const int i = idx / (PKC / 4), c = (idx % (PKC / 4)) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < nt && c < kc) v = *reinterpret_cast<const float4*>(h + (size_t)(t0 + i) * hidden + c0 + c);
-            *reinterpret_cast<float4*>(&xs[i][c]) = v;
+    for (int q = 0; q < 2; q++) {
+        const int r = min(r0 + q, rows - 1);
+        w[q] = r < num_experts ? wr + (size_t)r * hidden : wsg;
+        for (int c = lane * (128 / (int)sizeof(WT)); c < hidden; c += 32 * (128 / (int)sizeof(WT))) prefetch_l2(w[q] + c);
+    }
+    pdl_sync();
+    for (int e = threadIdx.x; e < RS_TOKENS * 2 * groups; e += blockDim.x) {
+        const int i = e / (2 * groups), u = e % (2 * groups);
+        const bool on = i < nt;
+        const float* src = h + (size_t)(t0 + (on ? i : 0)) * hidden + u * 4;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"((unsigned)__cvta_generic_to_shared(rs_x + (i * 2 + (u & 1)) * groups + (u >> 1))), "l"(src), "r"(on ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (r0 >= rows) return;
+    constexpr int UNITS = sizeof(WT) / 2, MB = 8 / UNITS;       // 16-byte units of 8 elements; a lane's groups in flight at a time
+    float acc[2][RS_TOKENS];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < RS_TOKENS; i++) acc[q][i] = 0.f;
+    for (int g0 = lane; g0 < groups; g0 += 32 * MB) {
+        uint4 raw[MB][2][UNITS];
+#pragma unroll
+        for (int m = 0; m < MB; m++) {
+            const int g = min(g0 + 32 * m, groups - 1);         // (past the end: read, not used)
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+#pragma unroll
+                for (int u = 0; u < UNITS; u++) raw[m][q][u] = __ldg(reinterpret_cast<const uint4*>(w[q] + g * 8) + u);
         }
-        __syncthreads();
-        if (r < rows) {
-            for (int c = lane * 8; c < kc; c += 256) {
-                float wv[8];
-                w_load8<WT>(w + c0 + c, wv);
 #pragma unroll
-                for (int i = 0; i < PT; i++) {
-                    const float4 a = *reinterpret_cast<const float4*>(&xs[i][c]);
-                    const float4 b = *reinterpret_cast<const float4*>(&xs[i][c + 4]);
-                    float s = acc[i];
-                    s = fmaf(a.x, wv[0], s), s = fmaf(a.y, wv[1], s), s = fmaf(a.z, wv[2], s), s = fmaf(a.w, wv[3], s);
-                    s = fmaf(b.x, wv[4], s), s = fmaf(b.y, wv[5], s), s = fmaf(b.z, wv[6], s), s = fmaf(b.w, wv[7], s);
-                    acc[i] = s;
+        for (int m = 0; m < MB; m++) {
+            const int g = g0 + 32 * m;
+            if (g >= groups) continue;
+            float wv[2][8];
+#pragma unroll
+            for (int q = 0; q < 2; q++) w_load8<WT>(reinterpret_cast<const WT*>(raw[m][q]), wv[q]);
+#pragma unroll
+            for (int i = 0; i < RS_TOKENS; i++) {
+                const float4 a = rs_x[i * 2 * groups + g], b = rs_x[(i * 2 + 1) * groups + g];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    float v = acc[q][i];
+                    v = fmaf(a.x, wv[q][0], v), v = fmaf(a.y, wv[q][1], v), v = fmaf(a.z, wv[q][2], v), v = fmaf(a.w, wv[q][3], v);
+                    v = fmaf(b.x, wv[q][4], v), v = fmaf(b.y, wv[q][5], v), v = fmaf(b.z, wv[q][6], v), v = fmaf(b.w, wv[q][7], v);
+                    acc[q][i] = v;
                 }
             }
         }
     }
+    float total[2][RS_TOKENS];
 #pragma unroll
-    for (int i = 0; i < PT; i++) {
-        const float s = warp_sum(acc[i]);
-        if (lane == 0 && i < nt && r < rows) logits[(size_t)(t0 + i) * rows + r] = s;
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < RS_TOKENS; i++) total[q][i] = warp_sum(acc[q][i]);
+    if (lane < 2 * RS_TOKENS) {
+        const int q = lane / RS_TOKENS, i = lane % RS_TOKENS;
+        float v = 0.f;
+#pragma unroll
+        for (int e = 0; e < 2 * RS_TOKENS; e++) v = e == lane ? total[e / RS_TOKENS][e % RS_TOKENS] : v;
+        if (i < nt && r0 + q < rows) logits[(size_t)(t0 + i) * rows + r0 + q] = v;
     }
 }
 
@@ -1063,16 +1095,21 @@ static int router_logits_impl(const float* h, const void* wr, const void* wsg, i
         }
         const size_t n = (size_t)num_tokens * rows;
         sum_slices_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(scratch, logits, n, slices);
+    } else if (vec_ok && num_tokens > 64 && hidden <= 12288 && (num_tokens + RS_TOKENS - 1) / RS_TOKENS <= 65535) {
+        const dim3 sg((rows + RS_ROWS - 1) / RS_ROWS, (num_tokens + RS_TOKENS - 1) / RS_TOKENS);
+        const int smem = RS_TOKENS * hidden * (int)sizeof(float);
+#define STAGED(WT)                                                                                                     \
+    do {                                                                                                               \
+        cudaError_t e = cudaFuncSetAttribute(router_logits_staged_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+        if (e != cudaSuccess) return (int)e;                                                                           \
+        return launch_pdl(router_logits_staged_kernel<WT>, sg, 256, (size_t)smem, stream, h, (const WT*)wr, (const WT*)wsg, \
+                          num_tokens, hidden, num_experts, rows, logits);                                              \
+    } while (0)
+        if (w_dt == DT_F32) STAGED(float);
+        STAGED(__nv_bfloat16);
+#undef STAGED
     } else if (num_tokens <= 64) {
         if (w_dt == DT_F32) LOGITS(float, 2, 4); else LOGITS(__nv_bfloat16, 2, 4);
-    } else if (vec_ok && (num_tokens + PT - 1) / PT <= 65535) {
-        const dim3 tg((rows + 7) / 8, (num_tokens + PT - 1) / PT);
-        if (w_dt == DT_F32)
-            router_logits_tiled_kernel<float><<<tg, 256, 0, stream>>>(h, (const float*)wr, (const float*)wsg,
-                                                                      num_tokens, hidden, num_experts, rows, logits);
-        else
-            router_logits_tiled_kernel<__nv_bfloat16><<<tg, 256, 0, stream>>>(
-                h, (const __nv_bfloat16*)wr, (const __nv_bfloat16*)wsg, num_tokens, hidden, num_experts, rows, logits);
     } else {
         if (w_dt == DT_F32) LOGITS(float, 8, 1); else LOGITS(__nv_bfloat16, 8, 1);
     }

@@ -138,3 +138,20 @@ def test_norm_and_router_with_several_blocks_a_token(core, T, E, k, H, post):
         src = row[p // k] * (wt.reshape(-1)[p] if post else 1.0)
         assert float((xs[i].float() - src).abs().max()) <= 2.0 ** -8 * float(src.abs().max())
     assert int(st[0]) == 0
+
+
+@pytest.mark.parametrize("T", [9, 64, 65, 131, 256])
+@pytest.mark.parametrize("E,H", [(60, 2048), (17, 264), (33, 3592), (4, 8)])
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+def test_router_logits_of_nine_tokens_and_more(core, T, E, H, wdt):
+    """Picks and weights against 64 bits; tokens and router rows that fill no whole block."""
+    torch.manual_seed(T + E)
+    h, wr = torch.randn(T, H, device=DEV), (torch.randn(E, H, device=DEV) * H ** -0.5).to(wdt)
+    wsg, k = (torch.randn(H, device=DEV) * H ** -0.5).to(wdt), min(3, E)
+    idx, w, sg = torch.empty(T, k, dtype=torch.int32, device=DEV), torch.empty(T, k, device=DEV), torch.empty(T, device=DEV)
+    core.router(h, wr, k, False, 1.0, idx, w, shared_gate_w=wsg, shared_gate=sg)
+    probs = torch.softmax(h.double() @ wr.double().T, -1)
+    # logits of size 1, H products added in 32 bits by 32 lanes: off by some 1e-6
+    assert torch.allclose(probs.gather(1, idx.long()), torch.topk(probs, k, -1).values, rtol=2e-5)
+    assert torch.allclose(w.double(), probs.gather(1, idx.long()), rtol=2e-5)
+    assert torch.allclose(sg.double(), torch.sigmoid(h.double() @ wsg.double()), rtol=2e-5)
