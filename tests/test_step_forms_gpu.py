@@ -140,6 +140,40 @@ def test_norm_and_router_with_several_blocks_a_token(core, T, E, k, H, post):
     assert int(st[0]) == 0
 
 
+@pytest.mark.parametrize("d,dv,taps,channel", [(128, 128, 4, True), (64, 40, 2, False), (36, 128, 3, True), (100, 12, 4, False)])
+def test_the_delta_rules_preparation_over_runs_of_tokens(core, d, dv, taps, channel):
+    """A step of 128 rows and more goes over runs of eight tokens, which sequences begin and end inside of; a step's pieces of fewer rows
+    do not: the same to the bit, rows of no sequence among them."""
+    torch.manual_seed(d)
+    H, Gk, lens = 3, 3, [1, 61, 2, 75, 20]
+    ch, T = 2 * Gk * d + H * dv, sum(lens)
+    ld = ch + 2 * H + (-(ch + 2 * H)) % 4
+    proj, tw = torch.randn(T, ld, device=DEV), torch.randn(taps, ch, device=DEV)
+    a_log, bias = torch.randn(H, device=DEV), torch.randn(H * d if channel else H, device=DEV)
+    a_rows = torch.randn(T, H * d, device=DEV) if channel else None
+    start = torch.randn(len(lens) + 1, ((taps - 1) * ch + 3) // 4 * 4, device=DEV)
+    kw = dict(heads=H, kv_heads=Gk, d=d, dv=dv, b_at=ch, a_at=ch + H, eps=1e-6, q_scale=d ** -0.5)
+
+    def run(proj, a_rows, batch):
+        n = proj.shape[0]
+        out, step = torch.full((n, ch), float("nan"), device=DEV), torch.full((n, 2 * H), float("nan"), device=DEV)
+        decay = torch.full((n, H * d), float("nan"), device=DEV) if channel else None
+        core.delta_prepare(proj, tw, a_log, bias, start.clone(), batch, out, step, a_rows=a_rows, decay=decay, **kw)
+        return [t for t in (out, step, decay) if t is not None]
+
+    whole = G.make_batch(DEV, list(range(len(lens))), [0] * len(lens), lens)
+    got = run(proj, a_rows, whole)
+    at = 0
+    for i, n in enumerate(lens):
+        alone = run(proj[at:at + n].contiguous(), a_rows[at:at + n].contiguous() if channel else None, G.make_batch(DEV, [i], [0], [n]))
+        for g, w in zip(got, alone):
+            assert torch.equal(g[at:at + n], w), i
+        at += n
+    whole.seq_of_token[140:] = -1                        # rows of no sequence: finite, and the others as before
+    for g, w in zip(run(proj, a_rows, whole), got):
+        assert torch.equal(g[:140], w[:140]) and bool(g[140:].isfinite().all())
+
+
 @pytest.mark.parametrize("T", [9, 64, 65, 131, 256])
 @pytest.mark.parametrize("E,H", [(60, 2048), (17, 264), (33, 3592), (4, 8)])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
