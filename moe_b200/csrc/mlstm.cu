@@ -519,7 +519,7 @@ __device__ __forceinline__ int mem_chunk_seq(const MemSeq& p, int num_seqs, int 
 __global__ void __launch_bounds__(256)
 mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
     extern __shared__ __align__(16) float sm[];               // k [64][d + 4], scaled | v [64][132]
-    __shared__ float s_a[QC], s_b[QC];
+    __shared__ float s_a[QC], s_b[QC], s_f[QC];
     __shared__ int s_seq;
     const int tid = threadIdx.x, number = c.first + blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
     pdl_sync();
@@ -540,11 +540,16 @@ mlstm_chunk_add_kernel(const MemSeq p, const MemChunks c, int num_seqs) {
             i < cnt && x < ncols ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.v_at + h * dv + c0 + x) : zero;
     }
     __syncthreads();
+    if (tid < QC) {                    // a token's factor: its b times the a after it
+        float f = s_b[tid];
+        for (int l = tid + 1; l < cnt; l++) f *= s_a[l];
+        s_f[tid] = f;
+    }
+    __syncthreads();
     for (int e = tid; e < QC * (d / 4); e += 256) {
         const int i = e / (d / 4), x = (e % (d / 4)) * 4;
         float4 k4 = i < cnt ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.k_at + h * d + x) : zero;
-        float f = s_b[i];
-        for (int l = i + 1; l < cnt; l++) f *= s_a[l];
+        const float f = s_f[i];
         k4.x *= f, k4.y *= f, k4.z *= f, k4.w *= f;
         *reinterpret_cast<float4*>(sk + i * dp + x) = k4;
     }
@@ -641,10 +646,13 @@ mlstm_chunk_state_kernel(const MemSeq p, const MemChunks c) {
 // counts as often as that is small beside its terms.  An output's own error (the median over tokens) is 0.7 - 0.8 of the
 // form's of four tokens; with 32-bit sums throughout, 118 us instead of 139, it was 1.2 - 1.3 times that.
 constexpr int QP = QC + 4;
+// The state takes the keys' place once the pair products are formed, and a thread's outputs take one set of accumulators, so that an SM
+// holds two blocks (keys of up to 64): one hides the other's loads (2,048 tokens 119 -> 87 us).
 __host__ __device__ constexpr size_t mlstm_chunk_out_floats(int d) {
-    return (size_t)2 * QC * (d + 4) + QC * QP + QC * (QV + 4) + (size_t)d * (QV + 4) + d;
+    const size_t keys = (size_t)QC * (d + 4), state = (size_t)d * (QV + 4);
+    return keys + (keys > state ? keys : state) + QC * QP + QC * (QV + 4) + d;
 }
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* __restrict__ o) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float s_a[QC], s_b[QC], s_den[QC];
@@ -652,11 +660,11 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
     __shared__ int s_seq;
     const int tid = threadIdx.x, number = c.first + blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * QV, d = p.d, dv = p.dv, dp = d + 4;
     float* sq = sm;                    // [64][d + 4]
-    float* sk = sq + QC * dp;          // [64][d + 4]
-    float* sP = sk + QC * dp;          // [64][68]
+    float* sP = sq + QC * dp;          // [64][68]
     float* sv = sP + QC * QP;          // [64][132]
-    float* sS = sv + QC * (QV + 4);    // [d][132]
-    float* sn = sS + d * (QV + 4);     // [d]
+    float* sn = sv + QC * (QV + 4);    // [d]
+    float* sk = sn + d;                // [64][d + 4], and then
+    float* sS = sk;                    // [d][132]
     pdl_sync();
     const int s = mem_chunk_seq(p, num_seqs, number, &s_seq);
     if (s < 0) return;
@@ -680,10 +688,6 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
         const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
         *reinterpret_cast<float4*>(sv + i * (QV + 4) + x) =
             i < cnt && x < ncols ? *reinterpret_cast<const float4*>(p.proj + (size_t)(tok + i) * p.ld + p.v_at + h * dv + c0 + x) : zero;
-    }
-    for (int e = tid; e < d * (QV / 4); e += 256) {
-        const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
-        *reinterpret_cast<float4*>(sS + i * (QV + 4) + x) = x < ncols ? *reinterpret_cast<const float4*>(c.add + (at + i) * dv + c0 + x) : zero;
     }
     for (int x = tid; x < d; x += 256) sn[x] = c.norm[at + x];
     __syncthreads();
@@ -740,6 +744,13 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
         }
     }
     __syncthreads();
+    for (int e = tid; e < d * (QV / 4); e += 256) {           // (the keys are no longer read)
+        const int i = e / (QV / 4), x = (e % (QV / 4)) * 4;
+        const bool on = x < ncols;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                     ::"r"((unsigned)__cvta_generic_to_shared(sS + i * (QV + 4) + x)), "l"(c.add + (at + i) * dv + c0 + (on ? x : 0)), "r"(on ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
     {                                  // n . q of a token by four neighbouring threads
         const int i = tid >> 2, part = tid & 3;
         double held = 0.;
@@ -749,15 +760,20 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
         __syncwarp();
         if (part == 0) s_den[i] = fmaxf(fabsf((float)fma(s_all[i], held, s_in[i])), s_den[i]) + READ_EPS;
     }
-    float in[4][8], held[4][8];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                   // the state is there, and the denominators
+    float acc[4][8], all[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < 4; i++) {
+        all[i] = (float)s_all[ty + 16 * i];
 #pragma unroll
-        for (int e = 0; e < 8; e++) in[i][e] = held[i][e] = 0.f;
+        for (int e = 0; e < 8; e++) acc[i][e] = 0.f;
+    }
     // Sixteen terms at a time, then their sums (one accumulator over 64 or 128 terms would be about twice as far off).
-    // CAUSAL: row i takes the right side's rows up to i, later ones not even with a factor of 0
-    auto product = [&](auto causal, const float* left, int pitch, int n, const float* right, float (&acc)[4][8]) {
-        constexpr bool CAUSAL = decltype(causal)::value;
+    // OWN: the chunk's own terms, onto what the state before it gives times the decay since; row i takes the right side's rows up to i,
+    // later ones not even with a factor of 0
+    auto product = [&](auto own, const float* left, int pitch, int n, const float* right) {
+        constexpr bool OWN = decltype(own)::value;
 #pragma unroll 1
         for (int x0 = 0; x0 < n; x0 += 16) {
             float part[4][8];
@@ -777,7 +793,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
                     const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        if (CAUSAL && x + z > ty + 16 * i) continue;
+                        if (OWN && x + z > ty + 16 * i) continue;
                         const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
 #pragma unroll
                         for (int e = 0; e < 8; e++) part[i][e] = fmaf(f, v[e], part[i][e]);
@@ -787,24 +803,22 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int e = 0; e < 8; e++) acc[i][e] += part[i][e];
+                for (int e = 0; e < 8; e++) acc[i][e] = OWN && x0 == 0 ? fmaf(all[i], acc[i][e], part[i][e]) : acc[i][e] + part[i][e];
         }
     };
-    product(std::true_type(), sP, QP, QC, sv, in);
-    product(std::false_type(), sq, dp, d, sS, held);
-    __syncthreads();                   // the denominators are there
+    product(std::false_type(), sq, dp, d, sS);
+    product(std::true_type(), sP, QP, QC, sv);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int t = ty + 16 * i;
         if (t >= cnt) continue;
-        const float all = (float)s_all[t], den = s_den[t];
+        const float den = s_den[t];
         float* dst = o + ((size_t)(tok + t) * p.H + h) * dv + c0;
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int x = e * 64 + tx * 4;
             if (x < ncols)
-                *reinterpret_cast<float4*>(dst + x) = make_float4(fmaf(all, held[i][4 * e], in[i][4 * e]) / den, fmaf(all, held[i][4 * e + 1], in[i][4 * e + 1]) / den,
-                                                                  fmaf(all, held[i][4 * e + 2], in[i][4 * e + 2]) / den, fmaf(all, held[i][4 * e + 3], in[i][4 * e + 3]) / den);
+                *reinterpret_cast<float4*>(dst + x) = make_float4(acc[i][4 * e] / den, acc[i][4 * e + 1] / den, acc[i][4 * e + 2] / den, acc[i][4 * e + 3] / den);
         }
     }
 }
