@@ -658,8 +658,10 @@ class SideBySideMixer(Part):
         return out.materialize(rt) if isinstance(out, LazyDelta) else out
 
     def forward_lazy(self, rt, h, batch, cache_view, state):
-        """The right mixer runs on a second stream beside the left one (inside a captured step: a fork
-        and a join); MOE_B200_SIDE_BY_SIDE_STREAMS=0 runs them one after the other."""
+        """One mixer runs on a second stream beside the other one (inside a captured step: a fork
+        and a join); MOE_B200_SIDE_BY_SIDE_STREAMS=0 runs them one after the other.  The main stream's first product starts at once, the
+        second stream's behind it, so the main stream takes the longer branch: of several tokens a sequence a recurrent mixer's scan, of
+        one token each the left mixer's attention."""
         states, at = [], 0
         for _, m in self.subs:
             r = m.state_request()
@@ -672,11 +674,17 @@ class SideBySideMixer(Part):
             side = rt.side_stream(1)
             rt = rt.beside()
             side.wait_stream(main)
-            with torch.cuda.stream(side):
+            a_beside = not batch.all_decode and right.state_request() is not None and left.kv_request() is not None
+            if a_beside:
+                with torch.cuda.stream(side):
+                    a = left.forward(rt, h, batch, views[0], states[0])
                 b = right.forward(rt, h, batch, views[1], states[1])
-            a = left.forward(rt, h, batch, views[0], states[0])
+            else:
+                with torch.cuda.stream(side):
+                    b = right.forward(rt, h, batch, views[1], states[1])
+                a = left.forward(rt, h, batch, views[0], states[0])
             main.wait_stream(side)
-            b.record_stream(main)
+            (a if a_beside else b).record_stream(main)
         else:
             a = left.forward(rt, h, batch, views[0], states[0])
             b = right.forward(rt, h, batch, views[1], states[1])
