@@ -32,6 +32,7 @@
 #include <cuda.h>
 
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "common.cuh"
@@ -49,12 +50,22 @@ constexpr int MAX_CLUSTER = 8;   // portable cluster size
 // 128-row weight tile (see gemm_tc_persistent_kernel), so that SwiGLU needs ONE accumulator.
 // MODE_ACT is MODE_PLAIN whose output passes plain_act: a mode of its own, so that the products without one carry
 // nothing of it (the exact GELU in every epilogue cost decode steps of other models 1 - 2 %).
-enum { MODE_PLAIN = 0, MODE_SWIGLU = 1, MODE_SWIGLU_IL = 2, MODE_ACT = 3 };
+// MODE_QKV (persistent and pair form): a step's queries, keys and values, heads of 128; see epilogue_part_qkv.
+enum { MODE_PLAIN = 0, MODE_SWIGLU = 1, MODE_SWIGLU_IL = 2, MODE_ACT = 3, MODE_QKV = 4 };
 __host__ __device__ constexpr bool plain_mode(int mode) { return mode == MODE_PLAIN || mode == MODE_ACT; }
 template <int MODE>
 __device__ __forceinline__ float plain_out(const int act, float v) {
     return MODE == MODE_ACT ? plain_act(act, v) : v;
 }
+
+// Where MODE_QKV leaves its heads, all bfloat16.
+struct QkvOut {
+    const float2* angles;       // [M][64]: cosine and sine of a token's angles
+    const int* rows;            // [M]: a token's row among a head's rows of the cache (head h: + h * page_size), -1: not kept; null: nothing is appended
+    __nv_bfloat16 *q, *k, *v;   // [M][heads][128]
+    __nv_bfloat16 *k_cache, *v_cache;
+    int nh, nkv, page_size;
+};
 
 struct Params {
     void* out;
@@ -81,6 +92,12 @@ struct Params {
     int act;                    // SWIGLU: the gate's activation (ACT_* in common.cuh)
     float act_param;            // its constant, if it has one (the limit of ACT_CLAMPED_SIGMOID)
 };
+// (A type of its own: with these fields in Params the other modes' persistent kernels came out 4 to 18 registers larger, SwiGLU 10 % slower.)
+struct QkvParams : Params {
+    QkvOut qkv;
+};
+template <int MODE>
+using ParamsOf = std::conditional_t<MODE == MODE_QKV, QkvParams, Params>;
 
 // ---- PTX wrappers ---------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -214,6 +231,12 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
         : "memory");
 }
 // D[256, N] (+)= A[256, 16] B[N, 16]^T over the pair: each CTA holds 128 rows of A and N / 2 rows of B
@@ -842,6 +865,62 @@ __device__ __forceinline__ void epilogue_part_il(const Params& p, uint32_t taddr
     }
 }
 
+// The same for MODE_QKV: the tile is one head, whose rows the load interleaves so that lanes 0..15 of quarter q hold features 16 q + lane and
+// lanes 16..31 the features 64 further on, their partners in the rotation.  Of each pair of tokens the lower lanes take the first, the upper
+// lanes the second, and write both features: rotated and rounded, to the step's own rows and, keys, to the cache.  Values are written as
+// they are.  (Bias, rotation and rounding one by one as rope_split4_kernel does them, so the results are the same to the bit; the
+// 32-bit rows, 50 MB at 2,048 tokens of 6,144 features, are neither written nor read again.)
+template <int BN>
+__device__ __forceinline__ void epilogue_part_qkv(const QkvParams& p, uint32_t taddr, int head, int quarter, int lane, int row0, int row_end,
+                                                  int c_lo, int c_hi) {
+    const QkvOut& o = p.qkv;
+    const bool upper = (lane & 16) != 0, live = head < o.nh + 2 * o.nkv;
+    const int i = quarter * 16 + (lane & 15), f = i + (upper ? 64 : 0);
+    const float bias = p.bias && live ? p.bias[head * 128 + f] : 0.f;
+    const bool rotated = head < o.nh + o.nkv, is_q = head < o.nh;
+    const int h = is_q ? head : rotated ? head - o.nh : head - o.nh - o.nkv, heads = is_q ? o.nh : o.nkv;
+    __nv_bfloat16* out = is_q ? o.q : rotated ? o.k : o.v;
+    __nv_bfloat16* cache = rotated ? o.k_cache : o.v_cache;
+    const int* rows = is_q ? nullptr : o.rows;
+    for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
+        float a[32];
+        __syncwarp();
+        tmem_ld32(taddr + c0, a);
+        if (!live) continue;
+        if (p.bias)
+#pragma unroll
+            for (int j = 0; j < 32; j++) a[j] = a[j] + bias;
+        if (!rotated) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) {
+                const int r = row0 + c0 + j;
+                if (r >= row_end) break;
+                const __nv_bfloat16 y = __float2bfloat16_rn(a[j]);
+                out[((size_t)r * heads + h) * 128 + f] = y;
+                if (rows && rows[r] >= 0) cache[((size_t)rows[r] + (size_t)h * o.page_size) * 128 + f] = y;
+            }
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            const float send = upper ? a[j] : a[j + 1];
+            const float recv = __shfl_xor_sync(0xffffffffu, send, 16);
+            const float lo = upper ? recv : a[j], hi = upper ? a[j + 1] : recv;
+            const int r = row0 + c0 + j + (upper ? 1 : 0);
+            if (r < row_end) {
+                const float2 t = __ldg(o.angles + (size_t)r * 64 + i);
+                const __nv_bfloat16 y0 = __float2bfloat16_rn(rot_lo(lo, hi, t.x, t.y)), y1 = __float2bfloat16_rn(rot_hi(lo, hi, t.x, t.y));
+                __nv_bfloat16* dst = out + ((size_t)r * heads + h) * 128;
+                dst[i] = y0, dst[i + 64] = y1;
+                if (rows && rows[r] >= 0) {
+                    __nv_bfloat16* at = cache + ((size_t)rows[r] + (size_t)h * o.page_size) * 128;
+                    at[i] = y0, at[i + 64] = y1;
+                }
+            }
+        }
+    }
+}
+
 // ---- the persistent form, for many tokens ------------------------------------------------------
 // One CTA per SM walks over the tiles (blockIdx.x, blockIdx.x + gridDim.x, ...).  The producer and
 // the MMA issuer run ahead across tile borders, and the accumulator in tensor memory is doubled,
@@ -895,7 +974,7 @@ __device__ __forceinline__ Tile tile_of(int item, int m_tiles, const Params& p, 
 template <int BN, int MODE>
 __global__ void __launch_bounds__(P_THREADS)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
-                          const Params p) {
+                          const ParamsOf<MODE> p) {
     using C = PCfg<BN, MODE>;
     // features of a tile: 128, or 64 where gate and up rows share the tile's 128 rows
     constexpr int TW = MODE == MODE_SWIGLU_IL ? TILE_W / 2 : TILE_W;
@@ -971,6 +1050,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
                         // tmW is five-dimensional here, (k, row of 16, gate|up, block of 16 features, group):
                         // one box is four times [16 gate rows, the 16 up rows of the same features]
                         tma_load_5d(st, &tmW, kb * BK, 0, 0, t.n0 / 16, t.g, full_bar(s), policy);
+                    } else if (MODE == MODE_QKV) {
+                        // the same map over heads of 128 rows: four times [16 rows, the 16 rows 64 further on]
+                        tma_load_5d(st, &tmW, kb * BK, 0, 0, 0, t.n0 / TILE_W, full_bar(s), policy);
                     } else {
                         tma_load_2d(st, &tmW, kb * BK, w_row, full_bar(s), policy);
                     }
@@ -1039,7 +1121,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
             const uint32_t taddr = tmem + b * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
             const int rows_here = min(BN, t.row_end - t.row0);
             const int part = ((rows_here + 32 * EPI_GROUPS - 1) / (32 * EPI_GROUPS)) * 32;      // a multiple of 32
-            if (MODE == MODE_SWIGLU_IL)
+            if constexpr (MODE == MODE_QKV)
+                epilogue_part_qkv<BN>(p, taddr, t.n0 / TILE_W, q, lane, t.row0, t.row_end, min(rows_here, h * part), min(rows_here, (h + 1) * part));
+            else if (MODE == MODE_SWIGLU_IL)
                 epilogue_part_il<BN>(p, taddr, t.n0 + q * 16 + (lane & 15), (lane & 16) != 0, t.row0, t.row_end,
                                      min(rows_here, h * part), min(rows_here, (h + 1) * part));
             else
@@ -1094,7 +1178,7 @@ struct PairCfg {
 
 template <int BN, int MODE>
 __global__ void __launch_bounds__(P_THREADS)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const ParamsOf<MODE> p) {
     using C = PairCfg<BN, MODE>;
     constexpr int PAIR_W = 2 * TILE_W;
     extern __shared__ uint8_t smem_raw[];
@@ -1179,7 +1263,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
                     const uint32_t st = base + s * C::STAGE_BYTES;
                     const uint32_t bar = mapa_cluster(full_bar(s), 0);
                     if (rank == 0) mbar_expect_tx(full_bar(s), 2 * cta_tx);
-                    tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
+                    if (MODE == MODE_QKV)
+                        tma_load_5d_pair(st, &tmW, kb * BK, 0, 0, 0, w_row / TILE_W, bar);     // (see gemm_tc_persistent_kernel)
+                    else
+                        tma_load_2d_pair(st, &tmW, kb * BK, w_row, bar);
                     if (MODE == MODE_SWIGLU) tma_load_2d_pair(st + C::W_BYTES, &tmW, kb * BK, w_row + p.N, bar);
                     for (int c = 0; c < xchunks; c++)
                         tma_load_2d_pair(st + C::NW * C::W_BYTES + c * C::XBOX * BK * 2, &tmX, kb * BK,
@@ -1238,8 +1325,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_consta
             const uint32_t taddr = tmem + b * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
             const int rows_here = min(BN, t.row_end - t.row0);
             const int part = ((rows_here + 32 * EPI_GROUPS - 1) / (32 * EPI_GROUPS)) * 32;
-            epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
-                                    min(rows_here, h * part), min(rows_here, (h + 1) * part));
+            if constexpr (MODE == MODE_QKV)
+                epilogue_part_qkv<BN>(p, taddr, t.n0 / TILE_W + (int)rank, q, lane, t.row0, t.row_end, min(rows_here, h * part),
+                                      min(rows_here, (h + 1) * part));
+            else
+                epilogue_part<BN, MODE>(p, taddr, t.n0 + (int)rank * TILE_W + q * 32 + lane, t.row0, t.row_end,
+                                        min(rows_here, h * part), min(rows_here, (h + 1) * part));
             // this warp has read its part of the buffer; the issuer waits for all epilogue warps of the pair
             tc_fence_before();
             __syncwarp();
@@ -1355,7 +1446,7 @@ int sm_count() {
 }
 
 template <int BN, int MODE>
-int launch_persistent(const CUtensorMap& tmW, const CUtensorMap& tmX, const Params& p, int max_items,
+int launch_persistent(const CUtensorMap& tmW, const CUtensorMap& tmX, const ParamsOf<MODE>& p, int max_items,
                       cudaStream_t stream) {
     using C = PCfg<BN, MODE>;
     static bool configured = false;
@@ -1385,7 +1476,7 @@ bool takes_pairs(int M, int num_groups, int mode) {       // num_groups: 0 for a
 }
 
 template <int BN, int MODE>
-int launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const Params& p, int max_items, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const ParamsOf<MODE>& p, int max_items, cudaStream_t stream) {
     using C = PairCfg<BN, MODE>;
     static bool configured = false;
     if (!configured) {
@@ -1488,6 +1579,29 @@ MOE_API int moe_gemm_tc(const void* X, int ldx, const void* W, int num_groups, i
     GO(16) GO(32) GO(64) GO(128) GO(256)
 #undef GO
     return -1;
+}
+
+// The projection of many rows to queries, keys and values, heads of 128 rotated over their whole width, in one launch: what moe_gemm_tc (32-bit
+// output, bias) and moe_rope_split leave, to the bit.  X: [M, K] bf16, row pitch ldx; W: [(nh + 2 nkv) * 128, K] bf16; angles: [M][64] pairs
+// (cosine, sine); rows (may be null: nothing is appended): see QkvOut; q: [M, nh, 128], k, v: [M, nkv, 128].  Returns 0, a CUDA error code, or -1 for
+// what it does not take (nothing is launched then).
+MOE_API int moe_gemm_qkv(const void* X, int ldx, const void* W, int M, int K, const float* bias, const float* angles, const int* rows, void* q,
+                         void* k, void* v, void* k_cache, void* v_cache, int nh, int nkv, int page_size, int* status, cudaStream_t stream) {
+    if (M <= 0) return 0;
+    if (nh <= 0 || nkv <= 0 || !angles || !q || !k || !v || (rows && (!k_cache || !v_cache))) return (int)cudaErrorInvalidValue;
+    if (!g_persistent || K <= 0 || K % 8 != 0 || ldx % 8 != 0 || ((uintptr_t)X & 15) || ((uintptr_t)W & 15) || ((uintptr_t)angles & 7)) return -1;
+    const int heads = nh + 2 * nkv;
+    CUtensorMap tmW, tmX;
+    if (!make_map_gate_up(&tmW, W, heads, 64, K) || !make_map(&tmX, X, M, K, ldx, 64)) return -1;
+    QkvParams p = {};
+    p.bias = bias, p.M = M, p.N = heads * 128, p.K = K, p.w_rows_per_group = p.N, p.splits = 1, p.kb_per_split = (K + BK - 1) / BK;
+    p.status = status, p.wait_limit = g_wait_limit, p.test_fault = g_test_fault;
+    p.qkv = QkvOut{(const float2*)angles, rows, (__nv_bfloat16*)q, (__nv_bfloat16*)k, (__nv_bfloat16*)v, (__nv_bfloat16*)k_cache,
+                   (__nv_bfloat16*)v_cache, nh, nkv, page_size};
+    const long long mt = (M + 255) / 256, items = mt * heads, pairs = mt * ((heads + 1) / 2);
+    if (items > (1 << 30)) return -1;
+    if (takes_pairs(M, 0, MODE_PLAIN) && sm_count() >= 2) return launch_pair<256, MODE_QKV>(tmW, tmX, p, (int)pairs, stream);
+    return launch_persistent<256, MODE_QKV>(tmW, tmX, p, (int)items, stream);
 }
 
 // Programmatic dependent launch on or off for the kernels of this library (on by default).

@@ -58,6 +58,9 @@ struct CommitArgs {
     const int* tables;
     int table_stride, ring, page_size, num_pages;
     int* status;
+    const int* pad_seq;       // with `zero`: a token's sequence, -1 for none
+    uint4* zero;              // rows of zero_units 16-byte units a token (or null): those of tokens of no sequence become zero
+    int zero_units;
 };
 
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
@@ -102,6 +105,8 @@ rope_split4_kernel(const float* __restrict__ qkv, const int* __restrict__ pos, c
             kc = (OT*)c.k_cache + at, vc = (OT*)c.v_cache + at;
         }
     }
+    if (c.zero && c.pad_seq[t] < 0)
+        for (int i = threadIdx.x; i < c.zero_units; i += blockDim.x) c.zero[(size_t)t * c.zero_units + i] = make_uint4(0, 0, 0, 0);
     const size_t head_step = (size_t)c.page_size * hd;
     const int rot_heads = nh + nkv, hq = half / 4;
     for (int idx = threadIdx.x; idx < rot_heads * hq; idx += blockDim.x) {
@@ -142,13 +147,42 @@ rope_split4_kernel(const float* __restrict__ qkv, const int* __restrict__ pos, c
     }
 }
 
+// What a product that rotates and appends its own output (moe_gemm_qkv) reads of every token: angles [T][half] pairs (cosine, sine), and
+// rows [T] (null: not wanted): the token's row among one head's rows of the cache, seen as [page][kv head][offset] of them, head 0; -1 for a token
+// that is not kept.  Four tokens a block.
+__global__ void __launch_bounds__(256)
+rope_angles_kernel(const int* __restrict__ pos, const float* __restrict__ inv_freq, int num_tokens, int half, float2* __restrict__ angles,
+                   const CommitArgs c, int nkv, int* __restrict__ rows) {
+    pdl_sync();
+    const int t = blockIdx.x * 4 + threadIdx.x / 64, i0 = threadIdx.x % 64;
+    if (t >= num_tokens) return;
+    const int p_int = pos[t];
+    const float p = (float)p_int;
+    for (int i = i0; i < half; i += 64) {
+        float sn, cs;
+        sincosf(p * inv_freq[i], &sn, &cs);
+        angles[(size_t)t * half + i] = make_float2(cs, sn);
+    }
+    if (rows && i0 == 0) {
+        const int s = c.seq_of_token[t];
+        int at = -1;
+        if (s >= 0 && !(c.ring > 0 && p_int < c.seq_end[s] - c.ring)) {
+            const CachePos cp = cache_pos(p_int, c.ring, c.tables + (size_t)c.slots[s] * c.table_stride, c.page_size, c.num_pages, c.status);
+            at = cp.page * nkv * c.page_size + cp.off;
+        }
+        rows[t] = at;
+    }
+}
+
+// With `zero` the rows of tokens of no sequence in another buffer become zero (an attention's output, which no attention kernel writes there): a
+// fill of the whole buffer was a launch of its own in every layer.
 // With cache arguments (k_cache not null) the keys and values are also appended to the cache, as
 // moe_kv_commit would: only for steps whose attention reads nothing from the cache.
 MOE_API int moe_rope_split(const float* qkv, const int* pos, const float* inv_freq, int num_tokens, int nh, int nkv,
                            int hd, int rot, void* q, void* k, void* v, int out_dt, void* k_cache, void* v_cache,
                            const int* seq_of_token, const int* seq_end, const int* slots, const int* tables,
-                           int table_stride, int ring, int page_size, int num_pages, int* status,
-                           cudaStream_t stream) {
+                           int table_stride, int ring, int page_size, int num_pages, int* status, const int* pad_seq, void* zero,
+                           int zero_units, cudaStream_t stream) {
     if (num_tokens <= 0) return 0;
     if (rot < 0 || rot > hd || (rot & 1)) return (int)cudaErrorInvalidValue;
     if (rot > 0 && !inv_freq) return (int)cudaErrorInvalidValue;
@@ -158,9 +192,11 @@ MOE_API int moe_rope_split(const float* qkv, const int* pos, const float* inv_fr
     const bool vec = hd % 8 == 0 && rot % 8 == 0 && ((uintptr_t)qkv % 16 == 0) && ((uintptr_t)q % 16 == 0) &&
                      ((uintptr_t)k % 16 == 0) && ((uintptr_t)v % 16 == 0) &&
                      (!k_cache || ((uintptr_t)k_cache % 16 == 0 && (uintptr_t)v_cache % 16 == 0));
-    if (k_cache && !vec) return -1;      // the caller commits with moe_kv_commit
+    if (zero && (!pad_seq || ((uintptr_t)zero & 15))) return (int)cudaErrorInvalidValue;
+    if ((k_cache || zero) && !vec) return -1;      // the caller commits with moe_kv_commit
     if (vec) {
         CommitArgs c;
+        c.pad_seq = pad_seq, c.zero = (uint4*)zero, c.zero_units = zero_units;
         c.k_cache = k_cache, c.v_cache = v_cache, c.seq_of_token = seq_of_token, c.seq_end = seq_end, c.slots = slots;
         c.tables = tables, c.table_stride = table_stride, c.ring = ring, c.page_size = page_size;
         c.num_pages = num_pages, c.status = status;
@@ -350,4 +386,17 @@ MOE_API int moe_clear_rows(void* const* rows, const long long* bytes, int n, cud
         if (code) return code;
     }
     return 0;
+}
+
+MOE_API int moe_rope_angles(const int* pos, const float* inv_freq, int num_tokens, int half, float* angles, int* rows, int nkv,
+                            const int* seq_of_token, const int* seq_end, const int* slots, const int* tables, int table_stride, int ring,
+                            int page_size, int num_pages, int* status, cudaStream_t stream) {
+    if (num_tokens <= 0) return 0;
+    if (half <= 0 || !pos || !inv_freq || !angles || ((uintptr_t)angles & 7) ||
+        (rows && (!seq_of_token || !seq_end || !slots || !tables || page_size <= 0 || (long long)num_pages * nkv * page_size > 0x7fffffffLL)))
+        return (int)cudaErrorInvalidValue;
+    CommitArgs c = {};
+    c.seq_of_token = seq_of_token, c.seq_end = seq_end, c.slots = slots, c.tables = tables, c.table_stride = table_stride, c.ring = ring;
+    c.page_size = page_size, c.num_pages = num_pages, c.status = status;
+    return launch_pdl(rope_angles_kernel, dim3((num_tokens + 3) / 4), dim3(256), 0, stream, pos, inv_freq, num_tokens, half, (float2*)angles, c, nkv, rows);
 }

@@ -39,6 +39,8 @@ class StepBatch:
     # mixer must leave something finite in those rows of its output, as rows of a tile are multiplied
     # by weights of exactly zero, and 0 x NaN is NaN
     has_padding: bool = False
+    # while a model runs the step: what one layer formed of the step's layout alone and the next layers use again
+    memo: Optional[dict] = None
 
 
 def layout(num_tokens: int, num_seqs: int, num_want: int) -> List[Tuple[str, int]]:

@@ -162,6 +162,13 @@ class DecoderModel:
     def forward(self, batch, cache) -> Optional[torch.Tensor]:
         """Run the batch's tokens through every scheduled layer, appending to the cache;
         return float32 logits [len(want_rows), vocab], or None if no row is wanted."""
+        batch.memo = {}
+        try:
+            return self._forward(batch, cache)
+        finally:
+            batch.memo = None
+
+    def _forward(self, batch, cache) -> Optional[torch.Tensor]:
         rt = self.rt
         if hasattr(self.embedding, "state_request"):
             x = self.embedding.forward(rt, batch.token_ids, batch.num_tokens, batch, state=cache.state("embedding"))

@@ -49,7 +49,7 @@ def lib():
             "moe_rmsnorm_combine": [P, P, P, P, I, P, P, P, P, P, P, I, I, I, F, I, P, P],
             "moe_add_inplace": [P, P, LL, P],
             "moe_gemm_generic": [P, I, I, P, I, P, I, LL, P, I, I, P, P, I, I, I, I, P, P, LL, P],
-            "moe_rope_split": [P, P, P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, P, P],
+            "moe_rope_split": [P, P, P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, P, P, P, I, P],
             "moe_kv_commit": [P, P, P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
             "moe_attention_generic": [P, P, P, P, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, I, F, I, P, I, P],
             "moe_router": [P, P, P, I, P, I, I, I, I, I, F, P, P, P, P, P, LL, P, I, I, P],
@@ -79,6 +79,7 @@ def lib():
             "moe_seed_rng": [P, P, P, I, P],
             "moe_table_update": [P, I, P, I, P],
             "moe_clear_rows": [P, P, I, P],
+            "moe_rope_angles": [P, P, I, I, P, P, I, P, P, P, P, I, I, I, I, P, P],
             "moe_whole_prepare": [P, I, P, P, P, P, F, P, I, P, I, I, I, I, I, I, P, P, P, LL, LL, I, P, P, P, P, P, I, I, I, I,
                                   I, P, P],
             "moe_whole_conv_prepare": [P, I, P, I, P, LL, I, P, P, P, P, P, P, F, P, I, I, I, I, I, I, I, I, I, P, P, P, LL, LL,
@@ -789,10 +790,11 @@ def gemm_generic(a, w, out, *, bias=None, a_rows=None, group_offsets=None, statu
                                _stream()), "gemm_generic")
 
 
-def rope_split(qkv, pos, inv_freq, nh, nkv, hd, rot, q, k, v, commit=None, status=None):
+def rope_split(qkv, pos, inv_freq, nh, nkv, hd, rot, q, k, v, commit=None, status=None, zero=None):
     """Rotate and split a step's projections.  ``commit=(view, batch)``: also append the keys and
-    values to that cache layer in the same launch (only for a step whose attention reads nothing
-    from the cache); returns False if this was asked for and the sizes do not allow it (nothing is
+    values to that cache layer in the same launch (only for a step whose attention reads none of the places
+    they go to: whole prompts, or a cache that is no ring), and with ``zero`` (contiguous rows of whole 16-byte units, one a token) to
+    make the rows of tokens of no sequence zero there; returns False if this was asked for and the sizes do not allow it (nothing is
     launched then), else True."""
     _chk(qkv, "qkv", torch.float32, 2), _chk(pos, "pos", torch.int32, 1)
     T = qkv.shape[0]
@@ -814,14 +816,32 @@ def rope_split(qkv, pos, inv_freq, nh, nkv, hd, rot, q, k, v, commit=None, statu
         code = lib().moe_rope_split(_p(qkv), _p(pos), _p(inv_freq) if rot else None, T, nh, nkv, hd, rot, _p(q),
                                     _p(k), _p(v), _dt(q), _p(view.k), _p(view.v), _p(batch.seq_of_token),
                                     _p(batch.seq_end), _p(batch.slots), _p(g.table), g.table.stride(0), g.ring,
-                                    g.page_size, g.num_pages, _p(status), _stream())
+                                    g.page_size, g.num_pages, _p(status), _p(batch.seq_of_token), _p(zero),
+                                    0 if zero is None else zero.numel() // zero.shape[0] * zero.element_size() // 16, _stream())
         if code == -1:
             return False
         _ok(code, "rope_split")
         return True
     _ok(lib().moe_rope_split(_p(qkv), _p(pos), _p(inv_freq) if rot else None, T, nh, nkv, hd, rot, _p(q), _p(k), _p(v),
-                             _dt(q), None, None, None, None, None, None, 0, 0, 0, 0, None, _stream()), "rope_split")
+                             _dt(q), None, None, None, None, None, None, 0, 0, 0, 0, None, None, None, 0, _stream()), "rope_split")
     return True
+
+
+def rope_angles(batch, inv_freq, half, view=None, status=None):
+    """(angles float32 [T, half, 2], rows int32 [T] or None): the cosines and sines of every token's position, and with ``view`` where each
+    token's keys and values go in that cache layer (the same in all layers of its group), for ``tc.gemm_qkv``."""
+    _chk(inv_freq, "inv_freq", torch.float32, 1)
+    T = batch.num_tokens
+    if inv_freq.numel() < half:
+        raise KernelError("rope_angles: inv_freq too short")
+    angles = torch.empty((T, half, 2), dtype=torch.float32, device=inv_freq.device)
+    rows, nkv, args = None, 0, [None, None, None, None, 0, 0, 0, 0]
+    if view is not None:
+        g = view.group
+        rows, nkv = torch.empty((T,), dtype=torch.int32, device=inv_freq.device), g.num_kv_heads
+        args = [_p(batch.seq_of_token), _p(batch.seq_end), _p(batch.slots), _p(g.table), g.table.stride(0), g.ring, g.page_size, g.num_pages]
+    _ok(lib().moe_rope_angles(_p(batch.pos), _p(inv_freq), T, int(half), _p(angles), _p(rows), nkv, *args, _p(status), _stream()), "rope_angles")
+    return angles, rows
 
 
 def kv_commit(k_new, v_new, view, batch, status):

@@ -27,6 +27,8 @@ def lib():
 
         L.moe_gemm_tc.argtypes = [P, I, P, I, I, I, I, P, I, I, P, P, I, I, I, P, P, P, I, I, _F, P]
         L.moe_gemm_tc.restype = c_int
+        L.moe_gemm_qkv.argtypes = [P, I, P, I, I, P, P, P, P, P, P, P, P, I, I, I, P, P]
+        L.moe_gemm_qkv.restype = c_int
         L.moe_gemm_tc_plan.argtypes = [I, I, I, I, I, I, P]
         L.moe_gemm_tc_plan.restype = c_int
         L.moe_gather_rows_bf16.argtypes = [P, I, P, P, I, I, I, P, P]
@@ -214,6 +216,35 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swiglu: bool
     if code == -1:
         return False
     core._ok(code, "gemm_tc")
+    return True
+
+
+def takes_qkv(x: torch.Tensor, w: torch.Tensor, beside: bool) -> bool:
+    """Whether ``gemm_qkv`` is the form for this projection: where ``gemm_tc`` would take the persistent form with tiles of 256 rows, from 1,280 rows
+    on.  (us, product and rotation one by one / in one: 48 heads of 2,048 features 1,024 rows 43.0 / 39.8, 1,536 47.9 / 43.8, 2,048 68.2 / 55.4,
+    8,192 222 / 199; 36 heads of 3,584 features 1,024 rows 40.2 / 41.8, 1,280 66.1 / 64.4, 8,192 248 / 203; 768 rows 27.5 / 29.3.)"""
+    M = x.shape[0]
+    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M >= 1280
+            and (beside or not mid_splits(M, -(-w.shape[0] // 128), -(-w.shape[1] // 64), num_sms(x.device))))
+
+
+def gemm_qkv(x, w, bias, angles, rows, q, k, v, view, *, nh: int, nkv: int, status) -> bool:
+    """Queries, keys and values of a step of many rows in one product (``csrc/gemm_tc.cu``, moe_gemm_qkv): heads of 128 rotated over their whole
+    width by ``angles`` (``core.rope_angles``) into q, k, v bf16, and, with ``rows``, keys and values into the cache layer ``view`` too.  False,
+    with nothing launched, for what the kernel does not take."""
+    for t, n in ((q, nh), (k, nkv), (v, nkv)):
+        if t.dtype != torch.bfloat16 or not t.is_contiguous() or t.numel() < x.shape[0] * n * 128:
+            raise core.KernelError("gemm_qkv: q, k and v are bfloat16 [M, heads, 128]")
+    if (w.shape[0] != (nh + 2 * nkv) * 128 or x.shape[1] != w.shape[1] or x.stride(1) != 1 or not w.is_contiguous()
+            or angles.numel() < x.shape[0] * 128 or (rows is not None and (view.group.dtype != torch.bfloat16 or view.group.head_dim != 128))):
+        raise core.KernelError("gemm_qkv: shapes")
+    code = lib().moe_gemm_qkv(x.data_ptr(), x.stride(0), w.data_ptr(), x.shape[0], w.shape[1], None if bias is None else bias.data_ptr(),
+                              angles.data_ptr(), None if rows is None else rows.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                              None if rows is None else view.k.data_ptr(), None if rows is None else view.v.data_ptr(), nh, nkv,
+                              view.group.page_size, status.data_ptr(), core._stream())
+    if code == -1:
+        return False
+    core._ok(code, "gemm_qkv")
     return True
 
 

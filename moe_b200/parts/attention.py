@@ -427,13 +427,16 @@ class GQAttention(Part):
             return self._forward_prepared(rt, h, batch, cache_view)
         T = batch.num_tokens
         nkv = self.nkv if self.own_kv else 0
+        done = self._project_rotated(rt, h, batch, cache_view)
+        if done is not None:
+            return self._attend_step(rt, batch, cache_view, *done)
         qkv = linear(rt, h.act, self.wqkv, bias=self.bqkv)
         table, rot = self.position.rotary_table()
         if table is None and hasattr(self.position, "apply"):
             self.position.apply(rt, qkv, self.nh, nkv, self.hd, batch.pos)
         ctx = rt.empty((T, self.nh * self.hd))
-        if getattr(batch, "has_padding", False) and not batch.all_decode:
-            ctx.zero_()      # rows of no sequence are written by no attention kernel
+        # rows of no sequence are written by no attention kernel: they become zero beside the rotation, or in front of it
+        padded = getattr(batch, "has_padding", False) and not batch.all_decode
         if batch.all_decode and self.own_kv:
             # one token per sequence: rotation, append, attention split along the keys and the
             # merge in ONE launch where the head size allows it
@@ -449,12 +452,48 @@ class GQAttention(Part):
         q = rt.empty((T, self.nh, self.hd))
         k_new = rt.empty((T, max(nkv, 1), self.hd))
         v_new = rt.empty((T, max(nkv, 1), self.hd))
-        # whole prompts read nothing from the cache, so their keys and values may go there at once
-        early = batch.all_fresh and self.own_kv and not batch.all_decode
-        committed = early and core.rope_split(qkv, batch.pos, table, self.nh, nkv, self.hd, rot, q, k_new, v_new,
-                                              commit=(cache_view, batch), status=rt.status)
+        committed = self._early(batch, cache_view) and core.rope_split(qkv, batch.pos, table, self.nh, nkv, self.hd, rot, q, k_new, v_new,
+                                                                       commit=(cache_view, batch), status=rt.status, zero=ctx if padded else None)
         if not committed:
+            if padded:
+                ctx.zero_()
             core.rope_split(qkv, batch.pos, table, self.nh, nkv, self.hd, rot, q, k_new, v_new)
+        return self._attend_step(rt, batch, cache_view, q, k_new, v_new, ctx, committed)
+
+    def _early(self, batch, cache_view) -> bool:
+        """Whether keys and values may go to the cache before the step's attention: where that writes over nothing the step still reads.  Whole
+        prompts read nothing from it, and sequences that go on read the step's own keys from its buffers; only in a ring a new key
+        takes an older one's place.  (A launch less: 5 us of 360 a layer for 400 tokens behind 1,500.)"""
+        return self.own_kv and not batch.all_decode and (batch.all_fresh or cache_view.group.ring == 0)
+
+    def _project_rotated(self, rt, h, batch, cache_view):
+        """Projection, rotation, split and append of a step of many rows in one product (``tc.gemm_qkv``): the arguments of ``_attend_step``, or
+        None where another form is the one."""
+        if not rt.is_bf16 or batch.all_decode or not self.own_kv or self.hd != 128:
+            return None
+        from ..ops import tc
+
+        table, rot = self.position.rotary_table()
+        if rot != 128 or not tc.takes_qkv(h.act, self.wqkv, getattr(rt, "forked", False)):
+            return None
+        T, early = batch.num_tokens, self._early(batch, cache_view)
+        # (a stream's own: branches of a layer run beside one another)
+        key = ("rope_angles", table.data_ptr(), cache_view.group.index if early else None, core._stream())
+        made = batch.memo.get(key) if batch.memo is not None else None
+        if made is None:
+            made = core.rope_angles(batch, table, 64, cache_view if early else None, rt.status)
+            if batch.memo is not None:
+                batch.memo[key] = made
+        q, k_new, v_new = rt.empty((T, self.nh, 128)), rt.empty((T, self.nkv, 128)), rt.empty((T, self.nkv, 128))
+        if not tc.gemm_qkv(h.act, self.wqkv, self.bqkv, *made, q, k_new, v_new, cache_view, nh=self.nh, nkv=self.nkv, status=rt.status):
+            return None
+        ctx = rt.empty((T, self.nh * self.hd))
+        if getattr(batch, "has_padding", False):
+            ctx.zero_()      # rows of no sequence are written by no attention kernel
+        return q, k_new, v_new, ctx, early
+
+    def _attend_step(self, rt, batch, cache_view, q, k_new, v_new, ctx, committed):
+        """Attention of a step of several tokens a sequence (or of a layer that reads another layer's cache), append, output projection."""
         if batch.all_decode:
             # a layer that reads another layer's cache: queries only
             core.attention_decode(q, cache_view, batch, ctx, nh=self.nh, window=self.window, scale=self.scale,

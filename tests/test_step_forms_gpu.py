@@ -189,3 +189,60 @@ def test_router_logits_of_nine_tokens_and_more(core, T, E, H, wdt):
     assert torch.allclose(probs.gather(1, idx.long()), torch.topk(probs, k, -1).values, rtol=2e-5)
     assert torch.allclose(w.double(), probs.gather(1, idx.long()), rtol=2e-5)
     assert torch.allclose(sg.double(), torch.sigmoid(h.double() @ wsg.double()), rtol=2e-5)
+
+
+@pytest.mark.parametrize("M,nh,nkv,K,bias,window", [(257, 4, 4, 264, True, None), (300, 7, 1, 512, False, None), (513, 3, 2, 136, True, 128),
+                                                    (3100, 2, 1, 520, True, None), (3073, 3, 3, 256, False, 256)])
+def test_queries_keys_and_values_in_one_product(core, M, nh, nkv, K, bias, window):
+    """The same as the product, then rotation, split and append, to the bit: single CTAs and pairs, an odd number of heads, a ring, rows of
+    no sequence, sequences that go on."""
+    from moe_b200.cache import KVCache, KVRequest
+    from moe_b200.ops import tc
+
+    torch.manual_seed(M)
+    x, w = torch.randn(M, K, device=DEV).bfloat16(), (torch.randn((nh + 2 * nkv) * 128, K, device=DEV) * K ** -0.5).bfloat16()
+    b = torch.randn((nh + 2 * nkv) * 128, device=DEV) if bias else None
+    freq = 10000.0 ** (-torch.arange(64, device=DEV, dtype=torch.float32) / 64)
+    lens, starts, st = [100, M - 107, 7], [0, 5, 77], core.new_status(DEV)
+    batch = G.make_batch(DEV, [1, 0, 2], starts, lens)
+    batch.seq_of_token[100 + 40] = -1
+    caches = []
+    for fused in (False, True):
+        cache = KVCache({0: KVRequest(nkv, 128, window)}, {0: None}, M + 1024, 3, torch.bfloat16, DEV)
+        for _ in range(3):
+            cache.acquire()
+        for slot, n0, n in zip([1, 0, 2], starts, lens):
+            G.give_pages(cache, slot, n0 + n)
+        cache.groups[0].storage.fill_(3.0)
+        view = cache.view(0)
+        q, k, v = (torch.full((M, n, 128), 9.0, device=DEV, dtype=torch.bfloat16) for n in (nh, nkv, nkv))
+        if fused:
+            angles, rows = core.rope_angles(batch, freq, 64, view, st)
+            assert tc.gemm_qkv(x, w, b, angles, rows, q, k, v, view, nh=nh, nkv=nkv, status=st)
+        else:
+            out = torch.empty(M, w.shape[0], device=DEV)
+            assert tc.gemm_tc(x, w, out, bias=b, bn=256, splits=1, status=st)
+            core.rope_split(out, batch.pos, freq, nh, nkv, 128, 128, q, k, v, commit=None)
+        caches.append((q, k, v, rows if fused else None))
+    for got, want in zip(caches[1][:3], caches[0][:3]):
+        assert torch.equal(got, want)
+    # the appended rows, each where the page table says
+    grp, rows = cache.groups[0], caches[1][3].tolist()
+    kc, vc = (t.reshape(-1, 128) for t in (view.k, view.v))
+    at, written = 0, {}
+    for i, (slot, s0, n) in enumerate(zip([1, 0, 2], starts, lens)):
+        for j in range(n):
+            t, pos = at + j, s0 + j
+            held = t != 140 and (grp.ring == 0 or pos >= s0 + n - grp.ring)
+            place = pos % grp.ring if grp.ring else pos
+            want = int(grp.table[slot, place // 64]) * nkv * 64 + place % 64 if held else -1
+            if t % 13 == 0 or n < 20:
+                assert rows[t] == want, (t, pos)
+            if rows[t] >= 0:
+                written[rows[t]] = t
+        at += n
+    for r, t in list(written.items())[::11]:
+        for h in range(nkv):
+            assert torch.equal(kc[r + h * 64], caches[1][1][t, h]) and torch.equal(vc[r + h * 64], caches[1][2][t, h])
+    untouched = kc.shape[0] - nkv * len(written)
+    assert int((kc == 3.0).all(-1).sum()) >= untouched and int(st[0]) == 0
