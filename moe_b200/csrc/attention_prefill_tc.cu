@@ -283,6 +283,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     auto x_bar = [&](int q) { return bars + 8u * (11 + q); };
 
     if (threadIdx.x == 0) {
+        auto prefetch_map = [](const CUtensorMap* m) { asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory"); };
+        prefetch_map(&tmQ), prefetch_map(&tmK), prefetch_map(&tmV);
+        if (n_cached > 0) prefetch_map(&tmKc), prefetch_map(&tmVc);
         mbar_init(q_full, 1);
         for (int i = 0; i < NST; i++) {
             mbar_init(k_full(i), 1);
@@ -474,7 +477,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                                             : (window <= 0 || j0 >= start + q0 + QT - window || (KEEP && j0 + KT <= keep)));
             auto tile_softmax = [&](auto masked_tag) -> bool {
                 constexpr bool MASKED = decltype(masked_tag)::value;
-                auto visible = [&](int j) { return j <= prow && j < jmax && (j >= lo_row || (KEEP && j < keep)); };
+                // the keys of this half row that the row sees, a bit each: positions up to its own, below jmax, from lo_row on (or kept ones).
+                // (One instruction a key and pass to look a bit up; three comparisons made the code of a masked tile half as long again,
+                // and a short prompt, one such tile a head, waits for its instructions.  8,192 tokens, 16 heads of 128: 478 -> 452 us.)
+                uint32_t seen[2];
+                if (MASKED) {
+                    auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; };      // bits 0 ... n - 1
+                    const int end = min(prow + 1, jmax) - jh, from = lo_row - jh;
+#pragma unroll
+                    for (int c = 0; c < 2; c++)
+                        seen[c] = below(end - 32 * c) & ~(below(from - 32 * c) & ~(KEEP ? below(keep - jh - 32 * c) : 0u));
+                }
+                auto visible = [&](int c, int i) { return (seen[c] >> i & 1u) != 0; };
                 float m_new = m, alpha = 1.f;
                 if (!sigmoid_w) {
                 // pass 1: the maximum of the half row (of the raw scores: the scale is positive)
@@ -488,8 +502,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     for (int c = 0; c < 2; c++) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 2) {
-                            if (!MASKED || visible(jh + c * 32 + i)) mx0 = fmaxf(mx0, s[c][i]);
-                            if (!MASKED || visible(jh + c * 32 + i + 1)) mx1 = fmaxf(mx1, s[c][i + 1]);
+                            if (!MASKED || visible(c, i)) mx0 = fmaxf(mx0, s[c][i]);
+                            if (!MASKED || visible(c, i + 1)) mx1 = fmaxf(mx1, s[c][i + 1]);
                         }
                     }
                 }
@@ -546,8 +560,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                         else
                             x0 = fmaf(sc[i], scale_log2, neg_m), x1 = fmaf(sc[i + 1], scale_log2, neg_m);
                         if (MASKED) {
-                            if (!visible(jh + c * 32 + i)) x0 = -INFINITY;
-                            if (!visible(jh + c * 32 + i + 1)) x1 = -INFINITY;
+                            if (!visible(c, i)) x0 = -INFINITY;
+                            if (!visible(c, i + 1)) x1 = -INFINITY;
                         }
                         // (sigmoid weights: 1 / (1 + 2^-(score + bias)), 0 for a key out of sight)
                         const float p0 = sigmoid_w ? __fdividef(1.0f, 1.0f + ex2_approx(-(x0 + bias_log2))) : ex2_approx(x0);
