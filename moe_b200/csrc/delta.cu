@@ -739,7 +739,7 @@ __global__ void __launch_bounds__(256, 2)
 delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
     constexpr int PK = NP + 4;
     __shared__ __align__(16) float sk[CC][PK], sq[CC][PK], sg[CH ? CC : 1][PK];
-    __shared__ __align__(16) double s_l[CC][CC], s_p[CC][CC];      // L, P, token j's column in row j; both 0 where j is later
+    __shared__ __align__(16) double s_l[CC][CC], s_p[CC][CC];      // L, P; both 0 where j is later
     __shared__ double s_beta[CC], s_lg[CC], s_eb[CC], s_er[CC];
     __shared__ int s_seq;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, at_chunk = blockIdx.x, number = wk.first + at_chunk, h = blockIdx.y;
@@ -818,39 +818,34 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
             dot *= exp(between);
         }
         if (lane < 16)
-            s_l[j][i] = i > j ? s_beta[i] * dot : 0.;
+            s_l[i][j] = i > j ? s_beta[i] * dot : 0.;
         else
-            s_p[j][i] = i >= j ? dot : 0.;
+            s_p[i][j] = i >= j ? dot : 0.;
     }
     __syncthreads();
-    // Both go through the columns, so that a step's terms are for different tokens: row by row every term waits for the one before, 256 of them
-    // one after the other.  A token's terms are added in the same order either way.
-    double x[CC], r[CC];
+    double x[CC];
     auto solve = [&]() {               // x <- (I + L)^-1 x
 #pragma unroll
-        for (int j = 0; j < CC - 1; j++) {
+        for (int i = 1; i < CC; i++) {
             asm volatile("" ::: "memory");       // (or all of L is fetched first)
 #pragma unroll
-            for (int i = (j + 1) & ~1; i < CC; i += 2) {
-                const double2 l2 = *reinterpret_cast<const double2*>(&s_l[j][i]);
-                if (i > j) x[i] = fma(-l2.x, x[j], x[i]);
-                x[i + 1] = fma(-l2.y, x[j], x[i + 1]);
+            for (int j = 0; j < i; j += 2) {
+                const double2 l2 = *reinterpret_cast<const double2*>(&s_l[i][j]);
+                x[i] = fma(-l2.x, x[j], x[i]);
+                if (j + 1 < i) x[i] = fma(-l2.y, x[j + 1], x[i]);
             }
         }
     };
-    auto pair_sums = [&]() {           // r <- P x
+    auto pair_sum = [&](int i) {       // (P x)_i
+        double r = 0.;
 #pragma unroll
-        for (int i = 0; i < CC; i++) r[i] = 0.;
-#pragma unroll
-        for (int j = 0; j < CC; j++) {
-            asm volatile("" ::: "memory");
-#pragma unroll
-            for (int i = j & ~1; i < CC; i += 2) {
-                const double2 p2 = *reinterpret_cast<const double2*>(&s_p[j][i]);
-                if (i >= j) r[i] = fma(p2.x, x[j], r[i]);
-                r[i + 1] = fma(p2.y, x[j], r[i + 1]);
+        for (int j = 0; j < CC; j += 2)
+            if (j <= i) {
+                const double2 p2 = *reinterpret_cast<const double2*>(&s_p[i][j]);
+                r = fma(p2.x, x[j], r);
+                if (j + 1 <= i) r = fma(p2.y, x[j + 1], r);
             }
-        }
+        return r;
     };
     if (tid < NP) {
         const int c = tid, at = chunk_place(c);
@@ -869,13 +864,12 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
             if (CH) since *= sg[CH ? i : 0][c];
         }
         solve();
-        pair_sums();
         all = 1.;
 #pragma unroll
         for (int i = 0; i < CC; i++) {
             asm volatile("" ::: "memory");
             if (CH) all *= sg[CH ? i : 0][c]; else all = s_eb[i];
-            const double q = sq[i][c] * all - r[i];
+            const double q = sq[i][c] * all - pair_sum(i);
             if (i < cnt) wk.w[row + i * pitch + at] = (float)x[i], wk.q[row + i * pitch + at] = (float)q;
         }
     } else {
@@ -884,12 +878,12 @@ delta_chunk_kernel(const DeltaSeq p, const DeltaWork wk, int num_seqs) {
 #pragma unroll
             for (int i = 0; i < CC; i++) x[i] = i < cnt ? s_beta[i] * v[(size_t)i * channels] : 0.;
             solve();
-            pair_sums();
             const size_t row = ((size_t)at_chunk * CC * p.H + h) * dv + c, pitch = (size_t)p.H * dv;
 #pragma unroll
             for (int i = 0; i < CC; i++) {
                 asm volatile("" ::: "memory");
-                if (i < cnt) wk.u[row + i * pitch] = (float)x[i], wk.pu[row + i * pitch] = (float)r[i];
+                const double r = pair_sum(i);
+                if (i < cnt) wk.u[row + i * pitch] = (float)x[i], wk.pu[row + i * pitch] = (float)r;
             }
         }
     }
