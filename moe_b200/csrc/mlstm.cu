@@ -644,10 +644,11 @@ mlstm_chunk_state_kernel(const MemSeq p, const MemChunks c) {
 // grid (chunks, heads, ceil(dv / 128)): the pair products of a chunk, 4 x 4 a thread; the outputs, 4 rows x 8 columns a thread.
 // The pair products and n . q are sums in 64 bits: an output is divided by n . q, which cancels, and whatever is lost in it
 // counts as often as that is small beside its terms.  An output's own error (the median over tokens) is 0.7 - 0.8 of the
-// form's of four tokens; with 32-bit sums throughout, 118 us instead of 139, it was 1.2 - 1.3 times that.
+// form's of four tokens; with 32-bit sums throughout it was 1.2 - 1.3 times that.
 constexpr int QP = QC + 4;
-// The state takes the keys' place once the pair products are formed, and a thread's outputs take one set of accumulators, so that an SM
-// holds two blocks (keys of up to 64): one hides the other's loads (2,048 tokens 119 -> 87 us).
+// The state takes the keys' place once the pair products are formed, and a thread's own sums wait in the place of the values while the
+// carried ones take the same accumulators, so that an SM holds two blocks (keys of up to 64): one hides the other's loads (2,048 tokens
+// of 16 heads of 64 x 128: 119.5 us with one block, 88.5 with two).
 __host__ __device__ constexpr size_t mlstm_chunk_out_floats(int d) {
     const size_t keys = (size_t)QC * (d + 4), state = (size_t)d * (QV + 4);
     return keys + (keys > state ? keys : state) + QC * QP + QC * (QV + 4) + d;
@@ -760,20 +761,15 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
         __syncwarp();
         if (part == 0) s_den[i] = fmaxf(fabsf((float)fma(s_all[i], held, s_in[i])), s_den[i]) + READ_EPS;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                   // the state is there, and the denominators
-    float acc[4][8], all[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        all[i] = (float)s_all[ty + 16 * i];
-#pragma unroll
-        for (int e = 0; e < 8; e++) acc[i][e] = 0.f;
-    }
+    float acc[4][8];
     // Sixteen terms at a time, then their sums (one accumulator over 64 or 128 terms would be about twice as far off).
-    // OWN: the chunk's own terms, onto what the state before it gives times the decay since; row i takes the right side's rows up to i,
-    // later ones not even with a factor of 0
-    auto product = [&](auto own, const float* left, int pitch, int n, const float* right) {
-        constexpr bool OWN = decltype(own)::value;
+    // CAUSAL: row i takes the right side's rows up to i, later ones not even with a factor of 0
+    auto product = [&](auto causal, const float* left, int pitch, int n, const float* right) {
+        constexpr bool CAUSAL = decltype(causal)::value;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int e = 0; e < 8; e++) acc[i][e] = 0.f;
 #pragma unroll 1
         for (int x0 = 0; x0 < n; x0 += 16) {
             float part[4][8];
@@ -793,7 +789,7 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
                     const float v[8] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        if (OWN && x + z > ty + 16 * i) continue;
+                        if (CAUSAL && x + z > ty + 16 * i) continue;
                         const float f = z == 0 ? a[i].x : z == 1 ? a[i].y : z == 2 ? a[i].z : a[i].w;
 #pragma unroll
                         for (int e = 0; e < 8; e++) part[i][e] = fmaf(f, v[e], part[i][e]);
@@ -803,22 +799,34 @@ mlstm_chunk_out_kernel(const MemSeq p, const MemChunks c, int num_seqs, float* _
 #pragma unroll
             for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int e = 0; e < 8; e++) acc[i][e] = OWN && x0 == 0 ? fmaf(all[i], acc[i][e], part[i][e]) : acc[i][e] + part[i][e];
+                for (int e = 0; e < 8; e++) acc[i][e] += part[i][e];
         }
     };
-    product(std::false_type(), sq, dp, d, sS);
+    // The chunk's own terms, which a thread then leaves in the place of the values until the carried ones are formed: the two sums meet
+    // once, so that small terms of a chunk are not lost one by one beside a large state.
     product(std::true_type(), sP, QP, QC, sv);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                   // the state is there, the denominators too, and the values are no longer read
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float* own = sv + (ty + 16 * i) * (QV + 4) + tx * 4;
+        *reinterpret_cast<float4*>(own) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        *reinterpret_cast<float4*>(own + 64) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    }
+    product(std::false_type(), sq, dp, d, sS);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int t = ty + 16 * i;
         if (t >= cnt) continue;
-        const float den = s_den[t];
+        const float all = (float)s_all[t], den = s_den[t];
         float* dst = o + ((size_t)(tok + t) * p.H + h) * dv + c0;
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int x = e * 64 + tx * 4;
+            const float4 own = *reinterpret_cast<const float4*>(sv + t * (QV + 4) + x);
             if (x < ncols)
-                *reinterpret_cast<float4*>(dst + x) = make_float4(acc[i][4 * e] / den, acc[i][4 * e + 1] / den, acc[i][4 * e + 2] / den, acc[i][4 * e + 3] / den);
+                *reinterpret_cast<float4*>(dst + x) = make_float4(fmaf(all, acc[i][4 * e], own.x) / den, fmaf(all, acc[i][4 * e + 1], own.y) / den,
+                                                                  fmaf(all, acc[i][4 * e + 2], own.z) / den, fmaf(all, acc[i][4 * e + 3], own.w) / den);
         }
     }
 }

@@ -326,6 +326,35 @@ def test_the_memory_over_chunks_is_no_further_off_than_four_at_a_time(core, forg
     assert chunks <= 1.02 * four, (chunks, four)
 
 
+@pytest.mark.parametrize("d,dv", [(64, 128), (12, 260), (128, 36)])
+def test_a_chunks_own_terms_of_the_memory_are_added_up_before_they_meet_the_carried_state(core, d, dv):
+    """Gates of exactly 1, queries and keys along one channel: an output is (carried + own) over one denominator, where sixteen own terms are
+    less than half a unit in the carried state's last place and sixty-four are several.  In 32 bits to the bit: products with
+    a power of two are exact, so the sums alone round."""
+    H, n = 2, 64
+    at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
+    proj = torch.zeros(n, -(-(at["f"] + H) // 4) * 4, device=DEV)
+    for h in range(H):
+        proj[:, at["q"] + h * d], proj[:, at["k"] + h * d] = 1.0, 2.0 ** -10       # |n . q| <= 2^-4, so the denominator is 1 + 1e-6
+    g = torch.Generator(device=DEV).manual_seed(d)
+    v = 1024 * (0.05 + 0.0125 * torch.rand(n, H * dv, device=DEV, generator=g))
+    proj[:, at["v"]:at["v"] + H * dv] = v
+    proj[:, at["f"]:at["f"] + H] = 1e4                                             # log f = -log(1 + e^-100): f = 1
+    zero = torch.zeros(H, device=DEV)
+    state, o = torch.zeros(2, -(-core.mlstm_state_floats(H, d, dv) // 4) * 4, device=DEV), torch.empty(n, H * dv, device=DEV)
+    state[1, :H * d * dv].view(H, d, dv)[:, 0] = 2.0 ** 24
+    core.mlstm_scan(proj, at, zero, zero, 100.0, 1.0, state, G.make_batch(DEV, [1], [0], [n]), o, heads=H, d=d, dv=dv, chunks=True)
+    terms, own, want = v.cpu() * 2.0 ** -10, torch.zeros(n, H * dv), torch.empty(n, H * dv)
+    for t in range(n):
+        for x0 in range(0, t + 1, 16):
+            part = torch.zeros(H * dv)
+            for x in range(x0, min(x0 + 16, t + 1)):
+                part = part + terms[x]
+            own[t] = own[t] + part
+        want[t] = (own[t] + 2.0 ** 24) / (torch.ones(()) + torch.tensor(1e-6))
+    assert float(own[15].max()) < 1.01 and float(own[63].min()) > 3 and torch.equal(o.cpu(), want)
+
+
 def test_segments_asked_for_by_the_environment_reach_the_memory(core, monkeypatch):
     H, d, dv, n = 2, 64, 128, 600
     at = {"q": 0, "k": H * d, "v": 2 * H * d, "i": 2 * H * d + H * dv, "f": 2 * H * d + H * dv + H}
