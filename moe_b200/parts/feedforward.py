@@ -384,8 +384,10 @@ class RoutedExperts(Part):
         """The block's offer to take the norm before this feed-forward along: for a step of few
         tokens, norm, router and dispatch are one launch.  None if the sizes or the kind of norm do
         not allow it (the block then runs the norm itself and calls ``forward``)."""
-        if x.shape[0] >= self.tc_router_tokens and self.split_router and not self.weight_input:
-            # a prompt: the norm leaves the three terms that the router's product reads, and no 32-bit row
+        if (x.shape[0] >= self.tc_router_tokens and self.split_router and not self.weight_input
+                and x.shape[0] > self.fused_norm_tokens and not self._picks_in_one_block(x.shape[0])):
+            # a prompt: the norm leaves the three terms that the router's product reads, and no 32-bit row (which the forms of few tokens
+            # read, whatever the environment says where they end)
             split = getattr(norm, "forward_split", None)
             h = split(rt, x, delta) if split is not None else None
             return None if h is None else self._run(rt, h, batch, None)
@@ -474,6 +476,9 @@ class RoutedExperts(Part):
         if self.trace is not None:
             self.trace.append((topk_idx.clone(), topk_w.clone()))
 
+    def _picks_in_one_block(self, T: int) -> bool:
+        return T <= 64 and self.E <= 256 and T <= self.route_dispatch_tokens and not self.table
+
     def _routed(self, rt, h, batch, routed, picked, after_logits=None):
         """The routed experts' outputs, not combined yet.  ``routed``: what ``core.norm_route`` returned behind the two norms, or None;
         ``picked`` is called with the picks and their weights, ``after_logits`` once the logits' product is launched."""
@@ -481,7 +486,7 @@ class RoutedExperts(Part):
         P = T * self.k
         if routed is not None:
             topk_idx, topk_w, sg, offsets, sorted_token, pos_of_pair, xs = routed
-        elif T <= 64 and self.E <= 256 and T <= self.route_dispatch_tokens and not self.table:
+        elif self._picks_in_one_block(T):
             # pick, table inversion and gather in one launch after the logits
             topk_idx, topk_w, sg, offsets, sorted_token, pos_of_pair, xs = core.route_dispatch(
                 h.f32, self.w_router, self.k, self.norm_topk, self.scale, shared_gate_w=self.w_sgate,

@@ -130,6 +130,29 @@ def test_routed_experts_part(dt, E, k, norm, shared, scale):
     assert int(rt.status[0]) == 0
 
 
+@pytest.mark.parametrize("T,from_,one_block", [(5, 4, 8), (8, 1, 8), (30, 16, 64), (64, 9, 64), (40, 9, 8)])
+def test_routed_experts_behind_a_norm_where_the_tensor_core_router_starts_early(T, from_, one_block):
+    """MOE_B200_TC_ROUTER_MIN and MOE_B200_ROUTE_DISPATCH_MAX may overlap: the forms of few tokens, which read the 32-bit row, go first."""
+    from moe_b200.config.spec import PartSpec
+    from moe_b200.parts import make_part
+
+    H, dt = 56, torch.bfloat16
+    params = {"hidden_size": H, "num_experts": 6, "top_k": 2, "expert_size": 24, "norm_topk_prob": True, "shared_size": 40, "shared_gate": True}
+    part, _, rt = build("ffn", "routed_experts", params, dt)
+    norm = make_part("norm", PartSpec("rmsnorm", {"size": H, "eps": 1e-6}, "n."))
+    norm.bind({"weight": torch.ones(H, device=DEV)}, rt)
+    x0, delta, batch = torch.randn(T, H, device=DEV), torch.randn(T, H, device=DEV), G.make_batch(DEV, [0], [0], [T])
+    want = part.forward(rt, norm.forward(rt, x0.clone(), delta=delta, want32=True), batch)
+    part.tc_router_tokens, part.route_dispatch_tokens = from_, one_block
+    x = x0.clone()
+    got = part.forward_prenorm(rt, x, delta, norm, batch)
+    if got is None:
+        got = part.forward(rt, norm.forward(rt, x, delta=delta, want32=True), batch)
+    else:
+        got = got.materialize(rt)
+    assert torch.equal(x, x0 + delta) and rel(got, want.double().cpu()) < tol(dt) and int(rt.status[0]) == 0
+
+
 @pytest.mark.parametrize("dt", DTYPES)
 def test_embedding_and_head_parts(dt):
     emb, ref, rt = build("embedding", "token_embedding", {"vocab_size": 77, "hidden_size": 40}, dt)
