@@ -99,21 +99,22 @@ router_logits_kernel(const float* __restrict__ h, const WT* __restrict__ wr, con
     }
 }
 
-// The same product for 65 to 256 tokens, hidden a multiple of 8: a block takes 4 tokens and 16 router rows, a warp two of the rows.  What bounds
+// The same product for 65 tokens and more, hidden a multiple of 8: a block takes 4 tokens and 16 router rows, a warp two of the rows.  What bounds
 // it is the chain of loads, so all rows of the block's tokens are asked for at once (cp.async; a row's 16-byte units of even and of odd
 // number lie apart, so that a lane's 8 elements are two reads without bank conflicts) and a lane's weights in batches of eight, asked into
-// L2 before the wait.  A lane's elements and the order of its sums are those of router_logits_kernel with KSPLIT = 1.  (Not for fewer tokens:
-// its shared memory does not fit beside the shared expert's CTAs of a decode step.)  128 rows, 6 layers: a pass 1,746 -> 1,665 us
-// against staging the tokens in chunks of 512 features, a barrier each.  Grid: (ceil(rows / 16), ceil(T / 4)).
-constexpr int RS_TOKENS = 4, RS_ROWS = 16;
-template <typename WT>
+// L2 before the wait.  Rows of more than RS_WIDTH features, which shared memory does not hold, come in slabs.  A lane's elements and the order
+// of its sums are those of router_logits_kernel with KSPLIT = 1.  (Not for fewer tokens: its shared memory does not fit beside the shared
+// expert's CTAs of a decode step.)  Grid: (ceil(rows / 16), ceil(T / 4)).  Measured, us, tokens staged in chunks of 512 features with a barrier
+// each / this way, 61 bfloat16 rows: 2,048 features 65, 256, 2,048 tokens 17.4 / 4.6, 17.5 / 7.5, 95 / 45; 8,192 features 60 / 13, 60 / 27, 369 /
+// 195; 16,384 features (two slabs) 116 / 26, 117 / 54, 720 / 385, where rows read from global memory take 72, 157, 781.
+constexpr int RS_TOKENS = 4, RS_ROWS = 16, RS_WIDTH = 12288;
+template <typename WT, bool SLABS>
 __global__ void __launch_bounds__(256)
 router_logits_staged_kernel(const float* __restrict__ h, const WT* __restrict__ wr, const WT* __restrict__ wsg,
                             int num_tokens, int hidden, int num_experts, int rows, float* __restrict__ logits) {
-    extern __shared__ __align__(16) float4 rs_x[];           // [RS_TOKENS][even | odd units][hidden / 8]
+    extern __shared__ __align__(16) float4 rs_x[];           // [RS_TOKENS][even | odd units][a slab's features / 8]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r0 = blockIdx.x * RS_ROWS + warp * 2, t0 = blockIdx.y * RS_TOKENS, nt = min(RS_TOKENS, num_tokens - t0);
-    const int groups = hidden / 8;
     const WT* w[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -122,52 +123,57 @@ router_logits_staged_kernel(const float* __restrict__ h, const WT* __restrict__ 
         for (int c = lane * (128 / (int)sizeof(WT)); c < hidden; c += 32 * (128 / (int)sizeof(WT))) prefetch_l2(w[q] + c);
     }
     pdl_sync();
-    for (int e = threadIdx.x; e < RS_TOKENS * 2 * groups; e += blockDim.x) {
-        const int i = e / (2 * groups), u = e % (2 * groups);
-        const bool on = i < nt;
-        const float* src = h + (size_t)(t0 + (on ? i : 0)) * hidden + u * 4;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                     ::"r"((unsigned)__cvta_generic_to_shared(rs_x + (i * 2 + (u & 1)) * groups + (u >> 1))), "l"(src), "r"(on ? 16 : 0) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    if (r0 >= rows) return;
     constexpr int UNITS = sizeof(WT) / 2, MB = 8 / UNITS;       // 16-byte units of 8 elements; a lane's groups in flight at a time
     float acc[2][RS_TOKENS];
 #pragma unroll
     for (int q = 0; q < 2; q++)
 #pragma unroll
         for (int i = 0; i < RS_TOKENS; i++) acc[q][i] = 0.f;
-    for (int g0 = lane; g0 < groups; g0 += 32 * MB) {
-        uint4 raw[MB][2][UNITS];
-#pragma unroll
-        for (int m = 0; m < MB; m++) {
-            const int g = min(g0 + 32 * m, groups - 1);         // (past the end: read, not used)
-#pragma unroll
-            for (int q = 0; q < 2; q++)
-#pragma unroll
-                for (int u = 0; u < UNITS; u++) raw[m][q][u] = __ldg(reinterpret_cast<const uint4*>(w[q] + g * 8) + u);
+    for (int c0 = 0; c0 < (SLABS ? hidden : 1); c0 += RS_WIDTH) {      // (whole rounds of 32 lanes: a lane's elements are its own throughout)
+        const int groups = (SLABS ? min(RS_WIDTH, hidden - c0) : hidden) / 8;
+        if (c0) __syncthreads();
+        for (int e = threadIdx.x; e < RS_TOKENS * 2 * groups; e += blockDim.x) {
+            const int i = e / (2 * groups), u = e % (2 * groups);
+            const bool on = i < nt;
+            const float* src = h + (size_t)(t0 + (on ? i : 0)) * hidden + c0 + u * 4;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                         ::"r"((unsigned)__cvta_generic_to_shared(rs_x + (i * 2 + (u & 1)) * groups + (u >> 1))), "l"(src), "r"(on ? 16 : 0) : "memory");
         }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (r0 >= rows) continue;
+        for (int g0 = lane; g0 < groups; g0 += 32 * MB) {
+            uint4 raw[MB][2][UNITS];
 #pragma unroll
-        for (int m = 0; m < MB; m++) {
-            const int g = g0 + 32 * m;
-            if (g >= groups) continue;
-            float wv[2][8];
+            for (int m = 0; m < MB; m++) {
+                const int g = min(g0 + 32 * m, groups - 1);         // (past the end: read, not used)
 #pragma unroll
-            for (int q = 0; q < 2; q++) w_load8<WT>(reinterpret_cast<const WT*>(raw[m][q]), wv[q]);
+                for (int q = 0; q < 2; q++)
 #pragma unroll
-            for (int i = 0; i < RS_TOKENS; i++) {
-                const float4 a = rs_x[i * 2 * groups + g], b = rs_x[(i * 2 + 1) * groups + g];
+                    for (int u = 0; u < UNITS; u++) raw[m][q][u] = __ldg(reinterpret_cast<const uint4*>(w[q] + c0 + g * 8) + u);
+            }
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    float v = acc[q][i];
-                    v = fmaf(a.x, wv[q][0], v), v = fmaf(a.y, wv[q][1], v), v = fmaf(a.z, wv[q][2], v), v = fmaf(a.w, wv[q][3], v);
-                    v = fmaf(b.x, wv[q][4], v), v = fmaf(b.y, wv[q][5], v), v = fmaf(b.z, wv[q][6], v), v = fmaf(b.w, wv[q][7], v);
-                    acc[q][i] = v;
+            for (int m = 0; m < MB; m++) {
+                const int g = g0 + 32 * m;
+                if (g >= groups) continue;
+                float wv[2][8];
+#pragma unroll
+                for (int q = 0; q < 2; q++) w_load8<WT>(reinterpret_cast<const WT*>(raw[m][q]), wv[q]);
+#pragma unroll
+                for (int i = 0; i < RS_TOKENS; i++) {
+                    const float4 a = rs_x[i * 2 * groups + g], b = rs_x[(i * 2 + 1) * groups + g];
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        float v = acc[q][i];
+                        v = fmaf(a.x, wv[q][0], v), v = fmaf(a.y, wv[q][1], v), v = fmaf(a.z, wv[q][2], v), v = fmaf(a.w, wv[q][3], v);
+                        v = fmaf(b.x, wv[q][4], v), v = fmaf(b.y, wv[q][5], v), v = fmaf(b.z, wv[q][6], v), v = fmaf(b.w, wv[q][7], v);
+                        acc[q][i] = v;
+                    }
                 }
             }
         }
     }
+    if (r0 >= rows) return;
     float total[2][RS_TOKENS];
 #pragma unroll
     for (int q = 0; q < 2; q++)
@@ -1095,14 +1101,15 @@ static int router_logits_impl(const float* h, const void* wr, const void* wsg, i
         }
         const size_t n = (size_t)num_tokens * rows;
         sum_slices_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(scratch, logits, n, slices);
-    } else if (vec_ok && num_tokens > 64 && hidden <= 12288 && (num_tokens + RS_TOKENS - 1) / RS_TOKENS <= 65535) {
+    } else if (vec_ok && num_tokens > 64 && (num_tokens + RS_TOKENS - 1) / RS_TOKENS <= 65535) {
         const dim3 sg((rows + RS_ROWS - 1) / RS_ROWS, (num_tokens + RS_TOKENS - 1) / RS_TOKENS);
-        const int smem = RS_TOKENS * hidden * (int)sizeof(float);
+        const int smem = RS_TOKENS * (hidden < RS_WIDTH ? hidden : RS_WIDTH) * (int)sizeof(float);
 #define STAGED(WT)                                                                                                     \
     do {                                                                                                               \
-        cudaError_t e = cudaFuncSetAttribute(router_logits_staged_kernel<WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); \
+        const auto kernel = hidden > RS_WIDTH ? router_logits_staged_kernel<WT, true> : router_logits_staged_kernel<WT, false>; \
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);               \
         if (e != cudaSuccess) return (int)e;                                                                           \
-        return launch_pdl(router_logits_staged_kernel<WT>, sg, 256, (size_t)smem, stream, h, (const WT*)wr, (const WT*)wsg, \
+        return launch_pdl(kernel, sg, 256, (size_t)smem, stream, h, (const WT*)wr, (const WT*)wsg,                     \
                           num_tokens, hidden, num_experts, rows, logits);                                              \
     } while (0)
         if (w_dt == DT_F32) STAGED(float);

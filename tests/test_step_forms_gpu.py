@@ -191,6 +191,22 @@ def test_router_logits_of_nine_tokens_and_more(core, T, E, H, wdt):
     assert torch.allclose(sg.double(), torch.sigmoid(h.double() @ wsg.double()), rtol=2e-5)
 
 
+@pytest.mark.parametrize("T,E", [(65, 17), (256, 128), (131, 1), (301, 33)])
+@pytest.mark.parametrize("H", [12280, 12288, 12296, 24576, 24840])
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+def test_router_logits_of_rows_wider_than_shared_memory(core, T, E, H, wdt):
+    """One slab of 12,288 features and several, the last one of one unit; without scratch, which 257 tokens and more otherwise use."""
+    torch.manual_seed(T + H)
+    h, wr, wsg = torch.randn(T, H, device=DEV), (torch.randn(E, H, device=DEV) * H ** -0.5).to(wdt), torch.randn(H, device=DEV).to(wdt)
+    out = torch.full((T, E + 1), float("nan"), device=DEV)
+    core._ok(core.lib().moe_router_logits(core._p(h), core._p(wr), core._p(wsg), core._dt(wr), T, H, E, core._p(out), None, 0,
+                                          core._stream()), "router_logits")
+    rows = torch.cat([wr, wsg[None]]).double().T
+    # a lane adds H / 32 products, the lanes' sums meet in five steps: each rounds by half a unit of at most all terms' size
+    bound = (H / 32 + 5) * 2.0 ** -24 * (h.double().abs() @ rows.abs())
+    assert bool(((out.double() - h.double() @ rows).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("M,nh,nkv,K,bias,window", [(257, 4, 4, 264, True, None), (300, 7, 1, 512, False, None), (513, 3, 2, 136, True, 128),
                                                     (3100, 2, 1, 520, True, None), (3073, 3, 3, 256, False, 256)])
 def test_queries_keys_and_values_in_one_product(core, M, nh, nkv, K, bias, window):
