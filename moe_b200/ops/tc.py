@@ -219,13 +219,12 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, swiglu: bool
     return True
 
 
-def takes_qkv(x: torch.Tensor, w: torch.Tensor, beside: bool) -> bool:
-    """Whether ``gemm_qkv`` is the form for this projection: where ``gemm_tc`` would take the persistent form with tiles of 256 rows, from 1,280 rows
-    on.  (us, product and rotation one by one / in one: 48 heads of 2,048 features 1,024 rows 43.0 / 39.8, 1,536 47.9 / 43.8, 2,048 68.2 / 55.4,
-    8,192 222 / 199; 36 heads of 3,584 features 1,024 rows 40.2 / 41.8, 1,280 66.1 / 64.4, 8,192 248 / 203; 768 rows 27.5 / 29.3.)"""
-    M = x.shape[0]
-    return (x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and M >= 1280
-            and (beside or not mid_splits(M, -(-w.shape[0] // 128), -(-w.shape[1] // 64), num_sms(x.device))))
+def takes_qkv(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``gemm_qkv`` is the form for this projection: in bfloat16 from 1,280 rows on, where ``gemm_tc`` takes the persistent form with
+    tiles of 256 rows.  (us, product and rotation one by one / in one: 48 heads of 2,048 features 1,024 rows 43.0 / 39.8, 1,536 47.9 / 43.8,
+    2,048 68.2 / 55.4, 8,192 222 / 199; 36 heads of 3,584 features 1,024 rows 40.2 / 41.8, 1,280 66.1 / 64.4, 8,192 248 / 203; 768 rows 27.5 /
+    29.3.)"""
+    return x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[0] >= 1280
 
 
 def gemm_qkv(x, w, bias, angles, rows, q, k, v, view, *, nh: int, nkv: int, status) -> bool:

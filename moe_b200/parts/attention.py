@@ -474,7 +474,7 @@ class GQAttention(Part):
         from ..ops import tc
 
         table, rot = self.position.rotary_table()
-        if rot != 128 or not tc.takes_qkv(h.act, self.wqkv, getattr(rt, "forked", False)):
+        if rot != 128 or not tc.takes_qkv(h.act, self.wqkv):
             return None
         T, early = batch.num_tokens, self._early(batch, cache_view)
         # (a stream's own: branches of a layer run beside one another)
