@@ -275,22 +275,26 @@ static inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 b
 }
 
 // ---- thread-block clusters -------------------------------------------------------------------
-__device__ __forceinline__ unsigned cl_rank() {
-    unsigned r;
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// all threads of all CTAs of the cluster; orders shared-memory writes before it against reads after
-__device__ __forceinline__ void cl_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// all threads of all CTAs of the cluster; orders shared-memory writes before it against reads after, in two halves and whole
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync_all() {
+    cluster_arrive();
+    cluster_wait();
 }
-// the 32-bit word at the same shared-memory address in CTA `rank` of the cluster
-__device__ __forceinline__ unsigned cl_peer_u32(const void* local, unsigned rank) {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(local);
-    unsigned pa, v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(pa) : "r"(a), "r"(rank));
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(pa) : "memory");
-    return v;
+// address of the same shared-memory location in the CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa_cluster(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
 
 // The rotation of one pair (a at i, b at i + half) by the angle whose cosine and sine are cs, sn:

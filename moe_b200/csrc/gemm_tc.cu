@@ -174,28 +174,7 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar), "l"(policy)
         : "memory");
 }
-// ---- thread-block clusters (the K splits of one tile) ----
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// (the same in two halves)
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// address of the same shared-memory location in the CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t mapa_cluster(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
+// ---- thread-block clusters (the K splits of one tile; the rest is in common.cuh) ----
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
@@ -347,7 +326,7 @@ struct Cfg {
 // sequence, 6 layers: 478 us, 488 where every CTA reads its peers' memory instead.
 // false: the wait for the accumulator ran out (the barriers are passed all the same).
 template <int BN, int MODE>
-__device__ __forceinline__ bool cluster_epilogue(const Params& p, uint32_t base, float* stage, const float* recv, uint32_t tmem, uint32_t acc_bar,
+__device__ __forceinline__ bool cluster_epilogue(const Params& p, float* stage, const float* recv, uint32_t tmem, uint32_t acc_bar,
                                                  volatile int* s_abort, int n0, int row0, int rows_here, int quarter, int lane) {
     using C = Cfg<BN, MODE>;
     constexpr int NW = C::NW, ROW = NW * TILE_W;
@@ -614,7 +593,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         }
     } else if (push) {
         uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
-        if (!cluster_epilogue<BN, MODE>(p, base, reinterpret_cast<float*>(aligned), reinterpret_cast<const float*>(aligned + C::STAGES * C::STAGE_BYTES + 256),
+        if (!cluster_epilogue<BN, MODE>(p, reinterpret_cast<float*>(aligned), reinterpret_cast<const float*>(aligned + C::STAGES * C::STAGE_BYTES + 256),
                                         tmem, acc_bar, &s_abort, n0, row0, rows_tile, warp & 3, lane) && lane == 0) {
             atomicOr(p.status, ST_WAIT_TIMEOUT);
             s_abort = 1;

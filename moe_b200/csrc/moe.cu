@@ -706,14 +706,6 @@ __device__ __noinline__ void route_token_once(const float* lg, float* sc, int la
                                               float* gate, float* wk) {
     route_token(lg, sc, lane, padding, p->num_experts, p->rows, p->top_k, p->norm_topk, p->scale, idx, w, gate, wk, nullptr, p->groups, p->keep);
 }
-__device__ __forceinline__ unsigned peer_addr(const void* local, unsigned rank) {
-    unsigned pa;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(pa) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
-    return pa;
-}
-__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 template <typename WT, bool POST>
 __global__ void __launch_bounds__(NRC_THREADS) norm_route_cluster_kernel(const __grid_constant__ NormRouteParams p) {
     extern __shared__ __align__(16) float nr_smem[];
@@ -731,7 +723,7 @@ __global__ void __launch_bounds__(NRC_THREADS) norm_route_cluster_kernel(const _
     float* gate = w_pick + pairs;                      // [T]
     int* picks = reinterpret_cast<int*>(gate + T);     // [pairs]
     int* place = picks + pairs;                        // [pairs]
-    cl_arrive();                                       // (a peer's memory may be written once it runs)
+    cluster_arrive();                                       // (a peer's memory may be written once it runs)
     const float* norm_w = POST ? p.post_w : p.norm_w;
     prefetch_router<WT>(p, rank, B, norm_w);
     constexpr int NV = 4;
@@ -795,17 +787,17 @@ __global__ void __launch_bounds__(NRC_THREADS) norm_route_cluster_kernel(const _
         for (int j = threadIdx.x + NV * blockDim.x; j < H; j += blockDim.x) one(j, norm_w[j]);
     }
     __syncthreads();
-    cl_wait();
+    cluster_wait();
 
     // ---- the router's logits, into everybody's shared memory ------------------------------------
     if (warp == nwarps - 1 && warp * C + part >= p.rows)       // (a warp without a router row: see above)
         route_token_once(all, sc, lane, false, &p, picks, w_pick, gate, wk);
     router_rows<WT>(p, row, warp * C + part, nwarps * C, lane, [&](int r, float v) {
-        if (lane < B) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_addr(all + t * p.rows + r, (unsigned)lane)), "f"(v) : "memory");
+        if (lane < B) st_cluster_f32(mapa_cluster((uint32_t)__cvta_generic_to_shared(all + t * p.rows + r), (uint32_t)lane), v);
     });
     __syncwarp();
-    cl_arrive();
-    cl_wait();                                         // (and all blocks of a token have read its row of the stream)
+    cluster_arrive();
+    cluster_wait();                                         // (and all blocks of a token have read its row of the stream)
     if (warp < T)
         route_token_once(all + warp * p.rows, sc + warp * E, lane, p.seq_of_token && p.seq_of_token[warp] < 0, &p, picks + warp * p.top_k,
                          w_pick + warp * p.top_k, p.shared_gate ? gate + warp : nullptr, wk + warp * p.top_k);
