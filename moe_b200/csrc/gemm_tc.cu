@@ -154,7 +154,8 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 }
 // The same with a say in what stays in L2.  Weights that one CTA reads once go first: a step streams more of them than L2 holds, and
 // what it pushes out otherwise are activations, the small weights and the kernels' instructions, which the chain of small kernels waits for.
-// (us a step of 6 layers, without / with: one sequence 509 / 478, eight 970 / 954, sixty-four 1,922 / 1,884, prompts of 113 tokens 1,675 / 1,635.)
+// (us a step of 6 layers, without / with: one sequence 486 / 463, eight 917 / 894, sixty-four 1,832 / 1,797, sixteen of a wide model 2,066 /
+// 1,990, prompts of 113 tokens 1,654 / 1,608.)
 __device__ __forceinline__ uint64_t l2_policy(bool read_once) {
     uint64_t first, normal;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
@@ -295,7 +296,8 @@ __host__ __device__ constexpr uint32_t instr_desc(int n, int m = TILE_W) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-template <int BN, int MODE>
+// PUSH: the form of a cluster that takes its tiles' K splits by cluster_epilogue (few rows; see pushes_splits).
+template <int BN, int MODE, bool PUSH>
 struct Cfg {
     static constexpr int NW = MODE == MODE_SWIGLU ? 2 : 1;
     static constexpr int W_BYTES = TILE_W * BK * 2;
@@ -309,10 +311,11 @@ struct Cfg {
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : (STAGES_RAW < 2 ? 2 : STAGES_RAW);
     static constexpr int TMEM_COLS_RAW = NW * BN;
     static constexpr int TMEM_COLS = TMEM_COLS_RAW < 32 ? 32 : TMEM_COLS_RAW;
-    // Where a cluster's other K splits put their rows of the partial tile (see cluster_epilogue).  Room for eight tokens (SwiGLU, with two numbers
-    // a feature: for one to three) and no more: with two CTAs on an SM the small kernels of the chain must still fit beside them.
+    // Where a cluster's other K splits put their rows of the partial tile: S - 1 of them, ceil(rows / S) rows each.  Plain products: up to 16, 12,
+    // 8, 10, 6, 7, 8 rows with 2 to 8 splits; SwiGLU, with two numbers a feature: 6, 3, 4 rows with 2 to 4, and none with more.  No more than
+    // that: with two CTAs on an SM the small kernels of the chain must still fit beside them.
     static constexpr int ROW_BYTES = NW * TILE_W * 4;
-    static constexpr int RECV_BYTES = BN > 64 ? 0 : MODE == MODE_SWIGLU ? 3 * 1024 : 4 * 1024;
+    static constexpr int RECV_BYTES = !PUSH ? 0 : MODE == MODE_SWIGLU ? 3 * 1024 : 4 * 1024;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/ + RECV_BYTES;
     // the partial tile of a K split fits in the (then free) pipeline stages
     static constexpr bool CLUSTER_OK = NW * BN * TILE_W * 4 <= STAGES * STAGE_BYTES;
@@ -322,13 +325,12 @@ struct Cfg {
 // split of rank r; every CTA writes the others' rows of its partial tile into their shared memory (recv: distributed stores, one barrier, and
 // nobody reads a peer's memory, so nobody waits to leave), keeps its own (in the pipeline stages, which are free by then) and adds its rows
 // up in split order.  The loop goes through the additions once BEFORE the accumulator is ready, on whatever lies there and without storing:
-// that brings the instructions to the SM while the main loop runs (read for the first time behind the barrier they took 1 - 2 us).  A step of one
-// sequence, 6 layers: 478 us, 488 where every CTA reads its peers' memory instead.
+// that brings the instructions to the SM while the main loop runs (read for the first time behind the barrier they took 1 - 2 us).
 // false: the wait for the accumulator ran out (the barriers are passed all the same).
 template <int BN, int MODE>
 __device__ __forceinline__ bool cluster_epilogue(const Params& p, float* stage, const float* recv, uint32_t tmem, uint32_t acc_bar,
                                                  volatile int* s_abort, int n0, int row0, int rows_here, int quarter, int lane) {
-    using C = Cfg<BN, MODE>;
+    using C = Cfg<BN, MODE, true>;
     constexpr int NW = C::NW, ROW = NW * TILE_W;
     const int S = p.splits, rank = (int)cluster_ctarank(), f = quarter * 32 + lane, n = n0 + f;
     const float bias = (plain_mode(MODE) && p.bias && n < p.N) ? p.bias[n] : 0.f;
@@ -433,10 +435,10 @@ __device__ __forceinline__ GroupTile find_group_tile(const int* offsets, int num
     return t;
 }
 
-template <int BN, int MODE>
+template <int BN, int MODE, bool PUSH>
 __global__ void __launch_bounds__(192, 3)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p) {
-    using C = Cfg<BN, MODE>;
+    using C = Cfg<BN, MODE, PUSH>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_work[4];          // group, first row, end row, is_last
     __shared__ int s_once;             // this tile holds all rows of its group: nobody else reads its weights
@@ -496,7 +498,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
     const int row0 = s_work[1], row_end = s_work[2];
     // few rows in a cluster: see cluster_epilogue
     const int rows_tile = min(BN, row_end - row0);
-    const bool push = p.cluster && (p.splits - 1) * ((rows_tile + p.splits - 1) / p.splits) * C::ROW_BYTES <= C::RECV_BYTES;
+    const bool push = PUSH && p.cluster && (p.splits - 1) * ((rows_tile + p.splits - 1) / p.splits) * C::ROW_BYTES <= C::RECV_BYTES;
     if (push) cluster_arrive();
 
     const int kb_total = (p.K + BK - 1) / BK;
@@ -591,7 +593,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                 s_abort = 1;
             }
         }
-    } else if (push) {
+    } else if (PUSH && push) {
         uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
         if (!cluster_epilogue<BN, MODE>(p, reinterpret_cast<float*>(aligned), reinterpret_cast<const float*>(aligned + C::STAGES * C::STAGE_BYTES + 256),
                                         tmem, acc_bar, &s_abort, n0, row0, rows_tile, warp & 3, lane) && lane == 0) {
@@ -1394,19 +1396,35 @@ bool make_map_gate_up(CUtensorMap* map, const void* ptr, uint64_t groups, uint64
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int MODE>
-int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, Params p, dim3 grid, cudaStream_t stream) {
-    using C = Cfg<BN, MODE>;
+template <int BN, int MODE, bool PUSH>
+int launch_form(const CUtensorMap& tmW, const CUtensorMap& tmX, const Params& p, dim3 grid, cudaStream_t stream) {
+    using C = Cfg<BN, MODE, PUSH>;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, MODE, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    p.cluster = (p.splits > 1 && p.splits <= MAX_CLUSTER && C::CLUSTER_OK) ? 1 : 0;
-    if (p.splits > 1 && !p.cluster && (!p.partials || !p.tickets)) return -1;
-    return launch_pdl_cluster(gemm_tc_kernel<BN, MODE>, grid, dim3(192), (size_t)C::SMEM, stream,
+    return launch_pdl_cluster(gemm_tc_kernel<BN, MODE, PUSH>, grid, dim3(192), (size_t)C::SMEM, stream,
                               p.cluster ? p.splits : 1, tmW, tmX, p);
+}
+
+// Whether a cluster's K splits push their rows (cluster_epilogue): dense products of up to 4 rows, grouped ones of up to 16 in all.  Beyond
+// that reading the peers' memory is as fast or faster, in a kernel that is smaller by that epilogue and its receive buffer.  Measured, us a step of
+// 6 layers (2,048 features), never / always push: 1, 2, 4 sequences 477 / 467, 549 / 545, 664.5 / 663.5, 8 of unequal length 888.5 / 895, 24
+// 1,400 / 1,405; prompts of 113 tokens 1,619 / 1,624.  This rule: 467, 548.5, 664.5, 889, 1,399, 1,619.  (SwiGLU with 5 splits and more never
+// finds room in RECV_BYTES and takes the smaller form: with the larger one 4 sequences take 669.)
+bool pushes_splits(const Params& p, int mode) {
+    return p.cluster && p.M <= (p.group_offsets ? 16 : 4) && (mode != MODE_SWIGLU || p.splits <= 4);
+}
+
+template <int BN, int MODE>
+int launch(const CUtensorMap& tmW, const CUtensorMap& tmX, Params p, dim3 grid, cudaStream_t stream) {
+    p.cluster = (p.splits > 1 && p.splits <= MAX_CLUSTER && Cfg<BN, MODE, false>::CLUSTER_OK) ? 1 : 0;
+    if (p.splits > 1 && !p.cluster && (!p.partials || !p.tickets)) return -1;
+    if constexpr (BN == 16)
+        if (pushes_splits(p, MODE)) return launch_form<BN, MODE, true>(tmW, tmX, p, grid, stream);
+    return launch_form<BN, MODE, false>(tmW, tmX, p, grid, stream);
 }
 
 int g_persistent = 1;
@@ -1503,7 +1521,7 @@ MOE_API int moe_gemm_tc(const void* X, int ldx, const void* W, int num_groups, i
     Params p;
     p.cluster = 0, p.early_offsets = (group_offsets && early_offsets) ? 1 : 0;
     // The routed experts' first product: its successor's CTAs, let in at its start, took the places of the shared expert's, which run beside it.
-    // (us a step, 6 layers, late / at the start: one sequence 509 / 511, eight 907 / 924.)
+    // (us a step of 6 layers, at the start / late: eight sequences 899 / 894.5; one, sixty-four, a wide model and short prompts the same.)
     p.late_dependents = mode == MODE_SWIGLU && group_offsets && !early_offsets;
     p.out = out, p.out_bf16 = out_bf16, p.ldo = ldo, p.bias = bias, p.group_offsets = group_offsets;
     p.num_groups = num_groups, p.M = M, p.N = N, p.K = K, p.w_rows_per_group = w_rows, p.splits = splits;

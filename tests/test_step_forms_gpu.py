@@ -91,6 +91,44 @@ def test_a_grouped_product_finds_its_rows_among_any_number_of_groups(groups):
     assert int(st[0]) == 0
 
 
+@pytest.mark.parametrize("S", [2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_k_splits_of_few_rows_push_or_are_read(core, S, swiglu, grouped):
+    """Every number of rows on both sides of the rule and of the receive buffer's size, groups that fill a tile and empty ones: against 64 bits, a row
+    the same to the bit in either form, nothing written past the last row."""
+    from moe_b200.ops import tc
+
+    torch.manual_seed(S)
+    groups, K, N, st = 4 if grouped else 1, 128 * S - 8, 136, core.new_status(DEV)       # two blocks of k a split, the last one ragged
+    shape = (groups, (2 if swiglu else 1) * N, K) if grouped else ((2 if swiglu else 1) * N, K)
+    rows, w = torch.randn(24, K, device=DEV).bfloat16(), (torch.randn(shape, device=DEV) * K ** -0.5).bfloat16()
+    wide = w.view(groups, -1, K)
+
+    def run(x, counts):
+        M, out = x.shape[0], torch.full((x.shape[0] + 3, N), 7.0, device=DEV)
+        offs = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32, device=DEV) if grouped else None
+        assert tc.gemm_tc(x, w, out, swiglu=swiglu, group_offsets=offs, bn=16, splits=S, status=st)
+        assert bool((out[M:] == 7.0).all())
+        return out[:M]
+
+    for M in range(1, 18):
+        x = rows[:M].contiguous()
+        # one group of M rows among empty ones (a grouped product of more than 16 rows in all has another form)
+        counts = [0, M, 0, 0]
+        got = run(x, counts)
+        ref = x.double() @ wide[1 if grouped else 0].double().T
+        slack = (K + S) * 2.0 ** -24 * (x.double().abs() @ wide[1 if grouped else 0].double().abs().T)      # exact products, K + S sums in 32 bits
+        if swiglu:
+            a, b, ea, eb = ref[:, :N], ref[:, N:], slack[:, :N], slack[:, N:]
+            ref = torch.nn.functional.silu(a) * b
+            slack = 1.1 * ea * b.abs() + a.abs() * eb + ea * eb + 1e-6 * ref.abs()       # |silu'| <= 1.1, |silu(a)| <= |a|
+        assert bool(((got.double() - ref).abs() <= slack).all()), M
+        more = run(torch.cat([x, rows[M:]]) if grouped else rows[:16 if M <= 16 else 24].contiguous(), [0, M, 0, 24 - M])
+        assert torch.equal(more[:M], got), M
+    assert int(st[0]) == 0
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 4, 5, 7, 8])
 @pytest.mark.parametrize("E,k,H,post", [(61, 4, 2048, False), (16, 2, 2056, True), (256, 8, 4104, False), (3, 3, 40, True)])
 def test_norm_and_router_with_several_blocks_a_token(core, T, E, k, H, post):
