@@ -143,16 +143,17 @@ __device__ __forceinline__ void rotated_chunk(const float* __restrict__ src, int
     }
 }
 
-// LPR: lanes per key row (row bytes / 16); GH: query heads handled together; KEEP: AttnVariant::keep may be set (a form of
-// its own, so that the others carry nothing of it).
 // 16 bytes of the cache, which a block reads once: they take no place in L1.  The loads stay in the order in which they stand, so all of
-// a tile are asked for before the first is used.  (us a step, plain loads / these: eight sequences 901 / 890, sixty-four 1,819 /
-// 1,809, sixteen of a wide model 1,991 / 1,960.)
+// a tile are asked for before the first is used.  (us a step of 6 layers, plain loads / these: eight sequences 909 / 894.5, sixty-four
+// 1,805 / 1,797, sixteen of a wide model of 3 layers 2,026 / 1,990; one sequence the same.)
 __device__ __forceinline__ uint4 load_once(const void* p) {
     uint4 v;
     asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
+
+// LPR: lanes per key row (row bytes / 16); GH: query heads handled together; KEEP: AttnVariant::keep may be set (a form of
+// its own, so that the others carry nothing of it).
 template <typename T, int LPR, int GH, bool FUSED, bool KEEP>
 __global__ void __launch_bounds__(WARPS * 32, (GH == 1 && LPR <= 16) ? 4 : 1)
 attn_decode_fast_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,

@@ -75,8 +75,9 @@ __global__ void __launch_bounds__(512, MINB) rmsnorm_kernel(float* __restrict__ 
     __shared__ float red[32];
     const int i = blockIdx.x;
     // The experts' combine with one 16-byte unit a thread: what does not come from the predecessor
-    // (the stream, the picks' places and weights, the gate and the norm's weight were all written
-    // at least two kernels ago) is read before the wait, so that only the experts' rows are left.
+    // is read before the wait, so that only the experts' rows are left: the stream and the norm's weight, and, by the norm
+    // and router of few tokens, the picks' places and weights and the gate were written at least two kernels ago on this stream.  With 9 tokens
+    // and more these come from a second stream, whose join in front of this launch is a full dependency.
     if (cs.y && !rows && hidden / 4 <= (int)blockDim.x && cs.top_k <= 8) {
         const int j = threadIdx.x;
         const bool mine = j < hidden / 4;

@@ -75,8 +75,9 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, float a, float b, float c,
 
 // The same as rope_split_kernel, four elements a thread (16-byte loads, 8- or 16-byte stores), for
 // head sizes and rotated widths that are multiples of 8; optionally it also appends the keys and
-// values to the cache (the arithmetic of kv_commit_kernel), which spares that launch where nothing
-// of this step's attention reads the cache (whole prompts).  One block per token.
+// values to the cache (the arithmetic of kv_commit_kernel), which spares that launch where nothing that
+// this step's attention still reads is written over: whole prompts, which read nothing from the cache, and any step
+// of a cache that is no ring, whose attention reads positions before the step there.  One block per token.
 template <typename OT>
 __global__ void __launch_bounds__(256)
 rope_split4_kernel(const float* __restrict__ qkv, const int* __restrict__ pos, const float* __restrict__ inv_freq,
@@ -177,7 +178,7 @@ rope_angles_kernel(const int* __restrict__ pos, const float* __restrict__ inv_fr
 // With `zero` the rows of tokens of no sequence in another buffer become zero (an attention's output, which no attention kernel writes there): a
 // fill of the whole buffer was a launch of its own in every layer.
 // With cache arguments (k_cache not null) the keys and values are also appended to the cache, as
-// moe_kv_commit would: only for steps whose attention reads nothing from the cache.
+// moe_kv_commit would: only where that writes over nothing that the step's attention still reads (whole prompts, or no ring).
 MOE_API int moe_rope_split(const float* qkv, const int* pos, const float* inv_freq, int num_tokens, int nh, int nkv,
                            int hd, int rot, void* q, void* k, void* v, int out_dt, void* k_cache, void* v_cache,
                            const int* seq_of_token, const int* seq_end, const int* slots, const int* tables,

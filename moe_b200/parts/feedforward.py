@@ -196,7 +196,12 @@ class RoutedExperts(Part):
         # from 16 on, where its single gathering block is the bottleneck
         self.fused_norm_tokens = int(os.environ.get("MOE_B200_NORM_ROUTE_MAX", "8"))
         self.shared_beside = os.environ.get("MOE_B200_SHARED_BESIDE", "1") != "0"
-        # up to this many tokens the shared expert's products start with the router's kernels, not behind them (see _run)
+        # Up to this many tokens the shared expert's products start with the router's kernels, not behind them (see _run).  Measured, us a
+        # step, behind / with, at 66, 128, 256, 400, 512, 700, 1,000 tokens: 6 layers of 60 experts of 1,408, width 2,048: 1,561 / 1,577,
+        # 1,619 / 1,632, 2,066 / 2,011, 2,067 / 2,021, 2,115 / 2,057, 2,326 / 2,268, 2,615 / 2,654; 3 of 64 of 2,560, width 3,584: 2,327 / 2,322,
+        # 2,527 / 2,520, 2,991 / 2,942, 3,224 / 3,185, 3,314 / 3,300, 3,732 / 3,690, 4,696 / 4,749; 6 of 32 of 704, width 1,024: 574 / 523, 635 / 601,
+        # 712 / 695, 827 / 809, 841 / 826, 2,028 / 2,029, 2,053 / 2,068; 3 of 32 of 1,408, width 4,096: 972 / 954, 1,025 / 1,006, 1,145 / 1,120,
+        # 1,347 / 1,318, 1,390 / 1,359, 1,520 / 1,557, 2,006 / 2,056.  (Beyond 512 steps are no longer replayed from a graph.)
         self.shared_first_tokens = int(os.environ.get("MOE_B200_SHARED_FIRST", "512"))
         # up to this many tokens one block picks, inverts and gathers (one launch after the logits);
         # beyond, a warp per token picks and the inversion and the gather are launches of their own
@@ -424,8 +429,8 @@ class RoutedExperts(Part):
         if not (T <= 64 and self.E <= 256) and not (self.shared_beside and rt.is_bf16 and T <= self.shared_first_tokens):
             # Many tokens: pick, table inversion and gather are small launches that leave the GPU
             # idle (37 us of a layer at 2,048 tokens), so the shared expert starts beside them on
-            # a second stream.  (Not before the logits' product: the shared expert's CTAs fill every
-            # SM's shared memory, and that product would wait for them to end.)
+            # a second stream.  (Not before the logits' product, which so many tokens do on the tensor cores: the shared expert's
+            # persistent CTAs fill every SM's shared memory, and that product would wait for them to end.)
             ys = side = None
 
             def shared_beside():
