@@ -153,6 +153,28 @@ def test_routed_experts_behind_a_norm_where_the_tensor_core_router_starts_early(
     assert torch.equal(x, x0 + delta) and rel(got, want.double().cpu()) < tol(dt) and int(rt.status[0]) == 0
 
 
+@pytest.mark.parametrize("limit,T", [(None, 65), (None, 512), (None, 513), (256, 256), (256, 257), (1000, 700)])
+def test_the_shared_expert_goes_first_up_to_a_number_of_tokens(monkeypatch, limit, T):
+    """Up to MOE_B200_SHARED_FIRST tokens (512) the routed experts run on the second stream, beyond it on the caller's: the same to the bit."""
+    if limit is not None:
+        monkeypatch.setenv("MOE_B200_SHARED_FIRST", str(limit))
+    H = 64
+    params = {"hidden_size": H, "num_experts": 6, "top_k": 2, "expert_size": 40, "norm_topk_prob": True, "shared_size": 72, "shared_gate": True}
+    part, _, rt = build("ffn", "routed_experts", params, torch.bfloat16)
+    x, batch = acts(rt, torch.randn(T, H)), G.make_batch(DEV, [0], [0], [T])
+    routed, streams = part._routed, []
+
+    def watched(*args, **kw):
+        streams.append(torch.cuda.current_stream() == torch.cuda.default_stream())
+        return routed(*args, **kw)
+
+    part._routed = watched
+    got = part.forward(rt, x, batch)
+    assert streams == [T > (limit or 512)]
+    part.shared_first_tokens = 10 ** 6 if streams[0] else 64
+    assert torch.equal(part.forward(rt, x, batch), got) and streams[1] != streams[0] and int(rt.status[0]) == 0
+
+
 @pytest.mark.parametrize("dt", DTYPES)
 def test_embedding_and_head_parts(dt):
     emb, ref, rt = build("embedding", "token_embedding", {"vocab_size": 77, "hidden_size": 40}, dt)

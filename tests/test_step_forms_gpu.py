@@ -300,3 +300,88 @@ def test_queries_keys_and_values_in_one_product(core, M, nh, nkv, K, bias, windo
             assert torch.equal(kc[r + h * 64], caches[1][1][t, h]) and torch.equal(vc[r + h * 64], caches[1][2][t, h])
     untouched = kc.shape[0] - nkv * len(written)
     assert int((kc == 3.0).all(-1).sum()) >= untouched and int(st[0]) == 0
+
+
+def test_long_steps_project_rotate_and_append_in_one_product_as_one_by_one(monkeypatch):
+    """A model whose layers share angles and cache rows within a step (windowed layers with a ring of their own among full ones): a prompt of 1,280
+    rows and more, a continued step of two sequences, another prompt, then a step of decoding, with the product that rotates and appends
+    and without it.  Logits and the whole cache to the bit."""
+    import moe_b200
+    from moe_b200.ops import tc
+
+    cfg = dict(architectures=["Qwen2MoeForCausalLM"], model_type="qwen2_moe", num_hidden_layers=4, hidden_size=264, num_attention_heads=3,
+               num_key_value_heads=1, head_dim=128, num_experts=4, num_experts_per_tok=2, norm_topk_prob=False, decoder_sparse_step=1,
+               moe_intermediate_size=72, shared_expert_intermediate_size=136, intermediate_size=136, vocab_size=301, rope_theta=1e4,
+               rms_norm_eps=1e-6, use_sliding_window=True, sliding_window=200, max_window_layers=2, tie_word_embeddings=False)
+    model = moe_b200.random_model(cfg, seed=3, dtype="bfloat16", device=DEV)
+    ids = torch.randint(0, 301, (6000,), generator=torch.Generator().manual_seed(1)).tolist()
+    fused, taken = tc.gemm_qkv, []
+
+    def counted(*args, **kw):
+        taken.append((args[0].shape[0], args[4] is not None))         # rows, and whether keys and values go to the cache at once
+        return fused(*args, **kw)
+
+    def steps():
+        engine = moe_b200.Engine(model, max_tokens=8192, max_slots=2)
+        a, b = engine.new_sequence(), engine.new_sequence()
+        out = [engine.step(s, t).clone() for s, t in (([a], [ids[:1300]]), ([a, b], [ids[1300:2700], ids[2700:2750]]),
+                                                      ([b], [ids[3000:4281]]), ([a, b], [[7], [9]]))]
+        engine.rt.check()
+        return out, [g.storage.clone() for g in engine.cache.groups], [g.ring for g in engine.cache.groups]
+
+    monkeypatch.setattr(tc, "gemm_qkv", counted)
+    got, kept, rings = steps()
+    assert len(rings) == 2 and sum(r > 0 for r in rings) == 1
+    # four layers each: a prompt appends everywhere at once, a step that goes on does so but in the ring of the two windowed layers
+    assert sorted(taken) == sorted([(1300, True)] * 4 + [(1450, True), (1450, False), (1281, True), (1281, False)] * 2)
+    monkeypatch.setattr(tc, "takes_qkv", lambda x, w: False)
+    del taken[:]
+    want, held, _ = steps()
+    assert not taken
+    for g, w in zip(got + kept, want + held):
+        assert torch.equal(g, w)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd,rot", [(3, 1, 128, 128), (5, 5, 24, 16)])
+def test_rope_split_zeroes_the_rows_of_no_sequence_and_no_others(core, dt, nh, nkv, hd, rot):
+    from moe_b200.cache import KVCache, KVRequest
+
+    T, st = 90, core.new_status(DEV)
+    cache = KVCache({0: KVRequest(nkv, hd, None)}, {0: None}, 256, 2, dt, DEV)
+    cache.acquire()
+    G.give_pages(cache, 0, T)
+    batch = G.make_batch(DEV, [0], [0], [T])
+    none = [0, 17, 88, 89]
+    batch.seq_of_token[none] = -1
+    qkv, freq = torch.randn(T, (nh + 2 * nkv) * hd, device=DEV), torch.rand(rot // 2, device=DEV)
+    q, k, v = (torch.empty(T, n, hd, device=DEV, dtype=dt) for n in (nh, nkv, nkv))
+    ctx = torch.full((T, nh * hd), float("nan"), device=DEV, dtype=dt)
+    assert core.rope_split(qkv, batch.pos, freq, nh, nkv, hd, rot, q, k, v, commit=(cache.view(0), batch), status=st, zero=ctx)
+    assert torch.equal(ctx[none], torch.zeros_like(ctx[none])) and int(ctx.isnan().all(1).sum()) == T - len(none) and int(st[0]) == 0
+
+
+@pytest.mark.parametrize("E,k", [(4, 3), (70, 8), (33, 1), (5, 5)])
+@pytest.mark.parametrize("score", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("norm", [False, True])
+def test_picks_from_logits_that_are_infinite_or_no_numbers(core, E, k, score, norm):
+    """The best score first, the lowest expert among equals, a score that is no number never; where none is left, expert j mod E with weight 0."""
+    inf, nan = float("inf"), float("nan")
+    rows = [[0.0] * E, [nan] * E, [-inf] * E, [inf] * E, [nan] + [-1.0] * (E - 1), [-inf] * (E - 1) + [2.0], [inf] + [0.5] * (E - 1),
+            [nan, inf] + [-inf] * (E - 2), [nan] * (E - 2) + [3.0, 3.0], [-200.0] * (E - 1) + [-0.0], [1e38, -1e38] + [0.0] * (E - 2)]
+    logits = torch.tensor(rows)
+    idx, w = torch.empty(len(rows), k, dtype=torch.int32, device=DEV), torch.empty(len(rows), k, device=DEV)
+    core.router_topk(logits.to(DEV), k, norm, 1.0, idx, w, num_experts=E, score=score)
+    for i, lg in enumerate(logits):
+        # (scores that vanish in 32 bits are equal)
+        sc = (torch.softmax(lg.double(), 0) if score == "softmax" else 1 / (1 + torch.exp(-lg).double())).float().tolist()
+        left, picks, weights = set(range(E)), [], []
+        for j in range(k):
+            best = max((e for e in left if sc[e] == sc[e]), key=lambda e: (sc[e], -e), default=None)
+            picks.append(j % E if best is None else best)
+            weights.append(0.0 if best is None else sc[best])
+            left.discard(picks[-1])
+        total = max(sum(weights), 1e-20) if norm else 1.0
+        assert idx[i].tolist() == picks, i
+        # E exponentials and their sum, in 32 bits
+        assert torch.allclose(w[i].double().cpu(), torch.tensor([x / total for x in weights], dtype=torch.float64), rtol=2e-5, atol=1e-30), i
