@@ -203,6 +203,7 @@ class RoutedExperts(Part):
         # 712 / 695, 827 / 809, 841 / 826, 2,028 / 2,029, 2,053 / 2,068; 3 of 32 of 1,408, width 4,096: 972 / 954, 1,025 / 1,006, 1,145 / 1,120,
         # 1,347 / 1,318, 1,390 / 1,359, 1,520 / 1,557, 2,006 / 2,056.  (Beyond 512 steps are no longer replayed from a graph.)
         self.shared_first_tokens = int(os.environ.get("MOE_B200_SHARED_FIRST", "512"))
+        self.routed_first_weights = 4 << 20       # an expert's weights from which on its branch goes first up to 64 tokens (see _run)
         # up to this many tokens one block picks, inverts and gathers (one launch after the logits);
         # beyond, a warp per token picks and the inversion and the gather are launches of their own
         # (measured on a B200, ms a decode step at 16 / 32 / 64 tokens: 4.65 / 5.89 / 7.38 with one
@@ -452,12 +453,18 @@ class RoutedExperts(Part):
         # Fewer: neither branch fills the GPU, so they run beside one another (inside a captured graph a fork and a join).  In bfloat16 the
         # shared expert's products follow the norm on the main stream, where a programmatic launch lets them fetch their first weights before
         # it has ended; what hangs on the picks (and, with 9 tokens and more, the picks themselves) runs on the second.  Measured, us a step
-        # of 6 layers, this way / the shared expert on the second stream: one sequence 465 / 478, eight 914 / 915, sixty-four 1,821 / 1,836.
+        # of 6 layers, this way / the shared expert on the second stream: one, two, four, eight sequences 465 / 479, 545 / 555, 666 / 680, 888.5 / 892.5.
         # (In 32 bits, whose products have no such launch, eight sequences take 1,069 / 1,055 us: there it is the shared expert's.)
+        # Where the picks do not come with the norm, up to 64 tokens, big experts keep the main stream themselves: their branch is the longer one, and a
+        # fork in front of the router is in its way.  Measured, this way / the other one, 9, 12, 16, 32, 64 sequences of 300 tokens: experts of 8.7 M
+        # weights (60, width 2,048) 941 / 923, 1,045 / 1,023, 1,148 / 1,136, 1,453 / 1,435, 1,711 / 1,701, of 9.4 M (128, width 4,096, 2 layers) 618 /
+        # 623, 690 / 691, 749 / 754, 947 / 941, 1,147 / 1,128, of 27.5 M (64, width 3,584, 3 layers) 1,650 / 1,654, 1,828 / 1,835, 1,992 / 1,995,
+        # 2,214 / 2,218, 2,478 / 2,499; of 2.2 M (32, width 1,024, 4 layers) 253 / 255, 264 / 265, 272 / 278, 326 / 329, 382 / 390, of 0.4 M (16, width 512)
+        # 196 / 198, 198 / 200, 200 / 203, 238 / 239, 282 / 283.
         main = torch.cuda.current_stream()
         side = rt.side_stream()
         side.wait_stream(main)
-        if not rt.is_bf16:
+        if not rt.is_bf16 or (routed is None and T <= 64 and 3 * self.size * self.hidden >= self.routed_first_weights):
             with torch.cuda.stream(side):
                 ys = self._shared(rt, h)
             out = self._routed(rt, h, batch, routed, self._record)

@@ -153,6 +153,22 @@ def test_routed_experts_behind_a_norm_where_the_tensor_core_router_starts_early(
     assert torch.equal(x, x0 + delta) and rel(got, want.double().cpu()) < tol(dt) and int(rt.status[0]) == 0
 
 
+@pytest.mark.parametrize("T", [1, 9, 64, 65])
+def test_big_experts_keep_the_main_stream_up_to_64_tokens(T):
+    params = {"hidden_size": 64, "num_experts": 6, "top_k": 2, "expert_size": 40, "norm_topk_prob": True, "shared_size": 72, "shared_gate": True}
+    part, _, rt = build("ffn", "routed_experts", params, torch.bfloat16)
+    x, batch, routed, streams, got = acts(rt, torch.randn(T, 64)), G.make_batch(DEV, [0], [0], [T]), part._routed, [], []
+
+    def watched(*args, **kw):
+        streams.append(torch.cuda.current_stream() == torch.cuda.default_stream())
+        return routed(*args, **kw)
+
+    part._routed = watched
+    for part.routed_first_weights in (3 * 64 * 40, 3 * 64 * 40 + 1):
+        got.append(part.forward(rt, x, batch))
+    assert streams == [T <= 64, False] and torch.equal(*got) and int(rt.status[0]) == 0
+
+
 @pytest.mark.parametrize("limit,T", [(None, 65), (None, 512), (None, 513), (256, 256), (256, 257), (1000, 700)])
 def test_the_shared_expert_goes_first_up_to_a_number_of_tokens(monkeypatch, limit, T):
     """Up to MOE_B200_SHARED_FIRST tokens (512) the routed experts run on the second stream, beyond it on the caller's: the same to the bit."""
